@@ -474,18 +474,52 @@ __global__ void __launch_bounds__(256) k_finalize(DevPtrs P) {
     }
 }
 
-// Canonical order: every (block, bucket) segment sorted by ascending id.
-// Rank sort in shared memory (particle ids are distinct inside a block).
+// Canonical order: every (block, bucket) segment sorted by ascending id, by
+// ranks (particle ids are distinct inside a block).  A warp takes a bucket of
+// up to kSegWarp ids (a slab holds some 128 at 8 particles a cell), so a
+// block's ten buckets sort side by side; the CTA sorts a longer one together
+// (the CTA sorting one bucket after another took 36 us for 100,003 particles).
 constexpr uint32_t kSegMax = 4096;
+constexpr uint32_t kSegWarp = kSegMax / 8;
 __global__ void __launch_bounds__(256) k_sort_segments(DevPtrs P) {
-    __shared__ uint32_t buf[kSegMax];
+    __shared__ uint4 buf4[kSegMax / 4];
+    uint32_t* buf = reinterpret_cast<uint32_t*>(buf4);
     const uint32_t total = P.counters->num_blocks;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t b = blockIdx.x; b < total; b += gridDim.x) {
-        uint32_t start = P.first[b];
+        bool longer = false;
+        const auto segment = [&](int k, uint32_t& start) {
+            start = k ? P.cursors[b * NUM_BUCKETS + k - 1] : P.first[b];
+            return P.cursors[b * NUM_BUCKETS + k] - start;
+        };
         for (int k = 0; k < NUM_BUCKETS; ++k) {
-            const uint32_t end = P.cursors[b * NUM_BUCKETS + k];
-            const uint32_t len = end - start;
-            if (len > 1 && len <= kSegMax) {
+            uint32_t start;
+            const uint32_t len = segment(k, start);
+            longer |= len > kSegWarp;
+            if ((uint32_t)k % 8u != warp || len < 2 || len > kSegWarp) continue;
+            uint32_t* mine = buf + warp * kSegWarp;
+            const uint4* mine4 = buf4 + warp * (kSegWarp / 4);
+            __syncwarp();  // the previous bucket's reads are done
+            for (uint32_t i = lane; i < ((len + 3u) & ~3u); i += 32u) mine[i] = i < len ? P.sorted[start + i] : NONE;
+            __syncwarp();
+            for (uint32_t i = lane; i < len; i += 64u) {
+                const uint32_t v0 = mine[i], v1 = i + 32u < len ? mine[i + 32u] : 0u;
+                uint32_t r0 = 0, r1 = 0;
+                for (uint32_t j = 0; j < (len + 3u) / 4u; ++j) {
+                    const uint4 q = mine4[j];
+                    r0 += (q.x < v0) + (q.y < v0) + (q.z < v0) + (q.w < v0);
+                    r1 += (q.x < v1) + (q.y < v1) + (q.z < v1) + (q.w < v1);
+                }
+                P.sorted[start + r0] = v0;
+                if (i + 32u < len) P.sorted[start + r1] = v1;
+            }
+        }
+        if (!longer) continue;
+        __syncthreads();
+        for (int k = 0; k < NUM_BUCKETS; ++k) {
+            uint32_t start;
+            const uint32_t len = segment(k, start);
+            if (len > kSegWarp && len <= kSegMax) {
                 for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) buf[i] = P.sorted[start + i];
                 __syncthreads();
                 for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
@@ -498,7 +532,6 @@ __global__ void __launch_bounds__(256) k_sort_segments(DevPtrs P) {
             } else if (len > kSegMax && threadIdx.x == 0) {
                 set_status(P.counters, STATUS_SORT_CAPACITY);
             }
-            start = end;
         }
     }
 }
