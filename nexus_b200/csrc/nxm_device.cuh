@@ -281,83 +281,79 @@ __device__ __forceinline__ Svd svd3(const m3& f) {
     return out;
 }
 
-// Fast-build SVD: the same Jacobi sweeps with the orthogonality test on
-// squares (no square roots), the rotation's division by an approximate
-// reciprocal (__fdividef), and the singular values and U columns from one
-// reciprocal square root per column.  Agrees with svd3 to a few ulp.
-__device__ __forceinline__ bool jacobi_pair_fast(float (&a)[3][3], float (&v)[3][3], int p, int q) {
-    const float alpha = a[0][p] * a[0][p] + a[1][p] * a[1][p] + a[2][p] * a[2][p];
-    const float beta = a[0][q] * a[0][q] + a[1][q] * a[1][q] + a[2][q] * a[2][q];
-    const float gamma = a[0][p] * a[0][q] + a[1][p] * a[1][q] + a[2][p] * a[2][q];
-    if (gamma * gamma <= 1.0e-12f * alpha * beta || fabsf(gamma) <= 1.0e-30f) return false;
-    const float zeta = __fdividef(beta - alpha, 2.0f * gamma);
-    const float t = __fdividef(copysignf(1.0f, zeta), fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
-    const float c = rsqrtf(1.0f + t * t);
-    const float s = c * t;
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const float ap = a[r][p], aq = a[r][q];
-        a[r][p] = c * ap - s * aq;
-        a[r][q] = s * ap + c * aq;
-        const float vp = v[r][p], vq = v[r][q];
-        v[r][p] = c * vp - s * vq;
-        v[r][q] = s * vp + c * vq;
-    }
+// Fast-build strain: eigenvalues e and vectors u (columns) of F F^T - I, by
+// cyclic Jacobi rotations of the symmetric matrix (Golub & Van Loan 8.5).  The
+// models need only functions of the left stretch, s = sqrt(1 + e) in the
+// frame u: a rotation updates 6 entries and one matrix where the one-sided
+// sweeps above update two matrices and form three dot products, and e keeps
+// the small strains that 1 + e would round away.  Stops when every
+// off-diagonal is below 3e-7 of the matrix (two to four sweeps).
+struct Strain {
+    v3 e;
+    m3 u;
+};
+
+__device__ __forceinline__ bool jacobi_sym(float& app, float& aqq, float& apq, float& arp, float& arq, v3& up, v3& uq,
+                                           float tol) {
+    if (apq * apq <= tol) return false;
+    const float d = aqq - app, g = 2.0f * apq;
+    const float ih = rsqrtf(d * d + g * g);
+    const float c2 = 0.5f + 0.5f * fabsf(d) * ih;  // cos^2 of the rotation, in [1/2, 1]
+    const float ic = rsqrtf(c2);
+    const float c = c2 * ic;
+    const float s = copysignf(0.5f * ih * ic, d) * g;
+    const float t = s * ic * apq;
+    app -= t;
+    aqq += t;
+    apq = 0.0f;
+    const float rp = arp, rq = arq;
+    arp = c * rp - s * rq;
+    arq = s * rp + c * rq;
+    const v3 p = up, q = uq;
+    up = p * c - q * s;
+    uq = p * s + q * c;
     return true;
 }
 
-__device__ __forceinline__ Svd svd3_fast(const m3& f) {
-    float a[3][3] = {{f.c0.x, f.c1.x, f.c2.x}, {f.c0.y, f.c1.y, f.c2.y}, {f.c0.z, f.c1.z, f.c2.z}};
-    float v[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
+__device__ __forceinline__ Strain strain_of(const m3& F) {
+    float xx = F.c0.x * F.c0.x - 1.0f, yy = F.c0.y * F.c0.y - 1.0f, zz = F.c0.z * F.c0.z - 1.0f;
+    xx += F.c1.x * F.c1.x; yy += F.c1.y * F.c1.y; zz += F.c1.z * F.c1.z;
+    xx += F.c2.x * F.c2.x; yy += F.c2.y * F.c2.y; zz += F.c2.z * F.c2.z;
+    float xy = F.c0.x * F.c0.y + F.c1.x * F.c1.y + F.c2.x * F.c2.y;
+    float xz = F.c0.x * F.c0.z + F.c1.x * F.c1.z + F.c2.x * F.c2.z;
+    float yz = F.c0.y * F.c0.z + F.c1.y * F.c1.z + F.c2.y * F.c2.z;
+    const float tol = 1.0e-13f * (xx * xx + yy * yy + zz * zz + 2.0f * (xy * xy + xz * xz + yz * yz));
+    Strain r;
+    r.u = mident();
 #pragma unroll 1
     for (int sweep = 0; sweep < 10; ++sweep) {
-        bool rot = jacobi_pair_fast(a, v, 0, 1);
-        rot |= jacobi_pair_fast(a, v, 0, 2);
-        rot |= jacobi_pair_fast(a, v, 1, 2);
+        bool rot = jacobi_sym(xx, yy, xy, xz, yz, r.u.c0, r.u.c1, tol);
+        rot |= jacobi_sym(xx, zz, xz, xy, yz, r.u.c0, r.u.c2, tol);
+        rot |= jacobi_sym(yy, zz, yz, xy, xz, r.u.c1, r.u.c2, tol);
         if (!rot) break;
     }
-    float sig[3], inv[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const float n2 = a[0][c] * a[0][c] + a[1][c] * a[1][c] + a[2][c] * a[2][c];
-        inv[c] = n2 > 1.0e-36f ? rsqrtf(n2) : 0.0f;
-        sig[c] = n2 * inv[c];
-    }
-    auto swapc = [&](int i, int j) {
-        float t = sig[i]; sig[i] = sig[j]; sig[j] = t;
-        t = inv[i]; inv[i] = inv[j]; inv[j] = t;
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            float ta = a[r][i]; a[r][i] = a[r][j]; a[r][j] = ta;
-            float tv = v[r][i]; v[r][i] = v[r][j]; v[r][j] = tv;
-        }
-    };
-    if (sig[1] > sig[0]) swapc(0, 1);
-    if (sig[2] > sig[0]) swapc(0, 2);
-    if (sig[2] > sig[1]) swapc(1, 2);
-    float u[3][3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int r = 0; r < 3; ++r) u[r][c] = a[r][c] * inv[c];
-    if (!(sig[1] > 1.0e-18f)) {
-        float ux = u[0][0], uy = u[1][0], uz = u[2][0];
-        float ox, oy, oz;
-        if (fabsf(ux) < 0.9f) { ox = 0; oy = -uz; oz = uy; } else { ox = uz; oy = 0; oz = -ux; }
-        float on = sqrtf(ox * ox + oy * oy + oz * oz);
-        if (on == 0.0f) { ox = 1; oy = 0; oz = 0; on = 1; }
-        u[0][1] = ox / on; u[1][1] = oy / on; u[2][1] = oz / on;
-    }
-    if (!(sig[2] > 1.0e-18f)) {
-        u[0][2] = u[1][0] * u[2][1] - u[2][0] * u[1][1];
-        u[1][2] = u[2][0] * u[0][1] - u[0][0] * u[2][1];
-        u[2][2] = u[0][0] * u[1][1] - u[1][0] * u[0][1];
-    }
-    Svd out;
-    out.u = mkm(mk(u[0][0], u[1][0], u[2][0]), mk(u[0][1], u[1][1], u[2][1]), mk(u[0][2], u[1][2], u[2][2]));
-    out.s = mk(sig[0], sig[1], sig[2]);
-    out.vt = mkm(mk(v[0][0], v[0][1], v[0][2]), mk(v[1][0], v[1][1], v[1][2]), mk(v[2][0], v[2][1], v[2][2]));
-    return out;
+    r.e = mk(xx, yy, zz);
+    return r;
+}
+
+// u diag(d) u^T.
+__device__ __forceinline__ m3 in_frame(const m3& u, v3 d) {
+    const v3 a = u.c0 * d.x, b = u.c1 * d.y, c = u.c2 * d.z;
+    const float xx = a.x * u.c0.x + b.x * u.c1.x + c.x * u.c2.x;
+    const float yy = a.y * u.c0.y + b.y * u.c1.y + c.y * u.c2.y;
+    const float zz = a.z * u.c0.z + b.z * u.c1.z + c.z * u.c2.z;
+    const float xy = a.x * u.c0.y + b.x * u.c1.y + c.x * u.c2.y;
+    const float xz = a.x * u.c0.z + b.x * u.c1.z + c.x * u.c2.z;
+    const float yz = a.y * u.c0.z + b.y * u.c1.z + c.y * u.c2.z;
+    return mkm(mk(xx, xy, xz), mk(xy, yy, yz), mk(xz, yz, zz));
+}
+
+// log(1 + e): the odd series of the area tangent, 2 artanh(e / (2 + e)), for
+// moderate strains (truncated below 1e-8 relative at |e| = 1/4).
+__device__ __forceinline__ float log_stretch(float e) {
+    if (fabsf(e) > 0.25f) return __logf(1.0f + e);
+    const float z = __fdividef(e, 2.0f + e), z2 = z * z;
+    return 2.0f * z * (1.0f + z2 * (1.0f / 3.0f + z2 * (0.2f + z2 * (1.0f / 7.0f))));
 }
 
 // ---------------------------------------------------------------------------
@@ -458,63 +454,89 @@ __device__ __forceinline__ m3 dp_project_svd(const float* pl, float* state, cons
     d.s = sv;
     return (d.u * diag(sv)) * d.vt;
 }
-// Fast-build Drucker-Prager projection: dp_project_svd's return map with the
-// hardware approximations of log, exp and sin (__logf, __expf, __sinf), and
-// the determinants' logarithms taken from the strains (log det = sum of the
-// log singular values), so no further logarithm is needed.
-// The paths that leave F unchanged return it as U S V^T (equal to rounding),
-// so F itself need not stay live across the SVD.
-__device__ __forceinline__ m3 dp_project_fast(const float* pl, float* state, const m3& F, Svd& d) {
-    d = svd3_fast(F);
-    if (pl[4] == 0.0f) return (d.u * diag(d.s)) * d.vt;
+// Fast-build models on the strain frame.  `s` is the stretch, `rs` its
+// reciprocal, `sm` = s - 1 formed without cancellation.
+struct Stretch {
+    v3 s, rs, sm;
+};
+__device__ __forceinline__ Stretch stretch_of(v3 e) {
+    Stretch r;
+    const v3 l = e + splat(1.0f);
+    r.rs = mk(rsqrtf(l.x), rsqrtf(l.y), rsqrtf(l.z));
+    r.s = mk(l.x * r.rs.x, l.y * r.rs.y, l.z * r.rs.z);
+    r.sm = mk(__fdividef(e.x, r.s.x + 1.0f), __fdividef(e.y, r.s.y + 1.0f), __fdividef(e.z, r.s.z + 1.0f));
+    return r;
+}
+
+// Corotated linear stress: with F = U S V^T, U (S - I) V^T F^T =
+// U diag((s - 1) s) U^T.
+__device__ __forceinline__ m3 linear_stress_fast(float lambda, float mu, const m3& u, v3 s, v3 sm) {
+    const float j = s.x * s.y * s.z;
+    m3 r = in_frame(u, mk(sm.x * s.x, sm.y * s.y, sm.z * s.z) * (2.0f * mu));
+    const float diag_val = lambda * (j - 1.0f) * j;
+    r.c0.x += diag_val;
+    r.c1.y += diag_val;
+    r.c2.z += diag_val;
+    return r;
+}
+
+// F with its stretches s replaced by `ns`: F + U diag(ns / s - 1) U^T F.
+__device__ __forceinline__ m3 restretch(const m3& F, const m3& u, v3 ns, v3 rs) {
+    return F + in_frame(u, mk(ns.x * rs.x - 1.0f, ns.y * rs.y - 1.0f, ns.z * rs.z - 1.0f)) * F;
+}
+
+// Drucker-Prager projection: dp_project_svd's return map with the hardware
+// approximations of exp and sin (__expf, __sinf), and the determinants'
+// logarithms taken from the strains (log det = sum of the log stretches), so
+// no further logarithm is needed.  `st` and F become the projected ones.
+__device__ __forceinline__ void dp_project_fast(const float* pl, float* state, m3& F, const Strain& d, Stretch& st) {
+    if (pl[4] == 0.0f) return;
     const float q = state[1];
     const float angle = pl[0] + (pl[1] * q - pl[3]) * __expf(-pl[2] * q);
     const float s_angle = __sinf(angle);
     const float alpha = sqrtf(2.0f / 3.0f) * __fdividef(2.0f * s_angle, 3.0f - s_angle);
     const float dd = 3.0f;
-    const v3 ls = mk(__logf(d.s.x), __logf(d.s.y), __logf(d.s.z));
+    const v3 ls = mk(log_stretch(d.e.x), log_stretch(d.e.y), log_stretch(d.e.z)) * 0.5f;
     const v3 strain = ls + splat(state[2] / dd);
     const float tr = strain.x + strain.y + strain.z;
     const v3 dev = strain - splat(tr / dd);
     const float shifted = tr - pl[6];
-    v3 sv;
-    float hard, log_new;
+    v3 h;
+    float hard;
     if (shifted > 0.0f || (dev.x == 0.0f && dev.y == 0.0f && dev.z == 0.0f)) {
-        sv = splat(__expf(pl[6] / dd));
+        h = splat(pl[6] / dd);
         hard = length(strain);
-        log_new = pl[6];
     } else {
         const float dnorm = length(dev);
         const float gamma = dnorm + (dd * pl[4] + 2.0f * pl[5]) / (2.0f * pl[5]) * shifted * alpha;
-        if (gamma <= 0.0f) return (d.u * diag(d.s)) * d.vt;  // invalid projection: state and F unchanged
-        const v3 h = strain - dev * __fdividef(gamma, dnorm);
-        sv = mk(__expf(h.x), __expf(h.y), __expf(h.z));
+        if (gamma <= 0.0f) return;  // invalid projection: state and F unchanged
+        h = strain - dev * __fdividef(gamma, dnorm);
         hard = gamma;
-        log_new = h.x + h.y + h.z;
     }
-    const float log_prev = ls.x + ls.y + ls.z;
+    const v3 sv = mk(__expf(h.x), __expf(h.y), __expf(h.z));
+    const float log_prev = ls.x + ls.y + ls.z, log_new = h.x + h.y + h.z;
     state[0] = state[0] * __expf(log_prev - log_new);
     state[1] = state[1] + hard;
     state[2] = state[2] + log_prev - log_new;
-    d.s = sv;
-    return (d.u * diag(sv)) * d.vt;
+    F = restretch(F, d.u, sv, st.rs);
+    st.s = sv;
+    st.sm = sv - splat(1.0f);
 }
 
-// Fast-build corotated linear stress from the SVD of F: with F = U S V^T,
-// U (S - I) V^T F^T = U diag((s - 1) s) U^T, a symmetric product.
-__device__ __forceinline__ m3 linear_stress_fast(float lambda, float mu, const Svd& d) {
-    const float j = d.s.x * d.s.y * d.s.z;
-    const v3 e = mk((d.s.x - 1.0f) * d.s.x, (d.s.y - 1.0f) * d.s.y, (d.s.z - 1.0f) * d.s.z) * (2.0f * mu);
-    const m3& U = d.u;
-    const v3 u0e = U.c0 * e.x, u1e = U.c1 * e.y, u2e = U.c2 * e.z;
-    const float xx = u0e.x * U.c0.x + u1e.x * U.c1.x + u2e.x * U.c2.x;
-    const float yy = u0e.y * U.c0.y + u1e.y * U.c1.y + u2e.y * U.c2.y;
-    const float zz = u0e.z * U.c0.z + u1e.z * U.c1.z + u2e.z * U.c2.z;
-    const float xy = u0e.x * U.c0.y + u1e.x * U.c1.y + u2e.x * U.c2.y;
-    const float xz = u0e.x * U.c0.z + u1e.x * U.c1.z + u2e.x * U.c2.z;
-    const float yz = u0e.y * U.c0.z + u1e.y * U.c1.z + u2e.y * U.c2.z;
-    const float diag_val = lambda * (j - 1.0f) * j;
-    return mkm(mk(xx + diag_val, xy, xz), mk(xy, yy + diag_val, yz), mk(xz, yz, zz + diag_val));
+// Snow projection (snow_project below): the stretches clamped to the elastic band.
+__device__ __forceinline__ float snow_project_fast(const float* pl, float* state, m3& F, const Strain& d, Stretch& st) {
+    if (!(pl[0] <= 0.0f && pl[1] <= 0.0f)) {
+        const v3 cl = vclamp(st.s, 1.0f - pl[0], 1.0f + pl[1]);
+        const float prev_det = st.s.x * st.s.y * st.s.z;
+        const float new_det = cl.x * cl.y * cl.z;
+        state[0] = rclamp(state[0] * prev_det / new_det, 0.1f, 4.0f);
+        F = restretch(F, d.u, cl, st.rs);
+        const v3 s = st.s;
+        st.s = cl;  // a stretch inside the band keeps its exact s - 1
+        st.sm = mk(cl.x == s.x ? st.sm.x : cl.x - 1.0f, cl.y == s.y ? st.sm.y : cl.y - 1.0f,
+                   cl.z == s.z ? st.sm.z : cl.z - 1.0f);
+    }
+    return expf(pl[2] * (1.0f - state[0]));
 }
 
 __device__ __forceinline__ m3 dp_project(const float* pl, float* state, const m3& F) {
@@ -542,35 +564,19 @@ __device__ __forceinline__ m3 snow_project(const float* pl, float* state, const 
 
 // models/default.rs:208-264.  `w` holds the material's 24 model words; the
 // per-particle state words (Drucker-Prager words 0..2, snow word 0) are in `st`
-// and updated in place.  kReuseSvd selects the fast build's forms, which
-// agree with the reference's to rounding: Drucker-Prager sand on a linear
-// backbone takes its stress from the projection's SVD instead of a second SVD
-// of the projected F, with the fast SVD, projection and stress above; the
-// deterministic build keeps the reference's operation order.
-template <bool kReuseSvd>
-__device__ __forceinline__ m3 model_update(uint32_t tag, const float* w, float* st, m3& F, const m3& vel_grad) {
+// and updated in place.  model_update_ref keeps the reference's operation
+// order (the deterministic build).
+__device__ __forceinline__ m3 model_update_ref(uint32_t tag, const float* w, float* st, m3& F, const m3& vel_grad) {
     switch (tag) {
     case MODEL_ELASTIC_LINEAR:
-        if (kReuseSvd) return linear_stress_fast(w[0], w[1], svd3_fast(F));
         return linear_stress(w[0], w[1], F);
     case MODEL_ELASTIC_NEO_HOOKEAN:
         return neo_hookean_stress(w[0], w[1], F);
     case MODEL_SAND_LINEAR:
-        if (kReuseSvd) {
-            Svd d;
-            F = dp_project_fast(&w[3], st, F, d);
-            return linear_stress_fast(w[10], w[11], d);
-        } else {
-            F = dp_project(&w[3], st, F);
-            return linear_stress(w[10], w[11], F);
-        }
+        F = dp_project(&w[3], st, F);
+        return linear_stress(w[10], w[11], F);
     case MODEL_SAND_NEO_HOOKEAN:
-        if (kReuseSvd) {
-            Svd d;
-            F = dp_project_fast(&w[3], st, F, d);
-        } else {
-            F = dp_project(&w[3], st, F);
-        }
+        F = dp_project(&w[3], st, F);
         return neo_hookean_stress(w[10], w[11], F);
     case MODEL_FLUID: {
         m3 sr = (vel_grad + transpose(vel_grad)) * 0.5f;
@@ -584,6 +590,55 @@ __device__ __forceinline__ m3 model_update(uint32_t tag, const float* w, float* 
     default:
         return mzero();
     }
+}
+
+struct ModelResult {
+    m3 F, tau;
+    v3 st;
+};
+static __device__ __noinline__ ModelResult model_update_far(uint32_t tag, const float* w, v3 st, m3 F) {
+    float s[4] = {st.x, st.y, st.z, 0.f};
+    ModelResult r;
+    r.tau = model_update_ref(tag, w, s, F, mzero());
+    r.F = F;
+    r.st = mk(s[0], s[1], s[2]);
+    return r;
+}
+
+// kFast selects the fast build's forms, which agree with the reference's to
+// rounding: the models with a stretch take it from one eigendecomposition of
+// F F^T - I (none decomposes a projected F again).  The square loses the
+// smallest stretch once it is far below the largest (under 0.3 of it: relative
+// error above 1e-6), so such an F takes the SVD forms, out of line.
+template <bool kFast>
+__device__ __forceinline__ m3 model_update(uint32_t tag, const float* w, float* st, m3& F, const m3& vel_grad) {
+    if (!kFast || tag > MODEL_SNOW) return model_update_ref(tag, w, st, F, vel_grad);
+    if (tag == MODEL_FLUID) {
+        m3 sr = (vel_grad + transpose(vel_grad)) * 0.5f;
+        return fluid_stress(&w[0], F, sr);
+    }
+    if (tag == MODEL_ELASTIC_NEO_HOOKEAN) return neo_hookean_stress(w[0], w[1], F);
+    const Strain d = strain_of(F);
+    const float lo = fminf(fminf(d.e.x, d.e.y), d.e.z) + 1.0f, hi = fmaxf(fmaxf(d.e.x, d.e.y), d.e.z) + 1.0f;
+    if (!(lo > 0.1f * hi)) {
+        const ModelResult r = model_update_far(tag, w, mk(st[0], st[1], st[2]), F);
+        F = r.F;
+        st[0] = r.st.x; st[1] = r.st.y; st[2] = r.st.z;
+        return r.tau;
+    }
+    Stretch x = stretch_of(d.e);
+    float lambda = w[0], mu = w[1];
+    if (tag == MODEL_SAND_LINEAR || tag == MODEL_SAND_NEO_HOOKEAN) {
+        dp_project_fast(&w[3], st, F, d, x);
+        lambda = w[10];
+        mu = w[11];
+        if (tag == MODEL_SAND_NEO_HOOKEAN) return neo_hookean_stress(lambda, mu, F);
+    } else if (tag == MODEL_SNOW) {
+        const float hard = snow_project_fast(&w[1], st, F, d, x);
+        lambda = w[4] * hard;
+        mu = w[5] * hard;
+    }
+    return linear_stress_fast(lambda, mu, d.u, x.s, x.sm);
 }
 
 // ---------------------------------------------------------------------------

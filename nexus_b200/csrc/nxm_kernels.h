@@ -26,14 +26,16 @@ struct DevPtrs {
     uint32_t* first;
     uint32_t* nprim;
     uint32_t* nwx;           // num_particles_with_extras
-    uint32_t* cursors;       // NUM_BUCKETS per block
+    uint32_t* cursors;       // NUM_BUCKETS per block: bucket ends after the sort
+    uint32_t* cells;         // 64 per block: particles per associated cell, then (scan) where each
+                             // cell's particles start in the sorted list, then (finalize) where they end
     uint32_t* nbh;           // NUM_NBH per block
     float4* nodes;           // 64 per block
     uint32_t* sorted;        // sorted ids with extras
     uint2* pcode;            // per particle: packed block key, assoc code (ax | ay<<2 | az<<4)
-    uint32_t* phdr;          // per particle: primary header id
+    uint32_t* phdr;          // per particle: primary header id * 64 + associated cell (NONE: no block)
     uint32_t* scan_tmp;      // per block: offset inside its scan tile
-    uint32_t* tile_sums;     // per scan tile of kScanTile blocks: its total
+    uint32_t* tile_sums;     // per scan tile of kScanTile (slab sort) or kCellTile (cell sort) blocks: its total
     // per run of kRangeChunk sorted positions: the block holding its first
     // position (written by the scan; the fast G2P walks the sorted list in
     // these runs)
@@ -72,7 +74,8 @@ struct DevPtrs {
     uint32_t* rp_sorted;
 };
 
-constexpr uint32_t kScanTile = 256;  // blocks per scan tile (one per thread of a scan CTA)
+constexpr uint32_t kScanTile = 256;  // blocks per scan tile of the slab sort (one per thread of a scan CTA)
+constexpr uint32_t kCellTile = 128;  // blocks per scan tile of the cell sort (16 per warp of a scan CTA)
 constexpr uint32_t kRangeChunk = 256;  // sorted positions per fast-G2P run (one per thread of its CTA)
 
 // Launch shapes the autotuner picks per state (nxm_state_autotune); the

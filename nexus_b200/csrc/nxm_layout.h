@@ -22,6 +22,7 @@ constexpr int NUM_EXTRA_BUCKETS = 6;
 constexpr int NUM_BUCKETS = 10;
 constexpr int NUM_NBH = 7;
 constexpr int MODEL_WORDS = 24;
+constexpr uint32_t kMaxBlocks = (1u << 26) - 1u;  // header id * 64 + cell fits 32 bits beside NONE
 constexpr float MAX_FLT = 1.0e18f;  // nexus_rbd_shaders::MAX_FLT
 constexpr int MAX_COLLIDERS = 16;   // solver/boundary_condition.rs:132
 
@@ -155,7 +156,8 @@ struct alignas(16) Counters {
                             // by the reordering G2P
     uint32_t dt_bound;      // CFL bound, (dt * 1e12) as u32 (written by the timestep-bound query)
     uint32_t rigid_len;     // CPIC: entries of the block-sorted rigid-particle list
-    uint32_t pad[3];
+    uint32_t p2g_next;      // units P2G's warps have taken beyond their first
+    uint32_t pad[2];
 };
 static_assert(sizeof(Counters) == 48, "Counters layout");
 

@@ -4,6 +4,10 @@
 // Same results as the reference: the set of active blocks (every particle's
 // 2x2x2 block neighbourhood), the per-block slab buckets (4 primary z-slabs,
 // 6 extra buckets), the +1 neighbour header ids and the sorted id list.
+//
+// Inside a slab the particles are also grouped by associated cell (64 counters
+// a block, z-major, so the slabs are runs of 16 cells): P2G takes a cell per
+// lane and G2P's neighbouring lanes read the same halo nodes.
 // Header order and the order inside a bucket come from atomics, as in the
 // reference; the canonical pass (deterministic mode) orders every bucket by
 // ascending particle id.  The extras (a particle listed again in each +1
@@ -146,6 +150,7 @@ __global__ void k_sort_reset(DevPtrs P, uint32_t hash_cap) {
         P.counters->sorted_len = 0;
         P.counters->unsorted = 0;
         P.counters->rigid_len = 0;
+        P.counters->p2g_next = 0;
     }
 }
 
@@ -233,6 +238,7 @@ __global__ void __launch_bounds__(256) k_block_prep(DevPtrs P) {
         if (P.nodes) P.nodes[t] = make_float4(0.f, 0.f, 0.f, 0.f);
         // the scatter P2G of CPIC accumulates the incompatible field too
         if (P.nodes_inc && P.params->use_cpic) P.nodes_inc[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (P.cells) P.cells[t] = 0;
         if (k < NUM_NBH) {
             int4 v = P.bvid[b];
             int sx, sy, sz;
@@ -283,14 +289,14 @@ __global__ void __launch_bounds__(256) k_count(DevPtrs P) {
             const uint32_t last = min(31u, hi - 1u - b32);
             known_key = __shfl_sync(0xFFFFFFFFu, key, last);
             known_h0 = __shfl_sync(0xFFFFFFFFu, h0, last);
+            const uint32_t ckey = (h0 != NONE) ? h0 * 64u + code.y : NONE;
             if (active) {
-                P.phdr[p] = h0;
+                P.phdr[p] = ckey;
                 if (h0 == NONE) set_status(P.counters, STATUS_MISSING_BLOCK);
             }
-            const uint32_t ax = code.y & 3u, ay = (code.y >> 2) & 3u, az = (code.y >> 4) & 3u;
-            const uint32_t bkey = (h0 != NONE) ? h0 * 16u + az : NONE;
-            warp_agg_red(bkey, bkey != NONE ? &P.cursors[h0 * NUM_BUCKETS + az] : nullptr);
+            warp_agg_red(ckey, ckey != NONE ? &P.cells[ckey] : nullptr);
             if (!kExtras) continue;
+            const uint32_t ax = code.y & 3u, ay = (code.y >> 2) & 3u, az = (code.y >> 4) & 3u;
             for (int i = 1; i < 8; ++i) {
                 int sx, sy, sz;
                 assoc_shift(i, sx, sy, sz);
@@ -311,7 +317,8 @@ __global__ void __launch_bounds__(256) k_count(DevPtrs P) {
 // sort.rs:382-420 gpu_copy_scan_values_to_first_particles, as a two-pass
 // tiled scan: pass 1 gives each block its offset inside a tile of kScanTile
 // blocks and each tile its total; pass 2 adds the tile's offset (the sum of
-// the tile totals before it) and turns the bucket counts into cursors.
+// the tile totals before it) and turns the bucket counts into cursors.  These
+// two serve the slab sort of launch_sort_positions.
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanPer = kScanTile / kScanThreads;  // blocks per thread
 
@@ -409,14 +416,123 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(DevPtrs P) {
                 running += cnt[j][k];
             }
             P.nwx[b] = running - first;
-            // the runs of kRangeChunk sorted positions that start inside this block
-            if (P.chunk_blk)
-                for (uint32_t c = (first + kRangeChunk - 1u) / kRangeChunk; c * kRangeChunk < running && c < P.chunk_cap; ++c)
-                    P.chunk_blk[c] = b;
             if (b == total - 1) {
                 P.counters->sorted_len = running;
                 if (running > P.params->sorted_capacity) set_status(P.counters, STATUS_SORT_CAPACITY);
             }
+        }
+    }
+}
+
+// The same two passes for the cell sort, one warp per block: a block's total
+// is the sum of its 64 cell counts (and 6 extra buckets); the second pass
+// turns the cell counts into cursors (a warp scan, two cells a lane) and
+// writes the slab ends.
+constexpr uint32_t kCellWarps = kScanThreads / 32;
+constexpr uint32_t kCellPerWarp = kCellTile / kCellWarps;  // blocks per warp of a scan CTA
+static_assert(kCellTile <= kScanThreads, "one block total per thread in the tile scan");
+
+template <bool kExtras>
+__global__ void __launch_bounds__(kScanThreads) k_scan_cell_tiles(DevPtrs P) {
+    __shared__ uint32_t warp_tot[33];
+    __shared__ uint32_t btot[kCellTile];
+    const uint32_t total = P.counters->num_blocks;
+    const uint32_t ntiles = (total + kCellTile - 1) / kCellTile;
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const uint2* cells = reinterpret_cast<const uint2*>(P.cells);
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const uint32_t b0 = tile * kCellTile;
+        uint32_t v[kCellPerWarp];
+#pragma unroll
+        for (uint32_t j = 0; j < kCellPerWarp; ++j) {
+            const uint32_t b = b0 + wid * kCellPerWarp + j;
+            v[j] = 0u;
+            if (b < total) {
+                const uint2 c = __ldcg(&cells[b * 32u + lane]);
+                v[j] = c.x + c.y;
+                if (kExtras && lane < NUM_EXTRA_BUCKETS)
+                    v[j] += __ldcg(&P.cursors[b * NUM_BUCKETS + NUM_PRIMARY_BUCKETS + lane]);
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kCellPerWarp; ++j) {
+            const uint32_t t = __reduce_add_sync(0xFFFFFFFFu, v[j]);
+            if (lane == 0) btot[wid * kCellPerWarp + j] = t;
+        }
+        __syncthreads();
+        const uint32_t mine = threadIdx.x < kCellTile ? btot[threadIdx.x] : 0u;
+        uint32_t tile_total;
+        const uint32_t off = cta_exclusive_scan(mine, warp_tot, &tile_total);
+        if (threadIdx.x < kCellTile && b0 + threadIdx.x < total) P.scan_tmp[b0 + threadIdx.x] = off;
+        if (threadIdx.x == 0) P.tile_sums[tile] = tile_total;
+    }
+}
+
+template <bool kExtras>
+__global__ void __launch_bounds__(kScanThreads) k_scan_cell_apply(DevPtrs P) {
+    __shared__ uint32_t warp_tot[33];
+    const uint32_t total = P.counters->num_blocks;
+    const uint32_t ntiles = (total + kCellTile - 1) / kCellTile;
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    uint2* cells = reinterpret_cast<uint2*>(P.cells);
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const uint32_t b0 = tile * kCellTile + wid * kCellPerWarp;
+        // all loads first: the stores below may alias them as far as the compiler knows
+        uint2 cnt[kCellPerWarp];
+        uint32_t ext[kCellPerWarp];
+#pragma unroll
+        for (uint32_t j = 0; j < kCellPerWarp; ++j) {
+            cnt[j] = make_uint2(0u, 0u);
+            ext[j] = 0u;
+            if (b0 + j < total) {
+                cnt[j] = __ldcg(&cells[(b0 + j) * 32u + lane]);
+                if (kExtras && lane < NUM_EXTRA_BUCKETS)
+                    ext[j] = __ldcg(&P.cursors[(b0 + j) * NUM_BUCKETS + NUM_PRIMARY_BUCKETS + lane]);
+            }
+        }
+        const uint32_t rel = lane < kCellPerWarp && b0 + lane < total ? __ldcg(&P.scan_tmp[b0 + lane]) : 0u;
+        uint32_t part = 0;
+        for (uint32_t i = threadIdx.x; i < tile; i += kScanThreads) part += __ldcg(&P.tile_sums[i]);
+        uint32_t offset;
+        cta_exclusive_scan(part, warp_tot, &offset);
+#pragma unroll
+        for (uint32_t j = 0; j < kCellPerWarp; ++j) {
+            const uint32_t b = b0 + j;
+            if (b >= total) break;
+            const uint32_t first = offset + __shfl_sync(0xFFFFFFFFu, rel, j);
+            uint32_t incl = cnt[j].x + cnt[j].y;
+            uint32_t einc = ext[j];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
+                if (kExtras && o < 8) {
+                    const uint32_t e = __shfl_up_sync(0xFFFFFFFFu, einc, o);
+                    if (lane >= (uint32_t)o) einc += e;
+                }
+            }
+            const uint32_t start = first + incl - cnt[j].x - cnt[j].y;
+            cells[b * 32u + lane] = make_uint2(start, start + cnt[j].x);
+            const uint32_t prim_end = first + __shfl_sync(0xFFFFFFFFu, incl, 31);
+            const uint32_t end = kExtras ? prim_end + __shfl_sync(0xFFFFFFFFu, einc, NUM_EXTRA_BUCKETS - 1) : prim_end;
+            // slab ends (a slab is 16 cells, 8 lanes); the extra buckets' cursors, empty without extras
+            if ((lane & 7u) == 7u) P.cursors[b * NUM_BUCKETS + (lane >> 3)] = first + incl;
+            if (lane < NUM_EXTRA_BUCKETS)
+                P.cursors[b * NUM_BUCKETS + NUM_PRIMARY_BUCKETS + lane] = prim_end + einc - ext[j];
+            if (lane == 0) {
+                P.first[b] = first;
+                P.nprim[b] = prim_end - first;
+                P.nwx[b] = end - first;
+                if (b == total - 1) {
+                    P.counters->sorted_len = end;
+                    if (end > P.params->sorted_capacity) set_status(P.counters, STATUS_SORT_CAPACITY);
+                }
+            }
+            // the runs of kRangeChunk sorted positions that start inside this block
+            if (P.chunk_blk)
+                for (uint32_t c = (first + kRangeChunk - 1u) / kRangeChunk + lane; c * kRangeChunk < end && c < P.chunk_cap;
+                     c += 32u)
+                    P.chunk_blk[c] = b;
         }
     }
 }
@@ -431,25 +547,21 @@ __global__ void __launch_bounds__(256) k_finalize(DevPtrs P) {
     uint32_t lo, hi;
     warp_range(n, lo, hi);
     for (uint32_t base = lo; base < hi; base += 32u * kSortBatch) {
-        uint32_t h0[kSortBatch], code[kSortBatch];
-#pragma unroll
-        for (int j = 0; j < kSortBatch; ++j) {
-            const uint32_t p = base + 32u * j + lane;
-            h0[j] = p < hi ? P.phdr[p] : NONE;
-            code[j] = p < hi ? P.pcode[p].y : 0u;
-        }
-        // the bucket atomics of all passes in flight together, then the scatter
+        // the cell atomics of all passes in flight together, then the scatter
         uint32_t key[kSortBatch], leader[kSortBatch], rank[kSortBatch], got[kSortBatch];
 #pragma unroll
         for (int j = 0; j < kSortBatch; ++j) {
-            const uint32_t az = (code[j] >> 4) & 3u;
-            key[j] = (h0[j] != NONE) ? h0[j] * 16u + az : NONE;
+            const uint32_t p = base + 32u * j + lane;
+            key[j] = p < hi ? P.phdr[p] : NONE;
+        }
+#pragma unroll
+        for (int j = 0; j < kSortBatch; ++j) {
             const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key[j]);
             leader[j] = __ffs(peers) - 1;
             rank[j] = __popc(peers & lt_mask);
             got[j] = 0u;
             if (key[j] != NONE && lane == leader[j])
-                got[j] = atomicAdd(&P.cursors[h0[j] * NUM_BUCKETS + az], (uint32_t)__popc(peers));
+                got[j] = atomicAdd(&P.cells[key[j]], (uint32_t)__popc(peers));
         }
 #pragma unroll
         for (int j = 0; j < kSortBatch; ++j) {
@@ -457,13 +569,13 @@ __global__ void __launch_bounds__(256) k_finalize(DevPtrs P) {
             const uint32_t slot = __shfl_sync(0xFFFFFFFFu, got[j], leader[j]) + rank[j];
             if (key[j] != NONE && slot < scap) P.sorted[slot] = p;
             if (!kExtras) continue;
-            const uint32_t ax = code[j] & 3u, ay = (code[j] >> 2) & 3u, az = (code[j] >> 4) & 3u;
+            const uint32_t h0 = key[j] >> 6, ax = key[j] & 3u, ay = (key[j] >> 2) & 3u, az = (key[j] >> 4) & 3u;
             for (int i = 1; i < 8; ++i) {
                 int sx, sy, sz;
                 assoc_shift(i, sx, sy, sz);
                 uint32_t hn = NONE, e = 0;
-                if (h0[j] != NONE && spills(ax, ay, az, sx, sy, sz)) {
-                    hn = P.nbh[h0[j] * NUM_NBH + (i - 1)];
+                if (key[j] != NONE && spills(ax, ay, az, sx, sy, sz)) {
+                    hn = P.nbh[h0 * NUM_NBH + (i - 1)];
                     e = extra_bucket(az, sz);
                 }
                 const uint32_t k2 = (hn != NONE) ? hn * 16u + e : NONE;
@@ -770,8 +882,13 @@ void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool ca
     case 24: k_count<true, 8><<<g, 256, 0, s>>>(P); break;
     default: k_count<false, 4><<<g, 256, 0, s>>>(P); break;
     }
-    k_scan_tiles<<<c.sm_count, kScanThreads, 0, s>>>(P);
-    k_scan_apply<<<c.sm_count, kScanThreads, 0, s>>>(P);
+    if (with_extras) {
+        k_scan_cell_tiles<true><<<c.sm_count * 2, kScanThreads, 0, s>>>(P);
+        k_scan_cell_apply<true><<<c.sm_count * 2, kScanThreads, 0, s>>>(P);
+    } else {
+        k_scan_cell_tiles<false><<<c.sm_count * 2, kScanThreads, 0, s>>>(P);
+        k_scan_cell_apply<false><<<c.sm_count * 2, kScanThreads, 0, s>>>(P);
+    }
     switch ((with_extras ? 16 : 0) + c.t.sort_batch) {
     case 2: k_finalize<false, 2><<<g, 256, 0, s>>>(P); break;
     case 8: k_finalize<false, 8><<<g, 256, 0, s>>>(P); break;

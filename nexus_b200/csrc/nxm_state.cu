@@ -391,7 +391,7 @@ struct nxm_state {
     uint32_t* hkey = nullptr;
     uint32_t* hval = nullptr;
     int4* bvid = nullptr;
-    uint32_t *first = nullptr, *nprim = nullptr, *nwx = nullptr, *cursors = nullptr, *nbh = nullptr;
+    uint32_t *first = nullptr, *nprim = nullptr, *nwx = nullptr, *cursors = nullptr, *cells = nullptr, *nbh = nullptr;
     float4* nodes = nullptr;
     uint32_t* scan_tmp = nullptr;
     uint32_t* tile_sums = nullptr;
@@ -566,6 +566,7 @@ DevPtrs dev_ptrs(nxm_state* s) {
     P.nprim = s->nprim;
     P.nwx = s->nwx;
     P.cursors = s->cursors;
+    P.cells = s->cells;
     P.nbh = s->nbh;
     P.nodes = s->nodes;
     P.sorted = s->sorted;
@@ -837,10 +838,11 @@ void grid_arrays(nxm_state* s, Slab& g) {
     g.add(&s->nprim, s->block_cap);
     g.add(&s->nwx, s->block_cap);
     g.add(&s->cursors, (size_t)s->block_cap * NUM_BUCKETS);
+    g.add(&s->cells, (size_t)s->block_cap * 64);
     g.add(&s->nbh, (size_t)s->block_cap * NUM_NBH);
     g.add(&s->nodes, (size_t)(s->block_cap + 1) * 64);  // + one block of zeros (halos of missing neighbours)
     g.add(&s->scan_tmp, s->block_cap);
-    g.add(&s->tile_sums, s->block_cap / kScanTile + 2);
+    g.add(&s->tile_sums, s->block_cap / kCellTile + 2);
 }
 
 int free_grid(nxm_state* s) {
@@ -1027,7 +1029,7 @@ int sync_params(nxm_state* s) {
     p.inv_dx = 1.0f / s->dx;
     p.n = s->n;
     p.ncol = (uint32_t)s->colliders.size();
-    p.block_capacity = s->block_cap;
+    p.block_capacity = std::min(s->block_cap, kMaxBlocks);
     p.hash_capacity = s->hash_cap;
     p.sorted_capacity = s->pcap * 8u;
     p.use_cpic = s->use_cpic ? 1u : 0u;

@@ -252,14 +252,17 @@ constexpr uint32_t kG2pThreads = NXM_G2P_THREADS;  // threads per G2P CTA
 // block (shared memory), then advects, updates F and the model, and writes the
 // particle (read from slot `src`, xm / vf = its first two kin words) to slot
 // `dst` of the output records, together with the block key of its new position.
+// The fast build takes the particle's cell from the sort: `vid` is its block,
+// `cell` its associated cell there.
 // kCpicBlock: the CPIC branches (a block whose halo carries affinity bits);
 // the plain instantiation serves every other block without their registers.
 template <bool kCpicBlock>
 __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm, const float4* __restrict__ halo,
-                                             uint32_t src, uint32_t dst, float4 xm, float4 vf, int3 key_off,
-                                             const CpicCtx& cx, volatile float* stash) {
+                                             uint32_t src, uint32_t dst, float4 xm, float4 vf, int4 vid, uint32_t cell,
+                                             int3 key_off, const CpicCtx& cx, volatile float* stash) {
     const float dx = prm.dx, dt = prm.dt;
     const float inv_d = 4.0f / (dx * dx);
+    const float lim2 = (dx / dt) * (dx / dt);
     float4* kr = reinterpret_cast<float4*>(&P.kin_out[dst]);
     uint32_t flags = __float_as_uint(vf.w);
     const v3 pt = mk(xm.x, xm.y, xm.z);
@@ -284,6 +287,8 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
 #else
     (void)cx;
 #endif
+    (void)vid;
+    (void)cell;
     // ---- G2P (g2p.rs:150-270)
     v3 velocity = splat(0.f);
     m3 grad = mzero();
@@ -301,12 +306,15 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
         // so each node costs one weight product and (1 + nonzero s) FMA pairs:
         // the x, y components accumulate as packed f32x2 (FFMA2), z on its own.
         const float inv_dx = prm.inv_dx;
-        const v3 ref = assoc_cell_of(dx, pt) * dx - pt;
+        const uint32_t ax = cell & 3u, ay = (cell >> 2) & 3u, az = cell >> 4;
+        v3 ref = mk((float)((vid.x - key_off.x) * 4 + (int)ax), (float)((vid.y - key_off.y) * 4 + (int)ay),
+                    (float)((vid.z - key_off.z) * 4 + (int)az)) * dx - pt;
+        // a block beyond the packed keys' range carries the aliased coordinates
+        if (fmaxf(fmaxf(fabsf(ref.x), fabsf(ref.y)), fabsf(ref.z)) > 4.0f * dx) ref = assoc_cell_of(dx, pt) * dx - pt;
         const v3 wx = kernel_eval_all(-ref.x * inv_dx);
         const v3 wy = kernel_eval_all(-ref.y * inv_dx);
         const v3 wz = kernel_eval_all(-ref.z * inv_dx);
-        const CellInfo ci = cell_info(dx, pt);
-        const uint32_t packed = ci.ax + 6u * ci.ay + 36u * ci.az;
+        const uint32_t packed = ax + 6u * ay + 36u * az;
         float2 vxy = make_float2(0.f, 0.f), sxxy = vxy, syxy = vxy, szxy = vxy;
         float vz = 0.f, sxz = 0.f, syz = 0.f, szz = 0.f;
 #pragma unroll
@@ -402,8 +410,16 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
     // particle_update.rs:98-102: reproject a penetrating particle
     if (cpic && crec0.w < -0.05f * dx) v = rigid_vel + bc_project(BC_SLIP, 0.0f, v - rigid_vel, pnormal);
 #endif
-    const float vl = length(v);
-    if (vl > dx / dt) v = ((v / vl) * dx) / dt;
+    if (NXM_FAST) {
+        // the square root only near or above the limit
+        if (dot(v, v) > 0.999f * lim2) {
+            const float vl = length(v);
+            if (vl > dx / dt) v = ((v / vl) * dx) / dt;
+        }
+    } else {
+        const float vl = length(v);
+        if (vl > dx / dt) v = ((v / vl) * dx) / dt;
+    }
     if (NXM_FAST) v = v * (1.0f / (1.0f + damping * dt));  // one division instead of three
     else v = v / (1.0f + damping * dt);
     if (flags & PFLAG_FIXED) v = splat(0.f);
@@ -607,7 +623,8 @@ __device__ __forceinline__ void g2p_block_loop(const DevPtrs& P, const Params& p
             nnp = __ldcg(&P.nprim[bn]);
         }
         const bool reorder = P.pid_in != nullptr;
-        const int3 key_off = prm.scene_blocks ? scene_base_of_block(prm, P.bvid[b]) : make_int3(0, 0, 0);
+        const int4 vid = P.bvid[b];
+        const int3 key_off = scene_base_of_block(prm, vid);
         uint32_t pid = tid < np ? __ldg(&P.sorted[first + tid]) : NONE;
         const uint32_t hblk = (tid < 216u && hoct != 0u) ? __ldg(&P.nbh[b * NUM_NBH + hoct - 1u]) : b;
         float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), vf = xm;
@@ -672,11 +689,13 @@ __device__ __forceinline__ void g2p_block_loop(const DevPtrs& P, const Params& p
                 xm = kr[0];
                 vf = kr[1];
             }
+            const uint32_t cell = NXM_FAST ? __ldcg(&P.phdr[pid]) & 63u : 0u;
 #if NXM_CPIC
-            if (cx.halo_cdf) g2p_particle<true>(P, prm, halo, pid, reorder ? first + k : pid, xm, vf, key_off, cx, stash);
+            if (cx.halo_cdf)
+                g2p_particle<true>(P, prm, halo, pid, reorder ? first + k : pid, xm, vf, vid, cell, key_off, cx, stash);
             else
 #endif
-                g2p_particle<false>(P, prm, halo, pid, reorder ? first + k : pid, xm, vf, key_off, cx, stash);
+                g2p_particle<false>(P, prm, halo, pid, reorder ? first + k : pid, xm, vf, vid, cell, key_off, cx, stash);
         }
         __syncthreads();
         b = bn;
@@ -811,8 +830,8 @@ __global__ void k_copy_wait_timeout(Counters* counters, uint32_t limit) {
 // block; run c spans the blocks [chunk_blk[c], chunk_blk[c + 1]] (the scan
 // records the block of each run's first position; the last run reaches the
 // last primary block), usually one or two.  Their halos are staged
-// kRangeHalos at a time, and each thread takes its particle's block from the
-// header id the sort's count pass stored for it (phdr).  A run's span is
+// kRangeHalos at a time, and each thread takes its particle's block and
+// cell from the word the sort's count pass stored for it (phdr).  A run's span is
 // loaded one run ahead, so that a run's own loads (ids, records, halos) are
 // issued together.
 //
@@ -820,6 +839,8 @@ __global__ void k_copy_wait_timeout(Counters* counters, uint32_t limit) {
 // (its particles in rounds of 256), through the same loop: a unit is a span
 // of blocks whose halos are staged in passes and a range of sorted positions
 // the threads step through, so the particle update has one call site.
+// Neighbouring positions are particles of the same cell or the next, so a
+// warp's halo reads are mostly broadcasts.
 //
 // Halo staging: plain loads by every thread (each node: its block id from the
 // neighbour table, then the node, both L2 hits) by default; with
@@ -894,12 +915,12 @@ __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_range(Dev
         // this thread's first particle, fetched while the halos load
         uint32_t pid = p0 + tid < p1 ? __ldg(&P.sorted[p0 + tid]) : NONE;
         float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), vf = xm;
-        uint32_t blk = lo;
+        uint32_t home = lo << 6;  // the particle's block and cell
         if (pid != NONE) {
             const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
             xm = kr[0];
             vf = kr[1];
-            if (!sparse) blk = __ldcg(&P.phdr[pid]);
+            home = __ldcg(&P.phdr[pid]);
         }
         bool pending = pid != NONE;  // dense: this thread's one particle not yet updated
         for (uint32_t b = lo; b <= hi; b += kRangeHalos) {
@@ -920,12 +941,14 @@ __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_range(Dev
                     const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
                     xm = kr[0];
                     vf = kr[1];
+                    home = __ldcg(&P.phdr[pid]);
                 }
+                const uint32_t blk = home >> 6;
                 if (blk >= b && blk - b < cnt) {
-                    const int3 key_off =
-                        prm.scene_blocks ? scene_base_of_block(prm, P.bvid[blk]) : make_int3(0, 0, 0);
-                    g2p_particle<false>(P, prm, halo + 216u * (blk - b), pid, reorder ? p : pid, xm, vf, key_off, cx,
-                                 stash);
+                    const int4 vid = P.bvid[blk];
+                    const int3 key_off = scene_base_of_block(prm, vid);
+                    g2p_particle<false>(P, prm, halo + 216u * (blk - b), pid, reorder ? p : pid, xm, vf, vid, home & 63u,
+                                        key_off, cx, stash);
                     pending = false;
                 }
             }

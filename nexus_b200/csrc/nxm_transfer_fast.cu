@@ -12,64 +12,17 @@ namespace {
 
 __device__ __forceinline__ void set_status_f(Counters* c, uint32_t bit) { atomicOr(&c->status, bit); }
 
-// P2G (solver/p2g.rs:64-351 computes the same node sums in gather form).
-//
-// One CTA per active block (grid-stride).  The block's primary particles are
-// staged in shared memory in chunks of kP2gChunk.  A staged record holds
-//   q = m v + C (x_0 - x_p)  (x_0 = stencil node (0,0,0)) and m,
-//   the three columns of C dx, each carrying one z weight w_z[k] alongside,
-//   the nine products w_x[i] w_y[j],
-// so the contribution to stencil node s is w_x[s.x] w_y[s.y] w_z[s.z]
-// (q + (C dx) s, m).  The chunk is binned by associated cell (counting sort
-// in shared memory).  Each warp then takes one cell at a time: lane l < 27
-// owns the stencil column (s.x, s.y) = ((l mod 9) mod 3, (l mod 9) / 3) for
-// particle group l / 9, so a pass reads three particles (three broadcast
-// addresses per load) and each lane accumulates its column's three nodes.  A
-// three-way shuffle exchange leaves lane l with the cell's full sum for node
-// (s.x, s.y, l / 9), which it adds to the warp's private 6x6x6 node tile
-// (the block plus the first two node layers of its +1 neighbours): the 27
-// lanes own distinct nodes and no other warp writes that tile, so no atomics.
-// At the end of the block the warp tiles are summed and each non-empty node
-// goes to global memory with one float4 atomic; nodes were zeroed by the sort.
-#ifndef NXM_P2G_WARPS
-#define NXM_P2G_WARPS 8
-#endif
-#ifndef NXM_P2G_CHUNK
-#define NXM_P2G_CHUNK 256
-#endif
-#ifndef NXM_P2G_MIN_CTAS
-#define NXM_P2G_MIN_CTAS 3
-#endif
-constexpr int kP2gWarps = NXM_P2G_WARPS;
-constexpr int kP2gThreads = 32 * kP2gWarps;
-constexpr int kP2gChunk = NXM_P2G_CHUNK;  // particles staged per pass
-constexpr int kP2gRec = 28;  // floats per staged particle
-// record: [0..3] q.xyz, m | [4..7] (C dx).c0, w_z[0] | [8..11] (C dx).c1, w_z[1]
-//       | [12..15] (C dx).c2, w_z[2] | [16 + i + 3 j] w_x[i] w_y[j] | [25..27] unused
-constexpr size_t kP2gSmem = (size_t)kP2gWarps * 216 * 16 + (size_t)kP2gChunk * kP2gRec * 4 + (64 + 68) * 4 +
-                            (size_t)kP2gChunk * (2 + 2 + 1);
-// CPIC adds the warps' incompatible-field tiles and the 216 tile nodes' affinity bits
-constexpr size_t kP2gSmemCpic = kP2gSmem + (size_t)kP2gWarps * 216 * 16 + 218 * 4 + 16;
-static_assert(kP2gChunk <= 65536, "staged particle indices are 16-bit");
-
 __device__ __forceinline__ float4 f4add(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
-// One staged particle's raw record (kin words 0..19, CPIC: its affinity
-// bits) and a block header.
+// The words of a particle's kinematic record that P2G reads (kin words 0..19).
 struct P2gRaw {
     float4 xm, vf, c0, c1, c2;
-    float aff;
-};
-struct P2gHdr {
-    uint32_t first, np;
 };
 
-template <bool kCpic>
 __device__ __forceinline__ P2gRaw p2g_load_raw(const DevPtrs& P, uint32_t pid) {
     P2gRaw r;
-    r.aff = 0.f;
     if (pid == NONE) {
-        r.vf = make_float4(0.f, 0.f, 0.f, 0.f);  // flags 0: not staged
+        r.vf = make_float4(0.f, 0.f, 0.f, 0.f);  // flags 0: contributes nothing
         return r;
     }
     const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
@@ -78,10 +31,221 @@ __device__ __forceinline__ P2gRaw p2g_load_raw(const DevPtrs& P, uint32_t pid) {
     r.c0 = __ldg(kr + 2);
     r.c1 = __ldg(kr + 3);
     r.c2 = __ldg(kr + 4);
-    // CPIC keeps particles in id order (slot = id): the affinity of this step's g2p_cdf
-    if (kCpic) r.aff = __ldg(&P.pcdf[3u * pid + 1u].w);
     return r;
 }
+
+// P2G (solver/p2g.rs:64-351 computes the same node sums in gather form).
+//
+// One warp per active block (taken from a counter), one cell per lane.  The
+// sort lists a block's particles by associated cell, so a lane walks its
+// cell's particles and keeps the cell's 27 nodes x (momentum, mass) in
+// registers: no particle is staged, binned or exchanged, and no two lanes
+// share an accumulator.  The contribution to stencil node s = (i, j, k) is
+// w_x[i] w_y[j] w_z[k] (q + (C dx) s, m) with q = m v + C (x_0 - x_p), x_0 =
+// node (0,0,0); per z layer k the factors w_z[k] (q + k C_z dx, m), w_z[k] C_x
+// dx and w_z[k] C_y dx are formed once.  At the end of a round the lanes add
+// their nodes into the warp's 6x6x6 tile (the block plus the first two node
+// layers of its +1 neighbours), one stencil offset at a time: distinct cells,
+// distinct nodes, so no atomics.  The tile goes to global memory with one
+// float4 atomic per non-zero node; nodes were zeroed by the sort.
+//
+// A round ends with its fullest cell, so the 64 cells are split by count: the
+// 32 fullest in the first round, the rest in the second (none when at most 32
+// hold particles).  Bound by FP32 issue and the record loads; 512 threads' worth
+// of registers an SM (the 108 sums) leave 12 warps, whose next records are in
+// flight while the current ones accumulate.
+#ifndef NXM_P2G_MIN_CTAS
+#define NXM_P2G_MIN_CTAS 3
+#endif
+constexpr int kP2gWarps = 4;
+constexpr int kP2gThreads = 32 * kP2gWarps;
+
+__global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P) {
+    __shared__ float4 tiles[kP2gWarps][216];
+    __shared__ uint8_t orders[kP2gWarps][64];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    float4* tile = tiles[warp];
+    uint8_t* order = orders[warp];
+    const float dx = P.params->dx;
+    const float inv_dx = P.params->inv_dx;
+    const uint32_t nbp = min(__ldcg(&P.counters->num_primary), __ldcg(&P.counters->num_blocks));
+    const uint32_t nwarps = gridDim.x * kP2gWarps;
+    // With fewer blocks than half the warps, a block's two rounds go to two warps.
+    const bool split = 2u * nbp <= nwarps;
+    const uint32_t units = split ? 2u * nbp : nbp;
+    for (uint32_t t = lane; t < 216u; t += 32u) tile[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t u = warp * gridDim.x + blockIdx.x;  // the first units go to different SMs
+    while (u < units) {
+        uint32_t next = units;
+        if (units > nwarps && lane == 0) next = nwarps + atomicAdd(&P.counters->p2g_next, 1u);
+        const uint32_t b = split ? u >> 1 : u;
+        int4 vid = P.bvid[b];
+        {
+            const int3 o = scene_base_of_block(*P.params, vid);  // scene-local block coordinates
+            vid.x -= o.x; vid.y -= o.y; vid.z -= o.z;
+        }
+        const uint32_t my_nbh = lane < NUM_NBH ? __ldg(&P.nbh[b * NUM_NBH + lane]) : b;
+        // the cells' ranges of the sorted list: lane's cells are `lane` and `lane + 32`
+        const uint32_t el = __ldg(&P.cells[b * 64u + lane]), eh = __ldg(&P.cells[b * 64u + 32u + lane]);
+        uint32_t sl = __shfl_up_sync(0xFFFFFFFFu, el, 1), sh = __shfl_up_sync(0xFFFFFFFFu, eh, 1);
+        const uint32_t mid = __shfl_sync(0xFFFFFFFFu, el, 31);
+        if (lane == 0) {
+            sl = __ldg(&P.first[b]);
+            sh = mid;
+        }
+        const uint32_t cl = el - sl, ch = eh - sh;
+        // the smallest threshold that at most 32 cells exceed
+        const auto above = [&](uint32_t t) {
+            return __popc(__ballot_sync(0xFFFFFFFFu, cl > t)) + __popc(__ballot_sync(0xFFFFFFFFu, ch > t));
+        };
+        uint32_t thr = 0;
+        if (above(0) > 32) {
+            uint32_t lo = 0, hi = __reduce_max_sync(0xFFFFFFFFu, max(cl, ch));
+            while (hi - lo > 1u) {
+                const uint32_t m = (lo + hi) >> 1;
+                if (above(m) > 32) lo = m; else hi = m;
+            }
+            thr = hi;
+        }
+        {  // the cells above it, then as many at it as fill 32 lanes; the others after them
+            const uint32_t need = 32u - above(thr);
+            const uint32_t eql = __ballot_sync(0xFFFFFFFFu, cl == thr), eqh = __ballot_sync(0xFFFFFFFFu, ch == thr);
+            const bool inl = cl > thr || (cl == thr && __popc(eql & lt) < need);
+            const bool inh = ch > thr || (ch == thr && __popc(eql) + __popc(eqh & lt) < need);
+            const uint32_t ml = __ballot_sync(0xFFFFFFFFu, inl), mh = __ballot_sync(0xFFFFFFFFu, inh);
+            const uint32_t nl = __popc(ml);
+            order[inl ? __popc(ml & lt) : 32u + __popc(~ml & lt)] = (uint8_t)lane;
+            order[inh ? nl + __popc(mh & lt) : 64u - nl + __popc(~mh & lt)] = (uint8_t)(lane + 32u);
+            __syncwarp();
+        }
+        const uint32_t r_end = split ? (u & 1u) + 1u : 2u;
+        for (uint32_t round = split ? (u & 1u) : 0u; round < r_end; ++round) {
+            if (round == 1u && thr == 0u) break;  // the second round's cells are empty
+            const uint32_t c = order[round * 32u + lane];
+            const uint32_t s0 = __shfl_sync(0xFFFFFFFFu, sl, c & 31u), s1 = __shfl_sync(0xFFFFFFFFu, sh, c & 31u);
+            const uint32_t n0 = __shfl_sync(0xFFFFFFFFu, cl, c & 31u), n1 = __shfl_sync(0xFFFFFFFFu, ch, c & 31u);
+            const uint32_t* list = P.sorted + (c < 32u ? s0 : s1);
+            const uint32_t n = c < 32u ? n0 : n1;
+            const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, n);
+            const uint32_t cx = c & 3u, cy = (c >> 2) & 3u, cz = c >> 4;
+            const v3 x0 = mk((float)(vid.x * 4 + (int)cx), (float)(vid.y * 4 + (int)cy), (float)(vid.z * 4 + (int)cz)) * dx;
+            float2 axy[27], azm[27];  // sums of node i + 3 j + 9 k: (x, y) and (z, mass)
+#pragma unroll
+            for (int t = 0; t < 27; ++t) axy[t] = azm[t] = make_float2(0.f, 0.f);
+            P2gRaw raw = p2g_load_raw(P, n > 0u ? __ldg(&list[0]) : NONE);
+            uint32_t pid = n > 1u ? __ldg(&list[1]) : NONE;
+#pragma unroll 1
+            for (uint32_t it = 0; it < nmax; ++it) {
+                const bool on = (__float_as_uint(raw.vf.w) & PFLAG_ENABLED) != 0u;
+                const v3 r = x0 - mk(raw.xm.x, raw.xm.y, raw.xm.z);
+                const v3 wx = kernel_eval_all(-r.x * inv_dx);
+                const v3 wy = kernel_eval_all(-r.y * inv_dx);
+                const v3 wz = kernel_eval_all(-r.z * inv_dx);
+                const float m = raw.xm.w;
+                const m3 C = mkm(mk(raw.c0.x, raw.c0.y, raw.c0.z), mk(raw.c1.x, raw.c1.y, raw.c1.z),
+                                 mk(raw.c2.x, raw.c2.y, raw.c2.z));
+                const v3 q = C * r + mk(raw.vf.x, raw.vf.y, raw.vf.z) * m;
+                const m3 K = C * dx;
+                raw = p2g_load_raw(P, pid);
+                pid = it + 2u < n ? __ldg(&list[it + 2u]) : NONE;
+                if (!on) continue;
+                float wxy[9];
+#pragma unroll
+                for (int t = 0; t < 9; ++t) wxy[t] = vget(wx, t % 3) * vget(wy, t / 3);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float wk = vget(wz, k);
+                    const v3 bk = k == 0 ? q : (k == 1 ? q + K.c2 : q + K.c2 * 2.0f);
+                    float2 pxy = make_float2(bk.x * wk, bk.y * wk), pzm = make_float2(bk.z * wk, m * wk);
+                    const float2 ixy = make_float2(K.c0.x * wk, K.c0.y * wk), izm = make_float2(K.c0.z * wk, 0.f);
+                    const float2 jxy = make_float2(K.c1.x * wk, K.c1.y * wk), jzm = make_float2(K.c1.z * wk, 0.f);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        if (j) {
+                            pxy = __fadd2_rn(pxy, jxy);
+                            pzm = __fadd2_rn(pzm, jzm);
+                        }
+                        float2 bxy = pxy, bzm = pzm;
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            if (i) {
+                                bxy = __fadd2_rn(bxy, ixy);
+                                bzm = __fadd2_rn(bzm, izm);
+                            }
+                            const float w = wxy[i + 3 * j];
+                            const int t = i + 3 * j + 9 * k;
+                            axy[t] = __ffma2_rn(make_float2(w, w), bxy, axy[t]);
+                            azm[t] = __ffma2_rn(make_float2(w, w), bzm, azm[t]);
+                        }
+                    }
+                }
+            }
+            float4* node = tile + cx + 6u * cy + 36u * cz;
+#pragma unroll
+            for (int t = 0; t < 27; ++t) {
+                const int off = t % 3 + 6 * ((t / 3) % 3) + 36 * (t / 9);
+                if (n) {
+                    const float4 o = node[off];
+                    node[off] = make_float4(o.x + axy[t].x, o.y + axy[t].y, o.z + azm[t].x, o.w + azm[t].y);
+                }
+                __syncwarp();  // the next offset's nodes are other lanes' nodes of this one
+            }
+        }
+        // the tile to global memory (clearing it)
+        for (uint32_t t = lane; t < 224u; t += 32u) {
+            const uint32_t tx = t % 6u, ty = (t / 6u) % 6u, tz = t / 36u;
+            const uint32_t ox = tx >= 4u, oy = ty >= 4u, oz = tz >= 4u;
+            const uint32_t oct = ox * 4u + oy * 2u + oz;
+            const uint32_t other = __shfl_sync(0xFFFFFFFFu, my_nbh, (oct + 31u) & 31u);
+            if (t >= 216u) continue;
+            const uint32_t blk = oct ? other : b;
+            const float4 sum = tile[t];
+            if (sum.x != 0.f || sum.y != 0.f || sum.z != 0.f || sum.w != 0.f) {
+                tile[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+                const uint32_t node = (tx - 4u * ox) + 4u * (ty - 4u * oy) + 16u * (tz - 4u * oz);
+                if (blk == NONE) set_status_f(P.counters, STATUS_MISSING_BLOCK);
+                else atomicAdd(&P.nodes[blk * 64u + node], sum);
+            }
+        }
+        __syncwarp();
+        u = __shfl_sync(0xFFFFFFFFu, next, 0);
+    }
+}
+
+// CPIC P2G (solver/p2g.rs:258-310): a particle whose affinity bits are
+// incompatible with a node's (aff_compatible) feeds that node's second,
+// incompatible field instead.
+//
+// One CTA per active block (grid-stride).  The block's primary particles are
+// staged in shared memory in chunks of kCpicChunk.  A staged record holds
+//   q = m v + C (x_0 - x_p)  (x_0 = stencil node (0,0,0)) and m,
+//   the three columns of C dx, each carrying one z weight w_z[k] alongside,
+//   the nine products w_x[i] w_y[j], the affinity bits,
+// so the contribution to stencil node s is w_x[s.x] w_y[s.y] w_z[s.z]
+// (q + (C dx) s, m).  The sort lists the particles by associated cell; each
+// warp takes one cell's staged particles at a time: lane l < 27
+// owns the stencil column (s.x, s.y) = ((l mod 9) mod 3, (l mod 9) / 3) for
+// particle group l / 9, so a pass reads three particles (three broadcast
+// addresses per load) and each lane accumulates its column's three nodes, the
+// compatible and the incompatible sums.  A
+// three-way shuffle exchange leaves lane l with the cell's full sum for node
+// (s.x, s.y, l / 9), which it adds to the warp's private 6x6x6 node tile (one
+// per field): the 27
+// lanes own distinct nodes and no other warp writes that tile, so no atomics.
+// At the end of the block the warp tiles are summed and each non-empty node
+// goes to global memory with one float4 atomic; nodes were zeroed by the sort.
+constexpr int kCpicWarps = 8;
+constexpr int kCpicThreads = 32 * kCpicWarps;
+constexpr int kCpicChunk = kCpicThreads;  // particles staged per pass, one per thread
+constexpr int kCpicRec = 28;  // floats per staged particle
+// record: [0..3] q.xyz, m | [4..7] (C dx).c0, w_z[0] | [8..11] (C dx).c1, w_z[1]
+//       | [12..15] (C dx).c2, w_z[2] | [16 + i + 3 j] w_x[i] w_y[j] | [25] affinity | [26..27] unused
+constexpr size_t kCpicSmem = (size_t)2 * kCpicWarps * 216 * 16 + (size_t)kCpicChunk * kCpicRec * 4 + 68 * 4 + 218 * 4;
+
+struct P2gHdr {
+    uint32_t first, np;
+};
 
 __device__ __forceinline__ P2gHdr p2g_load_hdr(const DevPtrs& P, uint32_t b, uint32_t nbp) {
     P2gHdr h{0u, 0u};
@@ -97,26 +261,15 @@ __device__ __forceinline__ P2gHdr p2g_load_hdr(const DevPtrs& P, uint32_t b, uin
 // grid strides ahead, the sorted id of the next chunk's particle right after
 // staging, and its 80-byte record at the start of the cell phase, so their
 // latency overlaps the current chunk's shared-memory work.
-//
-// CPIC (kCpic; solver/p2g.rs:258-310): a particle whose affinity bits are
-// incompatible with a node's (aff_compatible) feeds that node's second,
-// incompatible field instead: each lane keeps both sums for its three nodes,
-// and the warps keep a second tile flushed into nodes_inc.
-template <bool kCpic>
-__global__ void __launch_bounds__(kP2gThreads, kCpic ? 2 : NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P) {
-    static_assert(kP2gChunk == kP2gThreads, "one staged particle per thread");
-    static_assert(kP2gThreads >= 216, "one flushed tile node per thread");
+__global__ void __launch_bounds__(kCpicThreads, 2) k_p2g_cpic(DevPtrs P) {
+    static_assert(kCpicThreads >= 216, "one flushed tile node per thread");
     extern __shared__ float4 p2g_smem[];
-    float4* tiles = p2g_smem;  // kP2gWarps x 216 nodes of (x, y, z, m)
-    float4* tiles_inc = tiles + kP2gWarps * 216;  // CPIC only
-    float* rec = reinterpret_cast<float*>(tiles + (kCpic ? 2 : 1) * kP2gWarps * 216);
-    int* cnt = reinterpret_cast<int*>(rec + kP2gChunk * kP2gRec);
-    int* start = cnt + 64;  // 65 used
-    uint16_t* perm = reinterpret_cast<uint16_t*>(start + 68);
-    uint16_t* prank = perm + kP2gChunk;
-    uint8_t* pcell = reinterpret_cast<uint8_t*>(prank + kP2gChunk);
-    uint32_t* node_aff = reinterpret_cast<uint32_t*>(pcell + ((kP2gChunk + 15) & ~15));  // CPIC: 216 tile nodes
-    // CPIC: nonzero when a tile node of the current block carries an affinity
+    float4* tiles = p2g_smem;  // kCpicWarps x 216 nodes of (x, y, z, m)
+    float4* tiles_inc = tiles + kCpicWarps * 216;
+    float* rec = reinterpret_cast<float*>(tiles + 2 * kCpicWarps * 216);
+    int* start = reinterpret_cast<int*>(rec + kCpicChunk * kCpicRec);  // 65 used
+    uint32_t* node_aff = reinterpret_cast<uint32_t*>(start + 68);  // 216 tile nodes
+    // Nonzero when a tile node of the current block carries an affinity
     // bit; otherwise every particle is compatible with every node and the
     // block runs the plain accumulation (no incompatible sums, no flush).
     // Two flags by block parity: the one of the next block is cleared while
@@ -126,14 +279,6 @@ __global__ void __launch_bounds__(kP2gThreads, kCpic ? 2 : NXM_P2G_MIN_CTAS) k_p
 
     const float dx = P.params->dx;
     const float inv_dx = P.params->inv_dx;
-#ifndef NXM_P2G_POW2
-#define NXM_P2G_POW2 1
-#endif
-    // a power-of-two cell width divides exactly by multiplying with its
-    // reciprocal (the association must round as the reference's division)
-    const uint32_t dxb = __float_as_uint(dx);
-    const bool pow2 = NXM_P2G_POW2 && (dxb & 0x807FFFFFu) == 0u && (dxb >> 23) - 1u < 253u;
-    const float rdx = __uint_as_float((254u << 23) - dxb);
     const uint32_t nbp = min(__ldcg(&P.counters->num_primary), __ldcg(&P.counters->num_blocks));
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     // cell-phase roles; lanes 27..31 idle (zero weight, never write)
@@ -150,18 +295,20 @@ __global__ void __launch_bounds__(kP2gThreads, kCpic ? 2 : NXM_P2G_MIN_CTAS) k_p
     const uint32_t fox = ftx >= 4u, foy = fty >= 4u, foz = ftz >= 4u;
     const uint32_t foct = fox * 4u + foy * 2u + foz;
     const uint32_t fnode = (ftx - 4u * fox) + 4u * (fty - 4u * foy) + 16u * (ftz - 4u * foz);
+    // particles stay in id order (slot = id): the affinity of this step's g2p_cdf
+    const auto load_aff = [&](uint32_t pid) { return pid == NONE ? 0.f : __ldg(&P.pcdf[3u * pid + 1u].w); };
 
     uint32_t b = blockIdx.x;
     if (b >= nbp) return;
     const uint32_t stride = gridDim.x;
-    for (uint32_t t = tid; t < (kCpic ? 2u : 1u) * kP2gWarps * 216u; t += kP2gThreads)
-        tiles[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tid < 64) cnt[tid] = 0;
-    if (kCpic && tid == 0) blk_aff_pair[0] = 0u;
+    for (uint32_t t = tid; t < 2u * kCpicWarps * 216u; t += kCpicThreads) tiles[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tid == 0) blk_aff_pair[0] = 0u;
     P2gHdr h = p2g_load_hdr(P, b, nbp);
     P2gHdr hn = p2g_load_hdr(P, b + stride, nbp);
     P2gHdr hnn = p2g_load_hdr(P, b + 2u * stride, nbp);
-    P2gRaw raw = p2g_load_raw<kCpic>(P, tid < h.np ? __ldg(&P.sorted[h.first + tid]) : NONE);
+    uint32_t pid = tid < h.np ? __ldg(&P.sorted[h.first + tid]) : NONE;
+    P2gRaw raw = p2g_load_raw(P, pid);
+    float aff = load_aff(pid);
     __syncthreads();
     for (;;) {
         int4 vid = P.bvid[b];
@@ -170,24 +317,27 @@ __global__ void __launch_bounds__(kP2gThreads, kCpic ? 2 : NXM_P2G_MIN_CTAS) k_p
             vid.x -= o.x; vid.y -= o.y; vid.z -= o.z;
         }
         const uint32_t fblk = (tid < 216u && foct != 0u) ? __ldg(&P.nbh[b * NUM_NBH + foct - 1u]) : b;
+        // this thread's cell: the end of its particles in the block's list
+        const uint32_t cell_end = tid < 64u ? __ldg(&P.cells[b * 64u + tid]) - h.first : 0u;
         volatile uint32_t* blk_aff = blk_aff_pair + parity;
-        if (kCpic && tid == 0) blk_aff_pair[parity ^ 1u] = 0u;
-        if (kCpic && tid < 216u) {  // read after the staging barrier below
+        if (tid == 0) blk_aff_pair[parity ^ 1u] = 0u;
+        if (tid < 216u) {  // read after the staging barrier below
             const uint32_t na = fblk == NONE ? 0u : __ldg(&P.ncdf[fblk * 64u + fnode].y);
             node_aff[tid] = na;
             if (na & 0x0000FFFFu) *blk_aff = 1u;
         }
-        for (uint32_t base = 0; base < h.np; base += kP2gChunk) {
-            const uint32_t m_chunk = min(h.np - base, (uint32_t)kP2gChunk);
-            // 1. stage and bin this thread's particle (base + tid)
+        for (uint32_t base = 0; base < h.np; base += kCpicChunk) {
+            const uint32_t m_chunk = min(h.np - base, (uint32_t)kCpicChunk);
+            // 1. stage this thread's particle (base + tid); a disabled one as zeros
             if (tid < m_chunk) {
-                const uint32_t k = tid;
+                float4* rr = reinterpret_cast<float4*>(rec + tid * kCpicRec);
                 if (!(__float_as_uint(raw.vf.w) & PFLAG_ENABLED)) {
-                    pcell[k] = 255;
+#pragma unroll
+                    for (int w = 0; w < 7; ++w) rr[w] = make_float4(0.f, 0.f, 0.f, 0.f);
                 } else {
                     const v3 pt = mk(raw.xm.x, raw.xm.y, raw.xm.z);
                     const float m = raw.xm.w;
-                    const CellInfo ci = pow2 ? cell_info_scaled(pt * rdx) : cell_info(dx, pt);
+                    const CellInfo ci = cell_info(dx, pt);
                     const v3 r = mk((float)(vid.x * 4 + (int)ci.ax), (float)(vid.y * 4 + (int)ci.ay),
                                     (float)(vid.z * 4 + (int)ci.az)) * dx - pt;
                     const v3 wx = kernel_eval_all(-r.x * inv_dx);
@@ -196,56 +346,35 @@ __global__ void __launch_bounds__(kP2gThreads, kCpic ? 2 : NXM_P2G_MIN_CTAS) k_p
                     const m3 C = mkm(mk(raw.c0.x, raw.c0.y, raw.c0.z), mk(raw.c1.x, raw.c1.y, raw.c1.z),
                                      mk(raw.c2.x, raw.c2.y, raw.c2.z));
                     const v3 q = C * r + mk(raw.vf.x, raw.vf.y, raw.vf.z) * m;
-                    float4* rr = reinterpret_cast<float4*>(rec + k * kP2gRec);
                     rr[0] = make_float4(q.x, q.y, q.z, m);
                     rr[1] = make_float4(C.c0.x * dx, C.c0.y * dx, C.c0.z * dx, wz.x);
                     rr[2] = make_float4(C.c1.x * dx, C.c1.y * dx, C.c1.z * dx, wz.y);
                     rr[3] = make_float4(C.c2.x * dx, C.c2.y * dx, C.c2.z * dx, wz.z);
                     rr[4] = make_float4(wx.x * wy.x, wx.y * wy.x, wx.z * wy.x, wx.x * wy.y);
                     rr[5] = make_float4(wx.y * wy.y, wx.z * wy.y, wx.x * wy.z, wx.y * wy.z);
-                    rr[6] = make_float4(wx.z * wy.z, raw.aff, 0.f, 0.f);
-                    const uint32_t c = ci.ax + 4u * ci.ay + 16u * ci.az;
-                    pcell[k] = (uint8_t)c;
-                    prank[k] = (uint16_t)atomicAdd(&cnt[c], 1);
+                    rr[6] = make_float4(wx.z * wy.z, aff, 0.f, 0.f);
                 }
             }
+            // where each cell's particles lie in this chunk
+            if (tid < 64u) start[tid + 1] = (int)min(max(cell_end, base) - base, m_chunk);
+            if (tid == 64u) start[0] = 0;
             // sorted id of this thread's particle in the next chunk (this block or the next one)
             uint32_t pid_next = NONE;
-            if (base + kP2gChunk < h.np) {
-                if (base + kP2gChunk + tid < h.np) pid_next = __ldg(&P.sorted[h.first + base + kP2gChunk + tid]);
+            if (base + kCpicChunk < h.np) {
+                if (base + kCpicChunk + tid < h.np) pid_next = __ldg(&P.sorted[h.first + base + kCpicChunk + tid]);
             } else if (tid < hn.np) {
                 pid_next = __ldg(&P.sorted[hn.first + tid]);
             }
             __syncthreads();
-            // 2. exclusive scan of the 64 cell counts
-            if (warp == 0) {
-                const int v0 = cnt[2 * lane], v1 = cnt[2 * lane + 1];
-                int incl = v0 + v1;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                    if ((int)lane >= o) incl += y;
-                }
-                const int excl = incl - v0 - v1;
-                start[2 * lane] = excl;
-                start[2 * lane + 1] = excl + v0;
-                if (lane == 31) start[64] = incl;
-            }
-            __syncthreads();
-            if (tid < m_chunk) {
-                const uint32_t c = pcell[tid];
-                if (c != 255u) perm[start[c] + prank[tid]] = (uint16_t)tid;
-            }
-            __syncthreads();
-            if (tid < 64) cnt[tid] = 0;  // counts are consumed; ready for the next chunk
-            raw = p2g_load_raw<kCpic>(P, pid_next);
-            const bool split = kCpic && *blk_aff != 0u;
-            // 3. one warp per cell, three particles per pass
-            for (uint32_t c = warp; c < 64u; c += kP2gWarps) {
+            raw = p2g_load_raw(P, pid_next);
+            aff = load_aff(pid_next);
+            const bool split = *blk_aff != 0u;
+            // 2. one warp per cell, three particles per pass
+            for (uint32_t c = warp; c < 64u; c += kCpicWarps) {
                 const int s0 = start[c], s1 = start[c + 1];
                 if (s0 == s1) continue;
                 float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0, a2 = a0;  // s.z = 0, 1, 2
-                float4 i0 = a0, i1 = a0, i2 = a0;  // CPIC: the incompatible sums
+                float4 i0 = a0, i1 = a0, i2 = a0;  // the incompatible sums
                 const uint32_t cx = c & 3u, cy = (c >> 2) & 3u, cz = c >> 4;
                 const uint32_t col = (cx + sxy % 3u) + 6u * (cy + sxy / 3u) + 36u * cz;  // this lane's s.z = 0 node
                 uint32_t na0 = 0u, na1 = 0u, na2 = 0u;
@@ -257,7 +386,7 @@ __global__ void __launch_bounds__(kP2gThreads, kCpic ? 2 : NXM_P2G_MIN_CTAS) k_p
                 for (int i = s0; i < s1; i += 3) {
                     const int j = i + (int)grp;
                     const bool valid = worker && j < s1;
-                    const float* r = rec + (uint32_t)perm[valid ? j : s0] * kP2gRec;
+                    const float* r = rec + (valid ? j : s0) * kCpicRec;
                     const float4 qm = *reinterpret_cast<const float4*>(r);
                     const float4 k0 = *reinterpret_cast<const float4*>(r + 4);
                     const float4 k1 = *reinterpret_cast<const float4*>(r + 8);
@@ -314,15 +443,15 @@ __global__ void __launch_bounds__(kP2gThreads, kCpic ? 2 : NXM_P2G_MIN_CTAS) k_p
             }
             __syncthreads();
         }
-        // 4. sum the warp tiles (clearing them) and flush the block's nodes
-        const int nfields = kCpic && *blk_aff != 0u ? 2 : 1;
+        // 3. sum the warp tiles (clearing them) and flush the block's nodes
+        const int nfields = *blk_aff != 0u ? 2 : 1;
         if (tid < 216u) {
             for (int f = 0; f < nfields; ++f) {
                 float4* tt = f ? tiles_inc : tiles;
                 float4 sum = tt[tid];
                 tt[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int w = 1; w < kP2gWarps; ++w) {
+                for (int w = 1; w < kCpicWarps; ++w) {
                     sum = f4add(sum, tt[w * 216 + tid]);
                     tt[w * 216 + tid] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
@@ -345,13 +474,12 @@ __global__ void __launch_bounds__(kP2gThreads, kCpic ? 2 : NXM_P2G_MIN_CTAS) k_p
 }  // namespace
 
 void launch_p2g(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
-    cudaFuncSetAttribute(k_p2g<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2gSmem);
-    k_p2g<false><<<c.sm_count * (int)min(c.t.p2g_ctas, (uint32_t)NXM_P2G_MIN_CTAS), kP2gThreads, kP2gSmem, s>>>(P);
+    k_p2g<<<c.sm_count * (int)min(c.t.p2g_ctas, (uint32_t)NXM_P2G_MIN_CTAS), kP2gThreads, 0, s>>>(P);
 }
 
 void launch_p2g_cpic(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
-    cudaFuncSetAttribute(k_p2g<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2gSmemCpic);
-    k_p2g<true><<<c.sm_count * 2, kP2gThreads, kP2gSmemCpic, s>>>(P);
+    cudaFuncSetAttribute(k_p2g_cpic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCpicSmem);
+    k_p2g_cpic<<<c.sm_count * 2, kCpicThreads, kCpicSmem, s>>>(P);
 }
 
 
