@@ -66,6 +66,24 @@ __device__ __forceinline__ m3 diag(v3 d) { return mkm(mk(d.x, 0, 0), mk(0, d.y, 
 __device__ __forceinline__ float trace(const m3& a) { return a.c0.x + a.c1.y + a.c2.z; }
 __device__ __forceinline__ m3 outer(v3 a, v3 b) { return mkm(a * b.x, a * b.y, a * b.z); }
 
+// 32-byte records in one 256-bit access (sm_100).
+struct f8 {
+    float v[8];
+};
+// (through the read-only path: the record is not written before the load by this kernel)
+__device__ __forceinline__ f8 load8(const void* p) {
+    f8 r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
+        : "l"(p));
+    return r;
+}
+__device__ __forceinline__ void store8(void* p, float a, float b, float c, float d, float e, float f, float g, float h) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d),
+                 "f"(e), "f"(f), "f"(g), "f"(h)
+                 : "memory");
+}
+
 struct quat {
     float x, y, z, w;
 };
@@ -287,7 +305,7 @@ __device__ __forceinline__ Svd svd3(const m3& f) {
 // frame u: a rotation updates 6 entries and one matrix where the one-sided
 // sweeps above update two matrices and form three dot products, and e keeps
 // the small strains that 1 + e would round away.  Stops when every
-// off-diagonal is below 3e-7 of the matrix (two to four sweeps).
+// off-diagonal is below 3e-7 of the matrix or the rounding of its entries.
 struct Strain {
     v3 e;
     m3 u;
@@ -322,7 +340,7 @@ __device__ __forceinline__ Strain strain_of(const m3& F) {
     float xy = F.c0.x * F.c0.y + F.c1.x * F.c1.y + F.c2.x * F.c2.y;
     float xz = F.c0.x * F.c0.z + F.c1.x * F.c1.z + F.c2.x * F.c2.z;
     float yz = F.c0.y * F.c0.z + F.c1.y * F.c1.z + F.c2.y * F.c2.z;
-    const float tol = 1.0e-13f * (xx * xx + yy * yy + zz * zz + 2.0f * (xy * xy + xz * xz + yz * yz));
+    const float tol = 1.0e-13f * (xx * xx + yy * yy + zz * zz + 2.0f * (xy * xy + xz * xz + yz * yz)) + 1.0e-15f;
     Strain r;
     r.u = mident();
 #pragma unroll 1

@@ -7,11 +7,19 @@
 
 namespace nxm {
 
+// The records of the particles, one entry per storage slot.
+struct Particles {
+    PKin* kin;
+    PAff* aff;
+    PAffTail* tail;
+    PDef* def;
+    PMat* mat;
+    float4* pstate;          // model state words (plastic models)
+};
+
 // Device pointers of one state, passed by value to every kernel.
 struct DevPtrs {
-    PKin* kin;
-    PDef* def;
-    float4* pstate;          // model state words (plastic models)
+    Particles in;
     const Material* materials;
     DevCollider* colliders;
     const DevTri* tris;      // trimesh triangles of all trimesh colliders
@@ -41,12 +49,10 @@ struct DevPtrs {
     // these runs)
     uint32_t* chunk_blk;
     uint32_t chunk_cap;
-    // G2P output.  In place: the *_out pointers equal the inputs and pid_in is
-    // null.  Reordering: sorted entry j is written to slot j of the *_out
+    // G2P output.  In place: `out` equals `in` and pid_in is null.
+    // Reordering: sorted entry j is written to slot j of the `out`
     // records, pid_out[j] = pid_in[its source slot] (pid = particle id).
-    PKin* kin_out;
-    PDef* def_out;
-    float4* pstate_out;
+    Particles out;
     const uint32_t* pid_in;
     uint32_t* pid_out;
     // batched scenes: scene of each particle id, and each scene's colliders
@@ -157,8 +163,7 @@ enum : uint32_t {
     RENDER_CDF_SIGNS = 6,
 };
 struct RenderSrc {
-    const PKin* kin;
-    const PDef* def;
+    Particles p;
     const float4* pcdf;  // per id: normal + signed distance, rigid velocity + affinity, render properties
     const uint32_t* pid;
     uint32_t n;

@@ -1,11 +1,15 @@
 // Memory layout of one MPM state in HBM (shared by the host library and the kernels).
 //
-// Particles are stored as two 16-byte-aligned records so that a particle
-// gathered through the sorted index costs whole 32-byte sectors (in the fast
-// mode the records are kept in the previous step's sorted order, double
-// buffered, with the particle id of each slot alongside):
-//   PKin (80 B): x, mass | v, flags | C columns (c0.w = vel_grad_det)
-//   PDef (48 B): F columns | (f0.w = V0, f1.w = damping, f2.w = material id)
+// A particle is spread over arrays of records that each kernel reads or writes
+// whole, one 256-bit access per 32-byte record, so that neighbouring slots fill
+// whole sectors and a gathered slot wastes none (in the fast mode the records
+// are kept in the previous step's sorted order, double buffered, with the
+// particle id of each slot alongside):
+//   PKin (32 B): x, mass, v, flags            read by G2P and P2G
+//   PAff (32 B): C's first eight components   read by P2G
+//   PAffTail (8 B): C's last, vel_grad_det
+//   PDef (32 B): F's first eight components   read by G2P
+//   PMat (16 B): F's last, V0, damping, material id
 // plus, for plastic models only, a float4 of model state words.
 // The grid is a hash of 4x4x4-node blocks: packed block keys, per-block
 // headers (struct-of-arrays), 64 float4 nodes per block (momentum + mass,
@@ -50,21 +54,31 @@ enum : uint32_t {
     STATUS_COPY_TIMEOUT = 16u,    // a bulk copy did not complete within its wait limit
 };
 
-struct alignas(16) PKin {
+struct alignas(32) PKin {
     float x, y, z, mass;
-    float vx, vy, vz, flags;     // flags: PFLAG_* as u32 bits
-    float c00, c10, c20, vgd;    // C column 0; w = vel_grad_det
-    float c01, c11, c21, pad1;   // C column 1
-    float c02, c12, c22, pad2;   // C column 2
+    float vx, vy, vz, flags;  // flags: PFLAG_* as u32 bits
 };
-static_assert(sizeof(PKin) == 80, "PKin layout");
+static_assert(sizeof(PKin) == 32, "PKin layout");
 
-struct alignas(16) PDef {
-    float f00, f10, f20, init_volume;
-    float f01, f11, f21, damping;
-    float f02, f12, f22, material;  // material index (u32 bits)
+struct alignas(32) PAff {  // C, column-major
+    float c00, c10, c20, c01, c11, c21, c02, c12;
 };
-static_assert(sizeof(PDef) == 48, "PDef layout");
+static_assert(sizeof(PAff) == 32, "PAff layout");
+
+struct alignas(8) PAffTail {
+    float c22, vgd;  // vgd = vel_grad_det
+};
+static_assert(sizeof(PAffTail) == 8, "PAffTail layout");
+
+struct alignas(32) PDef {  // F, column-major
+    float f00, f10, f20, f01, f11, f21, f02, f12;
+};
+static_assert(sizeof(PDef) == 32, "PDef layout");
+
+struct alignas(16) PMat {
+    float f22, init_volume, damping, material;  // material index (u32 bits)
+};
+static_assert(sizeof(PMat) == 16, "PMat layout");
 
 // One deduplicated material: tag + the 24 model words as floats.  State
 // words (Drucker-Prager words 0..2, snow word 0) live per particle.

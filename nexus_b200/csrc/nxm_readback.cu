@@ -17,12 +17,12 @@ namespace {
 __device__ __forceinline__ void render_particle(const RenderSrc& in, uint32_t slot, uint32_t& id, float4& color,
                                                 m3& deform, v3& pos) {
     id = in.pid ? in.pid[slot] : slot;
-    const float4* kr = reinterpret_cast<const float4*>(&in.kin[slot]);
-    const float4 xm = kr[0], vf = kr[1];
-    const float4* dr = reinterpret_cast<const float4*>(&in.def[slot]);
-    const float4 f0 = dr[0], f1 = dr[1], f2 = dr[2];
+    const f8 k = load8(&in.p.kin[slot]);
+    const float4 xm = make_float4(k.v[0], k.v[1], k.v[2], k.v[3]), vf = make_float4(k.v[4], k.v[5], k.v[6], k.v[7]);
+    const f8 fr = load8(&in.p.def[slot]);
+    const float f22 = in.p.mat[slot].f22;
     const float4 props = in.pcdf[3u * id + 2u];  // boundary friction, init radius, phase, group id
-    const m3 F = mkm(mk(f0.x, f0.y, f0.z), mk(f1.x, f1.y, f1.z), mk(f2.x, f2.y, f2.z));
+    const m3 F = mkm(mk(fr.v[0], fr.v[1], fr.v[2]), mk(fr.v[3], fr.v[4], fr.v[5]), mk(fr.v[6], fr.v[7], f22));
     pos = mk(xm.x, xm.y, xm.z);
     const uint32_t ng = in.num_groups ? in.num_groups : 1u;
     const float4 base = in.palette[__float_as_uint(props.w) % ng];

@@ -42,11 +42,11 @@ __device__ __forceinline__ void assoc_shift(int i, int& dx, int& dy, int& dz) {
 // Insert `key` (block kx,ky,kz); allocates a header on first insertion.
 // Primary blocks take ids [0, num_primary); neighbour-pass blocks take ids
 // base + [0, num_extra) with base = num_primary.
-__device__ void hash_insert(const DevPtrs& P, uint32_t key, int kx, int ky, int kz, bool primary, uint32_t base,
-                            uint32_t hash_mask, uint32_t block_cap) {
-    uint32_t slot = hash_key(key) & hash_mask;
+// `slot` = hash_key(key) & hash_mask and `cur` = its entry, already read.
+__device__ void hash_insert_at(const DevPtrs& P, uint32_t key, int kx, int ky, int kz, bool primary, uint32_t base,
+                               uint32_t hash_mask, uint32_t block_cap, uint32_t slot, uint32_t cur) {
     for (uint32_t it = 0; it <= hash_mask; ++it) {
-        uint32_t cur = __ldcg(&P.hkey[slot]);
+        if (it) cur = __ldcg(&P.hkey[slot]);
         if (cur == key) return;
         if (cur == NONE) {
             uint32_t old = atomicCAS(&P.hkey[slot], NONE, key);
@@ -69,15 +69,27 @@ __device__ void hash_insert(const DevPtrs& P, uint32_t key, int kx, int ky, int 
     set_status(P.counters, STATUS_HASH_FULL);
 }
 
-__device__ __forceinline__ uint32_t hash_find(const DevPtrs& P, uint32_t key, uint32_t hash_mask) {
-    uint32_t slot = hash_key(key) & hash_mask;
+__device__ __forceinline__ void hash_insert(const DevPtrs& P, uint32_t key, int kx, int ky, int kz, bool primary,
+                                            uint32_t base, uint32_t hash_mask, uint32_t block_cap) {
+    const uint32_t slot = hash_key(key) & hash_mask;
+    hash_insert_at(P, key, kx, ky, kz, primary, base, hash_mask, block_cap, slot, __ldcg(&P.hkey[slot]));
+}
+
+// `cur`, `val` = the entry of `slot` = hash_key(key) & hash_mask, already read.
+__device__ __forceinline__ uint32_t hash_find_at(const DevPtrs& P, uint32_t key, uint32_t hash_mask, uint32_t slot,
+                                                 uint32_t cur, uint32_t val) {
     for (uint32_t it = 0; it <= hash_mask; ++it) {
-        uint32_t cur = __ldg(&P.hkey[slot]);
-        if (cur == key) return __ldg(&P.hval[slot]);
+        if (cur == key) return val;
         if (cur == NONE) return NONE;
         slot = (slot + 1) & hash_mask;
+        cur = __ldg(&P.hkey[slot]);
+        val = __ldg(&P.hval[slot]);
     }
     return NONE;
+}
+__device__ __forceinline__ uint32_t hash_find(const DevPtrs& P, uint32_t key, uint32_t hash_mask) {
+    const uint32_t slot = hash_key(key) & hash_mask;
+    return hash_find_at(P, key, hash_mask, slot, __ldg(&P.hkey[slot]), __ldg(&P.hval[slot]));
 }
 
 // Warp-aggregated atomicAdd: lanes with equal `key` (NONE = no-op) share one
@@ -156,9 +168,10 @@ __global__ void k_sort_reset(DevPtrs P, uint32_t hash_cap) {
 
 // sort.rs:104-121 gpu_touch_primary_blocks.  Block keys come from the cache
 // written by the previous step (or from the positions after an upload).
-// Each warp walks a contiguous range of particles, so consecutive passes
-// mostly see the block they inserted last: a pass whose lanes all carry the
-// key inserted by the previous pass skips the hash entirely.
+// Each warp walks a contiguous range of particles, so its passes mostly see
+// the block it inserted last (`known`).  The other keys of a batch (a block
+// border, particles that moved to another block) are probed together: one
+// L2 round trip a batch, not one a pass, and most are found present.
 template <int kSortBatch>
 __global__ void __launch_bounds__(256) k_touch_primary(DevPtrs P) {
     const uint32_t n = P.params->n;
@@ -180,7 +193,7 @@ __global__ void __launch_bounds__(256) k_touch_primary(DevPtrs P) {
                 if (cached) {
                     key = __ldg(&P.pcode[p].x);
                 } else {
-                    float4 xm = __ldg(reinterpret_cast<const float4*>(&P.kin[p]));
+                    float4 xm = __ldg(reinterpret_cast<const float4*>(&P.in.kin[p]));
                     CellInfo ci = cell_info(dx, mk(xm.x, xm.y, xm.z));
                     int3 o = make_int3(0, 0, 0);
                     if (P.params->scene_blocks) o = scene_base_of(*P.params, P.pscene[P.pid_in ? P.pid_in[p] : p]);
@@ -190,21 +203,34 @@ __global__ void __launch_bounds__(256) k_touch_primary(DevPtrs P) {
             }
             keys[j] = key;
         }
+        uint32_t slot[kSortBatch], cur[kSortBatch];
+        uint32_t lead = 0u;  // bit j: this lane inserts its key of pass j
 #pragma unroll
         for (int j = 0; j < kSortBatch; ++j) {
-            const uint32_t b32 = base + 32u * j;
-            if (b32 >= hi) break;
-            const bool active = b32 + lane < hi;
             const uint32_t key = keys[j];
-            const uint32_t need = (active && key != known) ? key : NONE;
-            if (!__all_sync(0xFFFFFFFFu, need == NONE)) {
-                const uint32_t peers = __match_any_sync(0xFFFFFFFFu, need);
-                if (need != NONE && lane == (uint32_t)(__ffs(peers) - 1))
-                    hash_insert(P, key, key_x(key), key_y(key), key_z(key), true, 0, hmask, bcap);
+            bool need = base + 32u * j + lane < hi && key != known;
+            if (j) need &= key != keys[j - 1];
+            slot[j] = hash_key(key) & hmask;
+            cur[j] = key;
+            if (!__any_sync(0xFFFFFFFFu, need)) continue;
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, need ? key : NONE);
+            if (need && lane == (uint32_t)(__ffs(peers) - 1)) {
+                lead |= 1u << j;
+                cur[j] = __ldcg(&P.hkey[slot[j]]);
             }
-            // the last active lane's key is now in the table
-            known = __shfl_sync(0xFFFFFFFFu, key, min(31u, hi - 1u - b32));
         }
+#pragma unroll
+        for (int j = 0; j < kSortBatch; ++j) {
+            const uint32_t key = keys[j];
+            if ((lead & (1u << j)) && cur[j] != key)
+                hash_insert_at(P, key, key_x(key), key_y(key), key_z(key), true, 0, hmask, bcap, slot[j], cur[j]);
+        }
+        // the last active lane's key is now in the table
+        uint32_t tail = keys[0];
+#pragma unroll
+        for (int j = 1; j < kSortBatch; ++j)
+            if (base + 32u * j < hi) tail = keys[j];
+        known = __shfl_sync(0xFFFFFFFFu, tail, min(hi - 1u - base, 32u * kSortBatch - 1u) & 31u);
     }
 }
 
@@ -260,13 +286,20 @@ __global__ void __launch_bounds__(256) k_count(DevPtrs P) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t lo, hi;
     warp_range(n, lo, hi);
-    uint32_t known_key = NONE, known_h0 = NONE;  // the last key this warp looked up
     for (uint32_t base = lo; base < hi; base += 32u * kSortBatch) {
         uint2 codes[kSortBatch];
 #pragma unroll
         for (int j = 0; j < kSortBatch; ++j) {
             const uint32_t p = base + 32u * j + lane;
             codes[j] = p < hi ? P.pcode[p] : make_uint2(NONE, 0u);
+        }
+        // every lane's first probe, all passes in flight together (lanes of a block share the address)
+        uint32_t slot[kSortBatch], cur[kSortBatch], val[kSortBatch];
+#pragma unroll
+        for (int j = 0; j < kSortBatch; ++j) {
+            slot[j] = hash_key(codes[j].x) & hmask;
+            cur[j] = __ldg(&P.hkey[slot[j]]);
+            val[j] = __ldg(&P.hval[slot[j]]);
         }
 #pragma unroll
         for (int j = 0; j < kSortBatch; ++j) {
@@ -276,19 +309,7 @@ __global__ void __launch_bounds__(256) k_count(DevPtrs P) {
             const bool active = p < hi;
             const uint2 code = codes[j];
             const uint32_t key = active ? code.x : NONE;
-            uint32_t h0;
-            if (__all_sync(0xFFFFFFFFu, !active || key == known_key)) {
-                h0 = active ? known_h0 : NONE;
-            } else {  // one probe per distinct block key in the warp
-                const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
-                const uint32_t leader = __ffs(peers) - 1;
-                uint32_t h = NONE;
-                if (active && lane == leader) h = hash_find(P, key, hmask);
-                h0 = __shfl_sync(0xFFFFFFFFu, h, leader);
-            }
-            const uint32_t last = min(31u, hi - 1u - b32);
-            known_key = __shfl_sync(0xFFFFFFFFu, key, last);
-            known_h0 = __shfl_sync(0xFFFFFFFFu, h0, last);
+            const uint32_t h0 = active ? hash_find_at(P, key, hmask, slot[j], cur[j], val[j]) : NONE;
             const uint32_t ckey = (h0 != NONE) ? h0 * 64u + code.y : NONE;
             if (active) {
                 P.phdr[p] = ckey;
@@ -649,6 +670,12 @@ __global__ void __launch_bounds__(256) k_sort_segments(DevPtrs P) {
 }
 
 inline int grid_for(int sm_count, int per_sm) { return sm_count * per_sm; }
+// At most `per_sm` CTAs of 256 threads an SM, and no more than `items` threads
+// need (a small scene's launch is mostly the cost of starting its CTAs).
+inline int grid_for(int sm_count, int per_sm, uint64_t items) {
+    const uint64_t want = (items + 255u) / 256u, cap = (uint64_t)sm_count * per_sm;
+    return (int)(want < 1u ? 1u : (want < cap ? want : cap));
+}
 
 
 // ---------------------------------------------------------------------------
@@ -858,22 +885,27 @@ namespace fast {
 
 void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool canonical, cudaStream_t s,
                  bool rigid) {
-    const int g = grid_for(c.sm_count, (int)c.t.sort_ctas);
-    int reset_grid = (int)((c.hash_capacity + 255u) / 256u);
-    if (reset_grid > g) reset_grid = g;
-    if (reset_grid < 1) reset_grid = 1;
+    const int per_sm = (int)c.t.sort_ctas;
+    const int g = grid_for(c.sm_count, per_sm, c.particle_capacity);
+    const int gr = grid_for(c.sm_count, per_sm, P.nrp);
+    const int reset_grid = grid_for(c.sm_count, per_sm, c.hash_capacity);
+    const int scan_grid = grid_for(c.sm_count, 2, ((uint64_t)c.block_capacity + kCellTile - 1) / kCellTile * 256u);
+    // a primary block holds a particle, and each has seven +1 neighbours
+    const uint64_t primaries = c.block_capacity < c.particle_capacity ? c.block_capacity : c.particle_capacity;
+    const int gn = grid_for(c.sm_count, per_sm, primaries * 7u);
+    const int gb = grid_for(c.sm_count, per_sm, (uint64_t)c.block_capacity * 64u);
     k_sort_reset<<<reset_grid, 256, 0, s>>>(P, c.hash_capacity);
     switch (c.t.sort_batch) {
     case 2: k_touch_primary<2><<<g, 256, 0, s>>>(P); break;
     case 8: k_touch_primary<8><<<g, 256, 0, s>>>(P); break;
     default: k_touch_primary<4><<<g, 256, 0, s>>>(P); break;
     }
-    k_touch_nbh<<<g, 256, 0, s>>>(P);
+    k_touch_nbh<<<gn, 256, 0, s>>>(P);
     if (rigid) {
-        k_rigid_mark<<<g, 256, 0, s>>>(P);
-        k_rigid_touch<<<g, 256, 0, s>>>(P);
+        k_rigid_mark<<<gr, 256, 0, s>>>(P);
+        k_rigid_touch<<<gr, 256, 0, s>>>(P);
     }
-    k_block_prep<<<g, 256, 0, s>>>(P);
+    k_block_prep<<<gb, 256, 0, s>>>(P);
     switch ((with_extras ? 16 : 0) + c.t.sort_batch) {
     case 2: k_count<false, 2><<<g, 256, 0, s>>>(P); break;
     case 8: k_count<false, 8><<<g, 256, 0, s>>>(P); break;
@@ -883,11 +915,11 @@ void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool ca
     default: k_count<false, 4><<<g, 256, 0, s>>>(P); break;
     }
     if (with_extras) {
-        k_scan_cell_tiles<true><<<c.sm_count * 2, kScanThreads, 0, s>>>(P);
-        k_scan_cell_apply<true><<<c.sm_count * 2, kScanThreads, 0, s>>>(P);
+        k_scan_cell_tiles<true><<<scan_grid, kScanThreads, 0, s>>>(P);
+        k_scan_cell_apply<true><<<scan_grid, kScanThreads, 0, s>>>(P);
     } else {
-        k_scan_cell_tiles<false><<<c.sm_count * 2, kScanThreads, 0, s>>>(P);
-        k_scan_cell_apply<false><<<c.sm_count * 2, kScanThreads, 0, s>>>(P);
+        k_scan_cell_tiles<false><<<scan_grid, kScanThreads, 0, s>>>(P);
+        k_scan_cell_apply<false><<<scan_grid, kScanThreads, 0, s>>>(P);
     }
     switch ((with_extras ? 16 : 0) + c.t.sort_batch) {
     case 2: k_finalize<false, 2><<<g, 256, 0, s>>>(P); break;
@@ -899,9 +931,9 @@ void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool ca
     }
     if (canonical) k_sort_segments<<<grid_for(c.sm_count, 4), 256, 0, s>>>(P);
     if (rigid) {
-        k_rigid_count<<<g, 256, 0, s>>>(P);
-        k_rigid_alloc<<<g, 256, 0, s>>>(P);
-        k_rigid_finalize<<<g, 256, 0, s>>>(P);
+        k_rigid_count<<<gr, 256, 0, s>>>(P);
+        k_rigid_alloc<<<grid_for(c.sm_count, per_sm, c.block_capacity), 256, 0, s>>>(P);
+        k_rigid_finalize<<<gr, 256, 0, s>>>(P);
     }
 }
 

@@ -105,25 +105,35 @@ int model_state_words(uint32_t tag) {
 
 // Packs selected 4-byte fields of the records of particles [first, first + n)
 // into a dense array.
-__global__ void k_pack_fields(const uint32_t* __restrict__ src, uint32_t stride_words, uint32_t first, uint32_t n,
+// Words of the records of one or two arrays: word w of `a`'s record for w <
+// a_words, word w - a_words of `b`'s from there on.
+struct FieldSrc {
+    const uint32_t* a;
+    const uint32_t* b;
+    uint32_t a_words, b_words;
+};
+__device__ __forceinline__ uint32_t field_of(const FieldSrc& s, size_t p, uint32_t w) {
+    return w < s.a_words ? s.a[p * s.a_words + w] : s.b[p * s.b_words + (w - s.a_words)];
+}
+__global__ void k_pack_fields(FieldSrc src, uint32_t first, uint32_t n,
                               const int* __restrict__ offsets, int nfields, uint32_t* __restrict__ dst) {
     const uint32_t total = n * (uint32_t)nfields;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
         const uint32_t p = first + t / (uint32_t)nfields, f = t % (uint32_t)nfields;
-        dst[t] = src[(size_t)p * stride_words + offsets[f]];
+        dst[t] = field_of(src, p, offsets[f]);
     }
 }
 
 // Permuted storage (slot p holds particle pid[p]): scatter the fields of the
 // particles with id in [first, first + count) by id (all n slots are scanned).
-__global__ void k_pack_fields_perm(const uint32_t* __restrict__ src, uint32_t stride_words, uint32_t n,
+__global__ void k_pack_fields_perm(FieldSrc src, uint32_t n,
                                    uint32_t first, uint32_t count, const int* __restrict__ offsets, int nfields,
                                    const uint32_t* __restrict__ pid, uint32_t* __restrict__ dst) {
     const uint32_t total = n * (uint32_t)nfields;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
         const uint32_t p = t / (uint32_t)nfields, f = t % (uint32_t)nfields;
         const uint32_t id = pid[p] - first;
-        if (id < count) dst[(size_t)id * nfields + f] = src[(size_t)p * stride_words + offsets[f]];
+        if (id < count) dst[(size_t)id * nfields + f] = field_of(src, p, offsets[f]);
     }
 }
 
@@ -227,12 +237,19 @@ __global__ void __launch_bounds__(1024) k_rm_scan(uint32_t* __restrict__ tiles, 
         __syncthreads();
     }
 }
-__global__ void __launch_bounds__(256) k_rm_move(uint32_t n, const PKin* __restrict__ kin, const PDef* __restrict__ def,
-                                                 const float4* __restrict__ pstate, const uint32_t* __restrict__ pid,
+// The records of slot `from` to slot `to` (of other buffers, or of the same).
+__device__ __forceinline__ void copy_slot(const Particles& a, uint32_t from, const Particles& b, uint32_t to) {
+    b.kin[to] = a.kin[from];
+    b.aff[to] = a.aff[from];
+    b.tail[to] = a.tail[from];
+    b.def[to] = a.def[from];
+    b.mat[to] = a.mat[from];
+    b.pstate[to] = a.pstate[from];
+}
+__global__ void __launch_bounds__(256) k_rm_move(uint32_t n, Particles from, const uint32_t* __restrict__ pid,
                                                  const uint2* __restrict__ ranges, const uint32_t* __restrict__ cum,
                                                  uint32_t nr, const uint32_t* __restrict__ tiles,
-                                                 PKin* __restrict__ kin_to, PDef* __restrict__ def_to,
-                                                 float4* __restrict__ pstate_to, uint32_t* __restrict__ pid_to) {
+                                                 Particles to, uint32_t* __restrict__ pid_to) {
     __shared__ uint32_t sh[9];
     bool keep[4];
     const uint32_t base = blockIdx.x * 1024u + threadIdx.x * 4u;
@@ -243,9 +260,7 @@ __global__ void __launch_bounds__(256) k_rm_move(uint32_t n, const PKin* __restr
     for (int k = 0; k < 4; ++k) {
         if (!keep[k]) continue;
         const uint32_t p = base + k;
-        kin_to[dst] = kin[p];
-        def_to[dst] = def[p];
-        pstate_to[dst] = pstate[p];
+        copy_slot(from, p, to, dst);
         if (pid) pid_to[dst] = new_id_of(pid[p], ranges, cum, nr);
         ++dst;
     }
@@ -266,13 +281,10 @@ __global__ void k_rm_ids(uint32_t n, const T* __restrict__ src, const uint2* __r
 // Swap-removal data movement: record pairs[i].y moves to slot pairs[i].x.
 // Every source is at or above the new length and every destination below it,
 // so the moves are independent.
-__global__ void k_move_records(PKin* __restrict__ kin, PDef* __restrict__ def, float4* __restrict__ pstate,
-                               float4* __restrict__ pcdf, const uint2* __restrict__ pairs, uint32_t count) {
+__global__ void k_move_records(Particles a, float4* __restrict__ pcdf, const uint2* __restrict__ pairs, uint32_t count) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint2 m = pairs[i];
-        kin[m.x] = kin[m.y];
-        def[m.x] = def[m.y];
-        pstate[m.x] = pstate[m.y];
+        copy_slot(a, m.y, a, m.x);
 #pragma unroll
         for (int k = 0; k < 3; ++k) pcdf[3u * m.x + k] = pcdf[3u * m.y + k];
     }
@@ -320,15 +332,9 @@ __global__ void k_iota(uint32_t* __restrict__ out, uint32_t first, uint32_t coun
 }
 
 // Back to id order: record of slot p goes to slot pid[p] of the other buffers.
-__global__ void k_unpermute(const PKin* __restrict__ kin, const PDef* __restrict__ def,
-                            const float4* __restrict__ pstate, const uint32_t* __restrict__ pid, uint32_t n,
-                            PKin* __restrict__ kin_to, PDef* __restrict__ def_to, float4* __restrict__ pstate_to) {
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        const uint32_t id = pid[p];
-        kin_to[id] = kin[p];
-        def_to[id] = def[p];
-        pstate_to[id] = pstate[p];
-    }
+__global__ void k_unpermute(Particles from, const uint32_t* __restrict__ pid, uint32_t n, Particles to) {
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
+        copy_slot(from, p, to, pid[p]);
 }
 
 }  // namespace
@@ -352,17 +358,13 @@ struct nxm_state {
     bool deterministic = false;
 
     // particles.  Fast mode keeps the records in the previous step's sorted
-    // order: each step's G2P writes them to the *_alt buffers, which then
+    // order: each step's G2P writes them to the `alt` buffers, which then
     // become current (`parity` counts the swaps mod 2); pid[slot] is the
     // particle id of a slot while `permuted`, otherwise slot == id.
     uint32_t n = 0, pcap = 0;
     char* pslab = nullptr;  // the one allocation the per-particle arrays below are carved from
-    PKin* kin = nullptr;
-    PDef* def = nullptr;
-    float4* pstate = nullptr;
-    PKin* kin_alt = nullptr;
-    PDef* def_alt = nullptr;
-    float4* pstate_alt = nullptr;
+    Particles cur{};
+    Particles alt{};
     uint32_t* pid = nullptr;
     uint32_t* pid_alt = nullptr;
     bool permuted = false;
@@ -523,19 +525,13 @@ bool reorders(const nxm_state* s) { return !s->deterministic && !s->use_cpic; }
 
 DevPtrs dev_ptrs(nxm_state* s) {
     DevPtrs P{};
-    P.kin = s->kin;
-    P.def = s->def;
-    P.pstate = s->pstate;
+    P.in = s->cur;
     if (reorders(s)) {
-        P.kin_out = s->kin_alt;
-        P.def_out = s->def_alt;
-        P.pstate_out = s->pstate_alt;
+        P.out = s->alt;
         P.pid_in = s->pid;
         P.pid_out = s->pid_alt;
     } else {
-        P.kin_out = s->kin;
-        P.def_out = s->def;
-        P.pstate_out = s->pstate;
+        P.out = s->cur;
         P.pid_in = nullptr;
         P.pid_out = nullptr;
     }
@@ -769,9 +765,7 @@ void invalidate_graph(nxm_state* s) {
 
 // The reordering G2P wrote the step's output to the *_alt buffers: make them current.
 void swap_buffers(nxm_state* s) {
-    std::swap(s->kin, s->kin_alt);
-    std::swap(s->def, s->def_alt);
-    std::swap(s->pstate, s->pstate_alt);
+    std::swap(s->cur, s->alt);
     std::swap(s->pid, s->pid_alt);
     s->parity ^= 1;
 }
@@ -785,14 +779,11 @@ int grid_for_n(nxm_state* s, uint32_t n) {
 int canonicalize(nxm_state* s) {
     if (!s->permuted) return NXM_OK;
     if (s->n) {
-        k_unpermute<<<grid_for_n(s, s->n), 256, 0, s->stream>>>(s->kin, s->def, s->pstate, s->pid, s->n, s->kin_alt,
-                                                                 s->def_alt, s->pstate_alt);
+        k_unpermute<<<grid_for_n(s, s->n), 256, 0, s->stream>>>(s->cur, s->pid, s->n, s->alt);
         s->launches += 1;
         NXM_TRY(cudaGetLastError());
     }
-    std::swap(s->kin, s->kin_alt);
-    std::swap(s->def, s->def_alt);
-    std::swap(s->pstate, s->pstate_alt);
+    std::swap(s->cur, s->alt);
     std::swap(s->pid, s->pid_alt);
     s->parity ^= 1;
     s->permuted = false;
@@ -900,17 +891,17 @@ int alloc_grid(nxm_state* s, uint32_t grid_capacity) {
 // The particle arrays of a state (owned; freed on destruction unless released).
 struct ParticleBuffers {
     char* slab = nullptr;
-    PKin *kin = nullptr, *kin_alt = nullptr;
-    PDef *def = nullptr, *def_alt = nullptr;
-    float4 *pstate = nullptr, *pstate_alt = nullptr;
+    Particles cur{}, alt{};
     uint32_t *pid = nullptr, *pid_alt = nullptr, *phdr = nullptr, *sorted = nullptr, *pscene = nullptr,
              *pscene_alt = nullptr, *tiles = nullptr, *chunk_blk = nullptr;
     uint2* pcode = nullptr;
     float4 *pcdf = nullptr, *pcdf_alt = nullptr;
     cudaError_t alloc(uint32_t cap) {
         Slab a;
-        a.add(&kin, cap); a.add(&def, cap); a.add(&pstate, cap);
-        a.add(&kin_alt, cap); a.add(&def_alt, cap); a.add(&pstate_alt, cap);
+        for (Particles* p : {&cur, &alt}) {
+            a.add(&p->kin, cap); a.add(&p->aff, cap); a.add(&p->tail, cap);
+            a.add(&p->def, cap); a.add(&p->mat, cap); a.add(&p->pstate, cap);
+        }
         a.add(&pid, cap); a.add(&pid_alt, cap); a.add(&pcode, cap); a.add(&phdr, cap);
         a.add(&sorted, (size_t)cap * 8);
         a.add(&pscene, cap);
@@ -927,9 +918,7 @@ struct ParticleBuffers {
 
 void free_particles(nxm_state* s) {
     dfree(s->pslab);
-    s->kin = s->kin_alt = nullptr;
-    s->def = s->def_alt = nullptr;
-    s->pstate = s->pstate_alt = nullptr;
+    s->cur = s->alt = Particles{};
     s->pid = s->pid_alt = s->phdr = s->sorted = s->d_pscene = s->d_pscene_alt = s->d_tiles = nullptr;
     s->d_chunk_blk = nullptr;
     s->pcode = nullptr;
@@ -946,17 +935,23 @@ int reserve_particles(nxm_state* s, uint32_t need) {
     ParticleBuffers t;
     NXM_TRY(t.alloc(cap));
     if (s->n) {
-        NXM_TRY(cudaMemcpyAsync(t.kin, s->kin, sizeof(PKin) * s->n, cudaMemcpyDeviceToDevice, s->stream));
-        NXM_TRY(cudaMemcpyAsync(t.def, s->def, sizeof(PDef) * s->n, cudaMemcpyDeviceToDevice, s->stream));
-        NXM_TRY(cudaMemcpyAsync(t.pstate, s->pstate, sizeof(float4) * s->n, cudaMemcpyDeviceToDevice, s->stream));
+        const auto keep = [&](void* to, const void* from, size_t bytes) {
+            return cudaMemcpyAsync(to, from, bytes * s->n, cudaMemcpyDeviceToDevice, s->stream);
+        };
+        NXM_TRY(keep(t.cur.kin, s->cur.kin, sizeof(PKin)));
+        NXM_TRY(keep(t.cur.aff, s->cur.aff, sizeof(PAff)));
+        NXM_TRY(keep(t.cur.tail, s->cur.tail, sizeof(PAffTail)));
+        NXM_TRY(keep(t.cur.def, s->cur.def, sizeof(PDef)));
+        NXM_TRY(keep(t.cur.mat, s->cur.mat, sizeof(PMat)));
+        NXM_TRY(keep(t.cur.pstate, s->cur.pstate, sizeof(float4)));
         NXM_TRY(cudaMemcpyAsync(t.pscene, s->d_pscene, 4 * (size_t)s->n, cudaMemcpyDeviceToDevice, s->stream));
         NXM_TRY(cudaMemcpyAsync(t.pcdf, s->d_pcdf, 48 * (size_t)s->n, cudaMemcpyDeviceToDevice, s->stream));
     }
     NXM_TRY(cudaStreamSynchronize(s->stream));
     free_particles(s);
     s->pslab = t.slab;
-    s->kin = t.kin; s->def = t.def; s->pstate = t.pstate;
-    s->kin_alt = t.kin_alt; s->def_alt = t.def_alt; s->pstate_alt = t.pstate_alt;
+    s->cur = t.cur;
+    s->alt = t.alt;
     s->pid = t.pid; s->pid_alt = t.pid_alt;
     s->pcode = t.pcode; s->phdr = t.phdr; s->sorted = t.sorted;
     s->d_pscene = t.pscene; s->d_pscene_alt = t.pscene_alt; s->d_tiles = t.tiles;
@@ -1139,8 +1134,7 @@ void finish_step(nxm_state* s) {
 }
 
 // Fields of particles [first, first + count) (ids), in id order, into `out`.
-int pack_read_range(nxm_state* s, const void* records, uint32_t stride_bytes, const int* offsets, int nfields,
-                    uint32_t first, uint32_t count, void* out, bool wait = true) {
+int pack_read_range(nxm_state* s, FieldSrc src, const int* offsets, int nfields, uint32_t first, uint32_t count, void* out, bool wait = true) {
     if (!out) return NXM_E_INVALID;
     if (first > s->n || count > s->n - first) return NXM_E_INVALID;
     if (count == 0) return NXM_OK;
@@ -1159,12 +1153,10 @@ int pack_read_range(nxm_state* s, const void* records, uint32_t stride_bytes, co
     int grid = (int)std::min<size_t>((threads + 255) / 256, (size_t)s->sm_count * 8);
     if (grid < 1) grid = 1;
     if (s->permuted)
-        k_pack_fields_perm<<<grid, 256, 0, s->stream>>>(reinterpret_cast<const uint32_t*>(records), stride_bytes / 4,
-                                                          s->n, first, count, s->d_offsets, nfields, s->pid,
+        k_pack_fields_perm<<<grid, 256, 0, s->stream>>>(src, s->n, first, count, s->d_offsets, nfields, s->pid,
                                                           s->d_pack);
     else
-        k_pack_fields<<<grid, 256, 0, s->stream>>>(reinterpret_cast<const uint32_t*>(records), stride_bytes / 4, first,
-                                                     count, s->d_offsets, nfields, s->d_pack);
+        k_pack_fields<<<grid, 256, 0, s->stream>>>(src, first, count, s->d_offsets, nfields, s->d_pack);
     s->launches += 1;
     NXM_TRY(cudaGetLastError());
     NXM_TRY(cudaMemcpyAsync(out, s->d_pack, words * 4, cudaMemcpyDeviceToHost, s->stream));
@@ -1172,9 +1164,19 @@ int pack_read_range(nxm_state* s, const void* records, uint32_t stride_bytes, co
     return NXM_OK;
 }
 
-int pack_read(nxm_state* s, const void* records, uint32_t stride_bytes, const int* offsets, int nfields, void* out) {
+int pack_read(nxm_state* s, FieldSrc src, const int* offsets, int nfields, void* out) {
     if (!out) return NXM_E_INVALID;
-    return pack_read_range(s, records, stride_bytes, offsets, nfields, 0, s->n, out);
+    return pack_read_range(s, src, offsets, nfields, 0, s->n, out);
+}
+
+// The words of one array of records, or of two.
+template <class A>
+FieldSrc field_src(const A* a) {
+    return FieldSrc{reinterpret_cast<const uint32_t*>(a), nullptr, sizeof(A) / 4, 0};
+}
+template <class A, class B>
+FieldSrc field_src(const A* a, const B* b) {
+    return FieldSrc{reinterpret_cast<const uint32_t*>(a), reinterpret_cast<const uint32_t*>(b), sizeof(A) / 4, sizeof(B) / 4};
 }
 
 // Removes the particles whose ids fall in `ranges` (sorted, disjoint), keeping
@@ -1211,8 +1213,7 @@ int remove_id_ranges(nxm_state* s, std::vector<uint2> ranges) {
     if (e == cudaSuccess) {
         k_rm_count<<<ntiles, 256, 0, s->stream>>>(n0, pid, d_r, nr, s->d_tiles);
         k_rm_scan<<<1, 1024, 0, s->stream>>>(s->d_tiles, ntiles);
-        k_rm_move<<<ntiles, 256, 0, s->stream>>>(n0, s->kin, s->def, s->pstate, pid, d_r, d_cum, nr, s->d_tiles,
-                                                 s->kin_alt, s->def_alt, s->pstate_alt, s->pid_alt);
+        k_rm_move<<<ntiles, 256, 0, s->stream>>>(n0, s->cur, pid, d_r, d_cum, nr, s->d_tiles, s->alt, s->pid_alt);
         s->launches += 3;
         if (s->scene_blocks) {  // the per-id scene index follows the ids
             k_rm_ids<uint32_t, 1><<<grid_for_n(s, n0), 256, 0, s->stream>>>(n0, s->d_pscene, d_r, d_cum, nr,
@@ -1285,7 +1286,7 @@ static int material_runs(nxm_state* s, const nxm_particle_model* models, uint32_
 
 // Device-side record packing of an upload: the SoA fields (null = the
 // ParticleDynamics::new default) of particles [base, base + count) of the
-// upload, written as PKin / PDef / model state / CPIC + properties records.
+// upload, written as the particle records and the CPIC + properties record.
 struct UploadSrc {
     const float *pos, *vel, *F, *A, *vgd, *v0, *rad, *mass, *damp, *phase, *bf;
     const uint32_t *gid, *en, *fx;
@@ -1295,8 +1296,7 @@ struct UploadSrc {
     uint32_t nruns;
 };
 
-__global__ void k_pack_particles(UploadSrc u, uint32_t base, uint32_t count, PKin* __restrict__ kin,
-                                 PDef* __restrict__ def, float4* __restrict__ pstate, float4* __restrict__ pcdf) {
+__global__ void k_pack_particles(UploadSrc u, uint32_t base, uint32_t count, Particles to, float4* __restrict__ pcdf) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         // the material run holding particle base + i
         uint32_t lo = 0, hi = u.nruns;
@@ -1311,17 +1311,13 @@ __global__ void k_pack_particles(UploadSrc u, uint32_t base, uint32_t count, PKi
         uint32_t flags = 0;
         if (!u.en || u.en[i]) flags |= PFLAG_ENABLED;
         if (u.fx && u.fx[i]) flags |= PFLAG_FIXED;
-        float4* k = reinterpret_cast<float4*>(&kin[i]);
-        k[0] = make_float4(x[0], x[1], x[2], u.mass[i]);
-        k[1] = make_float4(v ? v[0] : 0.f, v ? v[1] : 0.f, v ? v[2] : 0.f, __uint_as_float(flags));
-        k[2] = make_float4(a ? a[0] : 0.f, a ? a[1] : 0.f, a ? a[2] : 0.f, u.vgd ? u.vgd[i] : 0.f);
-        k[3] = make_float4(a ? a[3] : 0.f, a ? a[4] : 0.f, a ? a[5] : 0.f, 0.f);
-        k[4] = make_float4(a ? a[6] : 0.f, a ? a[7] : 0.f, a ? a[8] : 0.f, 0.f);
-        float4* d = reinterpret_cast<float4*>(&def[i]);
-        d[0] = make_float4(F ? F[0] : 1.f, F ? F[1] : 0.f, F ? F[2] : 0.f, u.v0[i]);
-        d[1] = make_float4(F ? F[3] : 0.f, F ? F[4] : 1.f, F ? F[5] : 0.f, u.damp ? u.damp[i] : 0.f);
-        d[2] = make_float4(F ? F[6] : 0.f, F ? F[7] : 0.f, F ? F[8] : 1.f, __uint_as_float(u.run_mid[lo]));
-        pstate[i] = u.run_state[lo];
+        to.kin[i] = PKin{x[0], x[1], x[2], u.mass[i], v ? v[0] : 0.f, v ? v[1] : 0.f, v ? v[2] : 0.f,
+                         __uint_as_float(flags)};
+        to.aff[i] = a ? PAff{a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]} : PAff{};
+        to.tail[i] = PAffTail{a ? a[8] : 0.f, u.vgd ? u.vgd[i] : 0.f};
+        to.def[i] = F ? PDef{F[0], F[1], F[2], F[3], F[4], F[5], F[6], F[7]} : PDef{1.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f};
+        to.mat[i] = PMat{F ? F[8] : 1.f, u.v0[i], u.damp ? u.damp[i] : 0.f, __uint_as_float(u.run_mid[lo])};
+        to.pstate[i] = u.run_state[lo];
         // CPIC fields start empty; then the properties: defaults of
         // ParticleDynamics::new (solver/particle.rs:100-122), the radius, when
         // not given, from init_volume = (2 r)^3
@@ -1431,8 +1427,9 @@ int upload_particles(nxm_state* s, const nxm_particles_soa* p, uint32_t count) {
         u.en = static_cast<const uint32_t*>(dst[12]);
         u.fx = static_cast<const uint32_t*>(dst[13]);
         const size_t at0 = (size_t)s->n + c0;
-        k_pack_particles<<<grid_for_n(s, cn), 256, 0, s->stream>>>(u, c0, cn, s->kin + at0, s->def + at0,
-                                                                   s->pstate + at0, s->d_pcdf + 3 * at0);
+        const Particles to{s->cur.kin + at0, s->cur.aff + at0, s->cur.tail + at0,
+                           s->cur.def + at0, s->cur.mat + at0, s->cur.pstate + at0};
+        k_pack_particles<<<grid_for_n(s, cn), 256, 0, s->stream>>>(u, c0, cn, to, s->d_pcdf + 3 * at0);
         s->launches += 1;
         err = cudaGetLastError();
     }
@@ -2062,8 +2059,7 @@ static int render_source(nxm_state* s, uint32_t mode, const float* palette, uint
         s->palette_cap = num_groups;
     }
     NXM_TRY(cudaMemcpyAsync(s->d_palette, palette, sizeof(float4) * num_groups, cudaMemcpyHostToDevice, s->stream));
-    in.kin = s->kin;
-    in.def = s->def;
+    in.p = s->cur;
     in.pcdf = s->d_pcdf;
     in.pid = s->permuted ? s->pid : nullptr;
     in.n = s->n;
@@ -2162,7 +2158,7 @@ int nxm_read_cdf(nxm_state* s, float* out) {
     if (!s) return NXM_E_INVALID;
     static const int off[8] = {0, 1, 2, 3, 4, 5, 6, 7};
     if (s->permuted) return NXM_E_INVALID;  // the fields are id-indexed; CPIC keeps id order
-    return pack_read(s, s->d_pcdf, 48, off, 8, out);
+    return pack_read(s, FieldSrc{reinterpret_cast<const uint32_t*>(s->d_pcdf), nullptr, 12, 0}, off, 8, out);
 }
 
 int nxm_state_set_deterministic(nxm_state* s, int enabled) {
@@ -2378,7 +2374,7 @@ int nxm_scene_set_collider_velocity(nxm_state* s, uint32_t scene, uint32_t index
 int nxm_read_positions_range(nxm_state* s, uint32_t first, uint32_t count, float* out) {
     if (!s) return NXM_E_INVALID;
     static const int off[3] = {0, 1, 2};
-    return pack_read_range(s, s->kin, sizeof(PKin), off, 3, first, count, out);
+    return pack_read_range(s, field_src(s->cur.kin), off, 3, first, count, out);
 }
 
 // ---- particle chunks (NexusState, src/state.rs:665-774) ---------------------
@@ -2511,7 +2507,7 @@ int nxm_particles_swap_remove(nxm_state* s, const uint32_t* slots, uint32_t coun
         cudaError_t e = cudaMemcpyAsync(d_pairs, pairs.data(), sizeof(uint2) * pairs.size(), cudaMemcpyHostToDevice,
                                         s->stream);
         if (e == cudaSuccess) {
-            k_move_records<<<grid_for_n(s, (uint32_t)pairs.size()), 256, 0, s->stream>>>(s->kin, s->def, s->pstate,
+            k_move_records<<<grid_for_n(s, (uint32_t)pairs.size()), 256, 0, s->stream>>>(s->cur,
                                                                                         s->d_pcdf, d_pairs,
                                                                                         (uint32_t)pairs.size());
             s->launches += 1;
@@ -2770,7 +2766,7 @@ int nxm_state_ticket_wait(nxm_state* s, uint64_t ticket) {
 int nxm_read_positions_range_async(nxm_state* s, uint32_t first, uint32_t count, float* out, uint64_t* ticket) {
     if (!s || !ticket) return NXM_E_INVALID;
     static const int off[3] = {0, 1, 2};
-    const int rc = pack_read_range(s, s->kin, sizeof(PKin), off, 3, first, count, out, /*wait=*/false);
+    const int rc = pack_read_range(s, field_src(s->cur.kin), off, 3, first, count, out, /*wait=*/false);
     if (rc) return rc;
     return nxm_state_fence(s, ticket);
 }
@@ -3010,51 +3006,51 @@ void* nxm_state_cuda_stream(const nxm_state* s) { return s ? reinterpret_cast<vo
 int nxm_read_positions(nxm_state* s, float* out) {
     if (!s) return NXM_E_INVALID;
     static const int off[3] = {0, 1, 2};
-    return pack_read(s, s->kin, sizeof(PKin), off, 3, out);
+    return pack_read(s, field_src(s->cur.kin), off, 3, out);
 }
 int nxm_read_velocities(nxm_state* s, float* out) {
     if (!s) return NXM_E_INVALID;
     static const int off[3] = {4, 5, 6};
-    return pack_read(s, s->kin, sizeof(PKin), off, 3, out);
+    return pack_read(s, field_src(s->cur.kin), off, 3, out);
 }
 int nxm_read_affine(nxm_state* s, float* out) {
     if (!s) return NXM_E_INVALID;
-    static const int off[9] = {8, 9, 10, 12, 13, 14, 16, 17, 18};
-    return pack_read(s, s->kin, sizeof(PKin), off, 9, out);
+    static const int off[9] = {0, 1, 2, 3, 4, 5, 6, 7, 8};
+    return pack_read(s, field_src(s->cur.aff, s->cur.tail), off, 9, out);
 }
 int nxm_read_vel_grad_det(nxm_state* s, float* out) {
     if (!s) return NXM_E_INVALID;
-    static const int off[1] = {11};
-    return pack_read(s, s->kin, sizeof(PKin), off, 1, out);
+    static const int off[1] = {1};
+    return pack_read(s, field_src(s->cur.tail), off, 1, out);
 }
 int nxm_read_mass(nxm_state* s, float* out) {
     if (!s) return NXM_E_INVALID;
     static const int off[1] = {3};
-    return pack_read(s, s->kin, sizeof(PKin), off, 1, out);
+    return pack_read(s, field_src(s->cur.kin), off, 1, out);
 }
 int nxm_read_enabled(nxm_state* s, uint32_t* out) {
     if (!s || !out) return NXM_E_INVALID;
     static const int off[1] = {7};
-    int rc = pack_read(s, s->kin, sizeof(PKin), off, 1, out);
+    int rc = pack_read(s, field_src(s->cur.kin), off, 1, out);
     if (rc) return rc;
     for (uint32_t i = 0; i < s->n; ++i) out[i] = (out[i] & PFLAG_ENABLED) ? 1u : 0u;
     return NXM_OK;
 }
 int nxm_read_def_grad(nxm_state* s, float* out) {
     if (!s) return NXM_E_INVALID;
-    static const int off[9] = {0, 1, 2, 4, 5, 6, 8, 9, 10};
-    return pack_read(s, s->def, sizeof(PDef), off, 9, out);
+    static const int off[9] = {0, 1, 2, 3, 4, 5, 6, 7, 8};
+    return pack_read(s, field_src(s->cur.def, s->cur.mat), off, 9, out);
 }
 int nxm_read_models(nxm_state* s, nxm_particle_model* out) {
     if (!s || !out) return NXM_E_INVALID;
     if (s->n == 0) return NXM_OK;
     std::vector<uint32_t> mid(s->n);
-    static const int off_m[1] = {11};
-    int rc = pack_read(s, s->def, sizeof(PDef), off_m, 1, mid.data());
+    static const int off_m[1] = {3};
+    int rc = pack_read(s, field_src(s->cur.mat), off_m, 1, mid.data());
     if (rc) return rc;
     std::vector<float> st(4 * (size_t)s->n);
     static const int off_s[4] = {0, 1, 2, 3};
-    rc = pack_read(s, s->pstate, sizeof(float4), off_s, 4, st.data());
+    rc = pack_read(s, field_src(s->cur.pstate), off_s, 4, st.data());
     if (rc) return rc;
     for (uint32_t i = 0; i < s->n; ++i) {
         if (mid[i] >= s->materials.size()) return NXM_E_INVALID;

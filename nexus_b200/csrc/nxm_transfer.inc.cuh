@@ -19,6 +19,16 @@ namespace nxm {
 namespace NXM_NS {
 namespace {
 
+// C and F of the particle in slot p.
+__device__ __forceinline__ m3 affine_of(const Particles& a, uint32_t p) {
+    const f8 c = load8(&a.aff[p]);
+    return mkm(mk(c.v[0], c.v[1], c.v[2]), mk(c.v[3], c.v[4], c.v[5]), mk(c.v[6], c.v[7], a.tail[p].c22));
+}
+__device__ __forceinline__ m3 def_grad_of(const Particles& a, uint32_t p, float f22) {
+    const f8 f = load8(&a.def[p]);
+    return mkm(mk(f.v[0], f.v[1], f.v[2]), mk(f.v[3], f.v[4], f.v[5]), mk(f.v[6], f.v[7], f22));
+}
+
 __device__ __forceinline__ void set_status(Counters* c, uint32_t bit) { atomicOr(&c->status, bit); }
 
 __device__ __forceinline__ v3 col_vel_at(const DevCollider& c, v3 p) {
@@ -263,13 +273,12 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
     const float dx = prm.dx, dt = prm.dt;
     const float inv_d = 4.0f / (dx * dx);
     const float lim2 = (dx / dt) * (dx / dt);
-    float4* kr = reinterpret_cast<float4*>(&P.kin_out[dst]);
     uint32_t flags = __float_as_uint(vf.w);
     const v3 pt = mk(xm.x, xm.y, xm.z);
     float mass = xm.w;
     // the deformation record, loaded ahead of the gather
-    const float4* dr = reinterpret_cast<const float4*>(&P.def[src]);
-    const float4 d0 = dr[0], d1 = dr[1], d2 = dr[2];
+    const float4 pm = *reinterpret_cast<const float4*>(&P.in.mat[src]);  // F's last, V0, damping, material
+    m3 F = def_grad_of(P.in, src, pm.x);
 
 #if NXM_CPIC
     // particle Cdf (normal, signed distance, affinity) from this step's g2p_cdf pass
@@ -399,9 +408,8 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
 #endif
 
     // ---- particle update (particle_update.rs:60-201, non-CPIC: Cdf = 0)
-    m3 F = mkm(mk(d0.x, d0.y, d0.z), mk(d1.x, d1.y, d1.z), mk(d2.x, d2.y, d2.z));
-    const float init_volume = d0.w, damping = d1.w;
-    const uint32_t mid = __float_as_uint(d2.w);
+    const float init_volume = pm.y, damping = pm.z;
+    const uint32_t mid = __float_as_uint(pm.w);
     const Material& mat = P.materials[mid];
     const uint32_t tag = mat.tag;
 
@@ -434,8 +442,7 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
     // written ahead of the constitutive update (fewer values live across it);
     // a particle that the check after it disables is rewritten there.
     const bool nan = (np_.x != np_.x) || (np_.y != np_.y) || (np_.z != np_.z);
-    kr[0] = make_float4(np_.x, np_.y, np_.z, mass);
-    kr[1] = make_float4(v.x, v.y, v.z, __uint_as_float(flags));
+    store8(&P.out.kin[dst], np_.x, np_.y, np_.z, mass, v.x, v.y, v.z, __uint_as_float(flags));
     {
         const CellInfo nc = cell_info(dx, np_);
         P.pcode[dst] = make_uint2(pack_key(nc.bx + key_off.x, nc.by + key_off.y, nc.bz + key_off.z),
@@ -453,7 +460,7 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
     }
     float st[4] = {0.f, 0.f, 0.f, 0.f};
     if (mat.has_state) {
-        float4 s4 = P.pstate[src];
+        float4 s4 = P.in.pstate[src];
         st[0] = s4.x; st[1] = s4.y; st[2] = s4.z; st[3] = s4.w;
     }
     m3 aff;
@@ -480,21 +487,17 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
         aff = mzero();
         // the fast build always writes to the other buffer: the old position
         // is re-read there instead of staying live across the model update
-        const v3 op = NXM_FAST ? mk(P.kin[src].x, P.kin[src].y, P.kin[src].z) : pt;
-        kr[0] = make_float4(op.x, op.y, op.z, 0.f);
-        kr[1] = make_float4(0.f, 0.f, 0.f, __uint_as_float(flags));
+        const v3 op = NXM_FAST ? mk(P.in.kin[src].x, P.in.kin[src].y, P.in.kin[src].z) : pt;
+        store8(&P.out.kin[dst], op.x, op.y, op.z, 0.f, 0.f, 0.f, 0.f, __uint_as_float(flags));
         const CellInfo oc = cell_info(dx, op);
         P.pcode[dst] = make_uint2(pack_key(oc.bx + key_off.x, oc.by + key_off.y, oc.bz + key_off.z),
                                   oc.ax | (oc.ay << 2) | (oc.az << 4));
     }
-    kr[2] = make_float4(aff.c0.x, aff.c0.y, aff.c0.z, vgd);
-    kr[3] = make_float4(aff.c1.x, aff.c1.y, aff.c1.z, 0.f);
-    kr[4] = make_float4(aff.c2.x, aff.c2.y, aff.c2.z, 0.f);
-    float4* dw = reinterpret_cast<float4*>(&P.def_out[dst]);
-    dw[0] = make_float4(F.c0.x, F.c0.y, F.c0.z, init_volume);
-    dw[1] = make_float4(F.c1.x, F.c1.y, F.c1.z, damping);
-    dw[2] = make_float4(F.c2.x, F.c2.y, F.c2.z, d2.w);
-    if (mat.has_state) P.pstate_out[dst] = make_float4(st[0], st[1], st[2], st[3]);
+    store8(&P.out.aff[dst], aff.c0.x, aff.c0.y, aff.c0.z, aff.c1.x, aff.c1.y, aff.c1.z, aff.c2.x, aff.c2.y);
+    *reinterpret_cast<float2*>(&P.out.tail[dst]) = make_float2(aff.c2.z, vgd);
+    store8(&P.out.def[dst], F.c0.x, F.c0.y, F.c0.z, F.c1.x, F.c1.y, F.c1.z, F.c2.x, F.c2.y);
+    *reinterpret_cast<float4*>(&P.out.mat[dst]) = make_float4(F.c2.z, init_volume, damping, pm.w);
+    if (mat.has_state) P.out.pstate[dst] = make_float4(st[0], st[1], st[2], st[3]);
     if (P.pid_in) P.pid_out[dst] = P.pid_in[src];
 }
 
@@ -548,17 +551,14 @@ __device__ __forceinline__ void g2p_finish(const DevPtrs& P, const Params& prm) 
             if (__ldcg(&P.phdr[p]) != NONE) continue;
             const uint32_t dst = sl + atomicAdd(&P.counters->unsorted, 1u);
             if (dst >= n) continue;  // not reached: exactly n - sl particles have no header
-            const float4* ks = reinterpret_cast<const float4*>(&P.kin[p]);
-            float4* kd = reinterpret_cast<float4*>(&P.kin_out[dst]);
-#pragma unroll
-            for (int w = 0; w < 5; ++w) kd[w] = ks[w];
-            const float4* ds = reinterpret_cast<const float4*>(&P.def[p]);
-            float4* dd = reinterpret_cast<float4*>(&P.def_out[dst]);
-#pragma unroll
-            for (int w = 0; w < 3; ++w) dd[w] = ds[w];
-            P.pstate_out[dst] = P.pstate[p];
+            P.out.kin[dst] = P.in.kin[p];
+            P.out.aff[dst] = P.in.aff[p];
+            P.out.tail[dst] = P.in.tail[p];
+            P.out.def[dst] = P.in.def[p];
+            P.out.mat[dst] = P.in.mat[p];
+            P.out.pstate[dst] = P.in.pstate[p];
             P.pid_out[dst] = P.pid_in[p];
-            const CellInfo nc = cell_info(prm.dx, mk(ks[0].x, ks[0].y, ks[0].z));
+            const CellInfo nc = cell_info(prm.dx, mk(P.in.kin[p].x, P.in.kin[p].y, P.in.kin[p].z));
             const int3 o = prm.scene_blocks ? scene_base_of(prm, P.pscene[P.pid_in[p]]) : make_int3(0, 0, 0);
             P.pcode[dst] = make_uint2(pack_key(nc.bx + o.x, nc.by + o.y, nc.bz + o.z),
                                       nc.ax | (nc.ay << 2) | (nc.az << 4));
@@ -629,7 +629,7 @@ __device__ __forceinline__ void g2p_block_loop(const DevPtrs& P, const Params& p
         const uint32_t hblk = (tid < 216u && hoct != 0u) ? __ldg(&P.nbh[b * NUM_NBH + hoct - 1u]) : b;
         float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), vf = xm;
         if (pid != NONE) {
-            const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
+            const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
             xm = kr[0];
             vf = kr[1];
         }
@@ -685,7 +685,7 @@ __device__ __forceinline__ void g2p_block_loop(const DevPtrs& P, const Params& p
         for (uint32_t k = tid; k < np; k += blockDim.x) {
             if (k != tid) {
                 pid = P.sorted[first + k];
-                const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
+                const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
                 xm = kr[0];
                 vf = kr[1];
             }
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_range(Dev
         float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), vf = xm;
         uint32_t home = lo << 6;  // the particle's block and cell
         if (pid != NONE) {
-            const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
+            const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
             xm = kr[0];
             vf = kr[1];
             home = __ldcg(&P.phdr[pid]);
@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_range(Dev
             for (uint32_t p = p0 + tid; p < p1; p += kG2pThreads) {
                 if (p != p0 + tid) {
                     pid = __ldg(&P.sorted[p]);
-                    const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
+                    const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
                     xm = kr[0];
                     vf = kr[1];
                     home = __ldcg(&P.phdr[pid]);

@@ -58,9 +58,9 @@ __global__ void __launch_bounds__(kGatherStage) k_p2g_gather(DevPtrs P) {
             bool on = false;
             v3 pt = splat(0.f);
             if (pid != NONE) {
-                const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
+                const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
                 const float4 xm = kr[0], vf = kr[1];
-                const float4 c0 = kr[2], c1 = kr[3], c2 = kr[4];
+                const m3 C = affine_of(P.in, pid);
                 const v3 at = mk(xm.x, xm.y, xm.z);
                 const v3 ac = assoc_cell_of(dx, at);
                 const int zk = f2i_sat(ac.z) - vid.z * 4;
@@ -70,9 +70,9 @@ __global__ void __launch_bounds__(kGatherStage) k_p2g_gather(DevPtrs P) {
                 if (__float_as_uint(vf.w) & PFLAG_ENABLED) {
                     const float m = xm.w;
                     pt = at;
-                    srow[tid][0] = make_float4(c0.x, c1.x, c2.x, vf.x * m);
-                    srow[tid][1] = make_float4(c0.y, c1.y, c2.y, vf.y * m);
-                    srow[tid][2] = make_float4(c0.z, c1.z, c2.z, vf.z * m);
+                    srow[tid][0] = make_float4(C.c0.x, C.c1.x, C.c2.x, vf.x * m);
+                    srow[tid][1] = make_float4(C.c0.y, C.c1.y, C.c2.y, vf.y * m);
+                    srow[tid][2] = make_float4(C.c0.z, C.c1.z, C.c2.z, vf.z * m);
                     srow[tid][3] = make_float4(0.f, 0.f, 0.f, m);
                 } else {  // a zero record at the origin, as the reference stages it
 #pragma unroll
@@ -156,17 +156,16 @@ __global__ void __launch_bounds__(256) k_timestep_bound(DevPtrs P) {
     const float cw = P.params->dx;
     uint32_t best = 0xFFFFFFFFu;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        const float4* kr = reinterpret_cast<const float4*>(&P.kin[p]);
+        const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[p]);
         const float4 xm = kr[0], vf = kr[1];
         if (!(__float_as_uint(vf.w) & PFLAG_ENABLED)) continue;
-        const float4 c0 = kr[2], c1 = kr[3], c2 = kr[4];
-        const float4* dr = reinterpret_cast<const float4*>(&P.def[p]);
-        const float4 d0 = dr[0], d1 = dr[1], d2 = dr[2];
-        const m3 F = mkm(mk(d0.x, d0.y, d0.z), mk(d1.x, d1.y, d1.z), mk(d2.x, d2.y, d2.z));
-        const Material& mat = P.materials[__float_as_uint(d2.w)];
+        const m3 C = affine_of(P.in, p);
+        const PMat pm = P.in.mat[p];
+        const m3 F = def_grad_of(P.in, p, pm.f22);
+        const Material& mat = P.materials[__float_as_uint(pm.material)];
         const float* w = mat.w;
         const float mass = xm.w;
-        const float density0 = mass / d0.w;
+        const float density0 = mass / pm.init_volume;
         const float jdet = det(F);
         const v3 vel = mk(vf.x, vf.y, vf.z);
         float dt;
@@ -179,14 +178,13 @@ __global__ void __launch_bounds__(256) k_timestep_bound(DevPtrs P) {
             dt = sound_speed_bound(w[3], w[0] * w[1], 0.0f, density0, jdet, vel, cw);
             break;
         case MODEL_SNOW: {  // snow.rs:77-79: hardening from the particle's plastic det
-            const float hard = expf(w[3] * (1.0f - P.pstate[p].x));
+            const float hard = expf(w[3] * (1.0f - P.in.pstate[p].x));
             dt = elastic_bound(w, 4, hard, density0, jdet, vel, cw);
             break;
         }
         default: dt = 0.0f; break;
         }
-        const v3 a0 = mk(c0.x, c0.y, c0.z), a1 = mk(c1.x, c1.y, c1.z), a2 = mk(c2.x, c2.y, c2.z);
-        const float na2 = dot(a0, a0) + dot(a1, a1) + dot(a2, a2);
+        const float na2 = dot(C.c0, C.c0) + dot(C.c1, C.c1) + dot(C.c2, C.c2);
         const float d = (cw * cw) / 4.0f;
         const float norm_b = d * sqrtf(na2) / mass;
         const float apic_v = norm_b * 6.0f * sqrtf(3.0f) / cw;
@@ -423,7 +421,7 @@ __global__ void __launch_bounds__(128) k_g2p_cdf(DevPtrs P) {
                 }
                 continue;
             }
-            const float4 xm = reinterpret_cast<const float4*>(&P.kin[pid])[0];
+            const float4 xm = reinterpret_cast<const float4*>(&P.in.kin[pid])[0];
             const v3 pt = mk(xm.x, xm.y, xm.z);
             const v3 ref = assoc_cell_of(dx, pt) * dx - pt;
             const v3 w0 = kernel_eval_all(-ref.x / dx), w1 = kernel_eval_all(-ref.y / dx),

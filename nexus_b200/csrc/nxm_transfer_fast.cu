@@ -14,26 +14,6 @@ __device__ __forceinline__ void set_status_f(Counters* c, uint32_t bit) { atomic
 
 __device__ __forceinline__ float4 f4add(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
-// The words of a particle's kinematic record that P2G reads (kin words 0..19).
-struct P2gRaw {
-    float4 xm, vf, c0, c1, c2;
-};
-
-__device__ __forceinline__ P2gRaw p2g_load_raw(const DevPtrs& P, uint32_t pid) {
-    P2gRaw r;
-    if (pid == NONE) {
-        r.vf = make_float4(0.f, 0.f, 0.f, 0.f);  // flags 0: contributes nothing
-        return r;
-    }
-    const float4* kr = reinterpret_cast<const float4*>(&P.kin[pid]);
-    r.xm = __ldg(kr);
-    r.vf = __ldg(kr + 1);
-    r.c0 = __ldg(kr + 2);
-    r.c1 = __ldg(kr + 3);
-    r.c2 = __ldg(kr + 4);
-    return r;
-}
-
 // P2G (solver/p2g.rs:64-351 computes the same node sums in gather form).
 //
 // One warp per active block (taken from a counter), one cell per lane.  The
@@ -54,19 +34,59 @@ __device__ __forceinline__ P2gRaw p2g_load_raw(const DevPtrs& P, uint32_t pid) {
 // hold particles).  Bound by FP32 issue and the record loads; 512 threads' worth
 // of registers an SM (the 108 sums) leave 12 warps, whose next records are in
 // flight while the current ones accumulate.
+//
+// The records of a lane's next particles are in flight while it accumulates:
+// asynchronous copies into a ring of kP2gRing slots a lane in shared memory
+// (slot words of one kind side by side over the lanes: no bank conflicts), so
+// that they cost no registers.
 #ifndef NXM_P2G_MIN_CTAS
 #define NXM_P2G_MIN_CTAS 3
 #endif
+#ifndef NXM_P2G_RING
+#define NXM_P2G_RING 4
+#endif
 constexpr int kP2gWarps = 4;
 constexpr int kP2gThreads = 32 * kP2gWarps;
+constexpr int kP2gRing = NXM_P2G_RING;  // kP2gRing - 1 records ahead
+struct P2gSlot {
+    float4 xm[32], vf[32], c0[32], c1[32];  // x, m; v, flags; C 0..3; C 4..7
+    float c2[32];                           // C 8
+};
+struct P2gWarp {
+    float4 tile[216];
+    P2gSlot ring[kP2gRing];
+    uint8_t order[64];
+};
+constexpr size_t kP2gSmem = sizeof(P2gWarp) * kP2gWarps;
+
+template <int kBytes>
+__device__ __forceinline__ void async_copy(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(kBytes)
+                 : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+__device__ __forceinline__ void p2g_fetch(const DevPtrs& P, P2gSlot& s, uint32_t lane, uint32_t pid) {
+    const float4* k = reinterpret_cast<const float4*>(&P.in.kin[pid]);
+    const float4* c = reinterpret_cast<const float4*>(&P.in.aff[pid]);
+    async_copy<16>(&s.xm[lane], k);
+    async_copy<16>(&s.vf[lane], k + 1);
+    async_copy<16>(&s.c0[lane], c);
+    async_copy<16>(&s.c1[lane], c + 1);
+    async_copy<4>(&s.c2[lane], &P.in.tail[pid].c22);
+}
 
 __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P) {
-    __shared__ float4 tiles[kP2gWarps][216];
-    __shared__ uint8_t orders[kP2gWarps][64];
+    extern __shared__ float4 p2g_smem[];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    float4* tile = tiles[warp];
-    uint8_t* order = orders[warp];
+    P2gWarp& sm = reinterpret_cast<P2gWarp*>(p2g_smem)[warp];
+    float4* tile = sm.tile;
+    uint8_t* order = sm.order;
     const float dx = P.params->dx;
     const float inv_dx = P.params->inv_dx;
     const uint32_t nbp = min(__ldcg(&P.counters->num_primary), __ldcg(&P.counters->num_blocks));
@@ -133,22 +153,36 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
             float2 axy[27], azm[27];  // sums of node i + 3 j + 9 k: (x, y) and (z, mass)
 #pragma unroll
             for (int t = 0; t < 27; ++t) axy[t] = azm[t] = make_float2(0.f, 0.f);
-            P2gRaw raw = p2g_load_raw(P, n > 0u ? __ldg(&list[0]) : NONE);
-            uint32_t pid = n > 1u ? __ldg(&list[1]) : NONE;
+            uint32_t pid[kP2gRing - 1];
+#pragma unroll
+            for (uint32_t t = 0; t + 1 < kP2gRing; ++t) pid[t] = t < n ? __ldg(&list[t]) : 0u;
+            uint32_t ahead = kP2gRing - 1u < n ? __ldg(&list[kP2gRing - 1]) : 0u;  // the id after the ring's
+#pragma unroll
+            for (uint32_t t = 0; t + 1 < kP2gRing; ++t) {
+                if (t < n) p2g_fetch(P, sm.ring[t], lane, pid[t]);
+                async_commit();
+            }
+            uint32_t at = 0;  // ring slot of the current particle
 #pragma unroll 1
             for (uint32_t it = 0; it < nmax; ++it) {
-                const bool on = (__float_as_uint(raw.vf.w) & PFLAG_ENABLED) != 0u;
-                const v3 r = x0 - mk(raw.xm.x, raw.xm.y, raw.xm.z);
+                async_wait<kP2gRing - 2>();  // this lane's copies of the current slot have landed
+                const P2gSlot& cur = sm.ring[at];
+                const float4 xm = cur.xm[lane], vf = cur.vf[lane], c0 = cur.c0[lane], c1 = cur.c1[lane];
+                const float c22 = cur.c2[lane];
+                // the slot read in the previous iteration takes the record kP2gRing - 1 ahead
+                if (it + kP2gRing - 1u < n) p2g_fetch(P, sm.ring[at == 0u ? kP2gRing - 1u : at - 1u], lane, ahead);
+                async_commit();
+                ahead = it + kP2gRing < n ? __ldg(&list[it + kP2gRing]) : 0u;
+                at = at + 1u == kP2gRing ? 0u : at + 1u;
+                const bool on = it < n && (__float_as_uint(vf.w) & PFLAG_ENABLED) != 0u;
+                const v3 r = x0 - mk(xm.x, xm.y, xm.z);
                 const v3 wx = kernel_eval_all(-r.x * inv_dx);
                 const v3 wy = kernel_eval_all(-r.y * inv_dx);
                 const v3 wz = kernel_eval_all(-r.z * inv_dx);
-                const float m = raw.xm.w;
-                const m3 C = mkm(mk(raw.c0.x, raw.c0.y, raw.c0.z), mk(raw.c1.x, raw.c1.y, raw.c1.z),
-                                 mk(raw.c2.x, raw.c2.y, raw.c2.z));
-                const v3 q = C * r + mk(raw.vf.x, raw.vf.y, raw.vf.z) * m;
+                const float m = xm.w;
+                const m3 C = mkm(mk(c0.x, c0.y, c0.z), mk(c0.w, c1.x, c1.y), mk(c1.z, c1.w, c22));
+                const v3 q = C * r + mk(vf.x, vf.y, vf.z) * m;
                 const m3 K = C * dx;
-                raw = p2g_load_raw(P, pid);
-                pid = it + 2u < n ? __ldg(&list[it + 2u]) : NONE;
                 if (!on) continue;
                 float wxy[9];
 #pragma unroll
@@ -211,6 +245,24 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
         __syncwarp();
         u = __shfl_sync(0xFFFFFFFFu, next, 0);
     }
+}
+
+// The words of a particle that the CPIC P2G reads.
+struct P2gRaw {
+    f8 k, c;  // x, m, v, flags; C's first eight
+    float c22;
+};
+
+__device__ __forceinline__ P2gRaw p2g_load_raw(const DevPtrs& P, uint32_t pid) {
+    P2gRaw r;
+    if (pid == NONE) {
+        r.k.v[7] = 0.f;  // flags 0: contributes nothing
+        return r;
+    }
+    r.k = load8(&P.in.kin[pid]);
+    r.c = load8(&P.in.aff[pid]);
+    r.c22 = __ldg(&P.in.tail[pid].c22);
+    return r;
 }
 
 // CPIC P2G (solver/p2g.rs:258-310): a particle whose affinity bits are
@@ -331,21 +383,21 @@ __global__ void __launch_bounds__(kCpicThreads, 2) k_p2g_cpic(DevPtrs P) {
             // 1. stage this thread's particle (base + tid); a disabled one as zeros
             if (tid < m_chunk) {
                 float4* rr = reinterpret_cast<float4*>(rec + tid * kCpicRec);
-                if (!(__float_as_uint(raw.vf.w) & PFLAG_ENABLED)) {
+                if (!(__float_as_uint(raw.k.v[7]) & PFLAG_ENABLED)) {
 #pragma unroll
                     for (int w = 0; w < 7; ++w) rr[w] = make_float4(0.f, 0.f, 0.f, 0.f);
                 } else {
-                    const v3 pt = mk(raw.xm.x, raw.xm.y, raw.xm.z);
-                    const float m = raw.xm.w;
+                    const v3 pt = mk(raw.k.v[0], raw.k.v[1], raw.k.v[2]);
+                    const float m = raw.k.v[3];
                     const CellInfo ci = cell_info(dx, pt);
                     const v3 r = mk((float)(vid.x * 4 + (int)ci.ax), (float)(vid.y * 4 + (int)ci.ay),
                                     (float)(vid.z * 4 + (int)ci.az)) * dx - pt;
                     const v3 wx = kernel_eval_all(-r.x * inv_dx);
                     const v3 wy = kernel_eval_all(-r.y * inv_dx);
                     const v3 wz = kernel_eval_all(-r.z * inv_dx);
-                    const m3 C = mkm(mk(raw.c0.x, raw.c0.y, raw.c0.z), mk(raw.c1.x, raw.c1.y, raw.c1.z),
-                                     mk(raw.c2.x, raw.c2.y, raw.c2.z));
-                    const v3 q = C * r + mk(raw.vf.x, raw.vf.y, raw.vf.z) * m;
+                    const m3 C = mkm(mk(raw.c.v[0], raw.c.v[1], raw.c.v[2]), mk(raw.c.v[3], raw.c.v[4], raw.c.v[5]),
+                                     mk(raw.c.v[6], raw.c.v[7], raw.c22));
+                    const v3 q = C * r + mk(raw.k.v[4], raw.k.v[5], raw.k.v[6]) * m;
                     rr[0] = make_float4(q.x, q.y, q.z, m);
                     rr[1] = make_float4(C.c0.x * dx, C.c0.y * dx, C.c0.z * dx, wz.x);
                     rr[2] = make_float4(C.c1.x * dx, C.c1.y * dx, C.c1.z * dx, wz.y);
@@ -474,7 +526,12 @@ __global__ void __launch_bounds__(kCpicThreads, 2) k_p2g_cpic(DevPtrs P) {
 }  // namespace
 
 void launch_p2g(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
-    k_p2g<<<c.sm_count * (int)min(c.t.p2g_ctas, (uint32_t)NXM_P2G_MIN_CTAS), kP2gThreads, 0, s>>>(P);
+    // at most a warp per round of a block, and no more blocks than particles
+    const uint64_t units = 2ull * min(c.block_capacity, c.particle_capacity);
+    const uint64_t want = max(units / kP2gWarps, (uint64_t)1);
+    const uint64_t cap = (uint64_t)c.sm_count * min(c.t.p2g_ctas, (uint32_t)NXM_P2G_MIN_CTAS);
+    cudaFuncSetAttribute(k_p2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2gSmem);
+    k_p2g<<<(int)min(want, cap), kP2gThreads, kP2gSmem, s>>>(P);
 }
 
 void launch_p2g_cpic(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
