@@ -98,21 +98,49 @@ __global__ void __launch_bounds__(256) k_prep_readback(RenderSrc in, float4* __r
 
 // prep_readback.rs:300-357 gpu_mpm_prep_render: positions (3 floats),
 // deformations (9, column-major 3x3) and colors (4) per particle.
+//
+// The results go to the particles' ids, which block-ordered storage scatters:
+// bound by the sectors the stores touch.  A warp's 12 words a particle pass
+// through shared memory so that neighbouring lanes store neighbouring words
+// (an instruction covers some 3.5 particles' deformations, or 10 positions,
+// instead of 32 separate words): 2 M particles 161 -> 114 us, 48 scenes of
+// 33,000 232 -> 132 us.
 __global__ void __launch_bounds__(256) k_prep_render(RenderSrc in, float* __restrict__ positions,
                                                      float* __restrict__ deformations, float* __restrict__ colors) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < in.n; t += gridDim.x * blockDim.x) {
-        uint32_t id;
-        float4 color;
-        m3 d;
-        v3 pos;
-        render_particle(in, t, id, color, d, pos);
-        float* p = positions + 3u * (size_t)id;
-        p[0] = pos.x; p[1] = pos.y; p[2] = pos.z;
-        float* m = deformations + 9u * (size_t)id;
-        m[0] = d.c0.x; m[1] = d.c0.y; m[2] = d.c0.z;
-        m[3] = d.c1.x; m[4] = d.c1.y; m[5] = d.c1.z;
-        m[6] = d.c2.x; m[7] = d.c2.y; m[8] = d.c2.z;
-        reinterpret_cast<float4*>(colors)[id] = color;
+    __shared__ float words[8][32 * 12];  // per warp: deformations, then positions
+    const uint32_t lane = threadIdx.x & 31u;
+    float* w = words[threadIdx.x >> 5];
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < in.n; base += stride) {
+        uint32_t id = 0;
+        if (base + lane < in.n) {
+            float4 color;
+            m3 d;
+            v3 pos;
+            render_particle(in, base + lane, id, color, d, pos);
+            float* m = w + 9u * lane;
+            m[0] = d.c0.x; m[1] = d.c0.y; m[2] = d.c0.z;
+            m[3] = d.c1.x; m[4] = d.c1.y; m[5] = d.c1.z;
+            m[6] = d.c2.x; m[7] = d.c2.y; m[8] = d.c2.z;
+            float* p = w + 288u + 3u * lane;
+            p[0] = pos.x; p[1] = pos.y; p[2] = pos.z;
+            reinterpret_cast<float4*>(colors)[id] = color;
+        }
+        __syncwarp();
+        const uint32_t live = min(in.n - base, 32u);
+#pragma unroll
+        for (uint32_t k = 0; k < 9; ++k) {
+            const uint32_t t = 32u * k + lane, who = t / 9u;
+            const uint32_t to = __shfl_sync(0xFFFFFFFFu, id, who);
+            if (who < live) deformations[9u * (size_t)to + (t - 9u * who)] = w[t];
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 3; ++k) {
+            const uint32_t t = 32u * k + lane, who = t / 3u;
+            const uint32_t to = __shfl_sync(0xFFFFFFFFu, id, who);
+            if (who < live) positions[3u * (size_t)to + (t - 3u * who)] = w[288u + t];
+        }
+        __syncwarp();
     }
 }
 

@@ -145,3 +145,21 @@ def test_canonical_buckets_of_every_length(pipe, per_slab):
     assert not errs, "\n".join(errs[:10])
     g = nodes_in_oracle_order(st.headers(), st.nodes(), o.headers())
     assert np.array_equal(g.view(np.uint32), o.nodes()[:, :, :4].view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 1000])
+def test_render_buffers_equal_the_records(pipe, n):
+    import torch
+    sc = scenes.elastic_cube(n_side=10)
+    sc.particles = sc.particles.take(np.arange(n))
+    st = state_from_scene(sc)
+    for _ in range(2):
+        pipe.step(st)
+    p, d, c = (torch.zeros((n, k), device="cuda") for k in (3, 9, 4))
+    torch.cuda.synchronize()
+    st.prep_render(2, p.data_ptr(), d.data_ptr(), c.data_ptr())
+    st.synchronize()
+    rec = st.prep_readback(2)
+    assert np.array_equal(p.cpu().numpy(), rec["position"])
+    assert np.array_equal(c.cpu().numpy(), rec["color"])
+    assert np.array_equal(d.cpu().numpy().reshape(n, 3, 3), rec["deformation"][:, :3, :3])
