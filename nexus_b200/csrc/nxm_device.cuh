@@ -791,39 +791,113 @@ __device__ __forceinline__ float aabb_distance(const DevBvhNode& n, v3 p) {
 // (the last one found wins ties, "dist <= best"), BVH traversal pruned by box
 // distance, then the inside test pn . (p - proj) <= 0 with the pseudo-normal
 // of the closest feature.  Returns false when no triangle is within max_dist.
+struct MeshBest {
+    float dist;
+    TriProj at;
+    uint32_t tri;
+};
+__device__ __forceinline__ void mesh_test(const DevTri* __restrict__ tris, uint32_t tri, v3 pt, MeshBest& m) {
+    const DevTri& t = tris[tri];
+    const TriProj pr = triangle_closest(mk(t.v[0][0], t.v[0][1], t.v[0][2]), mk(t.v[1][0], t.v[1][1], t.v[1][2]),
+                                        mk(t.v[2][0], t.v[2][1], t.v[2][2]), pt);
+    const float d = length(pr.point - pt);
+    if (d <= m.dist) {
+        m.dist = d;
+        m.at = pr;
+        m.tri = tri;
+    }
+}
+__device__ __forceinline__ bool mesh_result(const DevTri* __restrict__ tris, v3 pt, const MeshBest& m, Proj& out) {
+    if (m.tri == NONE) return false;
+    const DevTri& t = tris[m.tri];
+    const int k = m.at.feature == 0 ? m.at.id : (m.at.feature == 1 ? 3 + m.at.id : 6);
+    const v3 pn = mk(t.pn[k][0], t.pn[k][1], t.pn[k][2]);
+    out.point = m.at.point;
+    out.inside = dot(pn, pt - m.at.point) <= 0.f;
+    return true;
+}
 __device__ __forceinline__ bool trimesh_project_local(const DevTri* __restrict__ tris,
                                                       const DevBvhNode* __restrict__ bvh, uint32_t first,
                                                       uint32_t count, v3 pt, float max_dist, Proj& out) {
-    float best = max_dist;
-    TriProj bp;
-    bp.point = pt; bp.feature = 2; bp.id = 0;
-    uint32_t best_tri = NONE;
+    MeshBest m;
+    m.dist = max_dist;
+    m.at.point = pt; m.at.feature = 2; m.at.id = 0;
+    m.tri = NONE;
     const uint32_t end = first + count;
     uint32_t curr = first;
     for (uint32_t it = 0; it < count && curr < end; ++it) {
         const DevBvhNode n = bvh[curr];
         if (n.entry & kBvhLeaf) {
-            const DevTri& t = tris[n.entry & ~kBvhLeaf];
-            const TriProj pr = triangle_closest(mk(t.v[0][0], t.v[0][1], t.v[0][2]), mk(t.v[1][0], t.v[1][1], t.v[1][2]),
-                                                mk(t.v[2][0], t.v[2][1], t.v[2][2]), pt);
-            const float d = length(pr.point - pt);
-            if (d <= best) {
-                best = d;
-                bp = pr;
-                best_tri = n.entry & ~kBvhLeaf;
-            }
+            mesh_test(tris, n.entry & ~kBvhLeaf, pt, m);
             curr = n.exit;
         } else {
-            curr = aabb_distance(n, pt) <= best ? n.entry : n.exit;
+            curr = aabb_distance(n, pt) <= m.dist ? n.entry : n.exit;
         }
     }
-    if (best_tri == NONE) return false;
-    const DevTri& t = tris[best_tri];
-    const int k = bp.feature == 0 ? bp.id : (bp.feature == 1 ? 3 + bp.id : 6);
-    const v3 pn = mk(t.pn[k][0], t.pn[k][1], t.pn[k][2]);
-    out.point = bp.point;
-    out.inside = dot(pn, pt - bp.point) <= 0.f;
-    return true;
+    return mesh_result(tris, pt, m, out);
+}
+
+// The leaves within max_dist of any of a warp's points `pt` (one per lane, the
+// warp whole), as node indexes in traversal order: the nodes lie in depth-first
+// order, so the warp loads 32 consecutive ones at a time, tests them against
+// the box of its points, and walks the window by the skip links.  Returns
+// their number, or NONE when they do not fit kMeshLeaves.
+constexpr uint32_t kMeshLeaves = 192;
+__device__ __forceinline__ uint32_t warp_mesh_leaves(const DevBvhNode* __restrict__ bvh, uint32_t first, uint32_t count,
+                                                     v3 pt, float max_dist, uint32_t* leaves) {
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    v3 lo = pt, hi = pt;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = mk(fminf(lo.x, __shfl_xor_sync(0xFFFFFFFFu, lo.x, o)), fminf(lo.y, __shfl_xor_sync(0xFFFFFFFFu, lo.y, o)),
+                fminf(lo.z, __shfl_xor_sync(0xFFFFFFFFu, lo.z, o)));
+        hi = mk(fmaxf(hi.x, __shfl_xor_sync(0xFFFFFFFFu, hi.x, o)), fmaxf(hi.y, __shfl_xor_sync(0xFFFFFFFFu, hi.y, o)),
+                fmaxf(hi.z, __shfl_xor_sync(0xFFFFFFFFu, hi.z, o)));
+    }
+    const float reach = max_dist * 1.001f + 1.0e-6f;  // above the rounding of the per-point distances
+    lo = lo - splat(reach);
+    hi = hi + splat(reach);
+    const uint32_t end = first + count;
+    uint32_t curr = first, n = 0;
+    while (curr < end) {
+        const uint32_t at = curr + lane;
+        uint32_t to = NONE;  // where the traversal goes from this lane's node
+        bool leaf = false;
+        if (at < end) {
+            const DevBvhNode b = bvh[at];
+            const bool hit = !(b.mn[0] > hi.x || b.mx[0] < lo.x || b.mn[1] > hi.y || b.mx[1] < lo.y || b.mn[2] > hi.z ||
+                               b.mx[2] < lo.z);
+            leaf = hit && (b.entry & kBvhLeaf);
+            to = hit && !(b.entry & kBvhLeaf) ? b.entry : b.exit;
+        }
+        const uint32_t leaf_mask = __ballot_sync(0xFFFFFFFFu, leaf);
+        uint32_t take = 0u, pos = curr;
+        const uint32_t stop = min(curr + 32u, end);
+        for (uint32_t it = 0; it < 32u && pos >= curr && pos < stop; ++it) {
+            take |= leaf_mask & (1u << (pos - curr));
+            pos = __shfl_sync(0xFFFFFFFFu, to, pos - curr);
+        }
+        if (pos <= curr) break;  // not reached: the links go forward
+        if (n + __popc(take) > kMeshLeaves) return NONE;
+        if (take & (1u << lane)) leaves[n + __popc(take & lt)] = at;
+        n += __popc(take);
+        curr = pos;
+    }
+    __syncwarp();
+    return n;
+}
+// trimesh_project_local over the warp's leaves.
+__device__ __forceinline__ bool mesh_project_leaves(const DevTri* __restrict__ tris, const DevBvhNode* __restrict__ bvh,
+                                                    const uint32_t* leaves, uint32_t n, v3 pt, float max_dist, Proj& out) {
+    MeshBest m;
+    m.dist = max_dist;
+    m.at.point = pt; m.at.feature = 2; m.at.id = 0;
+    m.tri = NONE;
+    for (uint32_t k = 0; k < n; ++k) {
+        const DevBvhNode b = bvh[leaves[k]];
+        if (aabb_distance(b, pt) <= m.dist) mesh_test(tris, b.entry & ~kBvhLeaf, pt, m);
+    }
+    return mesh_result(tris, pt, m, out);
 }
 
 // CPIC affinity bits (grid/grid.rs:593-645): bit i = affinity to collider

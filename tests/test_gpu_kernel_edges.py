@@ -1,15 +1,16 @@
 """The kernels at the sizes where their splits change: P2G's two rounds of 32
-cells, the cell-ordered sort list, strains of every form (eigenvalues, SVD), the
-gather P2G's stages, long and short canonical buckets.  Against the CPU oracle,
-with the bounds of tests/parity.py (or bit for bit where the mode promises it)."""
+cells, the cell-ordered sort list, strains of every form (series, eigenvalues, SVD), the gather P2G's stages, long and
+short canonical buckets, mesh searches with more leaves than a warp keeps,
+render data at partial warps.  Against the CPU oracle, with the bounds of
+tests/parity.py (or bit for bit where the mode promises it)."""
 import numpy as np
 import pytest
 
 from nexus_b200 import scenes
 from nexus_b200.models import BoundaryCondition, ParticleModel
 from nexus_b200.mpm import MpmPipeline, state_from_scene
-from nexus_b200.particles import ParticleBatch, box_walls, collider_array
-from tests.parity import compare_sort, nodes_in_oracle_order, rel_l2
+from nexus_b200.particles import Collider, ParticleBatch, box_walls, collider_array
+from tests.parity import FAST_BOUNDS, assert_run_matches, compare_sort, nodes_in_oracle_order, rel_l2, start_state
 
 pytestmark = pytest.mark.gpu
 
@@ -145,6 +146,29 @@ def test_canonical_buckets_of_every_length(pipe, per_slab):
     assert not errs, "\n".join(errs[:10])
     g = nodes_in_oracle_order(st.headers(), st.nodes(), o.headers())
     assert np.array_equal(g.view(np.uint32), o.nodes()[:, :, :4].view(np.uint32))
+
+
+@pytest.mark.parametrize("vertices", [5, 21, 41])
+def test_mesh_floor_of_every_fineness(pipe, vertices):
+    """From a few triangles a block to more than a warp keeps (41 x 41 vertices:
+    about 600 triangles within reach of a warp's nodes, each node searches alone)."""
+    from oracle.oracle import OracleScene
+    sc = scenes.trimesh_floor(n_side=8, steps=20)
+    tri = scenes.height_field(vertices, 5, lo=0.3, hi=0.55)
+    walls = box_walls(0.0, 1.0, BoundaryCondition.slip(), BoundaryCondition.slip())
+    mesh = Collider.trimesh(0, len(tri), (0.0, 0.0, 0.0), BoundaryCondition.separate(0.3))
+    sc.colliders = collider_array(walls + [mesh])
+    sc.tri_vertices = tri.reshape(-1, 3)
+    st = state_from_scene(sc)
+    for _ in range(sc.steps):
+        pipe.step(st)
+    st.synchronize()
+    o32, o64 = OracleScene(sc, "f32"), OracleScene(sc, "f64")
+    o32.step(sc.steps)
+    o64.step(sc.steps)
+    p64 = o64.particles()
+    p64["pos"] = o64.positions_f64()
+    assert_run_matches(f"mesh floor {vertices}", st.read_particles(), o32.particles(), p64, start_state(sc), FAST_BOUNDS)
 
 
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 1000])
