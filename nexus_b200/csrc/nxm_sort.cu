@@ -608,64 +608,70 @@ __global__ void __launch_bounds__(256) k_finalize(DevPtrs P) {
 }
 
 // Canonical order: every (block, bucket) segment sorted by ascending id, by
-// ranks (particle ids are distinct inside a block).  A warp takes a bucket of
-// up to kSegWarp ids (a slab holds some 128 at 8 particles a cell), so a
-// block's ten buckets sort side by side; the CTA sorts a longer one together
-// (the CTA sorting one bucket after another took 36 us for 100,003 particles).
+// ranks (particle ids are distinct inside a block).  A block's whole list (some
+// 1,700 ids at 8 particles a cell) is taken into shared memory, every bucket
+// from a multiple of four, and the CTA's threads each rank some ids against
+// their bucket, four at a time; longer lists are sorted bucket by bucket.
+// Bound by the comparisons: 100,003 particles 28 us (one bucket after another,
+// a thread per id: 36 us; a warp per bucket: 31 us).
 constexpr uint32_t kSegMax = 4096;
-constexpr uint32_t kSegWarp = kSegMax / 8;
+constexpr uint32_t kSegList = kSegMax - 4 * NUM_BUCKETS - 4;
 __global__ void __launch_bounds__(256) k_sort_segments(DevPtrs P) {
     __shared__ uint4 buf4[kSegMax / 4];
+    __shared__ uint32_t ends[NUM_BUCKETS + 1];  // of the buckets in the block's list; ends[0] = 0
     uint32_t* buf = reinterpret_cast<uint32_t*>(buf4);
     const uint32_t total = P.counters->num_blocks;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t b = blockIdx.x; b < total; b += gridDim.x) {
-        bool longer = false;
-        const auto segment = [&](int k, uint32_t& start) {
-            start = k ? P.cursors[b * NUM_BUCKETS + k - 1] : P.first[b];
-            return P.cursors[b * NUM_BUCKETS + k] - start;
-        };
-        for (int k = 0; k < NUM_BUCKETS; ++k) {
-            uint32_t start;
-            const uint32_t len = segment(k, start);
-            longer |= len > kSegWarp;
-            if ((uint32_t)k % 8u != warp || len < 2 || len > kSegWarp) continue;
-            uint32_t* mine = buf + warp * kSegWarp;
-            const uint4* mine4 = buf4 + warp * (kSegWarp / 4);
-            __syncwarp();  // the previous bucket's reads are done
-            for (uint32_t i = lane; i < ((len + 3u) & ~3u); i += 32u) mine[i] = i < len ? P.sorted[start + i] : NONE;
-            __syncwarp();
-            for (uint32_t i = lane; i < len; i += 64u) {
-                const uint32_t v0 = mine[i], v1 = i + 32u < len ? mine[i + 32u] : 0u;
-                uint32_t r0 = 0, r1 = 0;
-                for (uint32_t j = 0; j < (len + 3u) / 4u; ++j) {
-                    const uint4 q = mine4[j];
-                    r0 += (q.x < v0) + (q.y < v0) + (q.z < v0) + (q.w < v0);
-                    r1 += (q.x < v1) + (q.y < v1) + (q.z < v1) + (q.w < v1);
-                }
-                P.sorted[start + r0] = v0;
-                if (i + 32u < len) P.sorted[start + r1] = v1;
-            }
-        }
-        if (!longer) continue;
+        const uint32_t first = P.first[b], len = P.nwx[b];
+        if (threadIdx.x <= NUM_BUCKETS)
+            ends[threadIdx.x] = threadIdx.x ? P.cursors[b * NUM_BUCKETS + threadIdx.x - 1] - first : 0u;
         __syncthreads();
-        for (int k = 0; k < NUM_BUCKETS; ++k) {
-            uint32_t start;
-            const uint32_t len = segment(k, start);
-            if (len > kSegWarp && len <= kSegMax) {
-                for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) buf[i] = P.sorted[start + i];
-                __syncthreads();
-                for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
-                    const uint32_t v = buf[i];
-                    uint32_t rank = 0;
-                    for (uint32_t j = 0; j < len; ++j) rank += buf[j] < v ? 1u : 0u;
-                    P.sorted[start + rank] = v;
+        if (len <= kSegList) {
+            // bucket k starts at the next multiple of four, four words of room a bucket
+            const auto at = [&](uint32_t k) { return (ends[k] + 4u * k + 3u) & ~3u; };
+            const auto bucket = [&](uint32_t i) {
+                uint32_t k = 0;
+                while (k + 1u < NUM_BUCKETS && i >= ends[k + 1u]) ++k;
+                return k;
+            };
+            for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
+                const uint32_t k = bucket(i);
+                buf[at(k) + i - ends[k]] = P.sorted[first + i];
+            }
+            if (threadIdx.x < 4u * NUM_BUCKETS) {  // the words after a bucket's last compare as larger
+                const uint32_t k = threadIdx.x >> 2, j = threadIdx.x & 3u, n = ends[k + 1u] - ends[k];
+                if (n + j < ((n + 3u) & ~3u)) buf[at(k) + n + j] = NONE;
+            }
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
+                const uint32_t k = bucket(i), s = at(k), n = ends[k + 1u] - ends[k];
+                const uint32_t v = buf[s + i - ends[k]];
+                uint32_t rank = 0;
+                for (uint32_t j = s / 4u; j < (s + n + 3u) / 4u; ++j) {
+                    const uint4 q = buf4[j];
+                    rank += (q.x < v) + (q.y < v) + (q.z < v) + (q.w < v);
                 }
-                __syncthreads();
-            } else if (len > kSegMax && threadIdx.x == 0) {
-                set_status(P.counters, STATUS_SORT_CAPACITY);
+                P.sorted[first + ends[k] + rank] = v;
+            }
+        } else {
+            for (uint32_t k = 0; k < NUM_BUCKETS; ++k) {
+                const uint32_t start = first + ends[k], n = ends[k + 1u] - ends[k];
+                if (n > 1u && n <= kSegMax) {
+                    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) buf[i] = P.sorted[start + i];
+                    __syncthreads();
+                    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+                        const uint32_t v = buf[i];
+                        uint32_t rank = 0;
+                        for (uint32_t j = 0; j < n; ++j) rank += buf[j] < v ? 1u : 0u;
+                        P.sorted[start + rank] = v;
+                    }
+                    __syncthreads();
+                } else if (n > kSegMax && threadIdx.x == 0) {
+                    set_status(P.counters, STATUS_SORT_CAPACITY);
+                }
             }
         }
+        __syncthreads();
     }
 }
 
