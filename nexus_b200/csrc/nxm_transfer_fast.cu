@@ -311,8 +311,9 @@ __device__ __forceinline__ P2gHdr p2g_load_hdr(const DevPtrs& P, uint32_t b, uin
 // Work runs over the primary blocks only (ids [0, num_primary); the others
 // hold no particles).  Loads run ahead of use: the headers of the blocks two
 // grid strides ahead, the sorted id of the next chunk's particle right after
-// staging, and its 80-byte record at the start of the cell phase, so their
-// latency overlaps the current chunk's shared-memory work.
+// staging, and its record at the start of the cell phase, so their latency
+// overlaps the current chunk's shared-memory work.  Two coupled fields of 27
+// sums do not fit a lane's registers, so this mode keeps a cell per warp.
 __global__ void __launch_bounds__(kCpicThreads, 2) k_p2g_cpic(DevPtrs P) {
     static_assert(kCpicThreads >= 216, "one flushed tile node per thread");
     extern __shared__ float4 p2g_smem[];

@@ -4,7 +4,7 @@
 // forms) and the CPIC branches.  A particle without affinity bits takes the
 // factored gather of the plain fast path; one with affinity takes the per-node
 // gather that substitutes incompatible nodes (solver/g2p.rs:206-257).  The
-// scatter P2G of this mode is k_p2g<true> (nxm_transfer_fast.cu).
+// scatter P2G of this mode is k_p2g_cpic (nxm_transfer_fast.cu).
 #define NXM_NS fast_cpic
 #define NXM_FAST true
 #define NXM_CPIC 1
