@@ -81,7 +81,7 @@ struct DevPtrs {
 };
 
 constexpr uint32_t kScanTile = 256;  // blocks per scan tile of the slab sort (one per thread of a scan CTA)
-constexpr uint32_t kCellTile = 128;  // blocks per scan tile of the cell sort (16 per warp of a scan CTA)
+constexpr uint32_t kCellTile = 64;   // blocks per scan tile of the cell sort (8 per warp of a scan CTA)
 constexpr uint32_t kRangeChunk = 256;  // sorted positions per fast-G2P run (one per thread of its CTA)
 
 // Launch shapes the autotuner picks per state (nxm_state_autotune); the
@@ -119,6 +119,8 @@ namespace fast {
 // by block (P.nrp > 0; their world positions already written).
 void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool canonical, cudaStream_t s,
                  bool rigid = false);
+// Kernels it issues (without the rigid ones).
+int sort_launches(const LaunchCfg& c, bool with_extras, bool canonical);
 constexpr int kRigidSortLaunches = 5;
 void launch_p2g(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s);
 void launch_grid_update(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s);
@@ -183,8 +185,7 @@ void launch_prep_readback_rigid(const RenderSrc& in, const float4* world, uint32
 void launch_sort_positions(const DevPtrs& P, const LaunchCfg& c, const float4* pos, cudaStream_t s);
 constexpr int kSortPositionsLaunches = 8;
 
-// Kernels issued per phase (sort counts the canonical segment sort when on).
-int sort_launches(bool canonical);
+// Kernels issued per phase.
 constexpr int kP2gLaunches = 1;
 constexpr int kGridLaunches = 1;
 

@@ -19,7 +19,7 @@
 // of lanes that hit the same block (or the same block bucket): one hash probe
 // or one atomicAdd per distinct key per warp instead of one per particle.
 // The block key of each particle is cached in `pcode` (8 bytes) by the
-// previous step's G2P, so activation does not re-read the 80-byte particle
+// previous step's G2P, so activation does not re-read the particle
 // records.  Counters, headers and the hash live in L2.
 #include "nxm_device.cuh"
 #include "nxm_kernels.h"
@@ -42,11 +42,11 @@ __device__ __forceinline__ void assoc_shift(int i, int& dx, int& dy, int& dz) {
 // Insert `key` (block kx,ky,kz); allocates a header on first insertion.
 // Primary blocks take ids [0, num_primary); neighbour-pass blocks take ids
 // base + [0, num_extra) with base = num_primary.
-// `slot` = hash_key(key) & hash_mask and `cur` = its entry, already read.
-__device__ void hash_insert_at(const DevPtrs& P, uint32_t key, int kx, int ky, int kz, bool primary, uint32_t base,
-                               uint32_t hash_mask, uint32_t block_cap, uint32_t slot, uint32_t cur) {
+__device__ void hash_insert(const DevPtrs& P, uint32_t key, int kx, int ky, int kz, bool primary, uint32_t base,
+                            uint32_t hash_mask, uint32_t block_cap) {
+    uint32_t slot = hash_key(key) & hash_mask;
     for (uint32_t it = 0; it <= hash_mask; ++it) {
-        if (it) cur = __ldcg(&P.hkey[slot]);
+        uint32_t cur = __ldcg(&P.hkey[slot]);
         if (cur == key) return;
         if (cur == NONE) {
             uint32_t old = atomicCAS(&P.hkey[slot], NONE, key);
@@ -69,27 +69,15 @@ __device__ void hash_insert_at(const DevPtrs& P, uint32_t key, int kx, int ky, i
     set_status(P.counters, STATUS_HASH_FULL);
 }
 
-__device__ __forceinline__ void hash_insert(const DevPtrs& P, uint32_t key, int kx, int ky, int kz, bool primary,
-                                            uint32_t base, uint32_t hash_mask, uint32_t block_cap) {
-    const uint32_t slot = hash_key(key) & hash_mask;
-    hash_insert_at(P, key, kx, ky, kz, primary, base, hash_mask, block_cap, slot, __ldcg(&P.hkey[slot]));
-}
-
-// `cur`, `val` = the entry of `slot` = hash_key(key) & hash_mask, already read.
-__device__ __forceinline__ uint32_t hash_find_at(const DevPtrs& P, uint32_t key, uint32_t hash_mask, uint32_t slot,
-                                                 uint32_t cur, uint32_t val) {
+__device__ __forceinline__ uint32_t hash_find(const DevPtrs& P, uint32_t key, uint32_t hash_mask) {
+    uint32_t slot = hash_key(key) & hash_mask;
     for (uint32_t it = 0; it <= hash_mask; ++it) {
-        if (cur == key) return val;
+        uint32_t cur = __ldg(&P.hkey[slot]);
+        if (cur == key) return __ldg(&P.hval[slot]);
         if (cur == NONE) return NONE;
         slot = (slot + 1) & hash_mask;
-        cur = __ldg(&P.hkey[slot]);
-        val = __ldg(&P.hval[slot]);
     }
     return NONE;
-}
-__device__ __forceinline__ uint32_t hash_find(const DevPtrs& P, uint32_t key, uint32_t hash_mask) {
-    const uint32_t slot = hash_key(key) & hash_mask;
-    return hash_find_at(P, key, hash_mask, slot, __ldg(&P.hkey[slot]), __ldg(&P.hval[slot]));
 }
 
 // Warp-aggregated atomicAdd: lanes with equal `key` (NONE = no-op) share one
@@ -168,10 +156,9 @@ __global__ void k_sort_reset(DevPtrs P, uint32_t hash_cap) {
 
 // sort.rs:104-121 gpu_touch_primary_blocks.  Block keys come from the cache
 // written by the previous step (or from the positions after an upload).
-// Each warp walks a contiguous range of particles, so its passes mostly see
-// the block it inserted last (`known`).  The other keys of a batch (a block
-// border, particles that moved to another block) are probed together: one
-// L2 round trip a batch, not one a pass, and most are found present.
+// Each warp walks a contiguous range of particles, so consecutive passes
+// mostly see the block they inserted last: a pass whose lanes all carry the
+// key inserted by the previous pass skips the hash entirely.
 template <int kSortBatch>
 __global__ void __launch_bounds__(256) k_touch_primary(DevPtrs P) {
     const uint32_t n = P.params->n;
@@ -203,34 +190,21 @@ __global__ void __launch_bounds__(256) k_touch_primary(DevPtrs P) {
             }
             keys[j] = key;
         }
-        uint32_t slot[kSortBatch], cur[kSortBatch];
-        uint32_t lead = 0u;  // bit j: this lane inserts its key of pass j
 #pragma unroll
         for (int j = 0; j < kSortBatch; ++j) {
+            const uint32_t b32 = base + 32u * j;
+            if (b32 >= hi) break;
+            const bool active = b32 + lane < hi;
             const uint32_t key = keys[j];
-            bool need = base + 32u * j + lane < hi && key != known;
-            if (j) need &= key != keys[j - 1];
-            slot[j] = hash_key(key) & hmask;
-            cur[j] = key;
-            if (!__any_sync(0xFFFFFFFFu, need)) continue;
-            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, need ? key : NONE);
-            if (need && lane == (uint32_t)(__ffs(peers) - 1)) {
-                lead |= 1u << j;
-                cur[j] = __ldcg(&P.hkey[slot[j]]);
+            const uint32_t need = (active && key != known) ? key : NONE;
+            if (!__all_sync(0xFFFFFFFFu, need == NONE)) {
+                const uint32_t peers = __match_any_sync(0xFFFFFFFFu, need);
+                if (need != NONE && lane == (uint32_t)(__ffs(peers) - 1))
+                    hash_insert(P, key, key_x(key), key_y(key), key_z(key), true, 0, hmask, bcap);
             }
+            // the last active lane's key is now in the table
+            known = __shfl_sync(0xFFFFFFFFu, key, min(31u, hi - 1u - b32));
         }
-#pragma unroll
-        for (int j = 0; j < kSortBatch; ++j) {
-            const uint32_t key = keys[j];
-            if ((lead & (1u << j)) && cur[j] != key)
-                hash_insert_at(P, key, key_x(key), key_y(key), key_z(key), true, 0, hmask, bcap, slot[j], cur[j]);
-        }
-        // the last active lane's key is now in the table
-        uint32_t tail = keys[0];
-#pragma unroll
-        for (int j = 1; j < kSortBatch; ++j)
-            if (base + 32u * j < hi) tail = keys[j];
-        known = __shfl_sync(0xFFFFFFFFu, tail, min(hi - 1u - base, 32u * kSortBatch - 1u) & 31u);
     }
 }
 
@@ -251,7 +225,10 @@ __global__ void __launch_bounds__(256) k_touch_nbh(DevPtrs P) {
 }
 
 // sort.rs:261-279 gpu_update_nbh_block_ids, plus zeroing of the block's
-// bucket counters and P2G accumulation nodes.  One thread per node.
+// bucket counters and P2G accumulation nodes.  One thread per node.  Without
+// extras only primary blocks have cell counts (kCells: which blocks' to clear).
+enum CellBlocks { kNoCells, kPrimaryCells, kAllCells };
+template <CellBlocks kCells>
 __global__ void __launch_bounds__(256) k_block_prep(DevPtrs P) {
     const uint32_t hmask = P.params->hash_capacity - 1;
     const uint32_t bcap = P.params->block_capacity;
@@ -264,7 +241,7 @@ __global__ void __launch_bounds__(256) k_block_prep(DevPtrs P) {
         if (P.nodes) P.nodes[t] = make_float4(0.f, 0.f, 0.f, 0.f);
         // the scatter P2G of CPIC accumulates the incompatible field too
         if (P.nodes_inc && P.params->use_cpic) P.nodes_inc[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (P.cells) P.cells[t] = 0;
+        if (kCells == kAllCells || (kCells == kPrimaryCells && b < nprim)) P.cells[t] = 0;
         if (k < NUM_NBH) {
             int4 v = P.bvid[b];
             int sx, sy, sz;
@@ -286,20 +263,13 @@ __global__ void __launch_bounds__(256) k_count(DevPtrs P) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t lo, hi;
     warp_range(n, lo, hi);
+    uint32_t known_key = NONE, known_h0 = NONE;  // the last key this warp looked up
     for (uint32_t base = lo; base < hi; base += 32u * kSortBatch) {
         uint2 codes[kSortBatch];
 #pragma unroll
         for (int j = 0; j < kSortBatch; ++j) {
             const uint32_t p = base + 32u * j + lane;
             codes[j] = p < hi ? P.pcode[p] : make_uint2(NONE, 0u);
-        }
-        // every lane's first probe, all passes in flight together (lanes of a block share the address)
-        uint32_t slot[kSortBatch], cur[kSortBatch], val[kSortBatch];
-#pragma unroll
-        for (int j = 0; j < kSortBatch; ++j) {
-            slot[j] = hash_key(codes[j].x) & hmask;
-            cur[j] = __ldg(&P.hkey[slot[j]]);
-            val[j] = __ldg(&P.hval[slot[j]]);
         }
 #pragma unroll
         for (int j = 0; j < kSortBatch; ++j) {
@@ -309,7 +279,19 @@ __global__ void __launch_bounds__(256) k_count(DevPtrs P) {
             const bool active = p < hi;
             const uint2 code = codes[j];
             const uint32_t key = active ? code.x : NONE;
-            const uint32_t h0 = active ? hash_find_at(P, key, hmask, slot[j], cur[j], val[j]) : NONE;
+            uint32_t h0;
+            if (__all_sync(0xFFFFFFFFu, !active || key == known_key)) {
+                h0 = active ? known_h0 : NONE;
+            } else {  // one probe per distinct block key in the warp
+                const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
+                const uint32_t leader = __ffs(peers) - 1;
+                uint32_t h = NONE;
+                if (active && lane == leader) h = hash_find(P, key, hmask);
+                h0 = __shfl_sync(0xFFFFFFFFu, h, leader);
+            }
+            const uint32_t last = min(31u, hi - 1u - b32);
+            known_key = __shfl_sync(0xFFFFFFFFu, key, last);
+            known_h0 = __shfl_sync(0xFFFFFFFFu, h0, last);
             const uint32_t ckey = (h0 != NONE) ? h0 * 64u + code.y : NONE;
             if (active) {
                 P.phdr[p] = ckey;
@@ -448,17 +430,18 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(DevPtrs P) {
 // The same two passes for the cell sort, one warp per block: a block's total
 // is the sum of its 64 cell counts (and 6 extra buckets); the second pass
 // turns the cell counts into cursors (a warp scan, two cells a lane) and
-// writes the slab ends.
-constexpr uint32_t kCellWarps = kScanThreads / 32;
-constexpr uint32_t kCellPerWarp = kCellTile / kCellWarps;  // blocks per warp of a scan CTA
-static_assert(kCellTile <= kScanThreads, "one block total per thread in the tile scan");
+// writes the slab ends.  Without extras only the primary blocks, which come
+// first, have counts: the others start where the list ends.
+constexpr uint32_t kCellPerWarp = 8;  // blocks per warp of a scan CTA
+static_assert(kCellTile == kCellPerWarp * (kScanThreads / 32), "a tile per scan CTA");
 
 template <bool kExtras>
 __global__ void __launch_bounds__(kScanThreads) k_scan_cell_tiles(DevPtrs P) {
     __shared__ uint32_t warp_tot[33];
     __shared__ uint32_t btot[kCellTile];
-    const uint32_t total = P.counters->num_blocks;
-    const uint32_t ntiles = (total + kCellTile - 1) / kCellTile;
+    const uint32_t total = __ldcg(&P.counters->num_blocks);
+    const uint32_t counted = kExtras ? total : min(__ldcg(&P.counters->num_primary), total);
+    const uint32_t ntiles = (counted + kCellTile - 1) / kCellTile;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint2* cells = reinterpret_cast<const uint2*>(P.cells);
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -468,7 +451,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_cell_tiles(DevPtrs P) {
         for (uint32_t j = 0; j < kCellPerWarp; ++j) {
             const uint32_t b = b0 + wid * kCellPerWarp + j;
             v[j] = 0u;
-            if (b < total) {
+            if (b < counted) {
                 const uint2 c = __ldcg(&cells[b * 32u + lane]);
                 v[j] = c.x + c.y;
                 if (kExtras && lane < NUM_EXTRA_BUCKETS)
@@ -489,11 +472,70 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_cell_tiles(DevPtrs P) {
     }
 }
 
+// The cursors, header fields and run starts of block b, whose particles start
+// at `first` (a warp; cnt: the counts of cells 2 lane and 2 lane + 1, ext: of
+// extra bucket `lane`).  Returns where the next block's start.
+template <bool kExtras>
+__device__ __forceinline__ uint32_t write_block_cursors(const DevPtrs& P, uint32_t b, uint32_t total, uint32_t first,
+                                                        uint2 cnt, uint32_t ext, uint32_t lane) {
+    uint2* cells = reinterpret_cast<uint2*>(P.cells);
+    uint32_t incl = cnt.x + cnt.y;
+    uint32_t einc = ext;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+        if (kExtras && o < 8) {
+            const uint32_t e = __shfl_up_sync(0xFFFFFFFFu, einc, o);
+            if (lane >= (uint32_t)o) einc += e;
+        }
+    }
+    const uint32_t start = first + incl - cnt.x - cnt.y;
+    cells[b * 32u + lane] = make_uint2(start, start + cnt.x);
+    const uint32_t prim_end = first + __shfl_sync(0xFFFFFFFFu, incl, 31);
+    const uint32_t end = kExtras ? prim_end + __shfl_sync(0xFFFFFFFFu, einc, NUM_EXTRA_BUCKETS - 1) : prim_end;
+    // slab ends (a slab is 16 cells, 8 lanes); the extra buckets' cursors, empty without extras
+    if ((lane & 7u) == 7u) P.cursors[b * NUM_BUCKETS + (lane >> 3)] = first + incl;
+    if (lane < NUM_EXTRA_BUCKETS)
+        P.cursors[b * NUM_BUCKETS + NUM_PRIMARY_BUCKETS + lane] = prim_end + einc - ext;
+    if (lane == 0) {
+        P.first[b] = first;
+        P.nprim[b] = prim_end - first;
+        P.nwx[b] = end - first;
+        if (b == total - 1) {
+            P.counters->sorted_len = end;
+            if (end > P.params->sorted_capacity) set_status(P.counters, STATUS_SORT_CAPACITY);
+        }
+    }
+    // the runs of kRangeChunk sorted positions that start inside this block
+    if (P.chunk_blk)
+        for (uint32_t c = (first + kRangeChunk - 1u) / kRangeChunk + lane; c * kRangeChunk < end && c < P.chunk_cap;
+             c += 32u)
+            P.chunk_blk[c] = b;
+    return end;
+}
+
+// The header of block b without particles, of a list that ends at `len` (a warp).
+__device__ __forceinline__ void write_block_empty(const DevPtrs& P, uint32_t b, uint32_t total, uint32_t len,
+                                                  uint32_t lane) {
+    if (lane < NUM_BUCKETS) P.cursors[b * NUM_BUCKETS + lane] = len;
+    if (lane == 0) {
+        P.first[b] = len;
+        P.nprim[b] = 0u;
+        P.nwx[b] = 0u;
+        if (b == total - 1) {
+            P.counters->sorted_len = len;
+            if (len > P.params->sorted_capacity) set_status(P.counters, STATUS_SORT_CAPACITY);
+        }
+    }
+}
+
 template <bool kExtras>
 __global__ void __launch_bounds__(kScanThreads) k_scan_cell_apply(DevPtrs P) {
     __shared__ uint32_t warp_tot[33];
-    const uint32_t total = P.counters->num_blocks;
-    const uint32_t ntiles = (total + kCellTile - 1) / kCellTile;
+    const uint32_t total = __ldcg(&P.counters->num_blocks);
+    const uint32_t counted = kExtras ? total : min(__ldcg(&P.counters->num_primary), total);
+    const uint32_t ntiles = (total + kCellTile - 1) / kCellTile, summed = (counted + kCellTile - 1) / kCellTile;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     uint2* cells = reinterpret_cast<uint2*>(P.cells);
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -505,15 +547,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_cell_apply(DevPtrs P) {
         for (uint32_t j = 0; j < kCellPerWarp; ++j) {
             cnt[j] = make_uint2(0u, 0u);
             ext[j] = 0u;
-            if (b0 + j < total) {
+            if (b0 + j < counted) {
                 cnt[j] = __ldcg(&cells[(b0 + j) * 32u + lane]);
                 if (kExtras && lane < NUM_EXTRA_BUCKETS)
                     ext[j] = __ldcg(&P.cursors[(b0 + j) * NUM_BUCKETS + NUM_PRIMARY_BUCKETS + lane]);
             }
         }
-        const uint32_t rel = lane < kCellPerWarp && b0 + lane < total ? __ldcg(&P.scan_tmp[b0 + lane]) : 0u;
+        const uint32_t rel =
+            tile < summed && lane < kCellPerWarp && b0 + lane < total ? __ldcg(&P.scan_tmp[b0 + lane]) : 0u;
         uint32_t part = 0;
-        for (uint32_t i = threadIdx.x; i < tile; i += kScanThreads) part += __ldcg(&P.tile_sums[i]);
+        for (uint32_t i = threadIdx.x; i < min(tile, summed); i += kScanThreads) part += __ldcg(&P.tile_sums[i]);
         uint32_t offset;
         cta_exclusive_scan(part, warp_tot, &offset);
 #pragma unroll
@@ -521,39 +564,60 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_cell_apply(DevPtrs P) {
             const uint32_t b = b0 + j;
             if (b >= total) break;
             const uint32_t first = offset + __shfl_sync(0xFFFFFFFFu, rel, j);
-            uint32_t incl = cnt[j].x + cnt[j].y;
-            uint32_t einc = ext[j];
+            if (b < counted) write_block_cursors<kExtras>(P, b, total, first, cnt[j], ext[j], lane);
+            else write_block_empty(P, b, total, first, lane);
+        }
+    }
+}
+
+// Both passes in one CTA, for states of few blocks (without extras): its warps
+// share the blocks out evenly, sum them, scan the sums and write the cursors,
+// which takes less than a second launch does (one state of 4,096 particles: sort
+// 39 us with two kernels, 34 us with this one; above some 2,000 blocks the one
+// CTA's walk costs more than the launch).
+constexpr uint32_t kOneCtaBlocks = 2048;
+constexpr uint32_t kOneCtaThreads = 1024;
+__global__ void __launch_bounds__(kOneCtaThreads) k_scan_cells(DevPtrs P) {
+    __shared__ uint32_t warp_tot[33];
+    const uint32_t total = P.counters->num_blocks;
+    const uint32_t counted = min(P.counters->num_primary, total);
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const uint32_t per = (counted + 31u) / 32u;  // blocks per warp, at most 64
+    const uint32_t b0 = min(wid * per, counted), b1 = min(b0 + per, counted);
+    uint2* cells = reinterpret_cast<uint2*>(P.cells);
+    uint32_t sum = 0;
+    for (uint32_t b = b0; b < b1; b += 8u) {
+        uint2 c[8];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                if (lane >= (uint32_t)o) incl += y;
-                if (kExtras && o < 8) {
-                    const uint32_t e = __shfl_up_sync(0xFFFFFFFFu, einc, o);
-                    if (lane >= (uint32_t)o) einc += e;
-                }
-            }
-            const uint32_t start = first + incl - cnt[j].x - cnt[j].y;
-            cells[b * 32u + lane] = make_uint2(start, start + cnt[j].x);
-            const uint32_t prim_end = first + __shfl_sync(0xFFFFFFFFu, incl, 31);
-            const uint32_t end = kExtras ? prim_end + __shfl_sync(0xFFFFFFFFu, einc, NUM_EXTRA_BUCKETS - 1) : prim_end;
-            // slab ends (a slab is 16 cells, 8 lanes); the extra buckets' cursors, empty without extras
-            if ((lane & 7u) == 7u) P.cursors[b * NUM_BUCKETS + (lane >> 3)] = first + incl;
-            if (lane < NUM_EXTRA_BUCKETS)
-                P.cursors[b * NUM_BUCKETS + NUM_PRIMARY_BUCKETS + lane] = prim_end + einc - ext[j];
-            if (lane == 0) {
-                P.first[b] = first;
-                P.nprim[b] = prim_end - first;
-                P.nwx[b] = end - first;
-                if (b == total - 1) {
-                    P.counters->sorted_len = end;
-                    if (end > P.params->sorted_capacity) set_status(P.counters, STATUS_SORT_CAPACITY);
-                }
-            }
-            // the runs of kRangeChunk sorted positions that start inside this block
-            if (P.chunk_blk)
-                for (uint32_t c = (first + kRangeChunk - 1u) / kRangeChunk + lane; c * kRangeChunk < end && c < P.chunk_cap;
-                     c += 32u)
-                    P.chunk_blk[c] = b;
+        for (uint32_t j = 0; j < 8; ++j) c[j] = b + j < b1 ? __ldcg(&cells[(b + j) * 32u + lane]) : make_uint2(0u, 0u);
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) sum += c[j].x + c[j].y;
+    }
+    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+    if (lane == 0) warp_tot[wid] = sum;
+    __syncthreads();
+    if (wid == 0) {
+        const uint32_t v = warp_tot[lane];
+        uint32_t incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        warp_tot[lane] = incl - v;
+        if (lane == 31) warp_tot[32] = incl;
+    }
+    __syncthreads();
+    for (uint32_t b = counted + wid; b < total; b += 32u) write_block_empty(P, b, total, warp_tot[32], lane);
+    uint32_t first = warp_tot[wid];
+    for (uint32_t b = b0; b < b1; b += 8u) {
+        uint2 c[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) c[j] = b + j < b1 ? __ldcg(&cells[(b + j) * 32u + lane]) : make_uint2(0u, 0u);
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            if (b + j >= b1) break;
+            first = write_block_cursors<false>(P, b + j, total, first, c[j], 0u, lane);
         }
     }
 }
@@ -738,7 +802,6 @@ __global__ void __launch_bounds__(256) k_bucket_pos(DevPtrs P, const float4* __r
 
 }  // namespace
 
-int sort_launches(bool canonical) { return canonical ? 9 : 8; }
 
 void launch_sort_positions(const DevPtrs& P, const LaunchCfg& c, const float4* pos, cudaStream_t s) {
     const int g = grid_for(c.sm_count, 8);
@@ -748,7 +811,7 @@ void launch_sort_positions(const DevPtrs& P, const LaunchCfg& c, const float4* p
     k_sort_reset<<<reset_grid, 256, 0, s>>>(P, c.hash_capacity);
     k_touch_primary_pos<<<g, 256, 0, s>>>(P, pos);
     k_touch_nbh<<<g, 256, 0, s>>>(P);
-    k_block_prep<<<g, 256, 0, s>>>(P);
+    k_block_prep<kNoCells><<<g, 256, 0, s>>>(P);
     k_bucket_pos<false><<<g, 256, 0, s>>>(P, pos);
     k_scan_tiles<<<c.sm_count, kScanThreads, 0, s>>>(P);
     k_scan_apply<<<c.sm_count, kScanThreads, 0, s>>>(P);
@@ -889,6 +952,12 @@ __global__ void __launch_bounds__(256) k_rigid_finalize(DevPtrs P) {
 
 namespace fast {
 
+bool one_cta_scan(const LaunchCfg& c) { return c.block_capacity <= kOneCtaBlocks; }
+
+int sort_launches(const LaunchCfg& c, bool with_extras, bool canonical) {
+    return (canonical ? 9 : 8) - (!with_extras && one_cta_scan(c) ? 1 : 0);
+}
+
 void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool canonical, cudaStream_t s,
                  bool rigid) {
     const int per_sm = (int)c.t.sort_ctas;
@@ -911,7 +980,8 @@ void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool ca
         k_rigid_mark<<<gr, 256, 0, s>>>(P);
         k_rigid_touch<<<gr, 256, 0, s>>>(P);
     }
-    k_block_prep<<<gb, 256, 0, s>>>(P);
+    if (with_extras) k_block_prep<kAllCells><<<gb, 256, 0, s>>>(P);
+    else k_block_prep<kPrimaryCells><<<gb, 256, 0, s>>>(P);
     switch ((with_extras ? 16 : 0) + c.t.sort_batch) {
     case 2: k_count<false, 2><<<g, 256, 0, s>>>(P); break;
     case 8: k_count<false, 8><<<g, 256, 0, s>>>(P); break;
@@ -924,8 +994,12 @@ void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool ca
         k_scan_cell_tiles<true><<<scan_grid, kScanThreads, 0, s>>>(P);
         k_scan_cell_apply<true><<<scan_grid, kScanThreads, 0, s>>>(P);
     } else {
-        k_scan_cell_tiles<false><<<scan_grid, kScanThreads, 0, s>>>(P);
-        k_scan_cell_apply<false><<<scan_grid, kScanThreads, 0, s>>>(P);
+        if (one_cta_scan(c)) {
+            k_scan_cells<<<1, kOneCtaThreads, 0, s>>>(P);
+        } else {
+            k_scan_cell_tiles<false><<<scan_grid, kScanThreads, 0, s>>>(P);
+            k_scan_cell_apply<false><<<scan_grid, kScanThreads, 0, s>>>(P);
+        }
     }
     switch ((with_extras ? 16 : 0) + c.t.sort_batch) {
     case 2: k_finalize<false, 2><<<g, 256, 0, s>>>(P); break;

@@ -1055,7 +1055,7 @@ int enqueue_step(nxm_state* s, cudaStream_t st, cudaEvent_t* ev /* 5 events or n
     const bool rigid = P.nrp > 0;  // CPIC with trimesh colliders
     if (rigid) { exact::launch_rigid_transform(P, c, st); ++k; }  // pipeline.rs:393-405
     fast::launch_sort(P, c, /*with_extras=*/exact_path, /*canonical=*/s->deterministic, st, rigid);
-    k += sort_launches(s->deterministic) + (rigid ? fast::kRigidSortLaunches : 0);
+    k += fast::sort_launches(c, exact_path, s->deterministic) + (rigid ? fast::kRigidSortLaunches : 0);
     if (s->use_cpic) {  // node and particle distance fields (pipeline.rs:433-460)
         exact::launch_grid_update_cdf(P, c, st);
         if (rigid) { exact::launch_p2g_cdf(P, c, st); ++k; }
@@ -2574,7 +2574,7 @@ int nxm_debug_sort(nxm_pipeline* pipeline, nxm_state* s, int with_p2g) {
     DevPtrs P = dev_ptrs(s);
     LaunchCfg c = launch_cfg(s);
     fast::launch_sort(P, c, /*with_extras=*/true, /*canonical=*/s->deterministic, s->stream);
-    s->launches += (uint64_t)sort_launches(s->deterministic);
+    s->launches += (uint64_t)fast::sort_launches(c, /*with_extras=*/true, s->deterministic);
     s->sort_pid = s->permuted ? s->pid : nullptr;
     if (with_p2g) {
         if (s->deterministic) exact::launch_p2g_gather(P, c, s->stream);

@@ -1,7 +1,8 @@
 """The kernels at the sizes where their splits change: P2G's two rounds of 32
-cells, the cell-ordered sort list, strains of every form (series, eigenvalues, SVD), the gather P2G's stages, long and
-short canonical buckets, mesh searches with more leaves than a warp keeps,
-render data at partial warps.  Against the CPU oracle, with the bounds of
+cells, the cell-ordered sort list and its two scans, strains of every form
+(series, eigenvalues, SVD), the gather P2G's stages, long and short canonical
+buckets, mesh searches with more leaves than a warp keeps, render data at
+partial warps.  Against the CPU oracle, with the bounds of
 tests/parity.py (or bit for bit where the mode promises it)."""
 import numpy as np
 import pytest
@@ -187,3 +188,26 @@ def test_render_buffers_equal_the_records(pipe, n):
     assert np.array_equal(p.cpu().numpy(), rec["position"])
     assert np.array_equal(c.cpu().numpy(), rec["color"])
     assert np.array_equal(d.cpu().numpy().reshape(n, 3, 3), rec["deformation"][:, :3, :3])
+
+
+@pytest.mark.parametrize("capacity", [2048, 4096])
+def test_step_headers_of_both_scans(pipe, capacity):
+    """A step lists primaries only, by one kernel up to 2,048 blocks and by two
+    above: the blocks of the full sort, the same particles in each, and the
+    blocks without particles empty at the list's end."""
+    sc = scenes.elastic_cube(n_side=12)
+    step, full = (state_from_scene(sc, grid_capacity=capacity) for _ in range(2))
+    pipe.step(step)
+    pipe.debug_sort(full)
+    hs, hf = step.headers(), full.headers()
+    ids, ids_f = step.sorted_ids(), full.sorted_ids()
+    assert len(ids) == sc.n and len(hs) == len(hf)
+    by_key = {tuple(h[:3]): h for h in hf}
+    at = 0
+    for h in hs:
+        f = by_key[tuple(h[:3])]
+        assert h[3] == at and h[4] == h[5] == f[4] and h[15] == at + h[4]
+        assert sorted(ids[at:at + h[4]]) == sorted(ids_f[f[3]:f[3] + f[4]])
+        assert all((a < 0) == (b < 0) and (a < 0 or tuple(hs[a][:3]) == tuple(hf[b][:3])) for a, b in zip(h[16:], f[16:]))
+        at += h[4]
+    assert at == sc.n
