@@ -299,6 +299,84 @@ __device__ __forceinline__ Svd svd3(const m3& f) {
     return out;
 }
 
+// Fast-build small strains.  The models are functions of the symmetric matrix
+// E = F F^T - I (or of the log strain X = log(I + E) / 2), and for the strains
+// a step meets they are short power series: evaluated as polynomials of degree
+// two by the Cayley-Hamilton theorem (X^3 = i1 X^2 - i2 X + i3 I), a Horner step
+// is four multiply-adds, so no eigenvectors, and no cancellation near E = 0.
+struct Sym {
+    float xx, yy, zz, xy, xz, yz;
+};
+struct Inv {
+    float i1, i2, i3;
+};
+struct Quad {  // a I + b X + c X^2
+    float a, b, c;
+};
+__device__ __forceinline__ Sym left_strain(const m3& F) {
+    Sym r;
+    r.xx = F.c0.x * F.c0.x - 1.0f; r.yy = F.c0.y * F.c0.y - 1.0f; r.zz = F.c0.z * F.c0.z - 1.0f;
+    r.xx += F.c1.x * F.c1.x; r.yy += F.c1.y * F.c1.y; r.zz += F.c1.z * F.c1.z;
+    r.xx += F.c2.x * F.c2.x; r.yy += F.c2.y * F.c2.y; r.zz += F.c2.z * F.c2.z;
+    r.xy = F.c0.x * F.c0.y + F.c1.x * F.c1.y + F.c2.x * F.c2.y;
+    r.xz = F.c0.x * F.c0.z + F.c1.x * F.c1.z + F.c2.x * F.c2.z;
+    r.yz = F.c0.y * F.c0.z + F.c1.y * F.c1.z + F.c2.y * F.c2.z;
+    return r;
+}
+__device__ __forceinline__ float norm2(const Sym& a) {
+    return a.xx * a.xx + a.yy * a.yy + a.zz * a.zz + 2.0f * (a.xy * a.xy + a.xz * a.xz + a.yz * a.yz);
+}
+__device__ __forceinline__ Sym square(const Sym& a) {
+    return Sym{a.xx * a.xx + a.xy * a.xy + a.xz * a.xz, a.xy * a.xy + a.yy * a.yy + a.yz * a.yz,
+               a.xz * a.xz + a.yz * a.yz + a.zz * a.zz, a.xx * a.xy + a.xy * a.yy + a.xz * a.yz,
+               a.xx * a.xz + a.xy * a.yz + a.xz * a.zz, a.xy * a.xz + a.yy * a.yz + a.yz * a.zz};
+}
+__device__ __forceinline__ Inv invariants(const Sym& a) {
+    const float mx = a.yy * a.zz - a.yz * a.yz, my = a.xy * a.zz - a.yz * a.xz, mz = a.xy * a.yz - a.yy * a.xz;
+    return Inv{a.xx + a.yy + a.zz, mx + (a.xx * a.zz - a.xz * a.xz) + (a.xx * a.yy - a.xy * a.xy),
+               a.xx * mx - a.xy * my + a.xz * mz};
+}
+__device__ __forceinline__ Quad times_x(const Quad& q, const Inv& v) {
+    return Quad{q.c * v.i3, q.a - q.c * v.i2, q.b + q.c * v.i1};
+}
+__device__ __forceinline__ Quad scaled(const Quad& q, float s) { return Quad{q.a * s, q.b * s, q.c * s}; }
+__device__ __forceinline__ Sym eval(const Quad& q, const Sym& x, const Sym& x2) {
+    return Sym{q.a + q.b * x.xx + q.c * x2.xx, q.a + q.b * x.yy + q.c * x2.yy, q.a + q.b * x.zz + q.c * x2.zz,
+               q.b * x.xy + q.c * x2.xy,       q.b * x.xz + q.c * x2.xz,       q.b * x.yz + q.c * x2.yz};
+}
+__device__ __forceinline__ m3 full(const Sym& a) {
+    return mkm(mk(a.xx, a.xy, a.xz), mk(a.xy, a.yy, a.yz), mk(a.xz, a.yz, a.zz));
+}
+// exp(x) - 1 for |x| <= 0.3 (the truncated term is below 5e-8 of it).
+__device__ __forceinline__ float expm1_small(float x) {
+    return x * (1.0f + x * (0.5f + x * (1.0f / 6.0f + x * (1.0f / 24.0f + x * (1.0f / 120.0f + x * (1.0f / 720.0f))))));
+}
+constexpr float kSmallStrain2 = 0.04f;  // |E|^2 up to which the series below hold (eigenvalues within 0.2)
+// log(1 + e) / e and ((1 + e) - sqrt(1 + e)) / e on [-0.2, 0.2], interpolated at
+// Chebyshev points (relative errors 2.4e-9 and 5e-10 before rounding).
+__device__ __forceinline__ Quad log_series(const Inv& v) {
+    Quad q{-1.344796503e-01f, 0.0f, 0.0f};
+    q = times_x(q, v); q.a += 1.521727398e-01f;
+    q = times_x(q, v); q.a -= 1.663773713e-01f;
+    q = times_x(q, v); q.a += 1.997634790e-01f;
+    q = times_x(q, v); q.a -= 2.500032420e-01f;
+    q = times_x(q, v); q.a += 3.333352402e-01f;
+    q = times_x(q, v); q.a -= 4.999999902e-01f;
+    q = times_x(q, v); q.a += 9.999999976e-01f;
+    return times_x(q, v);
+}
+__device__ __forceinline__ Quad corotated_series(const Inv& v) {
+    Quad q{1.396684888e-02f, 0.0f, 0.0f};
+    q = times_x(q, v); q.a -= 1.702353984e-02f;
+    q = times_x(q, v); q.a += 2.048115793e-02f;
+    q = times_x(q, v); q.a -= 2.732067537e-02f;
+    q = times_x(q, v); q.a += 3.906279847e-02f;
+    q = times_x(q, v); q.a -= 6.250018588e-02f;
+    q = times_x(q, v); q.a += 1.249999991e-01f;
+    q = times_x(q, v); q.a += 5.000000002e-01f;
+    return times_x(q, v);
+}
+
 // Fast-build strain: eigenvalues e and vectors u (columns) of F F^T - I, by
 // cyclic Jacobi rotations of the symmetric matrix (Golub & Van Loan 8.5).  The
 // models need only functions of the left stretch, s = sqrt(1 + e) in the
@@ -541,6 +619,95 @@ __device__ __forceinline__ void dp_project_fast(const float* pl, float* state, m
     st.sm = sv - splat(1.0f);
 }
 
+// The same for a small strain E of F, and the Kirchhoff stress of a linear
+// backbone into tau.  With X = log(I + E) / 2 the return map moves X to
+// rho X + tau0 I, so F is multiplied by exp(tau0 I - kappa X), kappa = 1 - rho,
+// and the stress is 2 mu (exp(2 X') - exp(X')) + lambda (j - 1) j.
+// False, with nothing changed, where a series would not hold.
+__device__ __forceinline__ bool dp_project_small(const float* pl, float* state, m3& F, const Sym& E, float lambda, float mu,
+                                                 m3& tau) {
+    const Sym X = eval(scaled(log_series(invariants(E)), 0.5f), E, square(E));
+    const float tr = X.xx + X.yy + X.zz, third = tr * (1.0f / 3.0f);
+    const Sym dev = Sym{X.xx - third, X.yy - third, X.zz - third, X.xy, X.xz, X.yz};
+    const float dnorm2 = norm2(dev);
+    float kappa = 0.0f, tau0 = 0.0f, hard = 0.0f, dlog = 0.0f;  // unchanged
+    if (pl[4] != 0.0f) {
+        const float q = state[1];
+        const float angle = pl[0] + (pl[1] * q - pl[3]) * __expf(-pl[2] * q);
+        const float s_angle = __sinf(angle);
+        const float alpha = sqrtf(2.0f / 3.0f) * __fdividef(2.0f * s_angle, 3.0f - s_angle);
+        const float total = tr + state[2], shifted = total - pl[6];
+        if (shifted > 0.0f || dnorm2 == 0.0f) {
+            kappa = 1.0f;
+            tau0 = pl[6] * (1.0f / 3.0f);
+            hard = sqrtf(dnorm2 + total * total * (1.0f / 3.0f));
+            dlog = tr - pl[6];
+        } else {
+            const float inv = rsqrtf(dnorm2), dnorm = dnorm2 * inv;
+            const float gamma = dnorm + (3.0f * pl[4] + 2.0f * pl[5]) / (2.0f * pl[5]) * shifted * alpha;
+            if (gamma > 0.0f) {
+                kappa = gamma * inv;
+                tau0 = kappa * third + state[2] * (1.0f / 3.0f);
+                hard = gamma;
+                dlog = -state[2];
+            }
+        }
+    }
+    const float rho = 1.0f - kappa;
+    const float y = rho * tr + 3.0f * tau0;  // log of the new determinant
+    if (!(fabsf(tau0) <= 0.1f && fabsf(y) <= 0.3f && fabsf(kappa) <= 2.0f)) return false;
+    if (kappa != 0.0f) {
+        state[0] = state[0] * __expf(dlog);
+        state[1] = state[1] + hard;
+        state[2] = state[2] + dlog;
+    }
+    const Inv v = invariants(X);
+    const Sym X2 = square(X);
+    const float bm1 = expm1_small(tau0), B = 1.0f + bm1, A = B * B;
+    Quad p{1.0f / 5040.0f, 0.0f, 0.0f};  // exp(-kappa X) - I
+    p = scaled(times_x(p, v), -kappa); p.a += 1.0f / 720.0f;
+    p = scaled(times_x(p, v), -kappa); p.a += 1.0f / 120.0f;
+    p = scaled(times_x(p, v), -kappa); p.a += 1.0f / 24.0f;
+    p = scaled(times_x(p, v), -kappa); p.a += 1.0f / 6.0f;
+    p = scaled(times_x(p, v), -kappa); p.a += 0.5f;
+    p = scaled(times_x(p, v), -kappa); p.a += 1.0f;
+    p = scaled(times_x(p, v), -kappa * B);
+    p.a += bm1;
+    // exp(2 X') - exp(X'): coefficients (A 2^n - B) / n!
+    Quad t{A * (256.0f / 40320.0f) - B * (1.0f / 40320.0f), 0.0f, 0.0f};
+    t = scaled(times_x(t, v), rho); t.a += A * (128.0f / 5040.0f) - B * (1.0f / 5040.0f);
+    t = scaled(times_x(t, v), rho); t.a += A * (64.0f / 720.0f) - B * (1.0f / 720.0f);
+    t = scaled(times_x(t, v), rho); t.a += A * (32.0f / 120.0f) - B * (1.0f / 120.0f);
+    t = scaled(times_x(t, v), rho); t.a += A * (16.0f / 24.0f) - B * (1.0f / 24.0f);
+    t = scaled(times_x(t, v), rho); t.a += A * (8.0f / 6.0f) - B * (1.0f / 6.0f);
+    t = scaled(times_x(t, v), rho); t.a += A * 2.0f - B * 0.5f;
+    t = scaled(times_x(t, v), rho); t.a += A * 2.0f - B;
+    t = scaled(times_x(t, v), rho); t.a += B * bm1;
+    const float jm1 = expm1_small(y);
+    Sym k = eval(scaled(t, 2.0f * mu), X, X2);
+    const float diag_val = lambda * jm1 * (1.0f + jm1);
+    k.xx += diag_val;
+    k.yy += diag_val;
+    k.zz += diag_val;
+    tau = full(k);
+    if (kappa != 0.0f) F = F + full(eval(p, X, X2)) * F;
+    return true;
+}
+
+// Corotated linear stress of a small strain: 2 mu (b - b^(1/2)) + lambda (j -
+// 1) j with b = I + E, j^2 = det b.
+__device__ __forceinline__ m3 linear_stress_small(float lambda, float mu, const Sym& E) {
+    const Inv v = invariants(E);
+    const float d = v.i1 + v.i2 + v.i3;  // j^2 - 1
+    const float j = sqrtf(1.0f + d), jm1 = __fdividef(d, 1.0f + j);
+    Sym k = eval(scaled(corotated_series(v), 2.0f * mu), E, square(E));
+    const float diag_val = lambda * jm1 * j;
+    k.xx += diag_val;
+    k.yy += diag_val;
+    k.zz += diag_val;
+    return full(k);
+}
+
 // Snow projection (snow_project below): the stretches clamped to the elastic band.
 __device__ __forceinline__ float snow_project_fast(const float* pl, float* state, m3& F, const Strain& d, Stretch& st) {
     if (!(pl[0] <= 0.0f && pl[1] <= 0.0f)) {
@@ -614,20 +781,40 @@ struct ModelResult {
     m3 F, tau;
     v3 st;
 };
-static __device__ __noinline__ ModelResult model_update_far(uint32_t tag, const float* w, v3 st, m3 F) {
-    float s[4] = {st.x, st.y, st.z, 0.f};
+// Snow and the strains beyond the series, out of line (inline it would keep
+// registers from everything else): one eigendecomposition of F F^T - I.  The
+// square loses the smallest stretch once it is far below the largest (under 0.3
+// of it: relative error above 1e-6), so such an F takes the SVD forms.
+static __device__ __noinline__ ModelResult model_update_large(uint32_t tag, const float* w, v3 st, m3 F) {
     ModelResult r;
-    r.tau = model_update_ref(tag, w, s, F, mzero());
+    float s[4] = {st.x, st.y, st.z, 0.f};
+    const Strain d = strain_of(F);
+    const float lo = fminf(fminf(d.e.x, d.e.y), d.e.z) + 1.0f, hi = fmaxf(fmaxf(d.e.x, d.e.y), d.e.z) + 1.0f;
+    if (!(lo > 0.1f * hi)) {
+        r.tau = model_update_ref(tag, w, s, F, mzero());
+    } else {
+        Stretch x = stretch_of(d.e);
+        float lambda = w[0], mu = w[1];
+        bool linear = true;
+        if (tag == MODEL_SAND_LINEAR || tag == MODEL_SAND_NEO_HOOKEAN) {
+            dp_project_fast(&w[3], s, F, d, x);
+            lambda = w[10];
+            mu = w[11];
+            linear = tag == MODEL_SAND_LINEAR;
+        } else if (tag == MODEL_SNOW) {
+            const float hard = snow_project_fast(&w[1], s, F, d, x);
+            lambda = w[4] * hard;
+            mu = w[5] * hard;
+        }
+        r.tau = linear ? linear_stress_fast(lambda, mu, d.u, x.s, x.sm) : neo_hookean_stress(lambda, mu, F);
+    }
     r.F = F;
     r.st = mk(s[0], s[1], s[2]);
     return r;
 }
 
 // kFast selects the fast build's forms, which agree with the reference's to
-// rounding: the models with a stretch take it from one eigendecomposition of
-// F F^T - I (none decomposes a projected F again).  The square loses the
-// smallest stretch once it is far below the largest (under 0.3 of it: relative
-// error above 1e-6), so such an F takes the SVD forms, out of line.
+// rounding: sand and linear elastic at small strains by series.
 template <bool kFast>
 __device__ __forceinline__ m3 model_update(uint32_t tag, const float* w, float* st, m3& F, const m3& vel_grad) {
     if (!kFast || tag > MODEL_SNOW) return model_update_ref(tag, w, st, F, vel_grad);
@@ -636,27 +823,19 @@ __device__ __forceinline__ m3 model_update(uint32_t tag, const float* w, float* 
         return fluid_stress(&w[0], F, sr);
     }
     if (tag == MODEL_ELASTIC_NEO_HOOKEAN) return neo_hookean_stress(w[0], w[1], F);
-    const Strain d = strain_of(F);
-    const float lo = fminf(fminf(d.e.x, d.e.y), d.e.z) + 1.0f, hi = fmaxf(fmaxf(d.e.x, d.e.y), d.e.z) + 1.0f;
-    if (!(lo > 0.1f * hi)) {
-        const ModelResult r = model_update_far(tag, w, mk(st[0], st[1], st[2]), F);
-        F = r.F;
-        st[0] = r.st.x; st[1] = r.st.y; st[2] = r.st.z;
-        return r.tau;
+    if (tag != MODEL_SNOW) {
+        const Sym E = left_strain(F);
+        if (norm2(E) <= kSmallStrain2) {
+            if (tag == MODEL_ELASTIC_LINEAR) return linear_stress_small(w[0], w[1], E);
+            m3 tau;
+            if (dp_project_small(&w[3], st, F, E, w[10], w[11], tau))
+                return tag == MODEL_SAND_LINEAR ? tau : neo_hookean_stress(w[10], w[11], F);
+        }
     }
-    Stretch x = stretch_of(d.e);
-    float lambda = w[0], mu = w[1];
-    if (tag == MODEL_SAND_LINEAR || tag == MODEL_SAND_NEO_HOOKEAN) {
-        dp_project_fast(&w[3], st, F, d, x);
-        lambda = w[10];
-        mu = w[11];
-        if (tag == MODEL_SAND_NEO_HOOKEAN) return neo_hookean_stress(lambda, mu, F);
-    } else if (tag == MODEL_SNOW) {
-        const float hard = snow_project_fast(&w[1], st, F, d, x);
-        lambda = w[4] * hard;
-        mu = w[5] * hard;
-    }
-    return linear_stress_fast(lambda, mu, d.u, x.s, x.sm);
+    const ModelResult r = model_update_large(tag, w, mk(st[0], st[1], st[2]), F);
+    F = r.F;
+    st[0] = r.st.x; st[1] = r.st.y; st[2] = r.st.z;
+    return r.tau;
 }
 
 // ---------------------------------------------------------------------------
