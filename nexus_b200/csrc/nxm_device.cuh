@@ -84,6 +84,20 @@ __device__ __forceinline__ void store8(void* p, float a, float b, float c, float
                  : "memory");
 }
 
+// Asynchronous copies of 4 or 16 bytes into shared memory (this thread's own
+// slots: visible to it once its commit group is waited for).
+template <int kBytes>
+__device__ __forceinline__ void async_copy(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(kBytes)
+                 : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+
 struct quat {
     float x, y, z, w;
 };
@@ -184,6 +198,27 @@ __device__ __forceinline__ CellInfo cell_info(float dx, v3 pt) {
     c.ax = (uint32_t)__float2uint_rz(dxl);
     c.ay = (uint32_t)__float2uint_rz(dyl);
     c.az = (uint32_t)__float2uint_rz(dzl);
+    return c;
+}
+
+// cell_info without the divisions: the product with 1 / dx (within 2^-22 of the
+// quotient, relative) rounds to the same integer unless it lies that close to
+// halfway between two; then, and beyond the integers it is exact for, the
+// divisions decide.
+__device__ __forceinline__ CellInfo cell_info_near(float dx, float inv_dx, v3 pt) {
+    const v3 q = pt * inv_dx;
+    const v3 k = mk(rintf(q.x), rintf(q.y), rintf(q.z));
+    const v3 far = vabs(q - k) + vabs(q) * 4.8e-7f;
+    const float most = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z));
+    if (!(fmaxf(fmaxf(far.x, far.y), far.z) < 0.5f && most < 1.0e6f)) return cell_info(dx, pt);
+    const int x = (int)k.x - 1, y = (int)k.y - 1, z = (int)k.z - 1;
+    CellInfo c;
+    c.bx = x >> 2;
+    c.by = y >> 2;
+    c.bz = z >> 2;
+    c.ax = (uint32_t)(x & 3);
+    c.ay = (uint32_t)(y & 3);
+    c.az = (uint32_t)(z & 3);
     return c;
 }
 

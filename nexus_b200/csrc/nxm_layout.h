@@ -154,7 +154,9 @@ struct alignas(16) Params {
     // the fast G2P takes one block per unit (instead of runs of the sorted
     // list) below this many particles per primary block on average (tuned)
     uint32_t range_min_fill;
-    uint32_t pad[3];
+    float inv_d;             // 4 / dx^2
+    float speed_limit2;      // (dx / dt)^2
+    uint32_t pad;
 };
 static_assert(sizeof(Params) == 96, "Params layout");
 

@@ -382,6 +382,7 @@ struct nxm_state {
 
     // materials (deduplicated model words)
     std::vector<Material> materials;
+    bool has_state = false;  // some material has model state words
     std::map<std::vector<uint32_t>, uint32_t> material_index;
     Material* d_materials = nullptr;
     uint32_t mat_cap = 0;
@@ -536,6 +537,7 @@ DevPtrs dev_ptrs(nxm_state* s) {
         P.pid_out = nullptr;
     }
     P.materials = s->d_materials;
+    P.has_state = s->has_state;
     P.colliders = s->d_colliders;
     P.pscene = s->d_pscene;
     P.ncdf = s->d_ncdf;
@@ -980,6 +982,10 @@ uint32_t material_of(nxm_state* s, const nxm_particle_model& m) {
     mat.tag = m.tag;
     mat.has_state = model_has_state(m.tag) ? 1u : 0u;
     for (int k = 0; k < MODEL_WORDS; ++k) mat.w[k] = bits_f(key[1 + k]);
+    if (mat.has_state && !s->has_state) {
+        s->has_state = true;
+        invalidate_graph(s);
+    }
     const uint32_t idx = (uint32_t)s->materials.size();
     s->materials.push_back(mat);
     s->material_index.emplace(std::move(key), idx);
@@ -1022,6 +1028,8 @@ int sync_params(nxm_state* s) {
     p.dt = s->dt;
     p.dx = s->dx;
     p.inv_dx = 1.0f / s->dx;
+    p.inv_d = 4.0f / (s->dx * s->dx);
+    p.speed_limit2 = (s->dx / s->dt) * (s->dx / s->dt);
     p.n = s->n;
     p.ncol = (uint32_t)s->colliders.size();
     p.block_capacity = std::min(s->block_cap, kMaxBlocks);

@@ -275,23 +275,68 @@ constexpr uint32_t kG2pThreads = NXM_G2P_THREADS;  // threads per G2P CTA
 // block (shared memory), then advects, updates F and the model, and writes the
 // particle (read from slot `src`, xm / vf = its first two kin words) to slot
 // `dst` of the output records, together with the block key of its new position.
-// The fast build takes the particle's cell from the sort: `vid` is its block,
-// `cell` its associated cell there.
+// The fast build takes the particle's cell from the sort: its block's
+// coordinates (in its scene) and its associated cell there.
 // kCpicBlock: the CPIC branches (a block whose halo carries affinity bits);
 // the plain instantiation serves every other block without their registers.
-template <bool kCpicBlock>
+// kSlots: `slots` holds 68 bytes a thread of shared memory: the deformation
+// record, the model state and the id come there by asynchronous copies while the
+// gather runs (instead of waiting in registers), and m A waits there across the
+// model update.
+struct G2pSlots {
+    float4 a[kG2pThreads], b[kG2pThreads], c[kG2pThreads];
+    float4 st[kG2pThreads];  // model state words, where any material has some (P.has_state)
+    uint32_t id[kG2pThreads];
+};
+__device__ __forceinline__ float4 reload(const float4* p) {  // a shared-memory read that stays one
+    float4 r;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+    return r;
+}
+// Where a particle's block is told from: its coordinates and key offset as
+// values, or in shared memory, read when they are needed.
+struct BlockHere {
+    int4 v;
+    int3 k;
+    __device__ __forceinline__ int4 vid() const { return v; }
+    __device__ __forceinline__ int3 key() const { return k; }
+};
+struct BlockStaged {
+    const int4* v;
+    const int4* k;
+    __device__ __forceinline__ int4 vid() const { return *v; }
+    __device__ __forceinline__ int3 key() const {
+        const float4 r = reload(reinterpret_cast<const float4*>(k));
+        return make_int3(__float_as_int(r.x), __float_as_int(r.y), __float_as_int(r.z));
+    }
+};
+template <bool kCpicBlock, bool kSlots, class Block>
 __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm, const float4* __restrict__ halo,
-                                             uint32_t src, uint32_t dst, float4 xm, float4 vf, int4 vid, uint32_t cell,
-                                             int3 key_off, const CpicCtx& cx, volatile float* stash) {
+                                             uint32_t src, uint32_t dst, float4 xm, uint32_t flags, const Block& block,
+                                             uint32_t cell, const CpicCtx& cx, volatile float* stash,
+                                             G2pSlots* slots) {
     const float dx = prm.dx, dt = prm.dt;
-    const float inv_d = 4.0f / (dx * dx);
-    const float lim2 = (dx / dt) * (dx / dt);
-    uint32_t flags = __float_as_uint(vf.w);
+    const float inv_d = prm.inv_d;
     const v3 pt = mk(xm.x, xm.y, xm.z);
     float mass = xm.w;
-    // the deformation record, loaded ahead of the gather
-    const float4 pm = *reinterpret_cast<const float4*>(&P.in.mat[src]);  // F's last, V0, damping, material
-    m3 F = def_grad_of(P.in, src, pm.x);
+    // the deformation record, fetched ahead of the gather; pm: F's last, V0, damping, material
+    float4 pm;
+    m3 F;
+    if (kSlots) {
+        const float4* f = reinterpret_cast<const float4*>(&P.in.def[src]);
+        async_copy<16>(&slots->a[threadIdx.x], f);
+        async_copy<16>(&slots->b[threadIdx.x], f + 1);
+        async_copy<16>(&slots->c[threadIdx.x], &P.in.mat[src]);
+        async_copy<4>(&slots->id[threadIdx.x], &P.pid_in[src]);
+        if (P.has_state) async_copy<16>(&slots->st[threadIdx.x], &P.in.pstate[src]);
+        async_commit();
+    } else {
+        pm = *reinterpret_cast<const float4*>(&P.in.mat[src]);
+        F = def_grad_of(P.in, src, pm.x);
+    }
 
 #if NXM_CPIC
     // particle Cdf (normal, signed distance, affinity) from this step's g2p_cdf pass
@@ -309,7 +354,6 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
 #else
     (void)cx;
 #endif
-    (void)vid;
     (void)cell;
     // ---- G2P (g2p.rs:150-270)
     v3 velocity = splat(0.f);
@@ -325,52 +369,38 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
         // Same sums, factored: with dpt_i = ref + s_i dx,
         //   grad = inv_d (v (x) ref + dx [Sx Sy Sz]),  S_a = sum_i w_i v_i s_i,a
         //   vgd  = inv_d (v . ref + dx (Sx.x + Sy.y + Sz.z))
-        // so each node costs one weight product and (1 + nonzero s) FMA pairs:
-        // the x, y components accumulate as packed f32x2 (FFMA2), z on its own.
+        // and, the weights being products, summed along x, then y, then z: 240
+        // multiply-adds (a weight product per node and the three moments summed
+        // over the 27 nodes take 310).
         const float inv_dx = prm.inv_dx;
         const uint32_t ax = cell & 3u, ay = (cell >> 2) & 3u, az = cell >> 4;
-        v3 ref = mk((float)((vid.x - key_off.x) * 4 + (int)ax), (float)((vid.y - key_off.y) * 4 + (int)ay),
-                    (float)((vid.z - key_off.z) * 4 + (int)az)) * dx - pt;
+        const int4 vid = block.vid();  // scene-local
+        v3 ref = mk((float)(vid.x * 4 + (int)ax), (float)(vid.y * 4 + (int)ay), (float)(vid.z * 4 + (int)az)) * dx - pt;
         // a block beyond the packed keys' range carries the aliased coordinates
         if (fmaxf(fmaxf(fabsf(ref.x), fabsf(ref.y)), fabsf(ref.z)) > 4.0f * dx) ref = assoc_cell_of(dx, pt) * dx - pt;
         const v3 wx = kernel_eval_all(-ref.x * inv_dx);
         const v3 wy = kernel_eval_all(-ref.y * inv_dx);
         const v3 wz = kernel_eval_all(-ref.z * inv_dx);
-        const uint32_t packed = ax + 6u * ay + 36u * az;
-        float2 vxy = make_float2(0.f, 0.f), sxxy = vxy, syxy = vxy, szxy = vxy;
-        float vz = 0.f, sxz = 0.f, syz = 0.f, szz = 0.f;
+        const float wx2 = 2.0f * wx.z, wy2 = 2.0f * wy.z, wz2 = 2.0f * wz.z;
+        const float4* node = halo + ax + 6u * ay + 36u * az;
+        v3 sxv = splat(0.f), syv = sxv, szv = sxv;
 #pragma unroll
-        for (int sz = 0; sz < 3; ++sz) {
+        for (int k = 0; k < 3; ++k) {
+            v3 a = splat(0.f), bx = a, by = a;
 #pragma unroll
-            for (int sy = 0; sy < 3; ++sy) {
-                const float wyz = vget(wy, sy) * vget(wz, sz);
-#pragma unroll
-                for (int sx = 0; sx < 3; ++sx) {
-                    const float4 h = halo[packed + (uint32_t)(sx + 6 * sy + 36 * sz)];
-                    const float2 hxy = make_float2(h.x, h.y);
-                    const float w = vget(wx, sx) * wyz;
-                    vxy = __ffma2_rn(make_float2(w, w), hxy, vxy);
-                    vz = fmaf(w, h.z, vz);
-                    if (sx) {
-                        const float ws = w * (float)sx;
-                        sxxy = __ffma2_rn(make_float2(ws, ws), hxy, sxxy);
-                        sxz = fmaf(ws, h.z, sxz);
-                    }
-                    if (sy) {
-                        const float ws = w * (float)sy;
-                        syxy = __ffma2_rn(make_float2(ws, ws), hxy, syxy);
-                        syz = fmaf(ws, h.z, syz);
-                    }
-                    if (sz) {
-                        const float ws = w * (float)sz;
-                        szxy = __ffma2_rn(make_float2(ws, ws), hxy, szxy);
-                        szz = fmaf(ws, h.z, szz);
-                    }
-                }
+            for (int j = 0; j < 3; ++j) {
+                const float4 h0 = node[6 * j + 36 * k], h1 = node[1 + 6 * j + 36 * k], h2 = node[2 + 6 * j + 36 * k];
+                const v3 s0 = mk(h0.x, h0.y, h0.z) * wx.x + mk(h1.x, h1.y, h1.z) * wx.y + mk(h2.x, h2.y, h2.z) * wx.z;
+                const v3 s1 = mk(h1.x, h1.y, h1.z) * wx.y + mk(h2.x, h2.y, h2.z) * wx2;
+                a = a + s0 * vget(wy, j);
+                bx = bx + s1 * vget(wy, j);
+                if (j) by = by + s0 * (j == 1 ? wy.y : wy2);
             }
+            velocity = velocity + a * vget(wz, k);
+            sxv = sxv + bx * vget(wz, k);
+            syv = syv + by * vget(wz, k);
+            if (k) szv = szv + a * (k == 1 ? wz.y : wz2);
         }
-        velocity = mk(vxy.x, vxy.y, vz);
-        const v3 sxv = mk(sxxy.x, sxxy.y, sxz), syv = mk(syxy.x, syxy.y, syz), szv = mk(szxy.x, szxy.y, szz);
         grad = (outer(velocity, ref) + mkm(sxv, syv, szv) * dx) * inv_d;
         vgd = (dot(velocity, ref) + dx * (sxv.x + syv.y + szv.z)) * inv_d;
     } else if (flags & PFLAG_ENABLED) {
@@ -421,6 +451,12 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
 #endif
 
     // ---- particle update (particle_update.rs:60-201, non-CPIC: Cdf = 0)
+    if (kSlots) {
+        async_wait<0>();
+        const float4 f0 = slots->a[threadIdx.x], f1 = slots->b[threadIdx.x];
+        pm = slots->c[threadIdx.x];
+        F = mkm(mk(f0.x, f0.y, f0.z), mk(f0.w, f1.x, f1.y), mk(f1.z, f1.w, pm.x));
+    }
     const float init_volume = pm.y, damping = pm.z;
     const uint32_t mid = __float_as_uint(pm.w);
     const Material& mat = P.materials[mid];
@@ -433,7 +469,7 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
 #endif
     if (NXM_FAST) {
         // the square root only near or above the limit
-        if (dot(v, v) > 0.999f * lim2) {
+        if (dot(v, v) > 0.999f * prm.speed_limit2) {
             const float vl = length(v);
             if (vl > dx / dt) v = ((v / vl) * dx) / dt;
         }
@@ -457,7 +493,8 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
     const bool nan = (np_.x != np_.x) || (np_.y != np_.y) || (np_.z != np_.z);
     store8(&P.out.kin[dst], np_.x, np_.y, np_.z, mass, v.x, v.y, v.z, __uint_as_float(flags));
     {
-        const CellInfo nc = cell_info(dx, np_);
+        const CellInfo nc = NXM_FAST ? cell_info_near(dx, prm.inv_dx, np_) : cell_info(dx, np_);
+        const int3 key_off = block.key();
         P.pcode[dst] = make_uint2(pack_key(nc.bx + key_off.x, nc.by + key_off.y, nc.bz + key_off.z),
                                   nc.ax | (nc.ay << 2) | (nc.az << 4));
     }
@@ -473,11 +510,20 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
     }
     float st[4] = {0.f, 0.f, 0.f, 0.f};
     if (mat.has_state) {
-        float4 s4 = P.in.pstate[src];
+        const float4 s4 = kSlots ? slots->st[threadIdx.x] : P.in.pstate[src];
         st[0] = s4.x; st[1] = s4.y; st[2] = s4.z; st[3] = s4.w;
     }
     m3 aff;
-    if (stash && tag != MODEL_FLUID) {
+    if (kSlots && tag != MODEL_FLUID) {
+        const m3 am = A * mass;
+        slots->a[threadIdx.x] = make_float4(am.c0.x, am.c0.y, am.c0.z, am.c1.x);
+        slots->b[threadIdx.x] = make_float4(am.c1.y, am.c1.z, am.c2.x, am.c2.y);
+        slots->c[threadIdx.x].x = am.c2.z;
+        const m3 tau = model_update<NXM_FAST>(tag, mat.w, st, F, mzero());
+        const float4 a = reload(&slots->a[threadIdx.x]), b = reload(&slots->b[threadIdx.x]);
+        const float4 c = reload(&slots->c[threadIdx.x]);
+        aff = mkm(mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x)) - tau * (init_volume * inv_d * dt);
+    } else if (!kSlots && stash && tag != MODEL_FLUID) {
         // m A waits in this thread's shared-memory slots (stride kG2pThreads) across
         // the model update instead of in registers
         const m3 am = A * mass;
@@ -500,9 +546,11 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
         aff = mzero();
         // the fast build always writes to the other buffer: the old position
         // is re-read there instead of staying live across the model update
-        const v3 op = NXM_FAST ? mk(P.in.kin[src].x, P.in.kin[src].y, P.in.kin[src].z) : pt;
+        const uint32_t from = kSlots ? P.sorted[dst] : src;
+        const v3 op = NXM_FAST ? mk(P.in.kin[from].x, P.in.kin[from].y, P.in.kin[from].z) : pt;
         store8(&P.out.kin[dst], op.x, op.y, op.z, 0.f, 0.f, 0.f, 0.f, __uint_as_float(flags));
         const CellInfo oc = cell_info(dx, op);
+        const int3 key_off = block.key();
         P.pcode[dst] = make_uint2(pack_key(oc.bx + key_off.x, oc.by + key_off.y, oc.bz + key_off.z),
                                   oc.ax | (oc.ay << 2) | (oc.az << 4));
     }
@@ -511,7 +559,8 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
     store8(&P.out.def[dst], F.c0.x, F.c0.y, F.c0.z, F.c1.x, F.c1.y, F.c1.z, F.c2.x, F.c2.y);
     *reinterpret_cast<float4*>(&P.out.mat[dst]) = make_float4(F.c2.z, init_volume, damping, pm.w);
     if (mat.has_state) P.out.pstate[dst] = make_float4(st[0], st[1], st[2], st[3]);
-    if (P.pid_in) P.pid_out[dst] = P.pid_in[src];
+    if (kSlots) P.pid_out[dst] = slots->id[threadIdx.x];
+    else if (P.pid_in) P.pid_out[dst] = P.pid_in[src];
 }
 
 // dynamics/body.rs Velocity::integrate for one-way coupled bodies
@@ -580,8 +629,11 @@ __device__ __forceinline__ void g2p_finish(const DevPtrs& P, const Params& prm) 
     if (blockIdx.x == 0 && threadIdx.x == 0) P.counters->codes_valid = 1u;
 }
 
+// CTAs per SM the register budget is sized for: at 4 (64 registers) the spills
+// around the constitutive update cost more than the fourth CTA's latency hiding
+// gives (2 M sand + water: 156 us at 4, 145 us at 3; 48 small scenes 121, 111).
 #ifndef NXM_G2P_MIN_CTAS
-#define NXM_G2P_MIN_CTAS 4  // CTAs per SM the register budget is sized for
+#define NXM_G2P_MIN_CTAS 3
 #endif
 
 // One CTA per primary block (ids [0, num_primary); the other blocks hold no
@@ -608,6 +660,7 @@ __device__ __forceinline__ bool g2p_sparse(const DevPtrs& P, const Params& prm) 
     return (uint64_t)len < (uint64_t)prm.range_min_fill * nbp;
 }
 
+#if !NXM_FAST || NXM_CPIC
 // The per-block loop: one CTA per primary block (grid-stride), halo of 216
 // nodes in `halo` (CPIC: the incompatible fields and node distance field in
 // halo_inc / halo_cdf).
@@ -636,8 +689,9 @@ __device__ __forceinline__ void g2p_block_loop(const DevPtrs& P, const Params& p
             nnp = __ldcg(&P.nprim[bn]);
         }
         const bool reorder = P.pid_in != nullptr;
-        const int4 vid = P.bvid[b];
-        const int3 key_off = scene_base_of_block(prm, vid);
+        BlockHere block{P.bvid[b], make_int3(0, 0, 0)};
+        block.k = scene_base_of_block(prm, block.v);
+        block.v.x -= block.k.x; block.v.y -= block.k.y; block.v.z -= block.k.z;
         uint32_t pid = tid < np ? __ldg(&P.sorted[first + tid]) : NONE;
         const uint32_t hblk = (tid < 216u && hoct != 0u) ? __ldg(&P.nbh[b * NUM_NBH + hoct - 1u]) : b;
         float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), vf = xm;
@@ -705,10 +759,12 @@ __device__ __forceinline__ void g2p_block_loop(const DevPtrs& P, const Params& p
             const uint32_t cell = NXM_FAST ? __ldcg(&P.phdr[pid]) & 63u : 0u;
 #if NXM_CPIC
             if (cx.halo_cdf)
-                g2p_particle<true>(P, prm, halo, pid, reorder ? first + k : pid, xm, vf, vid, cell, key_off, cx, stash);
+                g2p_particle<true, false>(P, prm, halo, pid, reorder ? first + k : pid, xm, __float_as_uint(vf.w), block,
+                                          cell, cx, stash, nullptr);
             else
 #endif
-                g2p_particle<false>(P, prm, halo, pid, reorder ? first + k : pid, xm, vf, vid, cell, key_off, cx, stash);
+                g2p_particle<false, false>(P, prm, halo, pid, reorder ? first + k : pid, xm, __float_as_uint(vf.w), block,
+                                           cell, cx, stash, nullptr);
         }
         __syncthreads();
         b = bn;
@@ -738,12 +794,12 @@ __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_update(De
     g2p_finish(P, prm);
 }
 
+#endif
+
 #if NXM_FAST && !NXM_CPIC
-// ---- bulk (TMA) copies of node blocks into shared memory -------------------
-// One elected thread issues 1-D cp.async.bulk copies of whole 1 KB node
-// blocks (global memory of this GPU only, no multicast) that complete on an
-// mbarrier in shared memory; every thread then waits on the barrier's phase,
-// with an iteration limit after which the kernel records
+// ---- a copy-barrier wait with an iteration limit ----------------------------
+// An mbarrier in shared memory that bulk copies would complete on; a wait on
+// its phase gives up after `limit` rounds, so that a kernel can record
 // STATUS_COPY_TIMEOUT instead of waiting on.
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar) {
@@ -752,12 +808,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar) {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
 }
 // Waits for the barrier's phase `parity` to complete; false when the limit ran out.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit) {
@@ -772,56 +822,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     }
     return false;
 }
-constexpr uint32_t kCopyWaitLimit = 1u << 20;  // try_wait rounds (each may suspend a few us): over a second
 
-// Stages the 6x6x6 node-velocity halos of blocks [b, b + cnt) into `halo`
-// by bulk copies: per group of kTmaGroup blocks, thread 0 copies the 8 node
-// blocks each halo draws from (the block and its 7 +1 neighbours; a missing
-// one from the zero block after the grid, index block_capacity) into `raw`,
-// 8 KB a block, completing on the CTA's barrier; every thread waits for the
-// phase, then the CTA rearranges them into halo order.  Ends with a CTA
-// barrier.
-constexpr uint32_t kTmaGroup = 2;
-__device__ __forceinline__ void stage_halos_tma(const DevPtrs& P, uint32_t b, uint32_t cnt, float4* halo, float4* raw,
-                                                uint64_t* bar, uint32_t& parity, uint32_t zero_blk) {
-    const uint32_t tid = threadIdx.x;
-    for (uint32_t g0 = 0; g0 < cnt; g0 += kTmaGroup) {
-        const uint32_t gc = min(cnt - g0, kTmaGroup);
-        if (tid == 0) {
-            // the raw area was last read by the generic proxy (the previous group's rearrangement)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(bar, gc * 8u * 1024u);
-            for (uint32_t j = 0; j < gc; ++j) {
-                const uint32_t blk = b + g0 + j;
-                uint32_t nb[7];
-#pragma unroll
-                for (uint32_t o = 0; o < 7; ++o) nb[o] = __ldcg(&P.nbh[blk * NUM_NBH + o]);
-                bulk_copy_g2s(raw + (j * 8u) * 64u, P.nodes + (size_t)blk * 64u, 1024u, bar);
-#pragma unroll
-                for (uint32_t o = 1; o < 8; ++o) {
-                    const uint32_t src = nb[o - 1] == NONE ? zero_blk : nb[o - 1];
-                    bulk_copy_g2s(raw + (j * 8u + o) * 64u, P.nodes + (size_t)src * 64u, 1024u, bar);
-                }
-            }
-        }
-        if (!mbar_wait(bar, parity, kCopyWaitLimit)) {
-            if (tid == 0) set_status(P.counters, STATUS_COPY_TIMEOUT);
-            mbar_wait(bar, parity, kCopyWaitLimit);  // the copies may still be in flight: wait once more
-        }
-        parity ^= 1u;
-        for (uint32_t t = tid; t < gc * 216u; t += blockDim.x) {
-            const uint32_t j = t / 216u, node = t - 216u * j;
-            const uint32_t tx = node % 6u, ty = (node / 6u) % 6u, tz = node / 36u;
-            const uint32_t ox = tx >= 4u, oy = ty >= 4u, oz = tz >= 4u;
-            const uint32_t oct = ox * 4u + oy * 2u + oz;
-            const float4 nd = raw[(j * 8u + oct) * 64u + (tx - 4u * ox) + 4u * (ty - 4u * oy) + 16u * (tz - 4u * oz)];
-            halo[(g0 + j) * 216u + node] = make_float4(nd.x, nd.y, nd.z, 0.f);
-        }
-        __syncthreads();  // raw is free again; the halos are complete
-    }
-}
-
-// The wait above, made to run out: a barrier that expects bytes no copy will
+// The wait made to run out: a barrier that expects bytes no copy will
 // deliver (nothing is issued), waited on with `limit` rounds; the kernel
 // records STATUS_COPY_TIMEOUT and returns with no copy in flight.
 __global__ void k_copy_wait_timeout(Counters* counters, uint32_t limit) {
@@ -855,113 +857,102 @@ __global__ void k_copy_wait_timeout(Counters* counters, uint32_t limit) {
 // Neighbouring positions are particles of the same cell or the next, so a
 // warp's halo reads are mostly broadcasts.
 //
-// Halo staging: plain loads by every thread (each node: its block id from the
-// neighbour table, then the node, both L2 hits) by default; with
-// NXM_G2P_TMA_HALO the bulk copies of stage_halos_tma instead (measured
-// slower on the 2 M-particle scene: the rearrangement pass and its barriers
-// cost more than the loads they replace).
-#ifndef NXM_G2P_TMA_HALO
-#define NXM_G2P_TMA_HALO 0
-#endif
+// Bound by instruction issue and the latency of a run's first loads; 2 M sand +
+// water particles: 190 us with the 27-node gather, the eigendecomposition of
+// every strain and records held in registers, 145 us now (0.25 GB, 1.7 TB/s).
+//
+// Halo staging: every thread below 216 loads one node of each staged block
+// (its block id from the neighbour table, then the node, both L2 hits).
 constexpr uint32_t kRangeHalos = 8;
 static_assert(kG2pThreads == kRangeChunk, "one sorted position per thread");
-#if NXM_G2P_TMA_HALO
-constexpr size_t kG2pRangeSmem = (size_t)kRangeHalos * 216 * 16 + (size_t)kTmaGroup * 8 * 64 * 16 +
-                                 (size_t)9 * 4 * kG2pThreads + 16;
-#endif
 __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_range(DevPtrs P) {
-#if NXM_G2P_TMA_HALO
-    extern __shared__ float4 g2p_smem[];
-    float4* halo = g2p_smem;                 // kRangeHalos x 216 nodes
-    float4* raw = halo + kRangeHalos * 216;  // kTmaGroup x 8 node blocks
-    float* stash_mem = reinterpret_cast<float*>(raw + kTmaGroup * 8 * 64);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(stash_mem + 9 * kG2pThreads);
-    if (threadIdx.x == 0) mbar_init(bar);
-    __syncthreads();
-    uint32_t parity = 0;
-    const uint32_t zero_blk = P.params->block_capacity;
-#else
     __shared__ float4 halo[kRangeHalos * 216];
-    __shared__ float stash_mem[9 * kG2pThreads];
-#endif
-#if NXM_G2P_STASH
-    volatile float* stash = stash_mem + threadIdx.x;
-#else
-    volatile float* stash = nullptr;
-#endif
-    const Params prm = *P.params;
+    __shared__ G2pSlots slots;
+    __shared__ int4 svid[kRangeHalos], skey[kRangeHalos];  // the staged blocks' coordinates and key offsets
+    // the parameters are read from shared memory where they are used: in
+    // registers they would push the particle's own values out to local memory
+    __shared__ Params prm;
+    if (threadIdx.x < sizeof(Params) / 4)
+        reinterpret_cast<uint32_t*>(&prm)[threadIdx.x] = reinterpret_cast<const uint32_t*>(P.params)[threadIdx.x];
+    __syncthreads();
     integrate_colliders(P, prm);
     const uint32_t nbp = min(__ldcg(&P.counters->num_primary), __ldcg(&P.counters->num_blocks));
     const uint32_t len = min(__ldcg(&P.counters->sorted_len), prm.n);
     const bool sparse = g2p_sparse(P, prm);
     const uint32_t nunits = !nbp ? 0u : (sparse ? nbp : min((len + kRangeChunk - 1u) / kRangeChunk, P.chunk_cap));
     const uint32_t tid = threadIdx.x;
-    const bool reorder = P.pid_in != nullptr;
+    // this thread's halo node: its octant and its place in that block
+    const uint32_t htx = tid % 6u, hty = (tid / 6u) % 6u, htz = tid / 36u;
+    const uint32_t hox = htx >= 4u, hoy = hty >= 4u, hoz = htz >= 4u;
+    const uint32_t hnode = (hox * 4u + hoy * 2u + hoz) << 8 | ((htx - 4u * hox) + 4u * (hty - 4u * hoy) + 16u * (htz - 4u * hoz));
     const CpicCtx cx{nullptr, nullptr, P.colliders, 0u};
-    // unit u: blocks [lo, hi], sorted positions [p0, p1), from two loaded
-    // words (dense: the run's first and last block; sparse: first, nprim of
-    // the block), loaded one unit ahead
-    auto words_of = [&](uint32_t u, uint32_t& a, uint32_t& b) {
+    // unit u: blocks [x, y], sorted positions [z, w), from two loaded words
+    // (dense: the run's first and last block; sparse: first, nprim of the
+    // block), loaded one unit ahead by one thread (a ring of four: others may
+    // still look at the previous unit)
+    __shared__ uint4 unit[4];
+    const auto unit_of = [&](uint32_t u) {
+        uint4 r = make_uint4(0u, 0u, 0u, 0u);
+        if (u >= nunits) return r;
         if (sparse) {
-            a = __ldcg(&P.first[u]);
-            b = __ldcg(&P.nprim[u]);
+            r.x = r.y = u;
+            r.z = __ldcg(&P.first[u]);
+            r.w = min(r.z + __ldcg(&P.nprim[u]), len);
         } else {
-            a = __ldcg(&P.chunk_blk[u]);
-            b = u + 1u < nunits ? __ldcg(&P.chunk_blk[u + 1u]) : nbp - 1u;
+            r.x = __ldcg(&P.chunk_blk[u]);
+            r.y = min(u + 1u < nunits ? __ldcg(&P.chunk_blk[u + 1u]) : nbp - 1u, nbp - 1u);
+            r.z = u * kRangeChunk;
+            r.w = min(r.z + kRangeChunk, len);
         }
+        return r;
     };
-    uint32_t u = blockIdx.x, wa = 0u, wb = 0u;
-    if (u < nunits) words_of(u, wa, wb);
-    for (; u < nunits; u += gridDim.x) {
-        uint32_t lo, hi, p0, p1;
-        if (sparse) {
-            lo = hi = u;
-            p0 = wa;
-            p1 = min(wa + wb, len);
-        } else {
-            lo = wa;
-            hi = min(wb, nbp - 1u);
-            p0 = u * kRangeChunk;
-            p1 = min(p0 + kRangeChunk, len);
-        }
-        if (u + gridDim.x < nunits) words_of(u + gridDim.x, wa, wb);
+    if (tid == 0) unit[0] = unit_of(blockIdx.x);
+    __syncthreads();
+    uint32_t slot = 0u;
+    for (uint32_t u = blockIdx.x; u < nunits; u += gridDim.x, slot = (slot + 1u) & 3u) {
+        if (tid == 0) unit[(slot + 1u) & 3u] = unit_of(u + gridDim.x);
+        const uint4 cur = unit[slot];
         // this thread's first particle, fetched while the halos load
-        uint32_t pid = p0 + tid < p1 ? __ldg(&P.sorted[p0 + tid]) : NONE;
-        float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), vf = xm;
-        uint32_t home = lo << 6;  // the particle's block and cell
-        if (pid != NONE) {
-            const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
-            xm = kr[0];
-            vf = kr[1];
+        uint32_t pid = cur.z + tid < cur.w ? __ldg(&P.sorted[cur.z + tid]) : NONE;
+        float4 xm = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t flags = 0u, home = cur.x << 6;  // home: the particle's block and cell
+        const auto load_head = [&] {
+            xm = *reinterpret_cast<const float4*>(&P.in.kin[pid]);
+            flags = __float_as_uint(P.in.kin[pid].flags);
             home = __ldcg(&P.phdr[pid]);
-        }
+        };
+        if (pid != NONE) load_head();
         bool pending = pid != NONE;  // dense: this thread's one particle not yet updated
-        for (uint32_t b = lo; b <= hi; b += kRangeHalos) {
-            const uint32_t cnt = min(hi - b + 1u, kRangeHalos);
-#if NXM_G2P_TMA_HALO
-            stage_halos_tma(P, b, cnt, halo, raw, bar, parity, zero_blk);
-#else
-            for (uint32_t t = tid; t < cnt * 216u; t += kG2pThreads) {
-                const uint32_t i = t / 216u;
-                halo[t] = halo_node(P, b + i, t - 216u * i);
+        for (uint32_t b = cur.x; b <= unit[slot].y; b += kRangeHalos) {
+            const uint32_t cnt = min(unit[slot].y - b + 1u, kRangeHalos);
+            if (tid >= kG2pThreads - kRangeHalos && tid - (kG2pThreads - kRangeHalos) < cnt) {  // no halo node of theirs
+                const uint32_t i = tid - (kG2pThreads - kRangeHalos);
+                const int4 v = P.bvid[b + i];
+                const int3 o = scene_base_of_block(prm, v);
+                svid[i] = make_int4(v.x - o.x, v.y - o.y, v.z - o.z, v.w);
+                skey[i] = make_int4(o.x, o.y, o.z, 0);
+            }
+            if (tid < 216u) {
+                const uint32_t oct = hnode >> 8, at = hnode & 255u;
+#pragma unroll 2
+                for (uint32_t i = 0; i < cnt; ++i) {
+                    const uint32_t blk = oct ? __ldg(&P.nbh[(b + i) * NUM_NBH + oct - 1u]) : b + i;
+                    float4 nd = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (blk != NONE) nd = P.nodes[blk * 64u + at];
+                    halo[216u * i + tid] = nd;
+                }
             }
             __syncthreads();
-#endif
             // dense: one position per thread; sparse: the block's positions in rounds
-            for (uint32_t p = p0 + tid; p < p1; p += kG2pThreads) {
-                if (p != p0 + tid) {
+            for (uint32_t p = unit[slot].z + tid; p < unit[slot].w; p += kG2pThreads) {
+                if (p >= unit[slot].z + kG2pThreads) {
                     pid = __ldg(&P.sorted[p]);
-                    const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
-                    xm = kr[0];
-                    vf = kr[1];
-                    home = __ldcg(&P.phdr[pid]);
+                    load_head();
                 }
-                const uint32_t blk = home >> 6;
-                if (blk >= b && blk - b < cnt) {
-                    const int4 vid = P.bvid[blk];
-                    const int3 key_off = scene_base_of_block(prm, vid);
-                    g2p_particle<false>(P, prm, halo + 216u * (blk - b), pid, reorder ? p : pid, xm, vf, vid, home & 63u,
-                                        key_off, cx, stash);
+                const uint32_t at = (home >> 6) - b;
+                if (at < cnt) {
+                    g2p_particle<false, true>(P, prm, halo + 216u * at, pid, p, xm, flags,
+                                              BlockStaged{svid + at, skey + at}, home & 63u, cx, nullptr, &slots);
                     pending = false;
                 }
             }
@@ -981,6 +972,8 @@ void launch_copy_wait_timeout(Counters* counters, uint32_t limit, cudaStream_t s
 }
 #endif
 
+// Grids stop at what the state's capacities can use: a CTA a block, or a run of
+// the sorted list each (a small scene's launch is mostly the start of its CTAs).
 void launch_grid_update(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
     // grid_ctas counts CTAs of 256 threads
     const uint32_t most = (uint32_t)c.sm_count * c.t.grid_ctas * (256 / kGridThreads);
@@ -988,20 +981,14 @@ void launch_grid_update(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
 }
 
 int launch_g2p_update(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
-#if NXM_FAST && !NXM_CPIC && !defined(NXM_G2P_PER_BLOCK)
-    if (P.chunk_blk) {  // runs of the sorted list, or one block per unit over sparse blocks
-#if NXM_G2P_TMA_HALO
-        cudaFuncSetAttribute(k_g2p_range, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG2pRangeSmem);
-        cudaFuncSetAttribute(k_g2p_range, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        k_g2p_range<<<c.sm_count * (int)min(c.t.g2p_ctas, (uint32_t)NXM_G2P_MIN_CTAS), kG2pThreads, kG2pRangeSmem,
-                      s>>>(P);
+    const uint32_t primaries = min(c.block_capacity, c.particle_capacity);
+    const uint32_t units = max(max(primaries, (c.particle_capacity + kRangeChunk - 1u) / kRangeChunk), 1u);
+#if NXM_FAST && !NXM_CPIC
+    const uint32_t most = (uint32_t)c.sm_count * min(c.t.g2p_ctas, (uint32_t)NXM_G2P_MIN_CTAS);
+    k_g2p_range<<<(int)min(units, most), kG2pThreads, 0, s>>>(P);
 #else
-        k_g2p_range<<<c.sm_count * (int)min(c.t.g2p_ctas, (uint32_t)NXM_G2P_MIN_CTAS), kG2pThreads, 0, s>>>(P);
+    k_g2p_update<<<(int)min(units, (uint32_t)c.sm_count * NXM_G2P_MIN_CTAS), kG2pThreads, 0, s>>>(P);
 #endif
-        return 1;
-    }
-#endif
-    k_g2p_update<<<c.sm_count * NXM_G2P_MIN_CTAS, kG2pThreads, 0, s>>>(P);
     return 1;
 }
 

@@ -31,14 +31,18 @@ __device__ __forceinline__ float4 f4add(float4 a, float4 b) { return make_float4
 //
 // A round ends with its fullest cell, so the 64 cells are split by count: the
 // 32 fullest in the first round, the rest in the second (none when at most 32
-// hold particles).  Bound by FP32 issue and the record loads; 512 threads' worth
-// of registers an SM (the 108 sums) leave 12 warps, whose next records are in
-// flight while the current ones accumulate.
+// hold particles).  The registers of the 108 sums leave 12 warps an SM.
 //
 // The records of a lane's next particles are in flight while it accumulates:
 // asynchronous copies into a ring of kP2gRing slots a lane in shared memory
 // (slot words of one kind side by side over the lanes: no bank conflicts), so
 // that they cost no registers.
+//
+// Bound by FP32 issue and the L1 lookups of 32 lanes' separate records.  2 M
+// sand + water particles: 168 us with a warp per cell and three lanes' groups a
+// stencil column, 111 us a cell per lane, 96 us with the ring (0.15 GB, 1.6
+// TB/s); 48 small scenes 152, 90, 81 us.  Whole blocks staged in shared memory
+// take 89 us alone, but 10% more than the ring for the 48 scenes.
 #ifndef NXM_P2G_MIN_CTAS
 #define NXM_P2G_MIN_CTAS 3
 #endif
@@ -59,17 +63,6 @@ struct P2gWarp {
 };
 constexpr size_t kP2gSmem = sizeof(P2gWarp) * kP2gWarps;
 
-template <int kBytes>
-__device__ __forceinline__ void async_copy(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
-                 "n"(kBytes)
-                 : "memory");
-}
-__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int kLeft>
-__device__ __forceinline__ void async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
-}
 __device__ __forceinline__ void p2g_fetch(const DevPtrs& P, P2gSlot& s, uint32_t lane, uint32_t pid) {
     const float4* k = reinterpret_cast<const float4*>(&P.in.kin[pid]);
     const float4* c = reinterpret_cast<const float4*>(&P.in.aff[pid]);
