@@ -484,6 +484,7 @@ struct nxm_state {
     size_t render_cap = 0;  // float4s
     float4* d_palette = nullptr;
     uint32_t palette_cap = 0;
+    std::vector<float> palette;  // the colors d_palette holds
 
     // pinned staging ring for host -> device copies (see upload_async)
     struct StagingSpan {
@@ -2063,10 +2064,19 @@ static int render_source(nxm_state* s, uint32_t mode, const float* palette, uint
     if (num_groups > s->palette_cap) {
         NXM_TRY(cudaStreamSynchronize(s->stream));
         dfree(s->d_palette);
+        s->palette.clear();
+        s->palette_cap = 0;
         NXM_TRY(dalloc(&s->d_palette, num_groups));
         s->palette_cap = num_groups;
     }
-    NXM_TRY(cudaMemcpyAsync(s->d_palette, palette, sizeof(float4) * num_groups, cudaMemcpyHostToDevice, s->stream));
+    // the device copy stands until the colors change (a copy from pageable memory costs a frame's
+    // host time what several launches do)
+    const std::vector<float> colors(palette, palette + 4 * (size_t)num_groups);
+    if (colors != s->palette) {
+        s->palette.clear();
+        NXM_TRY(cudaMemcpyAsync(s->d_palette, palette, sizeof(float4) * num_groups, cudaMemcpyHostToDevice, s->stream));
+        s->palette = colors;
+    }
     in.p = s->cur;
     in.pcdf = s->d_pcdf;
     in.pid = s->permuted ? s->pid : nullptr;
