@@ -84,6 +84,10 @@ __device__ __forceinline__ void store8(void* p, float a, float b, float c, float
                  : "memory");
 }
 
+// The first statement of a kernel that launch_after launches: waits until the
+// kernel before it in the stream is complete and its writes are visible.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Asynchronous copies of 4 or 16 bytes into shared memory (this thread's own
 // slots: visible to it once its commit group is waited for).
 template <int kBytes>

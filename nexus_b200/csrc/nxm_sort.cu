@@ -161,6 +161,7 @@ __global__ void k_sort_reset(DevPtrs P, uint32_t hash_cap) {
 // key inserted by the previous pass skips the hash entirely.
 template <int kSortBatch>
 __global__ void __launch_bounds__(256) k_touch_primary(DevPtrs P) {
+    after_previous();
     const uint32_t n = P.params->n;
     const float dx = P.params->dx;
     const uint32_t hmask = P.params->hash_capacity - 1;
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(256) k_touch_primary(DevPtrs P) {
 
 // sort.rs:133-163 gpu_touch_neighbor_blocks: one thread per (base block, neighbour).
 __global__ void __launch_bounds__(256) k_touch_nbh(DevPtrs P) {
+    after_previous();
     const uint32_t hmask = P.params->hash_capacity - 1;
     const uint32_t bcap = P.params->block_capacity;
     const uint32_t nprim = min(__ldcg(&P.counters->num_primary), bcap);
@@ -230,6 +232,7 @@ __global__ void __launch_bounds__(256) k_touch_nbh(DevPtrs P) {
 enum CellBlocks { kNoCells, kPrimaryCells, kAllCells };
 template <CellBlocks kCells>
 __global__ void __launch_bounds__(256) k_block_prep(DevPtrs P) {
+    after_previous();
     const uint32_t hmask = P.params->hash_capacity - 1;
     const uint32_t bcap = P.params->block_capacity;
     const uint32_t nprim = min(__ldcg(&P.counters->num_primary), bcap);
@@ -258,6 +261,7 @@ __global__ void __launch_bounds__(256) k_block_prep(DevPtrs P) {
 // sort.rs:287-349 gpu_update_block_particle_count.
 template <bool kExtras, int kSortBatch>
 __global__ void __launch_bounds__(256) k_count(DevPtrs P) {
+    after_previous();
     const uint32_t n = P.params->n;
     const uint32_t hmask = P.params->hash_capacity - 1;
     const uint32_t lane = threadIdx.x & 31u;
@@ -437,6 +441,7 @@ static_assert(kCellTile == kCellPerWarp * (kScanThreads / 32), "a tile per scan 
 
 template <bool kExtras>
 __global__ void __launch_bounds__(kScanThreads) k_scan_cell_tiles(DevPtrs P) {
+    after_previous();
     __shared__ uint32_t warp_tot[33];
     __shared__ uint32_t btot[kCellTile];
     const uint32_t total = __ldcg(&P.counters->num_blocks);
@@ -532,6 +537,7 @@ __device__ __forceinline__ void write_block_empty(const DevPtrs& P, uint32_t b, 
 
 template <bool kExtras>
 __global__ void __launch_bounds__(kScanThreads) k_scan_cell_apply(DevPtrs P) {
+    after_previous();
     __shared__ uint32_t warp_tot[33];
     const uint32_t total = __ldcg(&P.counters->num_blocks);
     const uint32_t counted = kExtras ? total : min(__ldcg(&P.counters->num_primary), total);
@@ -578,6 +584,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_cell_apply(DevPtrs P) {
 constexpr uint32_t kOneCtaBlocks = 2048;
 constexpr uint32_t kOneCtaThreads = 1024;
 __global__ void __launch_bounds__(kOneCtaThreads) k_scan_cells(DevPtrs P) {
+    after_previous();
     __shared__ uint32_t warp_tot[33];
     const uint32_t total = P.counters->num_blocks;
     const uint32_t counted = min(P.counters->num_primary, total);
@@ -625,6 +632,7 @@ __global__ void __launch_bounds__(kOneCtaThreads) k_scan_cells(DevPtrs P) {
 // sort.rs:430-491 gpu_finalize_particles_sort.
 template <bool kExtras, int kSortBatch>
 __global__ void __launch_bounds__(256) k_finalize(DevPtrs P) {
+    after_previous();
     const uint32_t n = P.params->n;
     const uint32_t scap = P.params->sorted_capacity;
     const uint32_t lane = threadIdx.x & 31u;
@@ -681,6 +689,7 @@ __global__ void __launch_bounds__(256) k_finalize(DevPtrs P) {
 constexpr uint32_t kSegMax = 4096;
 constexpr uint32_t kSegList = kSegMax - 4 * NUM_BUCKETS - 4;
 __global__ void __launch_bounds__(256) k_sort_segments(DevPtrs P) {
+    after_previous();
     __shared__ uint4 buf4[kSegMax / 4];
     __shared__ uint32_t ends[NUM_BUCKETS + 1];  // of the buckets in the block's list; ends[0] = 0
     uint32_t* buf = reinterpret_cast<uint32_t*>(buf4);
@@ -810,8 +819,8 @@ void launch_sort_positions(const DevPtrs& P, const LaunchCfg& c, const float4* p
     if (reset_grid < 1) reset_grid = 1;
     k_sort_reset<<<reset_grid, 256, 0, s>>>(P, c.hash_capacity);
     k_touch_primary_pos<<<g, 256, 0, s>>>(P, pos);
-    k_touch_nbh<<<g, 256, 0, s>>>(P);
-    k_block_prep<kNoCells><<<g, 256, 0, s>>>(P);
+    launch_after(k_touch_nbh, g, 256, 0, s, P);
+    launch_after(k_block_prep<kNoCells>, g, 256, 0, s, P);
     k_bucket_pos<false><<<g, 256, 0, s>>>(P, pos);
     k_scan_tiles<<<c.sm_count, kScanThreads, 0, s>>>(P);
     k_scan_apply<<<c.sm_count, kScanThreads, 0, s>>>(P);
@@ -846,6 +855,7 @@ __device__ __forceinline__ CellInfo rigid_cell(const DevPtrs& P, uint32_t i, flo
 // neighbours exists (without it the particle could not be listed there).
 // Runs on the hash as the particle passes left it, before any insertion.
 __global__ void __launch_bounds__(256) k_rigid_mark(DevPtrs P) {
+    after_previous();
     const uint32_t hmask = P.params->hash_capacity - 1;
     const float dx = P.params->dx;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.nrp; i += gridDim.x * blockDim.x) {
@@ -863,6 +873,7 @@ __global__ void __launch_bounds__(256) k_rigid_mark(DevPtrs P) {
 // sort.rs:165-198 gpu_touch_rigid_particle_blocks: the marked particles'
 // blocks join the neighbour-pass blocks (ids after the primaries).
 __global__ void __launch_bounds__(256) k_rigid_touch(DevPtrs P) {
+    after_previous();
     const uint32_t hmask = P.params->hash_capacity - 1;
     const uint32_t bcap = P.params->block_capacity;
     const uint32_t nprim = min(__ldcg(&P.counters->num_primary), bcap);
@@ -895,6 +906,7 @@ __device__ __forceinline__ int rigid_blocks(const DevPtrs& P, uint32_t i, float 
 
 // sort.rs:493-556 gpu_update_block_rigid_particle_count.
 __global__ void __launch_bounds__(256) k_rigid_count(DevPtrs P) {
+    after_previous();
     const uint32_t hmask = P.params->hash_capacity - 1;
     const float dx = P.params->dx;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.nrp; i += gridDim.x * blockDim.x) {
@@ -910,6 +922,7 @@ __global__ void __launch_bounds__(256) k_rigid_count(DevPtrs P) {
 // per warp on the list length, a warp scan for the lanes' offsets.  The
 // count becomes the placement cursor.
 __global__ void __launch_bounds__(256) k_rigid_alloc(DevPtrs P) {
+    after_previous();
     const uint32_t nb = __ldcg(&P.counters->num_blocks);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -936,6 +949,7 @@ __global__ void __launch_bounds__(256) k_rigid_alloc(DevPtrs P) {
 // sort.rs:602-667 gpu_finalize_rigid_particles_sort: the same block set as
 // the count pass, so every claimed slot stays inside its block's range.
 __global__ void __launch_bounds__(256) k_rigid_finalize(DevPtrs P) {
+    after_previous();
     const uint32_t hmask = P.params->hash_capacity - 1;
     const float dx = P.params->dx;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.nrp; i += gridDim.x * blockDim.x) {
@@ -971,49 +985,49 @@ void launch_sort(const DevPtrs& P, const LaunchCfg& c, bool with_extras, bool ca
     const int gb = grid_for(c.sm_count, per_sm, (uint64_t)c.block_capacity * 64u);
     k_sort_reset<<<reset_grid, 256, 0, s>>>(P, c.hash_capacity);
     switch (c.t.sort_batch) {
-    case 2: k_touch_primary<2><<<g, 256, 0, s>>>(P); break;
-    case 8: k_touch_primary<8><<<g, 256, 0, s>>>(P); break;
-    default: k_touch_primary<4><<<g, 256, 0, s>>>(P); break;
+    case 2: launch_after(k_touch_primary<2>, g, 256, 0, s, P); break;
+    case 8: launch_after(k_touch_primary<8>, g, 256, 0, s, P); break;
+    default: launch_after(k_touch_primary<4>, g, 256, 0, s, P); break;
     }
-    k_touch_nbh<<<gn, 256, 0, s>>>(P);
+    launch_after(k_touch_nbh, gn, 256, 0, s, P);
     if (rigid) {
-        k_rigid_mark<<<gr, 256, 0, s>>>(P);
-        k_rigid_touch<<<gr, 256, 0, s>>>(P);
+        launch_after(k_rigid_mark, gr, 256, 0, s, P);
+        launch_after(k_rigid_touch, gr, 256, 0, s, P);
     }
-    if (with_extras) k_block_prep<kAllCells><<<gb, 256, 0, s>>>(P);
-    else k_block_prep<kPrimaryCells><<<gb, 256, 0, s>>>(P);
+    if (with_extras) launch_after(k_block_prep<kAllCells>, gb, 256, 0, s, P);
+    else launch_after(k_block_prep<kPrimaryCells>, gb, 256, 0, s, P);
     switch ((with_extras ? 16 : 0) + c.t.sort_batch) {
-    case 2: k_count<false, 2><<<g, 256, 0, s>>>(P); break;
-    case 8: k_count<false, 8><<<g, 256, 0, s>>>(P); break;
-    case 18: k_count<true, 2><<<g, 256, 0, s>>>(P); break;
-    case 20: k_count<true, 4><<<g, 256, 0, s>>>(P); break;
-    case 24: k_count<true, 8><<<g, 256, 0, s>>>(P); break;
-    default: k_count<false, 4><<<g, 256, 0, s>>>(P); break;
+    case 2: launch_after(k_count<false, 2>, g, 256, 0, s, P); break;
+    case 8: launch_after(k_count<false, 8>, g, 256, 0, s, P); break;
+    case 18: launch_after(k_count<true, 2>, g, 256, 0, s, P); break;
+    case 20: launch_after(k_count<true, 4>, g, 256, 0, s, P); break;
+    case 24: launch_after(k_count<true, 8>, g, 256, 0, s, P); break;
+    default: launch_after(k_count<false, 4>, g, 256, 0, s, P); break;
     }
     if (with_extras) {
-        k_scan_cell_tiles<true><<<scan_grid, kScanThreads, 0, s>>>(P);
-        k_scan_cell_apply<true><<<scan_grid, kScanThreads, 0, s>>>(P);
+        launch_after(k_scan_cell_tiles<true>, scan_grid, kScanThreads, 0, s, P);
+        launch_after(k_scan_cell_apply<true>, scan_grid, kScanThreads, 0, s, P);
     } else {
         if (one_cta_scan(c)) {
-            k_scan_cells<<<1, kOneCtaThreads, 0, s>>>(P);
+            launch_after(k_scan_cells, 1, kOneCtaThreads, 0, s, P);
         } else {
-            k_scan_cell_tiles<false><<<scan_grid, kScanThreads, 0, s>>>(P);
-            k_scan_cell_apply<false><<<scan_grid, kScanThreads, 0, s>>>(P);
+            launch_after(k_scan_cell_tiles<false>, scan_grid, kScanThreads, 0, s, P);
+            launch_after(k_scan_cell_apply<false>, scan_grid, kScanThreads, 0, s, P);
         }
     }
     switch ((with_extras ? 16 : 0) + c.t.sort_batch) {
-    case 2: k_finalize<false, 2><<<g, 256, 0, s>>>(P); break;
-    case 8: k_finalize<false, 8><<<g, 256, 0, s>>>(P); break;
-    case 18: k_finalize<true, 2><<<g, 256, 0, s>>>(P); break;
-    case 20: k_finalize<true, 4><<<g, 256, 0, s>>>(P); break;
-    case 24: k_finalize<true, 8><<<g, 256, 0, s>>>(P); break;
-    default: k_finalize<false, 4><<<g, 256, 0, s>>>(P); break;
+    case 2: launch_after(k_finalize<false, 2>, g, 256, 0, s, P); break;
+    case 8: launch_after(k_finalize<false, 8>, g, 256, 0, s, P); break;
+    case 18: launch_after(k_finalize<true, 2>, g, 256, 0, s, P); break;
+    case 20: launch_after(k_finalize<true, 4>, g, 256, 0, s, P); break;
+    case 24: launch_after(k_finalize<true, 8>, g, 256, 0, s, P); break;
+    default: launch_after(k_finalize<false, 4>, g, 256, 0, s, P); break;
     }
-    if (canonical) k_sort_segments<<<grid_for(c.sm_count, 4), 256, 0, s>>>(P);
+    if (canonical) launch_after(k_sort_segments, grid_for(c.sm_count, 4), 256, 0, s, P);
     if (rigid) {
-        k_rigid_count<<<gr, 256, 0, s>>>(P);
-        k_rigid_alloc<<<grid_for(c.sm_count, per_sm, c.block_capacity), 256, 0, s>>>(P);
-        k_rigid_finalize<<<gr, 256, 0, s>>>(P);
+        launch_after(k_rigid_count, gr, 256, 0, s, P);
+        launch_after(k_rigid_alloc, grid_for(c.sm_count, per_sm, c.block_capacity), 256, 0, s, P);
+        launch_after(k_rigid_finalize, gr, 256, 0, s, P);
     }
 }
 

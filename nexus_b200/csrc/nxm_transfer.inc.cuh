@@ -177,6 +177,7 @@ __device__ __forceinline__ Collision collide(const DevPtrs& P, const DevCollider
 // six coupled scenes 80 us, 48 small scenes 24.6 us; 64: 77 us, 22.5 us).
 constexpr int kGridThreads = 64;
 __global__ void __launch_bounds__(kGridThreads, 16) k_grid_update(DevPtrs P) {
+    after_previous();
     __shared__ DevCollider scol[MAX_COLLIDERS];
     __shared__ uint32_t leaves[kGridThreads / 32][kMeshLeaves];
     const Params prm = *P.params;
@@ -774,6 +775,7 @@ __device__ __forceinline__ void g2p_block_loop(const DevPtrs& P, const Params& p
 }
 
 __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_update(DevPtrs P) {
+    after_previous();
     __shared__ float4 halo[216];
 #if NXM_G2P_STASH
     __shared__ float stash_mem[9 * kG2pThreads];
@@ -866,6 +868,7 @@ __global__ void k_copy_wait_timeout(Counters* counters, uint32_t limit) {
 constexpr uint32_t kRangeHalos = 8;
 static_assert(kG2pThreads == kRangeChunk, "one sorted position per thread");
 __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_range(DevPtrs P) {
+    after_previous();
     __shared__ float4 halo[kRangeHalos * 216];
     __shared__ G2pSlots slots;
     __shared__ int4 svid[kRangeHalos], skey[kRangeHalos];  // the staged blocks' coordinates and key offsets
@@ -977,7 +980,7 @@ void launch_copy_wait_timeout(Counters* counters, uint32_t limit, cudaStream_t s
 void launch_grid_update(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
     // grid_ctas counts CTAs of 256 threads
     const uint32_t most = (uint32_t)c.sm_count * c.t.grid_ctas * (256 / kGridThreads);
-    k_grid_update<<<(int)min(max(c.block_capacity, 1u), most), kGridThreads, 0, s>>>(P);
+    launch_after(k_grid_update, (int)min(max(c.block_capacity, 1u), most), kGridThreads, 0, s, P);
 }
 
 int launch_g2p_update(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
@@ -985,9 +988,9 @@ int launch_g2p_update(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
     const uint32_t units = max(max(primaries, (c.particle_capacity + kRangeChunk - 1u) / kRangeChunk), 1u);
 #if NXM_FAST && !NXM_CPIC
     const uint32_t most = (uint32_t)c.sm_count * min(c.t.g2p_ctas, (uint32_t)NXM_G2P_MIN_CTAS);
-    k_g2p_range<<<(int)min(units, most), kG2pThreads, 0, s>>>(P);
+    launch_after(k_g2p_range, (int)min(units, most), kG2pThreads, 0, s, P);
 #else
-    k_g2p_update<<<(int)min(units, (uint32_t)c.sm_count * NXM_G2P_MIN_CTAS), kG2pThreads, 0, s>>>(P);
+    launch_after(k_g2p_update, (int)min(units, (uint32_t)c.sm_count * NXM_G2P_MIN_CTAS), kG2pThreads, 0, s, P);
 #endif
     return 1;
 }

@@ -30,6 +30,7 @@ namespace {
 // time, 106 us with two entries' products in flight.
 constexpr int kGatherStage = 256;
 __global__ void __launch_bounds__(kGatherStage) k_p2g_gather(DevPtrs P) {
+    after_previous();
     __shared__ float4 srow[kGatherStage][4];  // per component: its row of C and of m v (mass: 0, 0, 0, m)
     __shared__ float4 spos[kGatherStage];     // position, affinity bits (CPIC)
     __shared__ float sw[12][kGatherStage];    // kernel weights: axis * 4 + coordinate
@@ -229,6 +230,7 @@ __device__ __forceinline__ const DevCollider* block_colliders(const DevPtrs& P, 
 // bit when inside); the closest by unsigned distance is kept.  Trimeshes
 // reach the node field through their rigid particles (k_p2g_cdf).
 __global__ void __launch_bounds__(256) k_grid_update_cdf(DevPtrs P) {
+    after_previous();
     const Params prm = *P.params;
     const float dx = prm.dx, cap = dx * 1.5f;
     const uint32_t total = P.counters->num_blocks * 64u;
@@ -302,6 +304,7 @@ __global__ void __launch_bounds__(256) k_rigid_transform(DevPtrs P) {
 // ascending-id order gives, and only a strictly closer one replaces the
 // analytic colliders' result.
 __global__ void __launch_bounds__(64) k_p2g_cdf(DevPtrs P) {
+    after_previous();
     // per staged entry: its triangle's vertices a, b, c, the face normal
     // n = (b - a) x (c - a) with |n|, and the three edge normals (edge x n);
     // a node's test then needs only differences and dot products, with the
@@ -408,6 +411,7 @@ __global__ void __launch_bounds__(64) k_p2g_cdf(DevPtrs P) {
 // threads an SM (the fit spills, where it runs): 70 -> 45 us for four scenes
 // of 100,000 particles.
 __global__ void __launch_bounds__(256, 4) k_g2p_cdf(DevPtrs P) {
+    after_previous();
     __shared__ uint4 halo[216];
     const Params prm = *P.params;
     const float dx = prm.dx;
@@ -557,11 +561,11 @@ __global__ void __launch_bounds__(256, 4) k_g2p_cdf(DevPtrs P) {
 }  // namespace
 
 void launch_grid_update_cdf(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
-    k_grid_update_cdf<<<c.sm_count * 8, 256, 0, s>>>(P);
+    launch_after(k_grid_update_cdf, c.sm_count * 8, 256, 0, s, P);
 }
 
 void launch_g2p_cdf(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
-    k_g2p_cdf<<<c.sm_count * 4, 256, 0, s>>>(P);
+    launch_after(k_g2p_cdf, c.sm_count * 4, 256, 0, s, P);
 }
 
 void launch_rigid_transform(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
@@ -569,7 +573,7 @@ void launch_rigid_transform(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s
 }
 
 void launch_p2g_cdf(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
-    k_p2g_cdf<<<c.sm_count * 16, 64, 0, s>>>(P);
+    launch_after(k_p2g_cdf, c.sm_count * 16, 64, 0, s, P);
 }
 
 void launch_timestep_bound(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
@@ -577,7 +581,7 @@ void launch_timestep_bound(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s)
 }
 
 void launch_p2g_gather(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
-    k_p2g_gather<<<c.sm_count * 6, kGatherStage, 0, s>>>(P);
+    launch_after(k_p2g_gather, c.sm_count * 6, kGatherStage, 0, s, P);
 }
 
 }  // namespace exact

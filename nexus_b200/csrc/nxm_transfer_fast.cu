@@ -74,6 +74,7 @@ __device__ __forceinline__ void p2g_fetch(const DevPtrs& P, P2gSlot& s, uint32_t
 }
 
 __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P) {
+    after_previous();
     extern __shared__ float4 p2g_smem[];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
@@ -308,6 +309,7 @@ __device__ __forceinline__ P2gHdr p2g_load_hdr(const DevPtrs& P, uint32_t b, uin
 // overlaps the current chunk's shared-memory work.  Two coupled fields of 27
 // sums do not fit a lane's registers, so this mode keeps a cell per warp.
 __global__ void __launch_bounds__(kCpicThreads, 2) k_p2g_cpic(DevPtrs P) {
+    after_previous();
     static_assert(kCpicThreads >= 216, "one flushed tile node per thread");
     extern __shared__ float4 p2g_smem[];
     float4* tiles = p2g_smem;  // kCpicWarps x 216 nodes of (x, y, z, m)
@@ -525,12 +527,12 @@ void launch_p2g(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
     const uint64_t want = max(units / kP2gWarps, (uint64_t)1);
     const uint64_t cap = (uint64_t)c.sm_count * min(c.t.p2g_ctas, (uint32_t)NXM_P2G_MIN_CTAS);
     cudaFuncSetAttribute(k_p2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2gSmem);
-    k_p2g<<<(int)min(want, cap), kP2gThreads, kP2gSmem, s>>>(P);
+    launch_after(k_p2g, (int)min(want, cap), kP2gThreads, kP2gSmem, s, P);
 }
 
 void launch_p2g_cpic(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
     cudaFuncSetAttribute(k_p2g_cpic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCpicSmem);
-    k_p2g_cpic<<<c.sm_count * 2, kCpicThreads, kCpicSmem, s>>>(P);
+    launch_after(k_p2g_cpic, c.sm_count * 2, kCpicThreads, kCpicSmem, s, P);
 }
 
 
