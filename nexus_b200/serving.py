@@ -45,11 +45,11 @@ from .mpm import MpmPipeline, MpmState, PinnedArray
 from .scenes import Scene
 
 # Estimated device bytes per particle of a batched state: two copies of the
-# 144-byte particle record, sort scratch (block key 8, header 4, sorted ids
+# 136-byte particle record, sort scratch (block key 8, header 4, sorted ids
 # reserved 32), ids 8, scene index 4.
-BYTES_PER_PARTICLE = 2 * 144 + 8 + 4 + 32 + 8 + 4
-# Per grid block: 64 nodes of 16 bytes, header arrays, hash slots.
-BYTES_PER_BLOCK = 64 * 16 + 16 + 4 * 3 + 4 * 10 + 4 * 7 + 4 + 2 * 8
+BYTES_PER_PARTICLE = 2 * 136 + 8 + 4 + 32 + 8 + 4
+# Per grid block: 64 nodes of 16 bytes, 64 cell counters, header arrays, hash slots.
+BYTES_PER_BLOCK = 64 * 16 + 64 * 4 + 16 + 4 * 3 + 4 * 10 + 4 * 7 + 4 + 2 * 8
 
 
 @dataclass
