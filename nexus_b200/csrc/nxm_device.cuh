@@ -1014,10 +1014,10 @@ struct MeshBest {
     TriProj at;
     uint32_t tri;
 };
-__device__ __forceinline__ void mesh_test(const DevTri* __restrict__ tris, uint32_t tri, v3 pt, MeshBest& m) {
-    const DevTri& t = tris[tri];
-    const TriProj pr = triangle_closest(mk(t.v[0][0], t.v[0][1], t.v[0][2]), mk(t.v[1][0], t.v[1][1], t.v[1][2]),
-                                        mk(t.v[2][0], t.v[2][1], t.v[2][2]), pt);
+template <int kStride>
+__device__ __forceinline__ void mesh_test(const float (&v)[3][kStride], uint32_t tri, v3 pt, MeshBest& m) {
+    const TriProj pr = triangle_closest(mk(v[0][0], v[0][1], v[0][2]), mk(v[1][0], v[1][1], v[1][2]),
+                                        mk(v[2][0], v[2][1], v[2][2]), pt);
     const float d = length(pr.point - pt);
     if (d <= m.dist) {
         m.dist = d;
@@ -1046,7 +1046,7 @@ __device__ __forceinline__ bool trimesh_project_local(const DevTri* __restrict__
     for (uint32_t it = 0; it < count && curr < end; ++it) {
         const DevBvhNode n = bvh[curr];
         if (n.entry & kBvhLeaf) {
-            mesh_test(tris, n.entry & ~kBvhLeaf, pt, m);
+            mesh_test(tris[n.entry & ~kBvhLeaf].v, n.entry & ~kBvhLeaf, pt, m);
             curr = n.exit;
         } else {
             curr = aabb_distance(n, pt) <= m.dist ? n.entry : n.exit;
@@ -1057,9 +1057,12 @@ __device__ __forceinline__ bool trimesh_project_local(const DevTri* __restrict__
 
 // The leaves within max_dist of any of a warp's points `pt` (one per lane, the
 // warp whole), as node indexes in traversal order: the nodes lie in depth-first
-// order, so the warp loads 32 consecutive ones at a time, tests them against
-// the box of its points, and walks the window by the skip links.  Returns
-// their number, or NONE when they do not fit kMeshLeaves.
+// order, so the warp loads 32 consecutive ones at a time and tests them against
+// the box of its points.  The links only go forward, so a node is visited unless
+// it lies before the exit of an earlier node that was missed: a running maximum
+// over the lanes.  The window after this one is loaded ahead, for where no link
+// skips it.  Returns the number of leaves, or NONE when they do not fit
+// kMeshLeaves.
 constexpr uint32_t kMeshLeaves = 192;
 __device__ __forceinline__ uint32_t warp_mesh_leaves(const DevBvhNode* __restrict__ bvh, uint32_t first, uint32_t count,
                                                      v3 pt, float max_dist, uint32_t* leaves) {
@@ -1077,43 +1080,63 @@ __device__ __forceinline__ uint32_t warp_mesh_leaves(const DevBvhNode* __restric
     hi = hi + splat(reach);
     const uint32_t end = first + count;
     uint32_t curr = first, n = 0;
+    DevBvhNode b{}, ahead{};
+    if (curr + lane < end) b = bvh[curr + lane];
     while (curr < end) {
         const uint32_t at = curr + lane;
-        uint32_t to = NONE;  // where the traversal goes from this lane's node
-        bool leaf = false;
-        if (at < end) {
-            const DevBvhNode b = bvh[at];
-            const bool hit = !(b.mn[0] > hi.x || b.mx[0] < lo.x || b.mn[1] > hi.y || b.mx[1] < lo.y || b.mn[2] > hi.z ||
-                               b.mx[2] < lo.z);
-            leaf = hit && (b.entry & kBvhLeaf);
-            to = hit && !(b.entry & kBvhLeaf) ? b.entry : b.exit;
+        if (at + 32u < end) ahead = bvh[at + 32u];
+        const bool in = at < end;
+        const bool hit = in && !(b.mn[0] > hi.x || b.mx[0] < lo.x || b.mn[1] > hi.y || b.mx[1] < lo.y ||
+                                 b.mn[2] > hi.z || b.mx[2] < lo.z);
+        uint32_t skip = in && !hit ? b.exit : 0u;  // the furthest exit of a missed node up to this lane
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t s = __shfl_up_sync(0xFFFFFFFFu, skip, o);
+            if (lane >= (uint32_t)o) skip = max(skip, s);
         }
-        const uint32_t leaf_mask = __ballot_sync(0xFFFFFFFFu, leaf);
-        uint32_t take = 0u, pos = curr;
-        const uint32_t stop = min(curr + 32u, end);
-        for (uint32_t it = 0; it < 32u && pos >= curr && pos < stop; ++it) {
-            take |= leaf_mask & (1u << (pos - curr));
-            pos = __shfl_sync(0xFFFFFFFFu, to, pos - curr);
-        }
-        if (pos <= curr) break;  // not reached: the links go forward
+        uint32_t before = __shfl_up_sync(0xFFFFFFFFu, skip, 1);
+        if (lane == 0) before = 0u;
+        const bool leaf = hit && (b.entry & kBvhLeaf) && before <= at;
+        const uint32_t take = __ballot_sync(0xFFFFFFFFu, leaf);
         if (n + __popc(take) > kMeshLeaves) return NONE;
-        if (take & (1u << lane)) leaves[n + __popc(take & lt)] = at;
+        if (leaf) leaves[n + __popc(take & lt)] = at;
         n += __popc(take);
-        curr = pos;
+        const uint32_t next = max(curr + 32u, __shfl_sync(0xFFFFFFFFu, skip, 31));
+        b = ahead;
+        if (next != curr + 32u && next + lane < end) b = bvh[next + lane];
+        curr = next;
     }
     __syncwarp();
     return n;
 }
-// trimesh_project_local over the warp's leaves.
+// A leaf's box and triangle, staged for the warp.
+struct MeshLeaf {
+    DevBvhNode box;
+    float v[3][3];
+};
+// trimesh_project_local over the warp's leaves: 32 at a time are brought to
+// shared memory together (`stage`, the warp's), then every node tests them there.
 __device__ __forceinline__ bool mesh_project_leaves(const DevTri* __restrict__ tris, const DevBvhNode* __restrict__ bvh,
-                                                    const uint32_t* leaves, uint32_t n, v3 pt, float max_dist, Proj& out) {
+                                                    const uint32_t* leaves, uint32_t n, v3 pt, float max_dist,
+                                                    MeshLeaf* stage, Proj& out) {
+    const uint32_t lane = threadIdx.x & 31u;
     MeshBest m;
     m.dist = max_dist;
     m.at.point = pt; m.at.feature = 2; m.at.id = 0;
     m.tri = NONE;
-    for (uint32_t k = 0; k < n; ++k) {
-        const DevBvhNode b = bvh[leaves[k]];
-        if (aabb_distance(b, pt) <= m.dist) mesh_test(tris, b.entry & ~kBvhLeaf, pt, m);
+    for (uint32_t k0 = 0; k0 < n; k0 += 32u) {
+        __syncwarp();  // the previous leaves are tested
+        if (k0 + lane < n) {
+            const DevBvhNode b = bvh[leaves[k0 + lane]];
+            const DevTri& t = tris[b.entry & ~kBvhLeaf];
+            stage[lane].box = b;
+#pragma unroll
+            for (int i = 0; i < 9; ++i) stage[lane].v[i / 3][i % 3] = t.v[i / 3][i % 3];
+        }
+        __syncwarp();
+        for (uint32_t k = 0; k < min(n - k0, 32u); ++k)
+            if (aabb_distance(stage[k].box, pt) <= m.dist)
+                mesh_test(stage[k].v, stage[k].box.entry & ~kBvhLeaf, pt, m);
     }
     return mesh_result(tris, pt, m, out);
 }
