@@ -819,8 +819,8 @@ void launch_sort_positions(const DevPtrs& P, const LaunchCfg& c, const float4* p
     if (reset_grid < 1) reset_grid = 1;
     k_sort_reset<<<reset_grid, 256, 0, s>>>(P, c.hash_capacity);
     k_touch_primary_pos<<<g, 256, 0, s>>>(P, pos);
-    launch_after(k_touch_nbh, g, 256, 0, s, P);
-    launch_after(k_block_prep<kNoCells>, g, 256, 0, s, P);
+    k_touch_nbh<<<g, 256, 0, s>>>(P);
+    k_block_prep<kNoCells><<<g, 256, 0, s>>>(P);
     k_bucket_pos<false><<<g, 256, 0, s>>>(P, pos);
     k_scan_tiles<<<c.sm_count, kScanThreads, 0, s>>>(P);
     k_scan_apply<<<c.sm_count, kScanThreads, 0, s>>>(P);
