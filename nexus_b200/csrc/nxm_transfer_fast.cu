@@ -40,9 +40,9 @@ __device__ __forceinline__ float4 f4add(float4 a, float4 b) { return make_float4
 //
 // Bound by FP32 issue and the L1 lookups of 32 lanes' separate records.  2 M
 // sand + water particles: 168 us with a warp per cell and three lanes' groups a
-// stencil column, 111 us a cell per lane, 96 us with the ring (0.15 GB, 1.6
-// TB/s); 48 small scenes 152, 90, 81 us.  Whole blocks staged in shared memory
-// take 89 us alone, but 10% more than the ring for the 48 scenes.
+// stencil column, 111 us a cell per lane, 96 us with the ring, 90 us with the
+// next round's records in flight while a round's sums go to the tile (0.15 GB,
+// 1.7 TB/s); 48 small scenes 152, 90, 81, 76 us; six coupled ones 70, -, 55, 45.
 #ifndef NXM_P2G_MIN_CTAS
 #define NXM_P2G_MIN_CTAS 3
 #endif
@@ -56,9 +56,15 @@ struct P2gSlot {
     float4 xm[32], vf[32], c0[32], c1[32];  // x, m; v, flags; C 0..3; C 4..7
     float c2[32];                           // C 8
 };
+struct P2gBlock {
+    uint32_t ends[65];  // ends[c]: where cell c's particles start in the sorted list
+    uint32_t blk[8];    // the block and its +1 neighbours
+    int x, y, z;        // scene-local block coordinates
+};
 struct P2gWarp {
     float4 tile[216];
     P2gSlot ring[kP2gRing];
+    P2gBlock block[2];  // of this unit and the next
     uint8_t order[64];
 };
 constexpr size_t kP2gSmem = sizeof(P2gWarp) * kP2gWarps;
@@ -90,30 +96,38 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
     const uint32_t units = split ? 2u * nbp : nbp;
     for (uint32_t t = lane; t < 216u; t += 32u) tile[t] = make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t u = warp * gridDim.x + blockIdx.x;  // the first units go to different SMs
-    while (u < units) {
-        uint32_t next = units;
-        if (units > nwarps && lane == 0) next = nwarps + atomicAdd(&P.counters->p2g_next, 1u);
-        const uint32_t b = split ? u >> 1 : u;
-        int4 vid = P.bvid[b];
-        {
-            const int3 o = scene_base_of_block(*P.params, vid);  // scene-local block coordinates
-            vid.x -= o.x; vid.y -= o.y; vid.z -= o.z;
-        }
-        const uint32_t my_nbh = lane < NUM_NBH ? __ldg(&P.nbh[b * NUM_NBH + lane]) : b;
-        // the cells' ranges of the sorted list: lane's cells are `lane` and `lane + 32`
-        const uint32_t el = __ldg(&P.cells[b * 64u + lane]), eh = __ldg(&P.cells[b * 64u + 32u + lane]);
-        uint32_t sl = __shfl_up_sync(0xFFFFFFFFu, el, 1), sh = __shfl_up_sync(0xFFFFFFFFu, eh, 1);
-        const uint32_t mid = __shfl_sync(0xFFFFFFFFu, el, 31);
+    // The block of a unit: loaded ahead, while the sums of the unit before go to
+    // the tile; its first records are then in flight while that tile is flushed.
+    uint32_t my_blk = 0, el = 0, eh = 0, first = 0;
+    int4 vid = make_int4(0, 0, 0, 0);
+    const auto load_block = [&](uint32_t v) {
+        const uint32_t b = split ? v >> 1 : v;
+        vid = P.bvid[b];
+        my_blk = lane - 1u < NUM_NBH ? __ldg(&P.nbh[b * NUM_NBH + lane - 1u]) : b;
+        // the cells' ends in the sorted list: lane's cells are `lane` and `lane + 32`
+        el = __ldg(&P.cells[b * 64u + lane]);
+        eh = __ldg(&P.cells[b * 64u + 32u + lane]);
+        first = __ldg(&P.first[b]);
+    };
+    uint32_t thr = 0;
+    const auto order_cells = [&](P2gBlock& k) {
+        k.ends[lane + 1u] = el;
+        k.ends[lane + 33u] = eh;
+        if (lane < 8u) k.blk[lane] = my_blk;
         if (lane == 0) {
-            sl = __ldg(&P.first[b]);
-            sh = mid;
+            k.ends[0] = first;
+            const int3 o = scene_base_of_block(*P.params, vid);
+            k.x = vid.x - o.x;
+            k.y = vid.y - o.y;
+            k.z = vid.z - o.z;
         }
-        const uint32_t cl = el - sl, ch = eh - sh;
+        __syncwarp();
+        const uint32_t cl = el - k.ends[lane], ch = eh - k.ends[lane + 32u];
         // the smallest threshold that at most 32 cells exceed
         const auto above = [&](uint32_t t) {
             return __popc(__ballot_sync(0xFFFFFFFFu, cl > t)) + __popc(__ballot_sync(0xFFFFFFFFu, ch > t));
         };
-        uint32_t thr = 0;
+        thr = 0;
         if (above(0) > 32) {
             uint32_t lo = 0, hi = __reduce_max_sync(0xFFFFFFFFu, max(cl, ch));
             while (hi - lo > 1u) {
@@ -133,29 +147,43 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
             order[inh ? nl + __popc(mh & lt) : 64u - nl + __popc(~mh & lt)] = (uint8_t)(lane + 32u);
             __syncwarp();
         }
-        const uint32_t r_end = split ? (u & 1u) + 1u : 2u;
+    };
+    uint32_t c = 0, n = 0, ahead = 0;  // this lane's cell of the round, its particles, the id after the ring's
+    const uint32_t* list = nullptr;
+    const auto begin_round = [&](const P2gBlock& k, uint32_t round) {
+        c = order[round * 32u + lane];
+        const uint32_t start = k.ends[c];
+        list = P.sorted + start;
+        n = k.ends[c + 1u] - start;
+        uint32_t pid[kP2gRing - 1];
+#pragma unroll
+        for (uint32_t t = 0; t + 1 < kP2gRing; ++t) pid[t] = t < n ? __ldg(&list[t]) : 0u;
+        ahead = kP2gRing - 1u < n ? __ldg(&list[kP2gRing - 1]) : 0u;
+#pragma unroll
+        for (uint32_t t = 0; t + 1 < kP2gRing; ++t) {
+            if (t < n) p2g_fetch(P, sm.ring[t], lane, pid[t]);
+            async_commit();
+        }
+    };
+    if (u < units) {
+        load_block(u);
+        order_cells(sm.block[0]);
+        begin_round(sm.block[0], split ? u & 1u : 0u);
+    }
+    uint32_t turn = 0;
+    while (u < units) {
+        uint32_t next = units;
+        if (units > nwarps && lane == 0) next = nwarps + atomicAdd(&P.counters->p2g_next, 1u);
+        const P2gBlock& now = sm.block[turn];
+        const uint32_t r_end = split ? (u & 1u) + 1u : (thr == 0u ? 1u : 2u);  // thr 0: the second round's cells are empty
         for (uint32_t round = split ? (u & 1u) : 0u; round < r_end; ++round) {
-            if (round == 1u && thr == 0u) break;  // the second round's cells are empty
-            const uint32_t c = order[round * 32u + lane];
-            const uint32_t s0 = __shfl_sync(0xFFFFFFFFu, sl, c & 31u), s1 = __shfl_sync(0xFFFFFFFFu, sh, c & 31u);
-            const uint32_t n0 = __shfl_sync(0xFFFFFFFFu, cl, c & 31u), n1 = __shfl_sync(0xFFFFFFFFu, ch, c & 31u);
-            const uint32_t* list = P.sorted + (c < 32u ? s0 : s1);
-            const uint32_t n = c < 32u ? n0 : n1;
             const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, n);
             const uint32_t cx = c & 3u, cy = (c >> 2) & 3u, cz = c >> 4;
-            const v3 x0 = mk((float)(vid.x * 4 + (int)cx), (float)(vid.y * 4 + (int)cy), (float)(vid.z * 4 + (int)cz)) * dx;
+            const bool held = n != 0u;
+            const v3 x0 = mk((float)(now.x * 4 + (int)cx), (float)(now.y * 4 + (int)cy), (float)(now.z * 4 + (int)cz)) * dx;
             float2 axy[27], azm[27];  // sums of node i + 3 j + 9 k: (x, y) and (z, mass)
 #pragma unroll
             for (int t = 0; t < 27; ++t) axy[t] = azm[t] = make_float2(0.f, 0.f);
-            uint32_t pid[kP2gRing - 1];
-#pragma unroll
-            for (uint32_t t = 0; t + 1 < kP2gRing; ++t) pid[t] = t < n ? __ldg(&list[t]) : 0u;
-            uint32_t ahead = kP2gRing - 1u < n ? __ldg(&list[kP2gRing - 1]) : 0u;  // the id after the ring's
-#pragma unroll
-            for (uint32_t t = 0; t + 1 < kP2gRing; ++t) {
-                if (t < n) p2g_fetch(P, sm.ring[t], lane, pid[t]);
-                async_commit();
-            }
             uint32_t at = 0;  // ring slot of the current particle
 #pragma unroll 1
             for (uint32_t it = 0; it < nmax; ++it) {
@@ -210,24 +238,34 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
                 }
             }
             float4* node = tile + cx + 6u * cy + 36u * cz;
+            // the next round's first records, or the next block, while these sums go to the tile
+            if (round + 1u < r_end) {
+                begin_round(now, round + 1u);
+            } else {
+                u = __shfl_sync(0xFFFFFFFFu, next, 0);
+                if (u < units) load_block(u);
+            }
 #pragma unroll
             for (int t = 0; t < 27; ++t) {
                 const int off = t % 3 + 6 * ((t / 3) % 3) + 36 * (t / 9);
-                if (n) {
+                if (held) {
                     const float4 o = node[off];
                     node[off] = make_float4(o.x + axy[t].x, o.y + axy[t].y, o.z + azm[t].x, o.w + azm[t].y);
                 }
                 __syncwarp();  // the next offset's nodes are other lanes' nodes of this one
             }
         }
+        if (u < units) {
+            __syncwarp();  // the cell order is read
+            order_cells(sm.block[turn ^ 1u]);
+            begin_round(sm.block[turn ^ 1u], split ? u & 1u : 0u);
+        }
         // the tile to global memory (clearing it)
-        for (uint32_t t = lane; t < 224u; t += 32u) {
+        for (uint32_t t = lane; t < 216u; t += 32u) {
             const uint32_t tx = t % 6u, ty = (t / 6u) % 6u, tz = t / 36u;
             const uint32_t ox = tx >= 4u, oy = ty >= 4u, oz = tz >= 4u;
             const uint32_t oct = ox * 4u + oy * 2u + oz;
-            const uint32_t other = __shfl_sync(0xFFFFFFFFu, my_nbh, (oct + 31u) & 31u);
-            if (t >= 216u) continue;
-            const uint32_t blk = oct ? other : b;
+            const uint32_t blk = now.blk[oct];
             const float4 sum = tile[t];
             if (sum.x != 0.f || sum.y != 0.f || sum.z != 0.f || sum.w != 0.f) {
                 tile[t] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -237,7 +275,7 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
             }
         }
         __syncwarp();
-        u = __shfl_sync(0xFFFFFFFFu, next, 0);
+        turn ^= 1u;
     }
 }
 
