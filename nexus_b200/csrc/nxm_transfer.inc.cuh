@@ -98,6 +98,12 @@ __device__ __forceinline__ uint32_t colliders_near_block(const DevPtrs& P, const
     return __ballot_sync(0xFFFFFFFFu, near);
 }
 
+// A warp's room for the leaves of a mesh search and the ones being tested.
+struct MeshWarp {
+    uint32_t leaves[kMeshLeaves];
+    MeshLeaf stage[32];
+};
+
 // `near` (bit i for collider i < 32, from colliders_near_block) leaves out
 // the colliders that cannot reach this node: their projections would find
 // no point within cap and no inside.
@@ -106,10 +112,6 @@ __device__ __forceinline__ uint32_t colliders_near_block(const DevPtrs& P, const
 // a node's own traversal is a chain of some hundred dependent loads (six scenes
 // over a 20,000-triangle floor: grid update 90 us, with the shared search 77 us,
 // with the leaves staged in shared memory and the windows in one scan 61 us).
-struct MeshWarp {
-    uint32_t leaves[kMeshLeaves];
-    MeshLeaf stage[32];
-};
 __device__ __forceinline__ Collision collide(const DevPtrs& P, const DevCollider* cols, uint32_t ncol, float dx,
                                              v3 point, uint32_t near, MeshWarp& mesh) {
     const float cap = dx * 1.5f;
