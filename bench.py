@@ -263,7 +263,7 @@ def workload_config(scene, world: int) -> dict:
     """The `config` of both arms' lines (the same dict, so that they compare)."""
     return {"workload": scene.name, "particles_per_gpu": scene.n, "dx": scene.dx, "dt": scene.dt,
             "parallelism": f"replicas{world}" if world > 1 else "single",
-            "l2": "inputs larger than L2 (particle state %.0f MB per GPU)" % (scene.n * 144 / 1e6)}
+            "l2": "inputs larger than L2 (particle state %.0f MB per GPU)" % (scene.n * 136 / 1e6)}
 
 
 # The reference arm times whole oracle steps of the full scene; it runs at
