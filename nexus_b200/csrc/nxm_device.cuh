@@ -338,157 +338,83 @@ __device__ __forceinline__ Svd svd3(const m3& f) {
     return out;
 }
 
-// Fast-build small strains.  The models are functions of the symmetric matrix
-// E = F F^T - I (or of the log strain X = log(I + E) / 2), and for the strains
-// a step meets they are short power series: evaluated as polynomials of degree
-// two by the Cayley-Hamilton theorem (X^3 = i1 X^2 - i2 X + i3 I), a Horner step
-// is four multiply-adds, so no eigenvectors, and no cancellation near E = 0.
-struct Sym {
-    float xx, yy, zz, xy, xz, yz;
-};
-struct Inv {
-    float i1, i2, i3;
-};
-struct Quad {  // a I + b X + c X^2
-    float a, b, c;
-};
-__device__ __forceinline__ Sym left_strain(const m3& F) {
-    Sym r;
-    r.xx = F.c0.x * F.c0.x - 1.0f; r.yy = F.c0.y * F.c0.y - 1.0f; r.zz = F.c0.z * F.c0.z - 1.0f;
-    r.xx += F.c1.x * F.c1.x; r.yy += F.c1.y * F.c1.y; r.zz += F.c1.z * F.c1.z;
-    r.xx += F.c2.x * F.c2.x; r.yy += F.c2.y * F.c2.y; r.zz += F.c2.z * F.c2.z;
-    r.xy = F.c0.x * F.c0.y + F.c1.x * F.c1.y + F.c2.x * F.c2.y;
-    r.xz = F.c0.x * F.c0.z + F.c1.x * F.c1.z + F.c2.x * F.c2.z;
-    r.yz = F.c0.y * F.c0.z + F.c1.y * F.c1.z + F.c2.y * F.c2.z;
-    return r;
-}
-__device__ __forceinline__ float norm2(const Sym& a) {
-    return a.xx * a.xx + a.yy * a.yy + a.zz * a.zz + 2.0f * (a.xy * a.xy + a.xz * a.xz + a.yz * a.yz);
-}
-__device__ __forceinline__ Sym square(const Sym& a) {
-    return Sym{a.xx * a.xx + a.xy * a.xy + a.xz * a.xz, a.xy * a.xy + a.yy * a.yy + a.yz * a.yz,
-               a.xz * a.xz + a.yz * a.yz + a.zz * a.zz, a.xx * a.xy + a.xy * a.yy + a.xz * a.yz,
-               a.xx * a.xz + a.xy * a.yz + a.xz * a.zz, a.xy * a.xz + a.yy * a.yz + a.yz * a.zz};
-}
-__device__ __forceinline__ Inv invariants(const Sym& a) {
-    const float mx = a.yy * a.zz - a.yz * a.yz, my = a.xy * a.zz - a.yz * a.xz, mz = a.xy * a.yz - a.yy * a.xz;
-    return Inv{a.xx + a.yy + a.zz, mx + (a.xx * a.zz - a.xz * a.xz) + (a.xx * a.yy - a.xy * a.xy),
-               a.xx * mx - a.xy * my + a.xz * mz};
-}
-__device__ __forceinline__ Quad times_x(const Quad& q, const Inv& v) {
-    return Quad{q.c * v.i3, q.a - q.c * v.i2, q.b + q.c * v.i1};
-}
-__device__ __forceinline__ Quad scaled(const Quad& q, float s) { return Quad{q.a * s, q.b * s, q.c * s}; }
-__device__ __forceinline__ Sym eval(const Quad& q, const Sym& x, const Sym& x2) {
-    return Sym{q.a + q.b * x.xx + q.c * x2.xx, q.a + q.b * x.yy + q.c * x2.yy, q.a + q.b * x.zz + q.c * x2.zz,
-               q.b * x.xy + q.c * x2.xy,       q.b * x.xz + q.c * x2.xz,       q.b * x.yz + q.c * x2.yz};
-}
-__device__ __forceinline__ m3 full(const Sym& a) {
-    return mkm(mk(a.xx, a.xy, a.xz), mk(a.xy, a.yy, a.yz), mk(a.xz, a.yz, a.zz));
-}
-// exp(x) - 1 for |x| <= 0.3 (the truncated term is below 5e-8 of it).
-__device__ __forceinline__ float expm1_small(float x) {
-    return x * (1.0f + x * (0.5f + x * (1.0f / 6.0f + x * (1.0f / 24.0f + x * (1.0f / 120.0f + x * (1.0f / 720.0f))))));
-}
-constexpr float kSmallStrain2 = 0.04f;  // |E|^2 up to which the series below hold (eigenvalues within 0.2)
-// log(1 + e) / e and ((1 + e) - sqrt(1 + e)) / e on [-0.2, 0.2], interpolated at
-// Chebyshev points (relative errors 2.4e-9 and 5e-10 before rounding).
-__device__ __forceinline__ Quad log_series(const Inv& v) {
-    Quad q{-1.344796503e-01f, 0.0f, 0.0f};
-    q = times_x(q, v); q.a += 1.521727398e-01f;
-    q = times_x(q, v); q.a -= 1.663773713e-01f;
-    q = times_x(q, v); q.a += 1.997634790e-01f;
-    q = times_x(q, v); q.a -= 2.500032420e-01f;
-    q = times_x(q, v); q.a += 3.333352402e-01f;
-    q = times_x(q, v); q.a -= 4.999999902e-01f;
-    q = times_x(q, v); q.a += 9.999999976e-01f;
-    return times_x(q, v);
-}
-__device__ __forceinline__ Quad corotated_series(const Inv& v) {
-    Quad q{1.396684888e-02f, 0.0f, 0.0f};
-    q = times_x(q, v); q.a -= 1.702353984e-02f;
-    q = times_x(q, v); q.a += 2.048115793e-02f;
-    q = times_x(q, v); q.a -= 2.732067537e-02f;
-    q = times_x(q, v); q.a += 3.906279847e-02f;
-    q = times_x(q, v); q.a -= 6.250018588e-02f;
-    q = times_x(q, v); q.a += 1.249999991e-01f;
-    q = times_x(q, v); q.a += 5.000000002e-01f;
-    return times_x(q, v);
-}
-
-// Fast-build strain: eigenvalues e and vectors u (columns) of F F^T - I, by
-// cyclic Jacobi rotations of the symmetric matrix (Golub & Van Loan 8.5).  The
-// models need only functions of the left stretch, s = sqrt(1 + e) in the
-// frame u: a rotation updates 6 entries and one matrix where the one-sided
-// sweeps above update two matrices and form three dot products, and e keeps
-// the small strains that 1 + e would round away.  Stops when every
-// off-diagonal is below 3e-7 of the matrix or the rounding of its entries.
-struct Strain {
-    v3 e;
-    m3 u;
-};
-
-__device__ __forceinline__ bool jacobi_sym(float& app, float& aqq, float& apq, float& arp, float& arq, v3& up, v3& uq,
-                                           float tol) {
-    if (apq * apq <= tol) return false;
-    const float d = aqq - app, g = 2.0f * apq;
-    const float ih = rsqrtf(d * d + g * g);
-    const float c2 = 0.5f + 0.5f * fabsf(d) * ih;  // cos^2 of the rotation, in [1/2, 1]
-    const float ic = rsqrtf(c2);
-    const float c = c2 * ic;
-    const float s = copysignf(0.5f * ih * ic, d) * g;
-    const float t = s * ic * apq;
-    app -= t;
-    aqq += t;
-    apq = 0.0f;
-    const float rp = arp, rq = arq;
-    arp = c * rp - s * rq;
-    arq = s * rp + c * rq;
-    const v3 p = up, q = uq;
-    up = p * c - q * s;
-    uq = p * s + q * c;
+// Fast-build SVD: the same Jacobi sweeps with the orthogonality test on
+// squares (no square roots), the rotation's division by an approximate
+// reciprocal (__fdividef), and the singular values and U columns from one
+// reciprocal square root per column.  Agrees with svd3 to a few ulp.
+__device__ __forceinline__ bool jacobi_pair_fast(float (&a)[3][3], float (&v)[3][3], int p, int q) {
+    const float alpha = a[0][p] * a[0][p] + a[1][p] * a[1][p] + a[2][p] * a[2][p];
+    const float beta = a[0][q] * a[0][q] + a[1][q] * a[1][q] + a[2][q] * a[2][q];
+    const float gamma = a[0][p] * a[0][q] + a[1][p] * a[1][q] + a[2][p] * a[2][q];
+    if (gamma * gamma <= 1.0e-12f * alpha * beta || fabsf(gamma) <= 1.0e-30f) return false;
+    const float zeta = __fdividef(beta - alpha, 2.0f * gamma);
+    const float t = __fdividef(copysignf(1.0f, zeta), fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
+    const float c = rsqrtf(1.0f + t * t);
+    const float s = c * t;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const float ap = a[r][p], aq = a[r][q];
+        a[r][p] = c * ap - s * aq;
+        a[r][q] = s * ap + c * aq;
+        const float vp = v[r][p], vq = v[r][q];
+        v[r][p] = c * vp - s * vq;
+        v[r][q] = s * vp + c * vq;
+    }
     return true;
 }
 
-__device__ __forceinline__ Strain strain_of(const m3& F) {
-    float xx = F.c0.x * F.c0.x - 1.0f, yy = F.c0.y * F.c0.y - 1.0f, zz = F.c0.z * F.c0.z - 1.0f;
-    xx += F.c1.x * F.c1.x; yy += F.c1.y * F.c1.y; zz += F.c1.z * F.c1.z;
-    xx += F.c2.x * F.c2.x; yy += F.c2.y * F.c2.y; zz += F.c2.z * F.c2.z;
-    float xy = F.c0.x * F.c0.y + F.c1.x * F.c1.y + F.c2.x * F.c2.y;
-    float xz = F.c0.x * F.c0.z + F.c1.x * F.c1.z + F.c2.x * F.c2.z;
-    float yz = F.c0.y * F.c0.z + F.c1.y * F.c1.z + F.c2.y * F.c2.z;
-    const float tol = 1.0e-13f * (xx * xx + yy * yy + zz * zz + 2.0f * (xy * xy + xz * xz + yz * yz)) + 1.0e-15f;
-    Strain r;
-    r.u = mident();
+__device__ __forceinline__ Svd svd3_fast(const m3& f) {
+    float a[3][3] = {{f.c0.x, f.c1.x, f.c2.x}, {f.c0.y, f.c1.y, f.c2.y}, {f.c0.z, f.c1.z, f.c2.z}};
+    float v[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
 #pragma unroll 1
     for (int sweep = 0; sweep < 10; ++sweep) {
-        bool rot = jacobi_sym(xx, yy, xy, xz, yz, r.u.c0, r.u.c1, tol);
-        rot |= jacobi_sym(xx, zz, xz, xy, yz, r.u.c0, r.u.c2, tol);
-        rot |= jacobi_sym(yy, zz, yz, xy, xz, r.u.c1, r.u.c2, tol);
+        bool rot = jacobi_pair_fast(a, v, 0, 1);
+        rot |= jacobi_pair_fast(a, v, 0, 2);
+        rot |= jacobi_pair_fast(a, v, 1, 2);
         if (!rot) break;
     }
-    r.e = mk(xx, yy, zz);
-    return r;
-}
-
-// u diag(d) u^T.
-__device__ __forceinline__ m3 in_frame(const m3& u, v3 d) {
-    const v3 a = u.c0 * d.x, b = u.c1 * d.y, c = u.c2 * d.z;
-    const float xx = a.x * u.c0.x + b.x * u.c1.x + c.x * u.c2.x;
-    const float yy = a.y * u.c0.y + b.y * u.c1.y + c.y * u.c2.y;
-    const float zz = a.z * u.c0.z + b.z * u.c1.z + c.z * u.c2.z;
-    const float xy = a.x * u.c0.y + b.x * u.c1.y + c.x * u.c2.y;
-    const float xz = a.x * u.c0.z + b.x * u.c1.z + c.x * u.c2.z;
-    const float yz = a.y * u.c0.z + b.y * u.c1.z + c.y * u.c2.z;
-    return mkm(mk(xx, xy, xz), mk(xy, yy, yz), mk(xz, yz, zz));
-}
-
-// log(1 + e): the odd series of the area tangent, 2 artanh(e / (2 + e)), for
-// moderate strains (truncated below 1e-8 relative at |e| = 1/4).
-__device__ __forceinline__ float log_stretch(float e) {
-    if (fabsf(e) > 0.25f) return __logf(1.0f + e);
-    const float z = __fdividef(e, 2.0f + e), z2 = z * z;
-    return 2.0f * z * (1.0f + z2 * (1.0f / 3.0f + z2 * (0.2f + z2 * (1.0f / 7.0f))));
+    float sig[3], inv[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float n2 = a[0][c] * a[0][c] + a[1][c] * a[1][c] + a[2][c] * a[2][c];
+        inv[c] = n2 > 1.0e-36f ? rsqrtf(n2) : 0.0f;
+        sig[c] = n2 * inv[c];
+    }
+    auto swapc = [&](int i, int j) {
+        float t = sig[i]; sig[i] = sig[j]; sig[j] = t;
+        t = inv[i]; inv[i] = inv[j]; inv[j] = t;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            float ta = a[r][i]; a[r][i] = a[r][j]; a[r][j] = ta;
+            float tv = v[r][i]; v[r][i] = v[r][j]; v[r][j] = tv;
+        }
+    };
+    if (sig[1] > sig[0]) swapc(0, 1);
+    if (sig[2] > sig[0]) swapc(0, 2);
+    if (sig[2] > sig[1]) swapc(1, 2);
+    float u[3][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) u[r][c] = a[r][c] * inv[c];
+    if (!(sig[1] > 1.0e-18f)) {
+        float ux = u[0][0], uy = u[1][0], uz = u[2][0];
+        float ox, oy, oz;
+        if (fabsf(ux) < 0.9f) { ox = 0; oy = -uz; oz = uy; } else { ox = uz; oy = 0; oz = -ux; }
+        float on = sqrtf(ox * ox + oy * oy + oz * oz);
+        if (on == 0.0f) { ox = 1; oy = 0; oz = 0; on = 1; }
+        u[0][1] = ox / on; u[1][1] = oy / on; u[2][1] = oz / on;
+    }
+    if (!(sig[2] > 1.0e-18f)) {
+        u[0][2] = u[1][0] * u[2][1] - u[2][0] * u[1][1];
+        u[1][2] = u[2][0] * u[0][1] - u[0][0] * u[2][1];
+        u[2][2] = u[0][0] * u[1][1] - u[1][0] * u[0][1];
+    }
+    Svd out;
+    out.u = mkm(mk(u[0][0], u[1][0], u[2][0]), mk(u[0][1], u[1][1], u[2][1]), mk(u[0][2], u[1][2], u[2][2]));
+    out.s = mk(sig[0], sig[1], sig[2]);
+    out.vt = mkm(mk(v[0][0], v[0][1], v[0][2]), mk(v[1][0], v[1][1], v[1][2]), mk(v[2][0], v[2][1], v[2][2]));
+    return out;
 }
 
 // ---------------------------------------------------------------------------
@@ -589,178 +515,63 @@ __device__ __forceinline__ m3 dp_project_svd(const float* pl, float* state, cons
     d.s = sv;
     return (d.u * diag(sv)) * d.vt;
 }
-// Fast-build models on the strain frame.  `s` is the stretch, `rs` its
-// reciprocal, `sm` = s - 1 formed without cancellation.
-struct Stretch {
-    v3 s, rs, sm;
-};
-__device__ __forceinline__ Stretch stretch_of(v3 e) {
-    Stretch r;
-    const v3 l = e + splat(1.0f);
-    r.rs = mk(rsqrtf(l.x), rsqrtf(l.y), rsqrtf(l.z));
-    r.s = mk(l.x * r.rs.x, l.y * r.rs.y, l.z * r.rs.z);
-    r.sm = mk(__fdividef(e.x, r.s.x + 1.0f), __fdividef(e.y, r.s.y + 1.0f), __fdividef(e.z, r.s.z + 1.0f));
-    return r;
-}
-
-// Corotated linear stress: with F = U S V^T, U (S - I) V^T F^T =
-// U diag((s - 1) s) U^T.
-__device__ __forceinline__ m3 linear_stress_fast(float lambda, float mu, const m3& u, v3 s, v3 sm) {
-    const float j = s.x * s.y * s.z;
-    m3 r = in_frame(u, mk(sm.x * s.x, sm.y * s.y, sm.z * s.z) * (2.0f * mu));
-    const float diag_val = lambda * (j - 1.0f) * j;
-    r.c0.x += diag_val;
-    r.c1.y += diag_val;
-    r.c2.z += diag_val;
-    return r;
-}
-
-// F with its stretches s replaced by `ns`: F + U diag(ns / s - 1) U^T F.
-__device__ __forceinline__ m3 restretch(const m3& F, const m3& u, v3 ns, v3 rs) {
-    return F + in_frame(u, mk(ns.x * rs.x - 1.0f, ns.y * rs.y - 1.0f, ns.z * rs.z - 1.0f)) * F;
-}
-
-// Drucker-Prager projection: dp_project_svd's return map with the hardware
-// approximations of exp and sin (__expf, __sinf), and the determinants'
-// logarithms taken from the strains (log det = sum of the log stretches), so
-// no further logarithm is needed.  `st` and F become the projected ones.
-__device__ __forceinline__ void dp_project_fast(const float* pl, float* state, m3& F, const Strain& d, Stretch& st) {
-    if (pl[4] == 0.0f) return;
+// Fast-build Drucker-Prager projection: dp_project_svd's return map with the
+// hardware approximations of log, exp and sin (__logf, __expf, __sinf), and
+// the determinants' logarithms taken from the strains (log det = sum of the
+// log singular values), so no further logarithm is needed.
+// The paths that leave F unchanged return it as U S V^T (equal to rounding),
+// so F itself need not stay live across the SVD.
+__device__ __forceinline__ m3 dp_project_fast(const float* pl, float* state, const m3& F, Svd& d) {
+    d = svd3_fast(F);
+    if (pl[4] == 0.0f) return (d.u * diag(d.s)) * d.vt;
     const float q = state[1];
     const float angle = pl[0] + (pl[1] * q - pl[3]) * __expf(-pl[2] * q);
     const float s_angle = __sinf(angle);
     const float alpha = sqrtf(2.0f / 3.0f) * __fdividef(2.0f * s_angle, 3.0f - s_angle);
     const float dd = 3.0f;
-    const v3 ls = mk(log_stretch(d.e.x), log_stretch(d.e.y), log_stretch(d.e.z)) * 0.5f;
+    const v3 ls = mk(__logf(d.s.x), __logf(d.s.y), __logf(d.s.z));
     const v3 strain = ls + splat(state[2] / dd);
     const float tr = strain.x + strain.y + strain.z;
     const v3 dev = strain - splat(tr / dd);
     const float shifted = tr - pl[6];
-    v3 h;
-    float hard;
+    v3 sv;
+    float hard, log_new;
     if (shifted > 0.0f || (dev.x == 0.0f && dev.y == 0.0f && dev.z == 0.0f)) {
-        h = splat(pl[6] / dd);
+        sv = splat(__expf(pl[6] / dd));
         hard = length(strain);
+        log_new = pl[6];
     } else {
         const float dnorm = length(dev);
         const float gamma = dnorm + (dd * pl[4] + 2.0f * pl[5]) / (2.0f * pl[5]) * shifted * alpha;
-        if (gamma <= 0.0f) return;  // invalid projection: state and F unchanged
-        h = strain - dev * __fdividef(gamma, dnorm);
+        if (gamma <= 0.0f) return (d.u * diag(d.s)) * d.vt;  // invalid projection: state and F unchanged
+        const v3 h = strain - dev * __fdividef(gamma, dnorm);
+        sv = mk(__expf(h.x), __expf(h.y), __expf(h.z));
         hard = gamma;
+        log_new = h.x + h.y + h.z;
     }
-    const v3 sv = mk(__expf(h.x), __expf(h.y), __expf(h.z));
-    const float log_prev = ls.x + ls.y + ls.z, log_new = h.x + h.y + h.z;
+    const float log_prev = ls.x + ls.y + ls.z;
     state[0] = state[0] * __expf(log_prev - log_new);
     state[1] = state[1] + hard;
     state[2] = state[2] + log_prev - log_new;
-    F = restretch(F, d.u, sv, st.rs);
-    st.s = sv;
-    st.sm = sv - splat(1.0f);
+    d.s = sv;
+    return (d.u * diag(sv)) * d.vt;
 }
 
-// The same for a small strain E of F, and the Kirchhoff stress of a linear
-// backbone into tau.  With X = log(I + E) / 2 the return map moves X to
-// rho X + tau0 I, so F is multiplied by exp(tau0 I - kappa X), kappa = 1 - rho,
-// and the stress is 2 mu (exp(2 X') - exp(X')) + lambda (j - 1) j.
-// False, with nothing changed, where a series would not hold.
-__device__ __forceinline__ bool dp_project_small(const float* pl, float* state, m3& F, const Sym& E, float lambda, float mu,
-                                                 m3& tau) {
-    const Sym X = eval(scaled(log_series(invariants(E)), 0.5f), E, square(E));
-    const float tr = X.xx + X.yy + X.zz, third = tr * (1.0f / 3.0f);
-    const Sym dev = Sym{X.xx - third, X.yy - third, X.zz - third, X.xy, X.xz, X.yz};
-    const float dnorm2 = norm2(dev);
-    float kappa = 0.0f, tau0 = 0.0f, hard = 0.0f, dlog = 0.0f;  // unchanged
-    if (pl[4] != 0.0f) {
-        const float q = state[1];
-        const float angle = pl[0] + (pl[1] * q - pl[3]) * __expf(-pl[2] * q);
-        const float s_angle = __sinf(angle);
-        const float alpha = sqrtf(2.0f / 3.0f) * __fdividef(2.0f * s_angle, 3.0f - s_angle);
-        const float total = tr + state[2], shifted = total - pl[6];
-        if (shifted > 0.0f || dnorm2 == 0.0f) {
-            kappa = 1.0f;
-            tau0 = pl[6] * (1.0f / 3.0f);
-            hard = sqrtf(dnorm2 + total * total * (1.0f / 3.0f));
-            dlog = tr - pl[6];
-        } else {
-            const float inv = rsqrtf(dnorm2), dnorm = dnorm2 * inv;
-            const float gamma = dnorm + (3.0f * pl[4] + 2.0f * pl[5]) / (2.0f * pl[5]) * shifted * alpha;
-            if (gamma > 0.0f) {
-                kappa = gamma * inv;
-                tau0 = kappa * third + state[2] * (1.0f / 3.0f);
-                hard = gamma;
-                dlog = -state[2];
-            }
-        }
-    }
-    const float rho = 1.0f - kappa;
-    const float y = rho * tr + 3.0f * tau0;  // log of the new determinant
-    if (!(fabsf(tau0) <= 0.1f && fabsf(y) <= 0.3f && fabsf(kappa) <= 2.0f)) return false;
-    if (kappa != 0.0f) {
-        state[0] = state[0] * __expf(dlog);
-        state[1] = state[1] + hard;
-        state[2] = state[2] + dlog;
-    }
-    const Inv v = invariants(X);
-    const Sym X2 = square(X);
-    const float bm1 = expm1_small(tau0), B = 1.0f + bm1, A = B * B;
-    Quad p{1.0f / 5040.0f, 0.0f, 0.0f};  // exp(-kappa X) - I
-    p = scaled(times_x(p, v), -kappa); p.a += 1.0f / 720.0f;
-    p = scaled(times_x(p, v), -kappa); p.a += 1.0f / 120.0f;
-    p = scaled(times_x(p, v), -kappa); p.a += 1.0f / 24.0f;
-    p = scaled(times_x(p, v), -kappa); p.a += 1.0f / 6.0f;
-    p = scaled(times_x(p, v), -kappa); p.a += 0.5f;
-    p = scaled(times_x(p, v), -kappa); p.a += 1.0f;
-    p = scaled(times_x(p, v), -kappa * B);
-    p.a += bm1;
-    // exp(2 X') - exp(X'): coefficients (A 2^n - B) / n!
-    Quad t{A * (256.0f / 40320.0f) - B * (1.0f / 40320.0f), 0.0f, 0.0f};
-    t = scaled(times_x(t, v), rho); t.a += A * (128.0f / 5040.0f) - B * (1.0f / 5040.0f);
-    t = scaled(times_x(t, v), rho); t.a += A * (64.0f / 720.0f) - B * (1.0f / 720.0f);
-    t = scaled(times_x(t, v), rho); t.a += A * (32.0f / 120.0f) - B * (1.0f / 120.0f);
-    t = scaled(times_x(t, v), rho); t.a += A * (16.0f / 24.0f) - B * (1.0f / 24.0f);
-    t = scaled(times_x(t, v), rho); t.a += A * (8.0f / 6.0f) - B * (1.0f / 6.0f);
-    t = scaled(times_x(t, v), rho); t.a += A * 2.0f - B * 0.5f;
-    t = scaled(times_x(t, v), rho); t.a += A * 2.0f - B;
-    t = scaled(times_x(t, v), rho); t.a += B * bm1;
-    const float jm1 = expm1_small(y);
-    Sym k = eval(scaled(t, 2.0f * mu), X, X2);
-    const float diag_val = lambda * jm1 * (1.0f + jm1);
-    k.xx += diag_val;
-    k.yy += diag_val;
-    k.zz += diag_val;
-    tau = full(k);
-    if (kappa != 0.0f) F = F + full(eval(p, X, X2)) * F;
-    return true;
-}
-
-// Corotated linear stress of a small strain: 2 mu (b - b^(1/2)) + lambda (j -
-// 1) j with b = I + E, j^2 = det b.
-__device__ __forceinline__ m3 linear_stress_small(float lambda, float mu, const Sym& E) {
-    const Inv v = invariants(E);
-    const float d = v.i1 + v.i2 + v.i3;  // j^2 - 1
-    const float j = sqrtf(1.0f + d), jm1 = __fdividef(d, 1.0f + j);
-    Sym k = eval(scaled(corotated_series(v), 2.0f * mu), E, square(E));
-    const float diag_val = lambda * jm1 * j;
-    k.xx += diag_val;
-    k.yy += diag_val;
-    k.zz += diag_val;
-    return full(k);
-}
-
-// Snow projection (snow_project below): the stretches clamped to the elastic band.
-__device__ __forceinline__ float snow_project_fast(const float* pl, float* state, m3& F, const Strain& d, Stretch& st) {
-    if (!(pl[0] <= 0.0f && pl[1] <= 0.0f)) {
-        const v3 cl = vclamp(st.s, 1.0f - pl[0], 1.0f + pl[1]);
-        const float prev_det = st.s.x * st.s.y * st.s.z;
-        const float new_det = cl.x * cl.y * cl.z;
-        state[0] = rclamp(state[0] * prev_det / new_det, 0.1f, 4.0f);
-        F = restretch(F, d.u, cl, st.rs);
-        const v3 s = st.s;
-        st.s = cl;  // a stretch inside the band keeps its exact s - 1
-        st.sm = mk(cl.x == s.x ? st.sm.x : cl.x - 1.0f, cl.y == s.y ? st.sm.y : cl.y - 1.0f,
-                   cl.z == s.z ? st.sm.z : cl.z - 1.0f);
-    }
-    return expf(pl[2] * (1.0f - state[0]));
+// Fast-build corotated linear stress from the SVD of F: with F = U S V^T,
+// U (S - I) V^T F^T = U diag((s - 1) s) U^T, a symmetric product.
+__device__ __forceinline__ m3 linear_stress_fast(float lambda, float mu, const Svd& d) {
+    const float j = d.s.x * d.s.y * d.s.z;
+    const v3 e = mk((d.s.x - 1.0f) * d.s.x, (d.s.y - 1.0f) * d.s.y, (d.s.z - 1.0f) * d.s.z) * (2.0f * mu);
+    const m3& U = d.u;
+    const v3 u0e = U.c0 * e.x, u1e = U.c1 * e.y, u2e = U.c2 * e.z;
+    const float xx = u0e.x * U.c0.x + u1e.x * U.c1.x + u2e.x * U.c2.x;
+    const float yy = u0e.y * U.c0.y + u1e.y * U.c1.y + u2e.y * U.c2.y;
+    const float zz = u0e.z * U.c0.z + u1e.z * U.c1.z + u2e.z * U.c2.z;
+    const float xy = u0e.x * U.c0.y + u1e.x * U.c1.y + u2e.x * U.c2.y;
+    const float xz = u0e.x * U.c0.z + u1e.x * U.c1.z + u2e.x * U.c2.z;
+    const float yz = u0e.y * U.c0.z + u1e.y * U.c1.z + u2e.y * U.c2.z;
+    const float diag_val = lambda * (j - 1.0f) * j;
+    return mkm(mk(xx + diag_val, xy, xz), mk(xy, yy + diag_val, yz), mk(xz, yz, zz + diag_val));
 }
 
 __device__ __forceinline__ m3 dp_project(const float* pl, float* state, const m3& F) {
@@ -788,19 +599,35 @@ __device__ __forceinline__ m3 snow_project(const float* pl, float* state, const 
 
 // models/default.rs:208-264.  `w` holds the material's 24 model words; the
 // per-particle state words (Drucker-Prager words 0..2, snow word 0) are in `st`
-// and updated in place.  model_update_ref keeps the reference's operation
-// order (the deterministic build).
-__device__ __forceinline__ m3 model_update_ref(uint32_t tag, const float* w, float* st, m3& F, const m3& vel_grad) {
+// and updated in place.  kReuseSvd selects the fast build's forms, which
+// agree with the reference's to rounding: Drucker-Prager sand on a linear
+// backbone takes its stress from the projection's SVD instead of a second SVD
+// of the projected F, with the fast SVD, projection and stress above; the
+// deterministic build keeps the reference's operation order.
+template <bool kReuseSvd>
+__device__ __forceinline__ m3 model_update(uint32_t tag, const float* w, float* st, m3& F, const m3& vel_grad) {
     switch (tag) {
     case MODEL_ELASTIC_LINEAR:
+        if (kReuseSvd) return linear_stress_fast(w[0], w[1], svd3_fast(F));
         return linear_stress(w[0], w[1], F);
     case MODEL_ELASTIC_NEO_HOOKEAN:
         return neo_hookean_stress(w[0], w[1], F);
     case MODEL_SAND_LINEAR:
-        F = dp_project(&w[3], st, F);
-        return linear_stress(w[10], w[11], F);
+        if (kReuseSvd) {
+            Svd d;
+            F = dp_project_fast(&w[3], st, F, d);
+            return linear_stress_fast(w[10], w[11], d);
+        } else {
+            F = dp_project(&w[3], st, F);
+            return linear_stress(w[10], w[11], F);
+        }
     case MODEL_SAND_NEO_HOOKEAN:
-        F = dp_project(&w[3], st, F);
+        if (kReuseSvd) {
+            Svd d;
+            F = dp_project_fast(&w[3], st, F, d);
+        } else {
+            F = dp_project(&w[3], st, F);
+        }
         return neo_hookean_stress(w[10], w[11], F);
     case MODEL_FLUID: {
         m3 sr = (vel_grad + transpose(vel_grad)) * 0.5f;
@@ -814,67 +641,6 @@ __device__ __forceinline__ m3 model_update_ref(uint32_t tag, const float* w, flo
     default:
         return mzero();
     }
-}
-
-struct ModelResult {
-    m3 F, tau;
-    v3 st;
-};
-// Snow and the strains beyond the series, out of line (inline it would keep
-// registers from everything else): one eigendecomposition of F F^T - I.  The
-// square loses the smallest stretch once it is far below the largest (under 0.3
-// of it: relative error above 1e-6), so such an F takes the SVD forms.
-static __device__ __noinline__ ModelResult model_update_large(uint32_t tag, const float* w, v3 st, m3 F) {
-    ModelResult r;
-    float s[4] = {st.x, st.y, st.z, 0.f};
-    const Strain d = strain_of(F);
-    const float lo = fminf(fminf(d.e.x, d.e.y), d.e.z) + 1.0f, hi = fmaxf(fmaxf(d.e.x, d.e.y), d.e.z) + 1.0f;
-    if (!(lo > 0.1f * hi)) {
-        r.tau = model_update_ref(tag, w, s, F, mzero());
-    } else {
-        Stretch x = stretch_of(d.e);
-        float lambda = w[0], mu = w[1];
-        bool linear = true;
-        if (tag == MODEL_SAND_LINEAR || tag == MODEL_SAND_NEO_HOOKEAN) {
-            dp_project_fast(&w[3], s, F, d, x);
-            lambda = w[10];
-            mu = w[11];
-            linear = tag == MODEL_SAND_LINEAR;
-        } else if (tag == MODEL_SNOW) {
-            const float hard = snow_project_fast(&w[1], s, F, d, x);
-            lambda = w[4] * hard;
-            mu = w[5] * hard;
-        }
-        r.tau = linear ? linear_stress_fast(lambda, mu, d.u, x.s, x.sm) : neo_hookean_stress(lambda, mu, F);
-    }
-    r.F = F;
-    r.st = mk(s[0], s[1], s[2]);
-    return r;
-}
-
-// kFast selects the fast build's forms, which agree with the reference's to
-// rounding: sand and linear elastic at small strains by series.
-template <bool kFast>
-__device__ __forceinline__ m3 model_update(uint32_t tag, const float* w, float* st, m3& F, const m3& vel_grad) {
-    if (!kFast || tag > MODEL_SNOW) return model_update_ref(tag, w, st, F, vel_grad);
-    if (tag == MODEL_FLUID) {
-        m3 sr = (vel_grad + transpose(vel_grad)) * 0.5f;
-        return fluid_stress(&w[0], F, sr);
-    }
-    if (tag == MODEL_ELASTIC_NEO_HOOKEAN) return neo_hookean_stress(w[0], w[1], F);
-    if (tag != MODEL_SNOW) {
-        const Sym E = left_strain(F);
-        if (norm2(E) <= kSmallStrain2) {
-            if (tag == MODEL_ELASTIC_LINEAR) return linear_stress_small(w[0], w[1], E);
-            m3 tau;
-            if (dp_project_small(&w[3], st, F, E, w[10], w[11], tau))
-                return tag == MODEL_SAND_LINEAR ? tau : neo_hookean_stress(w[10], w[11], F);
-        }
-    }
-    const ModelResult r = model_update_large(tag, w, mk(st[0], st[1], st[2]), F);
-    F = r.F;
-    st[0] = r.st.x; st[1] = r.st.y; st[2] = r.st.z;
-    return r.tau;
 }
 
 // ---------------------------------------------------------------------------

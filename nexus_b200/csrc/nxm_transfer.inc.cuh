@@ -639,7 +639,7 @@ __device__ __forceinline__ void g2p_finish(const DevPtrs& P, const Params& prm) 
 
 // CTAs per SM the register budget is sized for: at 4 (64 registers) the spills
 // around the constitutive update cost more than the fourth CTA's latency hiding
-// gives (2 M sand + water: 156 us at 4, 145 us at 3; 48 small scenes 121, 111).
+// gives (2 M sand + water: 178 us at 4, 166 us at 3; 48 small scenes 129, 124).
 #ifndef NXM_G2P_MIN_CTAS
 #define NXM_G2P_MIN_CTAS 3
 #endif
@@ -867,8 +867,8 @@ __global__ void k_copy_wait_timeout(Counters* counters, uint32_t limit) {
 // warp's halo reads are mostly broadcasts.
 //
 // Bound by instruction issue and the latency of a run's first loads; 2 M sand +
-// water particles: 190 us with the 27-node gather, the eigendecomposition of
-// every strain and records held in registers, 145 us now (0.25 GB, 1.7 TB/s).
+// water particles: 193 us with the 27-node gather and records held in
+// registers, 166 us now (0.25 GB, 1.5 TB/s); 500,000 snow particles 82, 73 us.
 //
 // Halo staging: every thread below 216 loads one node of each staged block
 // (its block id from the neighbour table, then the node, both L2 hits).

@@ -1,8 +1,7 @@
 """The kernels at the sizes where their splits change: P2G's two rounds of 32
-cells, the cell-ordered sort list and its two scans, strains of every form
-(series, eigenvalues, SVD), the gather P2G's stages, long and short canonical
-buckets, mesh searches with more leaves than a warp keeps, render data at
-partial warps.  Against the CPU oracle, with the bounds of
+cells, the cell-ordered sort list and its two scans, strains of every size,
+the gather P2G's stages, long and short canonical buckets, mesh searches with
+more leaves than a warp keeps, render data at partial warps.  Against the CPU oracle, with the bounds of
 tests/parity.py (or bit for bit where the mode promises it)."""
 import numpy as np
 import pytest
@@ -94,8 +93,7 @@ def test_p2g_over_cell_counts(pipe, kind, deterministic):
 @pytest.mark.parametrize("strain", ["none", "tiny", "small", "edge", "large", "far"])
 def test_strain_forms_match_the_oracle(pipe, model, strain):
     """One step from given deformation gradients: rotated, unstrained to strongly
-    strained, about the end of the series' range (edge), and with stretches so far
-    apart that the SVD forms take over (far)."""
+    strained, and with stretches far apart (far)."""
     from oracle.oracle import OracleScene
     mat = {"elastic": ParticleModel.elastic(2.0e4, 0.25), "sand": ParticleModel.sand(3.5e5, 0.3),
            "sand_neo_hookean": ParticleModel.sand_neo_hookean(2.0e5, 0.3), "snow": ParticleModel.snow(1.4e5, 0.2)}[model]
