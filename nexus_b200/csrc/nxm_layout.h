@@ -16,6 +16,7 @@
 // then velocity + mass after the grid update).
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 
 namespace nxm {
@@ -27,6 +28,8 @@ constexpr int NUM_BUCKETS = 10;
 constexpr int NUM_NBH = 7;
 constexpr int MODEL_WORDS = 24;
 constexpr uint32_t kMaxBlocks = (1u << 26) - 1u;  // header id * 64 + cell fits 32 bits beside NONE
+// Word w of block b's 64 float4 nodes: 2^24 blocks already hold 2^32 words.
+constexpr size_t node_word(uint32_t b, uint32_t w) { return (size_t)b * 256u + w; }
 constexpr float MAX_FLT = 1.0e18f;  // nexus_rbd_shaders::MAX_FLT
 constexpr int MAX_COLLIDERS = 16;   // solver/boundary_condition.rs:132
 

@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(kGatherStage) k_p2g_gather(DevPtrs P) {
             }
             __syncthreads();
         }
-        reinterpret_cast<float*>(P.nodes)[b * 256u + tid] = acc;
-        if (cpic) reinterpret_cast<float*>(P.nodes_inc)[b * 256u + tid] = acc_inc;
+        reinterpret_cast<float*>(P.nodes)[node_word(b, tid)] = acc;
+        if (cpic) reinterpret_cast<float*>(P.nodes_inc)[node_word(b, tid)] = acc_inc;
     }
 }
 

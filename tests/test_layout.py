@@ -1,0 +1,22 @@
+"""Index arithmetic of the layout header at the ends of its range, compiled for
+the host: states of that size do not fit a test."""
+import os
+import subprocess
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nexus_b200", "csrc")
+
+
+def _run(tmp_path, body):
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text('#include "nxm_layout.h"\n#include <cstdio>\nusing namespace nxm;\nint main() {\n' + body + "\n}\n")
+    subprocess.run(["g++", "-std=c++17", f"-I{CSRC}", str(src), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+
+
+def test_node_words_of_the_last_blocks(tmp_path):
+    """The gather P2G stores single words; a block's words follow the block before's up to kMaxBlocks."""
+    blocks = [0, 1, (1 << 24) - 1, 1 << 24, (1 << 24) + 5, (1 << 26) - 2]
+    got = _run(tmp_path, "".join(f'printf("%zu %zu ", node_word({b}u, 0u), node_word({b}u, 255u));' for b in blocks))
+    assert [int(x) for x in got] == [v for b in blocks for v in (b * 256, b * 256 + 255)]
+    det = open(os.path.join(CSRC, "nxm_transfer_det.cu")).read()
+    assert "* 256u" not in det  # no word index formed in 32 bits beside it
