@@ -27,7 +27,10 @@ constexpr int NUM_EXTRA_BUCKETS = 6;
 constexpr int NUM_BUCKETS = 10;
 constexpr int NUM_NBH = 7;
 constexpr int MODEL_WORDS = 24;
-constexpr uint32_t kMaxBlocks = (1u << 26) - 1u;  // header id * 64 + cell fits 32 bits beside NONE
+// header id * 64 + cell fits 32 bits beside NONE, and a loop over the nodes of
+// that many blocks can pass its end by a grid's stride without wrapping (at most
+// 16 CTAs of 256 threads an SM).
+constexpr uint32_t kMaxBlocks = (1u << 26) - (1u << 14);
 // Word w of block b's 64 float4 nodes: 2^24 blocks already hold 2^32 words.
 constexpr size_t node_word(uint32_t b, uint32_t w) { return (size_t)b * 256u + w; }
 constexpr float MAX_FLT = 1.0e18f;  // nexus_rbd_shaders::MAX_FLT

@@ -15,8 +15,17 @@ def _run(tmp_path, body):
 
 def test_node_words_of_the_last_blocks(tmp_path):
     """The gather P2G stores single words; a block's words follow the block before's up to kMaxBlocks."""
-    blocks = [0, 1, (1 << 24) - 1, 1 << 24, (1 << 24) + 5, (1 << 26) - 2]
+    blocks = [0, 1, (1 << 24) - 1, 1 << 24, (1 << 24) + 5, int(_run(tmp_path, 'printf("%u", kMaxBlocks);')[0]) - 1]
     got = _run(tmp_path, "".join(f'printf("%zu %zu ", node_word({b}u, 0u), node_word({b}u, 255u));' for b in blocks))
     assert [int(x) for x in got] == [v for b in blocks for v in (b * 256, b * 256 + 255)]
     det = open(os.path.join(CSRC, "nxm_transfer_det.cu")).read()
     assert "* 256u" not in det  # no word index formed in 32 bits beside it
+
+
+def test_node_loops_end_at_the_last_block(tmp_path):
+    """`for (t = thread; t < blocks * 64; t += stride)` in 32 bits: the first t past the end must not wrap
+    to a small one, or the loop starts again and never ends."""
+    blocks = int(_run(tmp_path, 'printf("%u", kMaxBlocks);')[0])
+    stride = 148 * 16 * 256  # the largest launch over nodes
+    assert blocks * 64 + stride <= 1 << 32
+    assert blocks * 64 + 63 < (1 << 32) - 1  # the last cell's key is not NONE
