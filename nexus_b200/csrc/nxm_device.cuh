@@ -70,12 +70,15 @@ __device__ __forceinline__ m3 outer(v3 a, v3 b) { return mkm(a * b.x, a * b.y, a
 struct f8 {
     float v[8];
 };
-// (through the read-only path: the record is not written before the load by this kernel)
+// (a plain load, kept in its place: in the modes that step in place the kernel
+// writes the record it read, and a read-only load is for data it does not write)
 __device__ __forceinline__ f8 load8(const void* p) {
     f8 r;
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
-        : "l"(p));
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]), "=f"(r.v[6]),
+                   "=f"(r.v[7])
+                 : "l"(p)
+                 : "memory");
     return r;
 }
 __device__ __forceinline__ void store8(void* p, float a, float b, float c, float d, float e, float f, float g, float h) {

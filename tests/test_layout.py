@@ -29,3 +29,13 @@ def test_node_loops_end_at_the_last_block(tmp_path):
     stride = 148 * 16 * 256  # the largest launch over nodes
     assert blocks * 64 + stride <= 1 << 32
     assert blocks * 64 + 63 < (1 << 32) - 1  # the last cell's key is not NONE
+
+
+def test_records_of_in_place_kernels_are_not_read_as_read_only():
+    """Deterministic and CPIC steps write the records they read: the read-only path
+    (ld.global.nc, __ldg) is only for arrays that a kernel does not write."""
+    for name in ("nxm_device.cuh", "nxm_transfer.inc.cuh", "nxm_transfer_det.cu"):
+        text = open(os.path.join(CSRC, name)).read()
+        assert "ld.global.nc" not in text, name
+        for record in ("in.kin", "in.aff", "in.tail", "in.def", "in.mat", "in.pstate", "out."):
+            assert f"__ldg(&P.{record}" not in text, (name, record)
