@@ -552,10 +552,14 @@ __device__ __forceinline__ void g2p_particle(const DevPtrs& P, const Params& prm
         flags &= ~PFLAG_ENABLED;
         F = mident();
         aff = mzero();
-        // the fast build always writes to the other buffer: the old position
-        // is re-read there instead of staying live across the model update
-        const uint32_t from = kSlots ? P.sorted[dst] : src;
-        const v3 op = NXM_FAST ? mk(P.in.kin[from].x, P.in.kin[from].y, P.in.kin[from].z) : pt;
+        // at its old position: kSlots writes to the other buffer, so it is re-read
+        // instead of staying live across the model update; in place (deterministic
+        // and CPIC) the record already holds the new one
+        v3 op = pt;
+        if (kSlots) {
+            const PKin& old = P.in.kin[P.sorted[dst]];
+            op = mk(old.x, old.y, old.z);
+        }
         store8(&P.out.kin[dst], op.x, op.y, op.z, 0.f, 0.f, 0.f, 0.f, __uint_as_float(flags));
         const CellInfo oc = cell_info(dx, op);
         const int3 key_off = block.key();

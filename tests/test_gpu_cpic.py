@@ -131,3 +131,31 @@ def test_cpic_trimesh_in_batched_scenes_matches_alone(gpu_lib, oracle_built):
         o.step(steps)
         assert_run_matches(f"batched cpic {sc.name}, fast", fst.read_scene_particles(sl), o.particles(),
                            _oracle64(sc, steps), start_state(sc), FAST_BOUNDS)
+
+
+@pytest.mark.parametrize("mode", ["plain", "deterministic", "cpic", "deterministic cpic"])
+def test_a_disabled_particle_keeps_its_old_position(gpu_lib, oracle_built, mode):
+    """Particles that a step disables (determinant of F not positive) stay where they
+    were, without velocity, affine matrix and mass, in the modes that step in place
+    as in the one that writes to another buffer."""
+    from oracle.oracle import OracleScene
+    sc = scenes.cpic_drop()
+    b = sc.particles
+    off = np.arange(5, b.n, 97)
+    b.def_grad[off, 0] = -1.0
+    cpic = "cpic" in mode
+    pipe, st = MpmPipeline(), state_from_scene(sc, deterministic="deterministic" in mode, use_cpic=cpic)
+    o = OracleScene(sc)
+    o.set_use_cpic(cpic)
+    for _ in range(2):
+        pipe.step(st)
+    st.synchronize()
+    o.step(2)
+    got, want = st.read_particles(), o.particles()
+    assert np.array_equal(np.flatnonzero(got["enabled"] == 0), off)
+    assert np.array_equal(np.flatnonzero(want["enabled"] == 0), off)
+    assert np.array_equal(got["pos"][off], b.pos[off]) and np.array_equal(want["pos"][off], b.pos[off])
+    assert not got["vel"][off].any() and not got["aff"][off].any()
+    assert np.array_equal(got["def_grad"][off], np.tile(np.eye(3, dtype=np.float32).reshape(9), (len(off), 1)))
+    # float rounding of positions up to 32 units
+    np.testing.assert_allclose(got["pos"], want["pos"], rtol=0, atol=8e-6)
