@@ -484,7 +484,9 @@ struct nxm_state {
     size_t render_cap = 0;  // float4s
     float4* d_palette = nullptr;
     uint32_t palette_cap = 0;
-    std::vector<float> palette;  // the colors d_palette holds
+    // the state's own copy of the colors that d_palette holds (kept_colors of them; 0: not known)
+    float palette[4 * 64] = {};
+    uint32_t kept_colors = 0;
 
     // pinned staging ring for host -> device copies (see upload_async)
     struct StagingSpan {
@@ -2064,18 +2066,23 @@ static int render_source(nxm_state* s, uint32_t mode, const float* palette, uint
     if (num_groups > s->palette_cap) {
         NXM_TRY(cudaStreamSynchronize(s->stream));
         dfree(s->d_palette);
-        s->palette.clear();
+        s->kept_colors = 0;
         s->palette_cap = 0;
         NXM_TRY(dalloc(&s->d_palette, num_groups));
         s->palette_cap = num_groups;
     }
-    // the device copy stands until the colors change (a copy from pageable memory costs a frame's
-    // host time what several launches do)
-    const std::vector<float> colors(palette, palette + 4 * (size_t)num_groups);
-    if (colors != s->palette) {
-        s->palette.clear();
-        NXM_TRY(cudaMemcpyAsync(s->d_palette, palette, sizeof(float4) * num_groups, cudaMemcpyHostToDevice, s->stream));
-        s->palette = colors;
+    // up to 64 colors: the device copy stands until their bytes change (a copy from pageable memory
+    // costs a frame's host time what several launches do).  It is made from the state's copy: the
+    // caller's memory may change before the stream reads it.
+    const size_t bytes = sizeof(float4) * num_groups;
+    if (bytes > sizeof(s->palette)) {
+        s->kept_colors = 0;
+        NXM_TRY(cudaMemcpyAsync(s->d_palette, palette, bytes, cudaMemcpyHostToDevice, s->stream));
+    } else if (s->kept_colors != num_groups || std::memcmp(s->palette, palette, bytes) != 0) {
+        s->kept_colors = 0;
+        std::memcpy(s->palette, palette, bytes);
+        NXM_TRY(cudaMemcpyAsync(s->d_palette, s->palette, bytes, cudaMemcpyHostToDevice, s->stream));
+        s->kept_colors = num_groups;
     }
     in.p = s->cur;
     in.pcdf = s->d_pcdf;

@@ -96,3 +96,37 @@ def test_prep_readback_rigid_matches_oracle(gpu_lib, oracle_built):
     st2 = state_from_scene(sc, use_cpic=True)  # before any step: the local samples
     np.testing.assert_array_equal(st2.prep_readback_rigid()["position"], st2.read_rigid_particles()["local"])
     assert st.prep_readback(RENDER_DEFAULT)["color"].shape == (sc.n, 4)
+
+
+@pytest.mark.parametrize("colors", [3, 64, 65])
+def test_palette_of_each_call(gpu_lib, colors):
+    """The colors of a call are those it was given, also when the caller's page-locked
+    array changes before the stream gets to the call, when a sign bit is all that
+    differs, and on both sides of the number of colors a state keeps."""
+    import torch
+    from nexus_b200.mpm import PinnedArray
+    sc = scenes.elastic_cube(n_side=24)
+    sc.particles.group_id = np.random.default_rng(4).integers(0, colors, sc.n).astype(np.uint32)
+    st, pipe = state_from_scene(sc), MpmPipeline()
+    first = np.random.default_rng(5).uniform(0.1, 1.0, (colors, 4)).astype(np.float32)
+    pinned = PinnedArray((colors, 4))
+    p, d, c = (torch.zeros((sc.n, k), device="cuda") for k in (3, 9, 4))
+    torch.cuda.synchronize()
+
+    def drawn(palette):
+        st.prep_render(RENDER_DEFAULT, p.data_ptr(), d.data_ptr(), c.data_ptr(), palette)
+        st.synchronize()
+        return c.cpu().numpy()
+
+    pinned.array[:] = first
+    for _ in range(300):  # some ms of queued work ahead of the call
+        pipe.step(st)
+    st.prep_render(RENDER_DEFAULT, p.data_ptr(), d.data_ptr(), c.data_ptr(), pinned.array)
+    pinned.array[:] = 0.0
+    st.synchronize()
+    assert np.array_equal(drawn(first), first[sc.particles.group_id])
+    zero = np.zeros((colors, 4), np.float32)
+    assert not np.signbit(drawn(zero)).any()
+    assert np.signbit(drawn(-zero)).all()
+    assert np.array_equal(drawn(first[:2]), first[sc.particles.group_id % 2])
+    assert np.array_equal(drawn(first), first[sc.particles.group_id])
