@@ -6,6 +6,8 @@
 #define NXM_FAST true
 #include "nxm_transfer.inc.cuh"
 
+#include <type_traits>
+
 namespace nxm {
 namespace fast {
 namespace {
@@ -32,6 +34,12 @@ __device__ __forceinline__ float4 f4add(float4 a, float4 b) { return make_float4
 // A round ends with its fullest cell, so the 64 cells are split by count: the
 // 32 fullest in the first round, the rest in the second (none when at most 32
 // hold particles).  The registers of the 108 sums leave 12 warps an SM.
+// A cell far fuller than the others (a collapsed or compressed scene) would
+// hold up 31 lanes: it gets a round of its own in which the lanes share its
+// particles and add up their sums, where that is less work (pick_heavy).  A step
+// of a scene of 8 particles a cell and one cell of 2,000 in every block: 228 us
+// with a warp per cell, 784 without such rounds, 163 with them; one cell of 20,000
+// alone 768, 7,300, 284 us.
 //
 // The records of a lane's next particles are in flight while it accumulates:
 // asynchronous copies into a ring of kP2gRing slots a lane in shared memory
@@ -56,10 +64,19 @@ struct P2gSlot {
     float4 xm[32], vf[32], c0[32], c1[32];  // x, m; v, flags; C 0..3; C 4..7
     float c2[32];                           // C 8
 };
+// A block with a cell above kHeavyCell particles looks for heavy ones; a round of
+// the whole warp for one costs some kHeavyCost particles of a lane (the 540
+// shuffles that add up the lanes' sums; 3 or 12 make no difference).
+constexpr uint32_t kHeavyCell = 32;
+constexpr uint32_t kHeavyCost = 6;
+constexpr uint32_t kHeavyRound = 2;  // beside rounds 0 and 1
 struct P2gBlock {
     uint32_t ends[65];  // ends[c]: where cell c's particles start in the sorted list
     uint32_t blk[8];    // the block and its +1 neighbours
     int x, y, z;        // scene-local block coordinates
+    uint32_t heavy;     // cells above this many particles get a round of the whole warp
+    uint32_t left[2];   // the ones still to come (cells 0..31, 32..63)
+    uint32_t rounds;    // 1 where the second round's cells are empty
 };
 struct P2gWarp {
     float4 tile[216];
@@ -109,8 +126,22 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
         eh = __ldg(&P.cells[b * 64u + 32u + lane]);
         first = __ldg(&P.first[b]);
     };
-    uint32_t thr = 0;
-    const auto order_cells = [&](P2gBlock& k) {
+    // The threshold, halving from the fullest cell, of the fewest steps: a heavy cell's particles over 32
+    // lanes and its cost, then two rounds of cells of at most the threshold.
+    const auto pick_heavy = [&](uint32_t cl, uint32_t ch, uint32_t most) {
+        uint32_t best = 2u * most, heavy = NONE;
+        for (uint32_t t = most >> 1; t >= kHeavyCell / 4u; t >>= 1) {
+            const uint32_t held = __reduce_add_sync(0xFFFFFFFFu, (cl > t ? cl : 0u) + (ch > t ? ch : 0u));
+            const uint32_t cells = __popc(__ballot_sync(0xFFFFFFFFu, cl > t)) + __popc(__ballot_sync(0xFFFFFFFFu, ch > t));
+            const uint32_t steps = held / 32u + kHeavyCost * cells + 2u * t;
+            if (steps < best) {
+                best = steps;
+                heavy = t;
+            }
+        }
+        return heavy;
+    };
+    const auto order_cells = [&](P2gBlock& k, uint32_t v) {
         k.ends[lane + 1u] = el;
         k.ends[lane + 33u] = eh;
         if (lane < 8u) k.blk[lane] = my_blk;
@@ -122,20 +153,36 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
             k.z = vid.z - o.z;
         }
         __syncwarp();
-        const uint32_t cl = el - k.ends[lane], ch = eh - k.ends[lane + 32u];
+        uint32_t cl = el - k.ends[lane], ch = eh - k.ends[lane + 32u];
+        const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, max(cl, ch));
+        uint32_t heavy = NONE, lo = 0, hi = 0;
+        if (most > kHeavyCell) {
+            heavy = pick_heavy(cl, ch, most);
+            lo = __ballot_sync(0xFFFFFFFFu, cl > heavy);
+            hi = __ballot_sync(0xFFFFFFFFu, ch > heavy);
+            if (split) (v & 1u ? lo : hi) = 0u;  // the block's two warps share them
+            if (cl > heavy) cl = 0u;
+            if (ch > heavy) ch = 0u;
+        }
+        if (lane == 0) {
+            k.heavy = heavy;
+            k.left[0] = lo;
+            k.left[1] = hi;
+        }
         // the smallest threshold that at most 32 cells exceed
         const auto above = [&](uint32_t t) {
             return __popc(__ballot_sync(0xFFFFFFFFu, cl > t)) + __popc(__ballot_sync(0xFFFFFFFFu, ch > t));
         };
-        thr = 0;
+        uint32_t thr = 0;
         if (above(0) > 32) {
-            uint32_t lo = 0, hi = __reduce_max_sync(0xFFFFFFFFu, max(cl, ch));
+            uint32_t lo = 0, hi = min(most, heavy);
             while (hi - lo > 1u) {
                 const uint32_t m = (lo + hi) >> 1;
                 if (above(m) > 32) lo = m; else hi = m;
             }
             thr = hi;
         }
+        if (lane == 0) k.rounds = thr == 0u ? 1u : 2u;
         {  // the cells above it, then as many at it as fill 32 lanes; the others after them
             const uint32_t need = 32u - above(thr);
             const uint32_t eql = __ballot_sync(0xFFFFFFFFu, cl == thr), eqh = __ballot_sync(0xFFFFFFFFu, ch == thr);
@@ -150,15 +197,25 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
     };
     uint32_t c = 0, n = 0, ahead = 0;  // this lane's cell of the round, its particles, the id after the ring's
     const uint32_t* list = nullptr;
-    const auto begin_round = [&](const P2gBlock& k, uint32_t round) {
-        c = order[round * 32u + lane];
-        const uint32_t start = k.ends[c];
-        list = P.sorted + start;
-        n = k.ends[c + 1u] - start;
+    // round 0 or 1, a cell per lane; kHeavyRound: the lanes share the next heavy cell, each every 32nd particle
+    const auto begin_round = [&](P2gBlock& k, uint32_t round) {
+        const bool shared = round == kHeavyRound;
+        if (shared) {
+            const uint32_t word = k.left[0] ? 0u : 1u, bits = k.left[word];
+            c = 32u * word + (uint32_t)__ffs(bits) - 1u;
+            __syncwarp();  // every lane has read the word
+            if (lane == 0) k.left[word] = bits & (bits - 1u);
+        } else {
+            c = order[round * 32u + lane];
+        }
+        const uint32_t start = k.ends[c], held = k.ends[c + 1u] - start;
+        list = P.sorted + start + (shared ? lane : 0u);
+        n = shared ? (held + 31u - lane) >> 5 : (held > k.heavy ? 0u : held);
+        const uint32_t apart = shared ? 5u : 0u;
         uint32_t pid[kP2gRing - 1];
 #pragma unroll
-        for (uint32_t t = 0; t + 1 < kP2gRing; ++t) pid[t] = t < n ? __ldg(&list[t]) : 0u;
-        ahead = kP2gRing - 1u < n ? __ldg(&list[kP2gRing - 1]) : 0u;
+        for (uint32_t t = 0; t + 1 < kP2gRing; ++t) pid[t] = t < n ? __ldg(&list[t << apart]) : 0u;
+        ahead = kP2gRing - 1u < n ? __ldg(&list[(kP2gRing - 1u) << apart]) : 0u;
 #pragma unroll
         for (uint32_t t = 0; t + 1 < kP2gRing; ++t) {
             if (t < n) p2g_fetch(P, sm.ring[t], lane, pid[t]);
@@ -167,19 +224,22 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
     };
     if (u < units) {
         load_block(u);
-        order_cells(sm.block[0]);
+        order_cells(sm.block[0], u);
         begin_round(sm.block[0], split ? u & 1u : 0u);
     }
     uint32_t turn = 0;
     while (u < units) {
         uint32_t next = units;
         if (units > nwarps && lane == 0) next = nwarps + atomicAdd(&P.counters->p2g_next, 1u);
-        const P2gBlock& now = sm.block[turn];
-        const uint32_t r_end = split ? (u & 1u) + 1u : (thr == 0u ? 1u : 2u);  // thr 0: the second round's cells are empty
-        for (uint32_t round = split ? (u & 1u) : 0u; round < r_end; ++round) {
+        P2gBlock& now = sm.block[turn];
+        const uint32_t r_end = split ? (u & 1u) + 1u : now.rounds;
+        // sums the round begun last, begins the one after it (or loads the next block) and returns which
+        const auto sum_round = [&](auto shared_cell, uint32_t round) {
+            constexpr bool kShared = decltype(shared_cell)::value;
+            constexpr uint32_t kApart = kShared ? 32u : 1u;  // from a lane's particle to its next in the list
             const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, n);
             const uint32_t cx = c & 3u, cy = (c >> 2) & 3u, cz = c >> 4;
-            const bool held = n != 0u;
+            const bool held = kShared ? lane == 0u : n != 0u;
             const v3 x0 = mk((float)(now.x * 4 + (int)cx), (float)(now.y * 4 + (int)cy), (float)(now.z * 4 + (int)cz)) * dx;
             float2 axy[27], azm[27];  // sums of node i + 3 j + 9 k: (x, y) and (z, mass)
 #pragma unroll
@@ -194,7 +254,7 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
                 // the slot read in the previous iteration takes the record kP2gRing - 1 ahead
                 if (it + kP2gRing - 1u < n) p2g_fetch(P, sm.ring[at == 0u ? kP2gRing - 1u : at - 1u], lane, ahead);
                 async_commit();
-                ahead = it + kP2gRing < n ? __ldg(&list[it + kP2gRing]) : 0u;
+                ahead = it + kP2gRing < n ? __ldg(&list[(it + kP2gRing) * kApart]) : 0u;
                 at = at + 1u == kP2gRing ? 0u : at + 1u;
                 const bool on = it < n && (__float_as_uint(vf.w) & PFLAG_ENABLED) != 0u;
                 const v3 r = x0 - mk(xm.x, xm.y, xm.z);
@@ -239,11 +299,26 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
             }
             float4* node = tile + cx + 6u * cy + 36u * cz;
             // the next round's first records, or the next block, while these sums go to the tile
-            if (round + 1u < r_end) {
-                begin_round(now, round + 1u);
+            uint32_t after = NONE;
+            if (!kShared && round + 1u < r_end) after = round + 1u;
+            else if (now.left[0] | now.left[1]) after = kHeavyRound;
+            if (after != NONE) {
+                begin_round(now, after);
             } else {
                 u = __shfl_sync(0xFFFFFFFFu, next, 0);
                 if (u < units) load_block(u);
+            }
+            if (kShared) {  // the lanes' sums of the one cell: all to lane 0
+#pragma unroll
+                for (int t = 0; t < 27; ++t) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        axy[t].x += __shfl_xor_sync(0xFFFFFFFFu, axy[t].x, o);
+                        axy[t].y += __shfl_xor_sync(0xFFFFFFFFu, axy[t].y, o);
+                        azm[t].x += __shfl_xor_sync(0xFFFFFFFFu, azm[t].x, o);
+                        azm[t].y += __shfl_xor_sync(0xFFFFFFFFu, azm[t].y, o);
+                    }
+                }
             }
 #pragma unroll
             for (int t = 0; t < 27; ++t) {
@@ -254,10 +329,15 @@ __global__ void __launch_bounds__(kP2gThreads, NXM_P2G_MIN_CTAS) k_p2g(DevPtrs P
                 }
                 __syncwarp();  // the next offset's nodes are other lanes' nodes of this one
             }
-        }
+            return after;
+        };
+        uint32_t round = split ? u & 1u : 0u;
+        do round = sum_round(std::false_type{}, round);
+        while (round < kHeavyRound);
+        while (round == kHeavyRound) round = sum_round(std::true_type{}, round);
         if (u < units) {
             __syncwarp();  // the cell order is read
-            order_cells(sm.block[turn ^ 1u]);
+            order_cells(sm.block[turn ^ 1u], u);
             begin_round(sm.block[turn ^ 1u], split ? u & 1u : 0u);
         }
         // the tile to global memory (clearing it)

@@ -89,6 +89,45 @@ def test_p2g_over_cell_counts(pipe, kind, deterministic):
         assert rel_l2(g[..., :3], want[..., :3]) < 1e-5
 
 
+@pytest.mark.parametrize("blocks", [40, 1200])
+def test_p2g_shares_heavy_cells_over_a_warp(pipe, blocks):
+    """Cells far fuller than their block's others, in either half of the block's cells,
+    alone or several, at counts about multiples of 32; with few blocks (two warps each)
+    and with many (one warp each)."""
+    from oracle.oracle import OracleScene
+    rng = np.random.default_rng(23)
+    at = rng.permutation(14 ** 3)[:blocks]
+    pos = []
+    for i, b in enumerate(at):
+        lo = 4 * (1 + np.array([b % 14, b // 14 % 14, b // 196]))
+        counts = rng.integers(0, 4, 64) * (rng.random(64) < 0.7)
+        for c in rng.permutation(64)[:(0, 0, 0, 1, 2, 5)[i % 6]]:
+            counts[c] = rng.choice([33, 63, 64, 65, 96, 127, 200])
+        if i % 50 == 7:  # nothing but heavy cells
+            counts = np.zeros(64, int)
+            counts[[5, 40]] = [70, 161]
+        cell = np.repeat(np.arange(64), counts)
+        pos.append((lo + np.stack([cell & 3, (cell >> 2) & 3, cell >> 4], 1) + 0.55 + 0.9 * rng.random((len(cell), 3))) * DX)
+    sc = _cells_scene(np.zeros(64, int))
+    sc.particles = ParticleBatch.from_positions(np.concatenate(pos).astype(np.float32), np.float32(DX / 4), 1000.0,
+                                                ParticleModel.elastic_neo_hookean(1.0e5, 0.3))
+    b = sc.particles
+    b.vel[:] = rng.standard_normal(b.vel.shape).astype(np.float32)
+    b.aff[:] = (0.1 * rng.standard_normal(b.aff.shape)).astype(np.float32)
+    b.enabled[::7] = 0
+    sc.grid_capacity = 8192
+    st = state_from_scene(sc)
+    pipe.debug_sort(st, with_p2g=True)
+    o = OracleScene(sc, "f64")
+    o.sort()
+    o.p2g()
+    g = nodes_in_oracle_order(st.headers(), st.nodes(), o.headers())
+    want = o.nodes()[:, :, :4]
+    # 32-bit sums of at most a few thousand products a node
+    assert rel_l2(g[..., 3], want[..., 3]) < 1e-6
+    assert rel_l2(g[..., :3], want[..., :3]) < 1e-5
+
+
 @pytest.mark.parametrize("model", ["elastic", "sand", "sand_neo_hookean", "snow"])
 @pytest.mark.parametrize("strain", ["none", "tiny", "small", "edge", "large", "far"])
 def test_strain_forms_match_the_oracle(pipe, model, strain):
