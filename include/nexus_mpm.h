@@ -358,7 +358,7 @@ NXM_API int nxm_debug_fail_allocation(int64_t after);
  * dispatch sizes are fixed per shader). */
 typedef struct nxm_tuning {
     uint32_t p2g_ctas_per_sm;   /* 1..3 */
-    uint32_t g2p_ctas_per_sm;   /* 1..4 (3 fit) */
+    uint32_t g2p_ctas_per_sm;   /* 1..4 (3 fit: 4 is the same launch) */
     uint32_t sort_ctas_per_sm;  /* 1, 2, 4, 8 or 16: the sort's particle passes */
     uint32_t grid_ctas_per_sm;  /* 1, 2, 4, 8 or 16: the grid update */
     uint32_t sort_batch;        /* 2, 4 or 8 passes of 32 particles a sort warp loads together */

@@ -89,7 +89,7 @@ constexpr uint32_t kRangeChunk = 256;  // sorted positions per fast-G2P run (one
 // defaults are the hand-measured best of the 2 M-particle sand + water scene.
 struct Tuning {
     uint32_t p2g_ctas = 3;    // P2G CTAs per SM (its launch bounds fit 3)
-    uint32_t g2p_ctas = 4;    // G2P CTAs per SM, at most what its launch bounds fit (3)
+    uint32_t g2p_ctas = 3;    // G2P CTAs per SM (its launch bounds fit 3; more are launched as 3)
     uint32_t sort_ctas = 8;   // CTAs per SM of the sort's particle passes
     uint32_t grid_ctas = 8;   // grid update CTAs per SM
     uint32_t sort_batch = 4;  // 2, 4 or 8 passes of 32 particles a sort warp loads together

@@ -2907,7 +2907,7 @@ int nxm_state_autotune(nxm_state* s, uint32_t trial_steps, nxm_tuning* out) {
     float before = 0.f;
     NXM_TRY_RC(time_steps(pipe, s, trial_steps, &before));
     float best_ms = before;
-    static const uint32_t kBatch[] = {2, 4, 8}, kSortCtas[] = {4, 8, 16}, kP2g[] = {2, 3}, kG2p[] = {3, 4},
+    static const uint32_t kBatch[] = {2, 4, 8}, kSortCtas[] = {4, 8, 16}, kP2g[] = {2, 3}, kG2p[] = {2, 3},
                           kGrid[] = {4, 8, 16}, kFill[] = {16, 32, 64, 128, 256};
     struct Knob {
         uint32_t* field;  // inside `trial`

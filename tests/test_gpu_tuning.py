@@ -56,6 +56,16 @@ def test_invalid_tuning_is_refused(gpu_lib):
         st.set_tuning(g2p_ctas_per_sm=5)
 
 
+def test_g2p_is_tuned_over_launches_that_differ(gpu_lib):
+    """Three G2P CTAs fit an SM: the default, and the most that the tuner tries; four is
+    accepted as before and stays what it was set to."""
+    st = state_from_scene(scenes.elastic_cube(n_side=12))
+    assert st.tuning()["g2p_ctas_per_sm"] == 3
+    assert st.autotune(trial_steps=2)["g2p_ctas_per_sm"] in (2, 3)
+    st.set_tuning(g2p_ctas_per_sm=4)
+    assert st.tuning()["g2p_ctas_per_sm"] == 4
+
+
 def test_autotune_fills_the_table_and_applies_it(gpu_lib):
     sc = scenes.sand_water(scale=0.2, steps=10)
     st = state_from_scene(sc)
