@@ -45,9 +45,10 @@ from .mpm import MpmPipeline, MpmState, PinnedArray
 from .scenes import Scene
 
 # Estimated device bytes per particle of a batched state: two copies of the
-# 136-byte particle record, sort scratch (block key 8, header 4, sorted ids
-# reserved 32), ids 8, scene index 4.
-BYTES_PER_PARTICLE = 2 * 136 + 8 + 4 + 32 + 8 + 4
+# 136-byte particle record and of the 48-byte CPIC and properties record, of the
+# id and of the scene index, and sort scratch (block key 8, header 4, sorted ids
+# reserved 32; a word per 256 and per 1,024 particles besides).
+BYTES_PER_PARTICLE = 2 * (136 + 48 + 4 + 4) + 8 + 4 + 32
 # Per grid block: 64 nodes of 16 bytes, 64 cell counters, header arrays, hash slots.
 BYTES_PER_BLOCK = 64 * 16 + 64 * 4 + 16 + 4 * 3 + 4 * 10 + 4 * 7 + 4 + 2 * 8
 

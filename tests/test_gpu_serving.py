@@ -98,3 +98,29 @@ def test_grid_overflow_evicts_and_reports_the_scene(gpu_lib):
     assert sorted(results) == [1, 2]
     for r in good:
         assert np.array_equal(results[r.rid].positions, _alone(r)), r.rid
+
+
+def test_footprint_is_what_a_state_allocates(gpu_lib):
+    """The admission estimate per particle and per grid block against the device memory
+    that states of other capacities take (1 %: allocation granularity and the words
+    per run of particles)."""
+    import torch
+    from nexus_b200.mpm import MpmState
+    from nexus_b200.serving import BYTES_PER_BLOCK, BYTES_PER_PARTICLE
+    torch.zeros(1, device="cuda")
+
+    def taken(particles, blocks):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        st = MpmState(grid_size=blocks, particles_capacity=particles)
+        st.enable_scenes(64)
+        got = before - torch.cuda.mem_get_info()[0]
+        st.close()
+        return got
+
+    taken(1 << 20, 1 << 12)  # what the context allocates once
+    base = taken(1 << 22, 1 << 14)
+    per_particle = (taken(3 << 22, 1 << 14) - base) / (2 << 22)
+    per_block = (taken(1 << 22, 1 << 19) - base) / ((1 << 19) - (1 << 14))
+    assert abs(per_particle / BYTES_PER_PARTICLE - 1.0) < 0.01, per_particle
+    assert abs(per_block / BYTES_PER_BLOCK - 1.0) < 0.01, per_block
