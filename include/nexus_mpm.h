@@ -47,7 +47,7 @@ extern "C" {
 #define NXM_STATUS_BLOCK_CAPACITY 2u
 #define NXM_STATUS_MISSING_BLOCK 4u
 #define NXM_STATUS_SORT_CAPACITY 8u
-#define NXM_STATUS_COPY_TIMEOUT 16u  /* a kernel's wait for its bulk copies ran out (reported as NXM_E_CUDA) */
+#define NXM_STATUS_COPY_TIMEOUT 16u  /* a kernel's wait on a copy barrier ran out (reported as NXM_E_CUDA); no step waits on one, see nxm_debug_copy_wait_timeout */
 
 /* ---- plain data -------------------------------------------------------- */
 
@@ -341,7 +341,7 @@ NXM_API int nxm_grid_read_nodes(nxm_state* state, float* out, uint32_t max_block
 /* Runs only the sort (+ P2G when `with_p2g`) of the next step on the current
  * particles, leaving the grid readable; particles are not advanced. */
 NXM_API int nxm_debug_sort(nxm_pipeline* pipeline, nxm_state* state, int with_p2g);
-/* Test of the bounded waits on bulk copies: enqueues a kernel whose wait on a
+/* Test of a bounded wait on a copy barrier and of its status bit: enqueues a kernel whose wait on a
  * copy barrier can never complete (no copy is issued) and runs out after
  * `limit` rounds, recording NXM_STATUS_COPY_TIMEOUT in the state's status word
  * (nxm_synchronize then returns NXM_E_CUDA until the status is cleared). */

@@ -57,7 +57,7 @@ enum : uint32_t {
     STATUS_BLOCK_CAPACITY = 2u,   // more active blocks than the grid capacity
     STATUS_MISSING_BLOCK = 4u,    // a particle's block was not found (follows 1 or 2)
     STATUS_SORT_CAPACITY = 8u,    // sorted-id list longer than its buffer
-    STATUS_COPY_TIMEOUT = 16u,    // a bulk copy did not complete within its wait limit
+    STATUS_COPY_TIMEOUT = 16u,    // a wait on a copy barrier ran out (nxm_debug_copy_wait_timeout)
 };
 
 struct alignas(32) PKin {

@@ -103,8 +103,6 @@ int model_state_words(uint32_t tag) {
     return 0;
 }
 
-// Packs selected 4-byte fields of the records of particles [first, first + n)
-// into a dense array.
 // Words of the records of one or two arrays: word w of `a`'s record for w <
 // a_words, word w - a_words of `b`'s from there on.
 struct FieldSrc {
@@ -115,6 +113,8 @@ struct FieldSrc {
 __device__ __forceinline__ uint32_t field_of(const FieldSrc& s, size_t p, uint32_t w) {
     return w < s.a_words ? s.a[p * s.a_words + w] : s.b[p * s.b_words + (w - s.a_words)];
 }
+// Packs selected 4-byte fields of the records of particles [first, first + n)
+// into a dense array.
 __global__ void k_pack_fields(FieldSrc src, uint32_t first, uint32_t n,
                               const int* __restrict__ offsets, int nfields, uint32_t* __restrict__ dst) {
     const uint32_t total = n * (uint32_t)nfields;
@@ -836,7 +836,7 @@ void grid_arrays(nxm_state* s, Slab& g) {
     g.add(&s->cursors, (size_t)s->block_cap * NUM_BUCKETS);
     g.add(&s->cells, (size_t)s->block_cap * 64);
     g.add(&s->nbh, (size_t)s->block_cap * NUM_NBH);
-    g.add(&s->nodes, (size_t)(s->block_cap + 1) * 64);  // + one block of zeros (halos of missing neighbours)
+    g.add(&s->nodes, (size_t)s->block_cap * 64);
     g.add(&s->scan_tmp, s->block_cap);
     g.add(&s->tile_sums, s->block_cap / kCellTile + 2);
 }
@@ -883,7 +883,6 @@ int alloc_grid(nxm_state* s, uint32_t grid_capacity) {
     grid_arrays(s, g);
     NXM_TRY(g.alloc(&s->gslab));
     NXM_TRY(cudaMemsetAsync(s->hkey, 0xFF, sizeof(uint32_t) * s->hash_cap, s->stream));
-    NXM_TRY(cudaMemsetAsync(s->nodes + (size_t)s->block_cap * 64, 0, 64 * sizeof(float4), s->stream));
     if (s->use_cpic) {
         int rc = alloc_cpic_grid(s);
         if (rc) return rc;

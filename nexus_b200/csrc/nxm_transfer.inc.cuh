@@ -811,9 +811,10 @@ __global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_update(De
 
 #if NXM_FAST && !NXM_CPIC
 // ---- a copy-barrier wait with an iteration limit ----------------------------
-// An mbarrier in shared memory that bulk copies would complete on; a wait on
-// its phase gives up after `limit` rounds, so that a kernel can record
-// STATUS_COPY_TIMEOUT instead of waiting on.
+// An mbarrier in shared memory as bulk copies complete on; a wait on its phase
+// gives up after `limit` rounds, so that a kernel can record STATUS_COPY_TIMEOUT
+// instead of waiting on.  Reached by nxm_debug_copy_wait_timeout alone: no step
+// kernel copies this way (halos by bulk copies were slower than plain loads).
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
