@@ -44,7 +44,7 @@ __device__ __forceinline__ float4 f4add(float4 a, float4 b) { return make_float4
 // The records of a lane's next particles are in flight while it accumulates:
 // asynchronous copies into a ring of kP2gRing slots a lane in shared memory
 // (slot words of one kind side by side over the lanes: no bank conflicts), so
-// that they cost no registers.
+// that the registers are left to the sums (168, some block words spilled).
 //
 // Bound by FP32 issue and the L1 lookups of 32 lanes' separate records.  2 M
 // sand + water particles: 168 us with a warp per cell and three lanes' groups a

@@ -166,9 +166,11 @@ def test_strain_forms_match_the_oracle(pipe, model, strain):
     assert np.allclose(sg, sw, rtol=2e-5, atol=2e-6)
 
 
-@pytest.mark.parametrize("per_slab", [300, 600, 1500])
+@pytest.mark.parametrize("per_slab", [300, 600, 1500, (1, 2, 3, 5), (33, 0, 4051, 7), (1013, 1013, 1013, 1013),
+                                      (1013, 1013, 1013, 1014), (1, 4095, 2, 4096)])
 def test_canonical_buckets_of_every_length(pipe, per_slab):
-    """Buckets a warp sorts (up to 512 ids) and buckets the CTA sorts."""
+    """A block's list sorted whole, up to 4,052 ids, and bucket by bucket above, on both
+    sides of the switch, with buckets of every remainder by four and up to 4,096 ids."""
     from oracle.oracle import OracleScene
     counts = np.zeros(64, int)
     counts[::16] = per_slab
