@@ -24,7 +24,8 @@ namespace {
 // entries, a ballot of the nonzero ones: the entries that can reach a node are
 // the AND of its three words, walked in ascending order.  An entry left out
 // has weight zero, which the reference skips too, so the sums are the same
-// bits; at 8 particles a cell a node meets about 220 of its block's 1,700
+// bits; an entry whose weights are no numbers (a coordinate that is not finite or
+// whose square overflows) reaches every node, as NaN times zero does; at 8 particles a cell a node meets about 220 of its block's 1,700
 // entries.  The bound is the serial chain of those sums.  100,003 particles, dx =
 // 1/128: 393 us with every node evaluating every entry, 97 us now, of which two
 // entries' products in flight instead of one give a quarter.
@@ -57,7 +58,7 @@ __global__ void __launch_bounds__(kGatherStage) k_p2g_gather(DevPtrs P) {
         const uint32_t node_aff = cpic ? P.ncdf[b * 64u + node].y : 0u;
         uint32_t pid = first + tid < last ? P.sorted[first + tid] : NONE;
         for (uint32_t base = first; base < last; base += kGatherStage) {
-            bool on = false;
+            bool on = false, everywhere = false;
             v3 pt = splat(0.f);
             if (pid != NONE) {
                 const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
@@ -81,6 +82,8 @@ __global__ void __launch_bounds__(kGatherStage) k_p2g_gather(DevPtrs P) {
                     for (int q = 0; q < 4; ++q) srow[tid][q] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
                 spos[tid] = make_float4(pt.x, pt.y, pt.z, aff);
+                const v3 far = vabs(cell_pos - pt) * inv_cell_width;
+                everywhere = !(far.x < 1.0e18f && far.y < 1.0e18f && far.z < 1.0e18f);
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -90,7 +93,7 @@ __global__ void __launch_bounds__(kGatherStage) k_p2g_gather(DevPtrs P) {
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     sw[4 * a + k][tid] = w[a];
-                    const uint32_t m = __ballot_sync(0xFFFFFFFFu, on && w[a] != 0.f);
+                    const uint32_t m = __ballot_sync(0xFFFFFFFFu, on && (w[a] != 0.f || everywhere));
                     if (lane == 0) smask[4 * a + k][warp] = m;
                 }
             }

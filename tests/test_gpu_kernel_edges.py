@@ -250,3 +250,21 @@ def test_step_headers_of_both_scans(pipe, capacity):
         assert all((a < 0) == (b < 0) and (a < 0 or tuple(hs[a][:3]) == tuple(hf[b][:3])) for a, b in zip(h[16:], f[16:]))
         at += h[4]
     assert at == sc.n
+
+
+@pytest.mark.parametrize("axes", [[0], [2], [0, 1], [0, 1, 2]])
+def test_gather_of_positions_that_are_no_numbers(pipe, axes):
+    """Deterministic P2G: a weight that is no number along one axis makes the node's
+    product no number wherever the other axes' weights are zero too."""
+    from oracle.oracle import OracleScene
+    sc = _cells_scene(np.full(64, 2), block=(0, 0, 0))
+    sc.particles.pos[37, axes] = np.nan
+    st = state_from_scene(sc, deterministic=True)
+    pipe.debug_sort(st, with_p2g=True)
+    o = OracleScene(sc)
+    o.sort()
+    o.p2g()
+    g, want = nodes_in_oracle_order(st.headers(), st.nodes(), o.headers()), o.nodes()[:, :, :4]
+    assert np.array_equal(np.isnan(g), np.isnan(want))
+    assert np.isnan(want).any()
+    assert np.array_equal(np.nan_to_num(g), np.nan_to_num(want))
