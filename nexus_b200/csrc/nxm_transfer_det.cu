@@ -13,9 +13,9 @@ namespace nxm {
 namespace exact {
 namespace {
 
-// The gather P2G: one CTA per block, four threads per node (tid = 4 node +
-// component; the components are the momentum's x, y, z and the mass, node = x +
-// 4y + 16z), each summing one component in the reference's order.
+// The gather P2G: four threads per node (tid = 4 node + component; the components
+// are the momentum's x, y, z and the mass, node = x + 4y + 16z), each summing one
+// component in the reference's order, one CTA per block.
 //
 // The list (primaries, then extras) is staged kGatherStage entries at a time;
 // the reference's chunks of 64 stay the unit of its z-slab culling.  A staged
@@ -25,125 +25,230 @@ namespace {
 // the AND of its three words, walked in ascending order.  An entry left out
 // has weight zero, which the reference skips too, so the sums are the same
 // bits; an entry whose weights are no numbers (a coordinate that is not finite or
-// whose square overflows) reaches every node, as NaN times zero does; at 8 particles a cell a node meets about 220 of its block's 1,700
-// entries.  The bound is the serial chain of those sums.  100,003 particles, dx =
-// 1/128: 393 us with every node evaluating every entry, 97 us now, of which two
-// entries' products in flight instead of one give a quarter.
+// whose square overflows) reaches every node, as NaN times zero does; at 8 particles
+// a cell a node meets about 220 of its block's 1,700 entries.  The bound is the
+// serial chain of those sums.  100,003 particles, dx = 1/128: 393 us with every
+// node evaluating every entry, 101 us now, of which two entries' products in flight
+// instead of one give a quarter.
+//
+// A block whose list is at most one chunk is bound by the latency of its loads
+// instead (a sparse scene has little else, a dense one them at its surface): such
+// blocks go first, four at a time in a CTA, 64 threads each with a thread per node.
+// 20,000 particles scattered over 110,000 blocks: 71 us with CTAs of 64 threads
+// that evaluate every entry, 338 us with 256 threads a block, 67 us now; 1.6 M
+// particles over 205,000 blocks: 1234, 1457, 573 us.
 constexpr int kGatherStage = 256;
-__global__ void __launch_bounds__(kGatherStage) k_p2g_gather(DevPtrs P) {
+constexpr uint32_t kGatherShort = 64;  // one chunk
+constexpr uint32_t kGatherTiny = 8;    // entries that a node evaluates faster than a lane stages their weights
+__global__ void __launch_bounds__(kGatherStage, 4) k_p2g_gather(DevPtrs P) {
     after_previous();
     __shared__ float4 srow[kGatherStage][4];  // per component: its row of C and of m v (mass: 0, 0, 0, m)
     __shared__ float4 spos[kGatherStage];     // position, affinity bits (CPIC)
     __shared__ float sw[12][kGatherStage];    // kernel weights: axis * 4 + coordinate
     __shared__ uint32_t smask[12][kGatherStage / 32];
     __shared__ int szkey[kGatherStage];
+    __shared__ uint32_t queue[kGatherStage], queued;
     const bool cpic = P.params->use_cpic != 0;
     const float dx = P.params->dx;
     const float inv_cell_width = 1.0f / dx;
     const uint32_t nb = P.counters->num_blocks;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t node = tid >> 2, comp = tid & 3u;
-    const int tx = (int)(node & 3u), ty = (int)((node >> 2) & 3u), tz = (int)(node >> 4);
-    for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
+    const auto block_coords = [&](uint32_t b) {  // scene-local
         int4 vid = P.bvid[b];
-        {
-            const int3 o = scene_base_of_block(*P.params, vid);  // scene-local block coordinates
-            vid.x -= o.x; vid.y -= o.y; vid.z -= o.z;
+        const int3 o = scene_base_of_block(*P.params, vid);
+        vid.x -= o.x; vid.y -= o.y; vid.z -= o.z;
+        return vid;
+    };
+    // This thread's entry (NONE: none) of the block at vid into its slot.
+    const auto stage = [&](uint32_t pid, int4 vid, bool weights) {
+        bool on = false, everywhere = false;
+        v3 pt = splat(0.f);
+        if (pid != NONE) {
+            const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
+            const float4 xm = kr[0], vf = kr[1];
+            const m3 C = affine_of(P.in, pid);
+            const v3 at = mk(xm.x, xm.y, xm.z);
+            const v3 ac = assoc_cell_of(dx, at);
+            const int zk = f2i_sat(ac.z) - vid.z * 4;
+            szkey[tid] = zk < -2 ? -2 : zk;
+            const float aff = cpic ? P.pcdf[3u * pid + 1u].w : 0.f;
+            on = true;
+            if (__float_as_uint(vf.w) & PFLAG_ENABLED) {
+                const float m = xm.w;
+                pt = at;
+                srow[tid][0] = make_float4(C.c0.x, C.c1.x, C.c2.x, vf.x * m);
+                srow[tid][1] = make_float4(C.c0.y, C.c1.y, C.c2.y, vf.y * m);
+                srow[tid][2] = make_float4(C.c0.z, C.c1.z, C.c2.z, vf.z * m);
+                srow[tid][3] = make_float4(0.f, 0.f, 0.f, m);
+            } else {  // a zero record at the origin, as the reference stages it
+#pragma unroll
+                for (int q = 0; q < 4; ++q) srow[tid][q] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            spos[tid] = make_float4(pt.x, pt.y, pt.z, aff);
+            const v3 far = vabs(mk((float)(vid.x * 4), (float)(vid.y * 4), (float)(vid.z * 4)) * dx - pt) * inv_cell_width;
+            everywhere = !(far.x < 1.0e18f && far.y < 1.0e18f && far.z < 1.0e18f);
         }
-        const v3 cell_pos = mk((float)(vid.x * 4 + tx), (float)(vid.y * 4 + ty), (float)(vid.z * 4 + tz)) * dx;
-        const uint32_t first = P.first[b];
-        const uint32_t last = first + P.nwx[b];
-        const uint32_t primaries_end = first + P.nprim[b];
-        float acc = 0.f, acc_inc = 0.f;
-        const uint32_t node_aff = cpic ? P.ncdf[b * 64u + node].y : 0u;
-        uint32_t pid = first + tid < last ? P.sorted[first + tid] : NONE;
-        for (uint32_t base = first; base < last; base += kGatherStage) {
-            bool on = false, everywhere = false;
-            v3 pt = splat(0.f);
-            if (pid != NONE) {
-                const float4* kr = reinterpret_cast<const float4*>(&P.in.kin[pid]);
-                const float4 xm = kr[0], vf = kr[1];
-                const m3 C = affine_of(P.in, pid);
-                const v3 at = mk(xm.x, xm.y, xm.z);
-                const v3 ac = assoc_cell_of(dx, at);
-                const int zk = f2i_sat(ac.z) - vid.z * 4;
-                szkey[tid] = zk < -2 ? -2 : zk;
-                const float aff = cpic ? P.pcdf[3u * pid + 1u].w : 0.f;
-                on = true;
-                if (__float_as_uint(vf.w) & PFLAG_ENABLED) {
-                    const float m = xm.w;
-                    pt = at;
-                    srow[tid][0] = make_float4(C.c0.x, C.c1.x, C.c2.x, vf.x * m);
-                    srow[tid][1] = make_float4(C.c0.y, C.c1.y, C.c2.y, vf.y * m);
-                    srow[tid][2] = make_float4(C.c0.z, C.c1.z, C.c2.z, vf.z * m);
-                    srow[tid][3] = make_float4(0.f, 0.f, 0.f, m);
-                } else {  // a zero record at the origin, as the reference stages it
+        if (!weights) return;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) srow[tid][q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                spos[tid] = make_float4(pt.x, pt.y, pt.z, aff);
-                const v3 far = vabs(cell_pos - pt) * inv_cell_width;
-                everywhere = !(far.x < 1.0e18f && far.y < 1.0e18f && far.z < 1.0e18f);
+        for (int k = 0; k < 4; ++k) {
+            const v3 c = mk((float)(vid.x * 4 + k), (float)(vid.y * 4 + k), (float)(vid.z * 4 + k)) * dx;
+            const float w[3] = {kernel_eval((c.x - pt.x) * inv_cell_width), kernel_eval((c.y - pt.y) * inv_cell_width),
+                                kernel_eval((c.z - pt.z) * inv_cell_width)};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                sw[4 * a + k][tid] = w[a];
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, on && (w[a] != 0.f || everywhere));
+                if (lane == 0) smask[4 * a + k][warp] = m;
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const v3 c = mk((float)(vid.x * 4 + k), (float)(vid.y * 4 + k), (float)(vid.z * 4 + k)) * dx;
-                const float w[3] = {kernel_eval((c.x - pt.x) * inv_cell_width), kernel_eval((c.y - pt.y) * inv_cell_width),
-                                    kernel_eval((c.z - pt.z) * inv_cell_width)};
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    sw[4 * a + k][tid] = w[a];
-                    const uint32_t m = __ballot_sync(0xFFFFFFFFu, on && (w[a] != 0.f || everywhere));
-                    if (lane == 0) smask[4 * a + k][warp] = m;
-                }
-            }
-            __syncthreads();
-            const uint32_t next = base + kGatherStage + tid;
-            pid = next < last ? P.sorted[next] : NONE;
-            const uint32_t staged = min(last - base, (uint32_t)kGatherStage);
-            for (uint32_t c0 = 0; c0 < staged; c0 += 64u) {  // the reference's chunks
-                const uint32_t chunk_len = min(staged - c0, 64u);
-                int zmin = szkey[c0];
-                int zmax = szkey[c0 + chunk_len - 1u];
-                if (primaries_end > base + c0 && primaries_end < base + c0 + chunk_len) {
-                    const uint32_t bb = primaries_end - base;
-                    zmin = min(zmin, szkey[bb]);
-                    zmax = max(zmax, szkey[bb - 1u]);
-                }
-                if (tz < zmin || tz > zmax + 2) continue;
-#pragma unroll
-                for (uint32_t h = 0; h < 2; ++h) {
-                    const uint32_t w32 = c0 / 32u + h;
-                    // two entries at a time: their products are independent, only the
-                    // sums are a chain
-                    for (uint32_t m = smask[tx][w32] & smask[4 + ty][w32] & smask[8 + tz][w32]; m;) {
-                        float w[2], add[2];
-                        bool inc[2];
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const uint32_t p = 32u * w32 + (m ? (uint32_t)__ffs(m) - 1u : 0u);
-                            w[e] = m ? sw[tx][p] * sw[4 + ty][p] * sw[8 + tz][p] : 0.f;
-                            m &= m - 1u;  // 0 stays 0
-                            const float4 ps = spos[p], r = srow[p][comp];
-                            const v3 dpt = cell_pos - mk(ps.x, ps.y, ps.z);
-                            const float a = r.x * dpt.x + r.y * dpt.y + r.z * dpt.z;
-                            add[e] = comp < 3u ? (a + r.w) * w[e] : r.w * w[e];
-                            // p2g.rs:268-305: an incompatible particle feeds the node's second field
-                            inc[e] = cpic && !aff_compatible(__float_as_uint(ps.w), node_aff);
+        }
+    };
+    // The reference's culling of a chunk of `len` staged entries from slot c0 on, `split` of them
+    // primaries (0: all or none).
+    const auto culled = [&](uint32_t c0, uint32_t len, uint32_t split, int tz) {
+        int zmin = szkey[c0];
+        int zmax = szkey[c0 + len - 1u];
+        if (split) {
+            zmin = min(zmin, szkey[c0 + split]);
+            zmax = max(zmax, szkey[c0 + split - 1u]);
+        }
+        return tz < zmin || tz > zmax + 2;
+    };
+
+    {  // short lists
+        const uint32_t group = tid / kGatherShort, node = tid % kGatherShort, slot0 = group * kGatherShort;
+        const int tx = (int)(node & 3u), ty = (int)((node >> 2) & 3u), tz = (int)(node >> 4);
+        const auto group_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(group + 1u) : "memory"); };
+        constexpr uint32_t kGroups = kGatherStage / kGatherShort;
+        const uint32_t step = gridDim.x * kGroups;
+        uint32_t b = blockIdx.x * kGroups + group;
+        uint3 ahead = make_uint3(0u, 0u, 0u);  // the next block's entries, where they start, its primaries
+        if (b < nb) ahead = make_uint3(P.nwx[b], P.first[b], P.nprim[b]);
+        for (; b < nb; b += step) {
+            const uint32_t num = ahead.x, first = ahead.y, prim = ahead.z;
+            if (b + step < nb) ahead = make_uint3(P.nwx[b + step], P.first[b + step], P.nprim[b + step]);
+            if (num > kGatherShort) continue;
+            v3 mv = splat(0.f), mv_inc = mv;
+            float mass = 0.f, mass_inc = 0.f;
+            if (num) {
+                const uint32_t pid = node < num ? P.sorted[first + node] : NONE;
+                const int4 vid = block_coords(b);
+                const uint32_t node_aff = cpic ? P.ncdf[b * 64u + node].y : 0u;
+                const bool tiny = num <= kGatherTiny;
+                stage(pid, vid, !tiny);
+                group_sync();
+                if (!culled(slot0, num, prim < num ? prim : 0u, tz)) {
+                    const v3 cell_pos = mk((float)(vid.x * 4 + tx), (float)(vid.y * 4 + ty), (float)(vid.z * 4 + tz)) * dx;
+                    // one entry, in the reference's order of operations
+                    const auto add_entry = [&](uint32_t p, v3 dpt, float w) {
+                        if (w == 0.f) return;
+                        const float4 rx = srow[p][0], ry = srow[p][1], rz = srow[p][2];
+                        const v3 add = mk(rx.x * dpt.x + rx.y * dpt.y + rx.z * dpt.z + rx.w,
+                                          ry.x * dpt.x + ry.y * dpt.y + ry.z * dpt.z + ry.w,
+                                          rz.x * dpt.x + rz.y * dpt.y + rz.z * dpt.z + rz.w) * w;
+                        const float add_m = srow[p][3].w * w;
+                        if (cpic && !aff_compatible(__float_as_uint(spos[p].w), node_aff)) {
+                            mv_inc = mv_inc + add;
+                            mass_inc += add_m;
+                        } else {
+                            mv = mv + add;
+                            mass += add_m;
                         }
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            if (w[e] == 0.f) continue;
-                            if (inc[e]) acc_inc += add[e];
-                            else acc += add[e];
+                    };
+                    const auto from_node = [&](uint32_t p) {
+                        const float4 ps = spos[p];
+                        return cell_pos - mk(ps.x, ps.y, ps.z);
+                    };
+                    if (tiny) {
+#pragma unroll 1
+                        for (uint32_t p = slot0; p < slot0 + num; ++p) {
+                            const v3 dpt = from_node(p);
+                            add_entry(p, dpt, kernel_eval(dpt.x * inv_cell_width) * kernel_eval(dpt.y * inv_cell_width) *
+                                                  kernel_eval(dpt.z * inv_cell_width));
+                        }
+                    } else {
+#pragma unroll 1
+                        for (uint32_t w32 = slot0 / 32u; w32 < (slot0 + num + 31u) / 32u; ++w32) {
+                            for (uint32_t m = smask[tx][w32] & smask[4 + ty][w32] & smask[8 + tz][w32]; m; m &= m - 1u) {
+                                const uint32_t p = 32u * w32 + (uint32_t)__ffs(m) - 1u;
+                                add_entry(p, from_node(p), sw[tx][p] * sw[4 + ty][p] * sw[8 + tz][p]);
+                            }
                         }
                     }
                 }
+                group_sync();
             }
-            __syncthreads();
+            P.nodes[b * 64u + node] = make_float4(mv.x, mv.y, mv.z, mass);
+            if (cpic) P.nodes_inc[b * 64u + node] = make_float4(mv_inc.x, mv_inc.y, mv_inc.z, mass_inc);
         }
-        reinterpret_cast<float*>(P.nodes)[node_word(b, tid)] = acc;
-        if (cpic) reinterpret_cast<float*>(P.nodes_inc)[node_word(b, tid)] = acc_inc;
+        __syncthreads();
+    }
+
+    const uint32_t node = tid >> 2, comp = tid & 3u;
+    const int tx = (int)(node & 3u), ty = (int)((node >> 2) & 3u), tz = (int)(node >> 4);
+    // this CTA's blocks with longer lists, found 256 at a time
+    for (uint32_t b0 = blockIdx.x; b0 < nb; b0 += gridDim.x * kGatherStage) {
+        if (tid == 0) queued = 0u;
+        __syncthreads();
+        const uint32_t mine = b0 + gridDim.x * tid;
+        if (mine < nb && P.nwx[mine] > kGatherShort) queue[atomicAdd(&queued, 1u)] = mine;
+        __syncthreads();
+        for (uint32_t q = 0; q < queued; ++q) {
+            const uint32_t b = queue[q];
+            const uint32_t num = P.nwx[b];
+            const int4 vid = block_coords(b);
+            const v3 cell_pos = mk((float)(vid.x * 4 + tx), (float)(vid.y * 4 + ty), (float)(vid.z * 4 + tz)) * dx;
+            const uint32_t first = P.first[b];
+            const uint32_t last = first + num;
+            const uint32_t primaries_end = first + P.nprim[b];
+            float acc = 0.f, acc_inc = 0.f;
+            const uint32_t node_aff = cpic ? P.ncdf[b * 64u + node].y : 0u;
+            uint32_t pid = first + tid < last ? P.sorted[first + tid] : NONE;
+            for (uint32_t base = first; base < last; base += kGatherStage) {
+                stage(pid, vid, true);
+                __syncthreads();
+                const uint32_t next = base + kGatherStage + tid;
+                pid = next < last ? P.sorted[next] : NONE;
+                const uint32_t staged = min(last - base, (uint32_t)kGatherStage);
+                for (uint32_t c0 = 0; c0 < staged; c0 += 64u) {  // the reference's chunks
+                    const uint32_t chunk_len = min(staged - c0, 64u);
+                    const uint32_t chunk = base + c0;
+                    const bool split = primaries_end > chunk && primaries_end < chunk + chunk_len;
+                    if (culled(c0, chunk_len, split ? primaries_end - chunk : 0u, tz)) continue;
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; ++h) {
+                        const uint32_t w32 = c0 / 32u + h;
+                        // two entries at a time: their products are independent, only the
+                        // sums are a chain
+                        for (uint32_t m = smask[tx][w32] & smask[4 + ty][w32] & smask[8 + tz][w32]; m;) {
+                            float w[2], add[2];
+                            bool inc[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const uint32_t p = 32u * w32 + (m ? (uint32_t)__ffs(m) - 1u : 0u);
+                                w[e] = m ? sw[tx][p] * sw[4 + ty][p] * sw[8 + tz][p] : 0.f;
+                                m &= m - 1u;  // 0 stays 0
+                                const float4 ps = spos[p], r = srow[p][comp];
+                                const v3 dpt = cell_pos - mk(ps.x, ps.y, ps.z);
+                                const float a = r.x * dpt.x + r.y * dpt.y + r.z * dpt.z;
+                                add[e] = comp < 3u ? (a + r.w) * w[e] : r.w * w[e];
+                                // p2g.rs:268-305: an incompatible particle feeds the node's second field
+                                inc[e] = cpic && !aff_compatible(__float_as_uint(ps.w), node_aff);
+                            }
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                if (w[e] == 0.f) continue;
+                                if (inc[e]) acc_inc += add[e];
+                                else acc += add[e];
+                            }
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+            reinterpret_cast<float*>(P.nodes)[node_word(b, tid)] = acc;
+            if (cpic) reinterpret_cast<float*>(P.nodes_inc)[node_word(b, tid)] = acc_inc;
+        }
+        __syncthreads();  // the queue is read
     }
 }
 

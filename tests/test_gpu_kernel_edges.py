@@ -268,3 +268,32 @@ def test_gather_of_positions_that_are_no_numbers(pipe, axes):
     assert np.array_equal(np.isnan(g), np.isnan(want))
     assert np.isnan(want).any()
     assert np.array_equal(np.nan_to_num(g), np.nan_to_num(want))
+
+
+def test_gather_of_short_and_long_lists(pipe):
+    """Deterministic P2G of blocks with no entry, a few, one chunk of the reference (64)
+    or just more, primaries and extras in every proportion, bit for bit."""
+    from oracle.oracle import OracleScene
+    rng = np.random.default_rng(31)
+    pos = []
+    for i, b in enumerate(rng.permutation(14 ** 3)[:400]):
+        lo = 4 * (1 + np.array([b % 14, b // 14 % 14, b // 196]))
+        n = (0, 1, 2, 3, 7, 8, 9, 31, 32, 33, 63, 64, 65, 66, 127, 128, 129, 257)[i % 18]
+        pos.append((lo + 0.5 + 4.0 * rng.random((n, 3))) * DX)
+    sc = _cells_scene(np.zeros(64, int))
+    sc.particles = ParticleBatch.from_positions(np.concatenate(pos).astype(np.float32), np.float32(DX / 4), 1000.0,
+                                                ParticleModel.elastic_neo_hookean(1.0e5, 0.3))
+    b = sc.particles
+    b.vel[:] = rng.standard_normal(b.vel.shape).astype(np.float32)
+    b.aff[:] = (0.1 * rng.standard_normal(b.aff.shape)).astype(np.float32)
+    b.enabled[::7] = 0
+    sc.grid_capacity = 4096
+    st = state_from_scene(sc, deterministic=True)
+    pipe.debug_sort(st, with_p2g=True)
+    o = OracleScene(sc)
+    o.sort()
+    o.p2g()
+    lists = o.headers()[:, 5]
+    assert (lists <= 64).sum() > 100 and (lists > 64).sum() > 100
+    g = nodes_in_oracle_order(st.headers(), st.nodes(), o.headers())
+    assert np.array_equal(g.view(np.uint32), o.nodes()[:, :, :4].view(np.uint32))
