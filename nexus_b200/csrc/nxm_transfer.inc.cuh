@@ -647,6 +647,12 @@ __device__ __forceinline__ void g2p_finish(const DevPtrs& P, const Params& prm) 
 #ifndef NXM_G2P_MIN_CTAS
 #define NXM_G2P_MIN_CTAS 3
 #endif
+// k_g2p_update (a block a CTA) at 4: sparse scenes wait for each block's loads, and
+// their step loses more at 3 than crowded ones gain (deterministic, 100,000
+// particles over 198,000 blocks: 881 us at 3, 695 at 4; 110,000 in 64 blocks 76, 82).
+#ifndef NXM_G2P_BLOCK_CTAS
+#define NXM_G2P_BLOCK_CTAS 4
+#endif
 
 // One CTA per primary block (ids [0, num_primary); the other blocks hold no
 // particles), grid-stride: the halo of the block and its +1 neighbours is
@@ -785,7 +791,7 @@ __device__ __forceinline__ void g2p_block_loop(const DevPtrs& P, const Params& p
     }
 }
 
-__global__ void __launch_bounds__(kG2pThreads, NXM_G2P_MIN_CTAS) k_g2p_update(DevPtrs P) {
+__global__ void __launch_bounds__(kG2pThreads, NXM_G2P_BLOCK_CTAS) k_g2p_update(DevPtrs P) {
     after_previous();
     __shared__ float4 halo[216];
 #if NXM_G2P_STASH
@@ -1002,7 +1008,7 @@ int launch_g2p_update(const DevPtrs& P, const LaunchCfg& c, cudaStream_t s) {
     const uint32_t most = (uint32_t)c.sm_count * min(c.t.g2p_ctas, (uint32_t)NXM_G2P_MIN_CTAS);
     launch_after(k_g2p_range, (int)min(units, most), kG2pThreads, 0, s, P);
 #else
-    launch_after(k_g2p_update, (int)min(units, (uint32_t)c.sm_count * NXM_G2P_MIN_CTAS), kG2pThreads, 0, s, P);
+    launch_after(k_g2p_update, (int)min(units, (uint32_t)c.sm_count * NXM_G2P_BLOCK_CTAS), kG2pThreads, 0, s, P);
 #endif
     return 1;
 }
