@@ -159,3 +159,29 @@ def test_a_disabled_particle_keeps_its_old_position(gpu_lib, oracle_built, mode)
     assert np.array_equal(got["def_grad"][off], np.tile(np.eye(3, dtype=np.float32).reshape(9), (len(off), 1)))
     # float rounding of positions up to 32 units
     np.testing.assert_allclose(got["pos"], want["pos"], rtol=0, atol=8e-6)
+
+
+def test_fast_cpic_with_crowded_cells(gpu_lib, oracle_built):
+    """A chunk of the fast CPIC P2G that one or two cells fill, which its warps share:
+    hundreds of particles in single cells, over the floor and away from every collider."""
+    from oracle.oracle import OracleScene
+    from nexus_b200.models import ParticleModel
+    from nexus_b200.particles import ParticleBatch
+    sc = scenes.cpic_drop(steps=20)
+    rng = np.random.default_rng(3)
+    piles = [(np.array(c) + 0.05 + 0.4 * rng.random((n, 3))).astype(np.float32)
+             for c, n in (((18.25, 9.25, 0.75), 700), ((18.25, 9.75, 0.75), 60), ((24.25, 24.25, 12.25), 257))]
+    crowd = ParticleBatch.from_positions(np.concatenate(piles), np.float32(sc.dx / 16), 1000.0,
+                                         ParticleModel.elastic_neo_hookean(1.0e5, 0.3))
+    crowd.vel[:, 2] = -10.0
+    sc.particles = ParticleBatch.concat([sc.particles, crowd])
+    start = start_state(sc)
+    pipe, st = MpmPipeline(), state_from_scene(sc, use_cpic=True)
+    for _ in range(sc.steps):
+        pipe.step(st)
+    st.synchronize()
+    o = OracleScene(sc)
+    o.set_use_cpic(True)
+    o.step(sc.steps)
+    assert_run_matches("cpic with crowded cells", st.read_particles(), o.particles(), _oracle64(sc, sc.steps), start,
+                       FAST_BOUNDS)
